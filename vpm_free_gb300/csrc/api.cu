@@ -147,8 +147,8 @@ void prepare(vpmg_handle* h) {
   } else {
     h->vel_ff.release(); h->def_ff.release();
   }
-  h->rhs_bl.ensure(B * 3 * NB); h->sol_bl.ensure(B * 3 * NB); h->sol0.ensure(NB);
-  h->samp.ensure(B * 3 * NC); h->crhs.ensure(3 * NC); h->csol.ensure(3 * NC); h->csol0.ensure(NC);
+  h->rhs_bl.ensure(B * 3 * NB); h->sol_bl.ensure(B * 3 * NB); h->sol0.ensure(3 * NB);
+  h->samp.ensure(B * 3 * NC); h->crhs.ensure(3 * NC); h->csol.ensure(3 * NC); h->csol0.ensure(3 * NC);
   h->sampsum.ensure(3 * NC);
   for (DBuf<double>* b : {&h->rhs, &h->sol, &h->vel, &h->def, &h->rhs_bl, &h->sol_bl, &h->sol0, &h->samp, &h->crhs,
                           &h->csol, &h->csol0, &h->sampsum})
@@ -163,7 +163,7 @@ void prepare(vpmg_handle* h) {
   dirichlet_prepare(h->dp_c, s.nn_coarse, c_full, s.dpm_coarse, st, h->arith);
   size_t wmax = 0;
   for (DirichletPlan* p : {&h->dp_bl, &h->dp_inner, &h->dp_c}) wmax = std::max(wmax, (size_t)p->m[0] * p->m[1] * p->m[2]);
-  h->work.ensure(wmax);
+  h->work.ensure(3 * wmax);
   if (h->nblk == 1) {
     h->bsolve.prepare(h->dp_bl, s.nnbl_bl, h->cfg.ncoarse);
     h->fsolve.prepare(h->dp_inner);
@@ -233,13 +233,11 @@ void ev_mark(vpmg_handle* h, int i) {
 void infinite_domain(vpmg_handle* h, DirichletPlan& dp, BoundaryOp& bo, const Grid& g, double* rhs3, double* sol3,
                      double* sol0, size_t n) {
   cudaStream_t st = h->stream;
-  for (int c = 0; c < 3; ++c) {
-    dirichlet_solve(dp, rhs3 + c * n, sol0, true, h->work.p, st);
-    boundary_panels(bo, g, sol0, c, st);
-  }
+  dirichlet_solve(dp, rhs3, sol0, true, h->work.p, st, 3, n, n);
+  boundary_panels(bo, g, sol0, n, st);
   double* sp[3] = {sol3, sol3 + n, sol3 + 2 * n};
   boundary_apply(bo, g, sp, st);
-  for (int c = 0; c < 3; ++c) dirichlet_solve(dp, rhs3 + c * n, sol3 + c * n, false, h->work.p, st);
+  dirichlet_solve(dp, rhs3, sol3, false, h->work.p, st, 3, n, n);
 }
 
 // The vector-potential solve: global RHS (h->rhs) -> global SOL (h->sol),
@@ -258,12 +256,10 @@ void poisson_part_multi(vpmg_handle* h) {
     double* SB[3] = {h->sol_bl.p + (size_t)b * 3 * NB, h->sol_bl.p + ((size_t)b * 3 + 1) * NB,
                      h->sol_bl.p + ((size_t)b * 3 + 2) * NB};
     BoundaryOp& bo = *h->bo_blk[b];
-    for (int c = 0; c < 3; ++c) {
-      dirichlet_solve(h->dp_bl, RB + c * NB, h->sol0.p, true, h->work.p, st);
-      boundary_panels(bo, h->g_blk[b], h->sol0.p, c, st);
-    }
+    dirichlet_solve(h->dp_bl, RB, h->sol0.p, true, h->work.p, st, 3, NB, NB);
+    boundary_panels(bo, h->g_blk[b], h->sol0.p, NB, st);
     boundary_apply(bo, h->g_blk[b], SB, st);
-    for (int c = 0; c < 3; ++c) dirichlet_solve(h->dp_bl, RB + c * NB, SB[c], false, h->work.p, st);
+    dirichlet_solve(h->dp_bl, RB, SB[0], false, h->work.p, st, 3, NB, NB);
   }
   if (h->keep_intermediates) {
     h->bl_sol1_copy.ensure(3 * NB);
@@ -275,11 +271,10 @@ void poisson_part_multi(vpmg_handle* h) {
   infinite_domain(h, h->dp_c, h->bo_c, h->gco, h->crhs.p, h->csol.p, h->csol0.p, NC);
   yaps_multi_faces(h->ym, s.nn_coarse, h->csol.p, h->sampsum.p, h->samp.p, h->sol_bl.p, NB, st);
   ev_mark(h, 5);
-  for (int b = 0; b < h->nblk; ++b)
-    for (int c = 0; c < 3; ++c) {
-      const size_t off = ((size_t)b * 3 + c) * NB;
-      dirichlet_solve(h->dp_inner, h->rhs_bl.p + off, h->sol_bl.p + off, false, h->work.p, st);
-    }
+  for (int b = 0; b < h->nblk; ++b) {
+    const size_t off = (size_t)b * 3 * NB;
+    dirichlet_solve(h->dp_inner, h->rhs_bl.p + off, h->sol_bl.p + off, false, h->work.p, st, 3, NB, NB);
+  }
   yaps_multi_solget(h->sol_bl.p, s.nnbl, s.nnbl_bl, h->nb3, s.nn, s.nn_bl, h->sol.p, st);
   (void)N;
   ev_mark(h, 6);
@@ -291,21 +286,18 @@ void poisson_head(vpmg_handle* h) {
   cudaStream_t st = h->stream;
   const vpmg_sizes& s = h->sz;
   const size_t N = h->gglob.count(), NB = h->gbl.count();
-  double* R[3] = {comp(h->rhs, N, 0), comp(h->rhs, N, 1), comp(h->rhs, N, 2)};
   // rhsscat_3d: global interior -> block inner box; the block padding stays zero
   const int go[3] = {s.nn_bl[0] - 1, s.nn_bl[1] - 1, s.nn_bl[2] - 1};
-  for (int c = 0; c < 3; ++c) box_copy(R[c], s.nn, go, comp(h->rhs_bl, NB, c), s.nnbl, h->inner_lo, h->inner_ext, st);
+  box_copy(h->rhs.p, s.nn, go, h->rhs_bl.p, s.nnbl, h->inner_lo, h->inner_ext, st, 3, N, NB);
   fill_zero(h->sol_bl.p, 3 * NB, st);
   ev_mark(h, 1);
   // yaps3d (a): fine infinite-domain solve on the padded block.  By default
   // both block solves are evaluated only where the step reads them
   // (block_solve.cu); the full solves remain for parity checks.
   const bool full = h->full_block_solves || h->keep_intermediates;
-  for (int c = 0; c < 3; ++c) {
-    if (full) dirichlet_solve(h->dp_bl, comp(h->rhs_bl, NB, c), h->sol0.p, true, h->work.p, st);
-    else block_solve_zero_bc(h->bsolve, h->dp_bl, comp(h->rhs_bl, NB, c), c, h->sol0.p, st);
-    boundary_panels(h->bo_bl, h->gbl, h->sol0.p, c, st);
-  }
+  if (full) dirichlet_solve(h->dp_bl, h->rhs_bl.p, h->sol0.p, true, h->work.p, st, 3, NB, NB);
+  else block_solve_zero_bc(h->bsolve, h->dp_bl, h->rhs_bl.p, NB, h->sol0.p, NB, 3, st);
+  boundary_panels(h->bo_bl, h->gbl, h->sol0.p, NB, st);
   ev_mark(h, 2);
 }
 
@@ -319,10 +311,8 @@ void poisson_tail(vpmg_handle* h) {
   const bool full = h->full_block_solves || h->keep_intermediates;
   double* SB[3] = {comp(h->sol_bl, NB, 0), comp(h->sol_bl, NB, 1), comp(h->sol_bl, NB, 2)};
   ev_mark(h, 3);
-  for (int c = 0; c < 3; ++c) {
-    if (full) dirichlet_solve(h->dp_bl, comp(h->rhs_bl, NB, c), SB[c], false, h->work.p, st);
-    else block_solve_bc(h->bsolve, h->dp_bl, c, SB[c], st);
-  }
+  if (full) dirichlet_solve(h->dp_bl, h->rhs_bl.p, h->sol_bl.p, false, h->work.p, st, 3, NB, NB);
+  else block_solve_bc(h->bsolve, h->dp_bl, h->sol_bl.p, NB, 3, st);
   if (h->keep_intermediates) {
     h->bl_sol1_copy.ensure(3 * NB);
     VPMG_CUDA(cudaMemcpyAsync(h->bl_sol1_copy.p, h->sol_bl.p, sizeof(double) * 3 * NB, cudaMemcpyDeviceToDevice, st));
@@ -343,15 +333,12 @@ void poisson_tail(vpmg_handle* h) {
   // (e): final Dirichlet solve on the inner block box: the RHS (zero away
   // from the vorticity) transformed alone, the faces' values in DST space
   // (the block's transform scratch W is free by now)
-  for (int c = 0; c < 3; ++c) {
-    if (h->fsolve.ready && h->bsolve.ready)
-      dirichlet_solve_faces(h->dp_inner, h->fsolve, comp(h->rhs_bl, NB, c), SB[c], h->work.p, h->bsolve.W.p, st);
-    else
-      dirichlet_solve(h->dp_inner, comp(h->rhs_bl, NB, c), SB[c], false, h->work.p, st);
-  }
+  if (h->fsolve.ready && h->bsolve.ready)
+    dirichlet_solve_faces(h->dp_inner, h->fsolve, h->rhs_bl.p, NB, h->sol_bl.p, NB, 3, h->work.p, h->bsolve.W.p, st);
+  else
+    dirichlet_solve(h->dp_inner, h->rhs_bl.p, h->sol_bl.p, false, h->work.p, st, 3, NB, NB);
   // solget_3d
-  double* S[3] = {comp(h->sol, N, 0), comp(h->sol, N, 1), comp(h->sol, N, 2)};
-  for (int c = 0; c < 3; ++c) box_copy(SB[c], s.nnbl, h->inner_lo, S[c], s.nn, go, h->inner_ext, st);
+  box_copy(h->sol_bl.p, s.nnbl, h->inner_lo, h->sol.p, s.nn, go, h->inner_ext, st, 3, NB, N);
   ev_mark(h, 6);
 }
 
@@ -1344,7 +1331,7 @@ int vpmg_bench_kernel(vpmg_handle* h, int which, int reps, double* ms, double* f
       VPMG_CHECK(h->nblk == 1 && h->bsolve.ready, VPMG_ERR_UNSUPPORTED, "one-block handle needed");
       h->bench_scratch.ensure(NB);
       double* o = h->bench_scratch.p;
-      f = [h, o, NB, st] { block_solve_zero_bc(h->bsolve, h->dp_bl, h->rhs_bl.p, 0, o, st); };
+      f = [h, o, NB, st] { block_solve_zero_bc(h->bsolve, h->dp_bl, h->rhs_bl.p, NB, o, NB, 1, st); };
       const DirichletPlan& P = h->dp_bl;
       const double nint = (double)P.m[0] * P.m[1] * P.m[2];
       // forward x and y transforms, the Thomas sweep, 8 x-layer and 8 y-layer dot products
@@ -1641,7 +1628,7 @@ int vpmg_pmesh(vpmg_handle* h, double* const sol[3], const double* const rhs[3],
     const Grid g = make_grid(xbound, dpm, nn);
     const size_t n = g.count();
     DBuf<double> r, s, s0, w;
-    r.ensure(3 * n); s.ensure(3 * n); s0.ensure(n);
+    r.ensure(3 * n); s.ensure(3 * n); s0.ensure(3 * n);
     for (int c = 0; c < 3; ++c) {
       VPMG_CUDA(cudaMemcpyAsync(r.p + c * n, rhs[c], sizeof(double) * n, cudaMemcpyHostToDevice, h->stream));
       VPMG_CUDA(cudaMemcpyAsync(s.p + c * n, sol[c], sizeof(double) * n, cudaMemcpyHostToDevice, h->stream));
@@ -1650,23 +1637,21 @@ int vpmg_pmesh(vpmg_handle* h, double* const sol[3], const double* const rhs[3],
     if (iynbc == 1) {
       const int full[6] = {0, 0, 0, nn[0] - 1, nn[1] - 1, nn[2] - 1};
       dirichlet_prepare(dp, nn, full, dpm, h->stream, h->arith);
-      w.ensure((size_t)dp.m[0] * dp.m[1] * dp.m[2]);
-      fill_zero(s0.p, n, h->stream);
+      w.ensure(3 * (size_t)dp.m[0] * dp.m[1] * dp.m[2]);
+      fill_zero(s0.p, 3 * n, h->stream);
       BoundaryOp bo;
       boundary_prepare(bo, g, itree == 1 ? levmax : 0, h->op_budget, h->stream, h->cfg.ibctyp, itree == 1, h->arith);
-      for (int c = 0; c < 3; ++c) {
-        dirichlet_solve(dp, r.p + c * n, s0.p, true, w.p, h->stream);
-        boundary_panels(bo, g, s0.p, c, h->stream);
-      }
+      dirichlet_solve(dp, r.p, s0.p, true, w.p, h->stream, 3, n, n);
+      boundary_panels(bo, g, s0.p, n, h->stream);
       double* sp[3] = {s.p, s.p + n, s.p + 2 * n};
       boundary_apply(bo, g, sp, h->stream);
-      for (int c = 0; c < 3; ++c) dirichlet_solve(dp, r.p + c * n, s.p + c * n, false, w.p, h->stream);
+      dirichlet_solve(dp, r.p, s.p, false, w.p, h->stream, 3, n, n);
       VPMG_CUDA(cudaStreamSynchronize(h->stream));
     } else {
       const int box[6] = {nn_bl[0] - 1, nn_bl[1] - 1, nn_bl[2] - 1, nn_bl[3] - 1, nn_bl[4] - 1, nn_bl[5] - 1};
       dirichlet_prepare(dp, nn, box, dpm, h->stream, h->arith);
-      w.ensure((size_t)dp.m[0] * dp.m[1] * dp.m[2]);
-      for (int c = 0; c < 3; ++c) dirichlet_solve(dp, r.p + c * n, s.p + c * n, false, w.p, h->stream);
+      w.ensure(3 * (size_t)dp.m[0] * dp.m[1] * dp.m[2]);
+      dirichlet_solve(dp, r.p, s.p, false, w.p, h->stream, 3, n, n);
     }
     for (int c = 0; c < 3; ++c)
       VPMG_CUDA(cudaMemcpyAsync(sol[c], s.p + c * n, sizeof(double) * n, cudaMemcpyDeviceToHost, h->stream));

@@ -39,7 +39,8 @@ __device__ __forceinline__ float2 shfl_xor(float2 v, int m) {
 // sine rows are stored in it (doubles, or float-float pairs), W enters it
 // as it is staged, and each result is joined back into a double.
 
-// out[i + nsel*(q + m1*kk)] = sum_p S[i][p] * W[p + m0*(q + m1*k)],  k = klist ? klist[kk] : kk
+// out[i + nsel*(q + m1*kk)] = sum_p S[i][p] * W[p + m0*(q + m1*k)],  k = klist ? klist[kk] : kk,
+// for nc components of W (wcs doubles apart; their outputs follow each other).
 // Persistent CTAs walk tiles of up to kLines lines; the sine rows are
 // staged once per CTA.  In FP64 (dbl) the next tile is staged with
 // asynchronous copies (cp.async, 8 bytes each) while the current one is
@@ -56,7 +57,10 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 
 template <class A>
 __device__ __forceinline__ void stage_x_tile(typename A::R* tile, const double* __restrict__ W, int m0, int m1,
-                                             int nlines, const int* __restrict__ klist, int l0, int lines) {
+                                             int nlines, const int* __restrict__ klist, int tile_id, int ntile1,
+                                             size_t wcs, int lines) {
+  W += (size_t)(tile_id / ntile1) * wcs;
+  const int l0 = (tile_id % ntile1) * lines;
   for (int t = threadIdx.x; t < lines * m0; t += blockDim.x) {
     const int li = t / m0, p = t - li * m0;
     const int l = l0 + li;
@@ -76,18 +80,20 @@ __device__ __forceinline__ void stage_x_tile(typename A::R* tile, const double* 
 template <class A>
 __global__ void __launch_bounds__(128) k_partial_x(const double* __restrict__ W, int m0, int m1, int nk,
                                                    const int* __restrict__ klist, const typename A::R* __restrict__ S,
-                                                   int nsel, double* __restrict__ out, int lines, int dbl) {
+                                                   int nsel, double* __restrict__ out, int lines, int dbl, int nc,
+                                                   size_t wcs) {
   using R = typename A::R;
   extern __shared__ double smx[];
   R* Ss = reinterpret_cast<R*>(smx);               // nsel x m0
   R* const buf0 = Ss + (size_t)nsel * m0;           // one or two (dbl) tiles of `lines` x m0 (lines <= kLines)
   R* const buf1 = buf0 + (size_t)lines * m0;
   const int nlines = m1 * nk;
-  const int ntiles = (nlines + lines - 1) / lines;
+  const int ntile1 = (nlines + lines - 1) / lines, ntiles = ntile1 * nc;
+  const size_t ocs = (size_t)nsel * nlines;
   for (int t = threadIdx.x; t < nsel * m0; t += blockDim.x) Ss[t] = S[t];
   int cur = 0;
   if (dbl && (int)blockIdx.x < ntiles)
-    stage_x_tile<A>(buf0, W, m0, m1, nlines, klist, blockIdx.x * lines, lines);
+    stage_x_tile<A>(buf0, W, m0, m1, nlines, klist, blockIdx.x, ntile1, wcs, lines);
   // R adjacent threads share one dot product (R = 128 / outputs, a power of
   // two up to 8, when the CTA has fewer outputs than threads), each summing
   // every R-th term; their partials meet in a fixed shuffle tree.
@@ -99,18 +105,19 @@ __global__ void __launch_bounds__(128) k_partial_x(const double* __restrict__ W,
     const int next = tile + gridDim.x;
     if (dbl) {
       if (next < ntiles) {
-        stage_x_tile<A>(cur ? buf0 : buf1, W, m0, m1, nlines, klist, next * lines, lines);
+        stage_x_tile<A>(cur ? buf0 : buf1, W, m0, m1, nlines, klist, next, ntile1, wcs, lines);
         if constexpr (!A::kFF) cp_async_wait<1>();  // the current tile's copies are done
       } else {
         if constexpr (!A::kFF) cp_async_wait<0>();
       }
     } else {
-      stage_x_tile<A>(buf0, W, m0, m1, nlines, klist, tile * lines, lines);
+      stage_x_tile<A>(buf0, W, m0, m1, nlines, klist, tile, ntile1, wcs, lines);
       if constexpr (!A::kFF) cp_async_wait<0>();
     }
     __syncthreads();
     const R* tl = cur ? buf1 : buf0;
-    const int l0 = tile * lines;
+    const int l0 = (tile % ntile1) * lines;
+    double* const oc = out + (size_t)(tile / ntile1) * ocs;
     for (int o0 = 0; o0 < nout; o0 += blockDim.x / Rs) {
       const int o = o0 + threadIdx.x / Rs;
       const int li = o % lines, i = o / lines;
@@ -136,7 +143,7 @@ __global__ void __launch_bounds__(128) k_partial_x(const double* __restrict__ W,
       }
       if (ok && r == 0) {
         const int q = l % m1, kk = l / m1;
-        out[i + (size_t)nsel * (q + (size_t)m1 * kk)] = A::to(v);
+        oc[i + (size_t)nsel * (q + (size_t)m1 * kk)] = A::to(v);
       }
     }
     __syncthreads();  // the buffer is refilled next (one buffer) or two tiles on (dbl)
@@ -177,14 +184,15 @@ __global__ void __launch_bounds__(256) k_partial_y(const double* __restrict__ W,
                                                    const int* __restrict__ klist, const typename A::R* __restrict__ S,
                                                    int nsel, double* __restrict__ out,
                                                    const typename A::R* __restrict__ S2, int nsel2,
-                                                   double* __restrict__ out2, int dbl) {
+                                                   double* __restrict__ out2, int dbl, int nc, size_t wcs) {
   using R = typename A::R;
   extern __shared__ double smy[];
   R* const buf0 = reinterpret_cast<R*>(smy);              // [q][lane], m1 x kColTile
   R* const buf1 = buf0 + (size_t)m1 * kColTile;             // the second tile (dbl)
   R* const partial = (dbl ? buf1 : buf0) + (size_t)m1 * kColTile;  // partial sums [row][lane]
   const int nbx = (m0 + kColTile - 1) / kColTile;
-  const int ntiles = nbx * nk;
+  const int ntile1 = nbx * nk, ntiles = ntile1 * nc;
+  const size_t ocs = (size_t)m0 * nsel * nk, ocs2 = (size_t)m0 * nsel2 * nk;
   const int lane = threadIdx.x % kColTile, row = threadIdx.x / kColTile, rows = blockDim.x / kColTile;
   // R rows share one output row set when there are fewer outputs than rows
   // (R a power of two), each summing every R-th q; the partials are added
@@ -195,19 +203,22 @@ __global__ void __launch_bounds__(256) k_partial_y(const double* __restrict__ W,
   const int r = row % Rs;
   int cur = 0;
   if (dbl && (int)blockIdx.x < ntiles)
-    stage_y_tile<A>(buf0, W, m0, m1, klist, ((int)blockIdx.x % nbx) * kColTile, (int)blockIdx.x / nbx);
+    stage_y_tile<A>(buf0, W + (size_t)((int)blockIdx.x / ntile1) * wcs, m0, m1, klist,
+                    ((int)blockIdx.x % nbx) * kColTile, ((int)blockIdx.x % ntile1) / nbx);
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int p0 = (tile % nbx) * kColTile, kk = tile / nbx;
+    const int comp = tile / ntile1;
+    const int p0 = (tile % nbx) * kColTile, kk = (tile % ntile1) / nbx;  // nbx divides ntile1
     const int next = tile + gridDim.x;
     if (dbl) {
       if (next < ntiles) {
-        stage_y_tile<A>(cur ? buf0 : buf1, W, m0, m1, klist, (next % nbx) * kColTile, next / nbx);
+        stage_y_tile<A>(cur ? buf0 : buf1, W + (size_t)(next / ntile1) * wcs, m0, m1, klist, (next % nbx) * kColTile,
+                        (next % ntile1) / nbx);
         if constexpr (!A::kFF) cp_async_wait<1>();
       } else {
         if constexpr (!A::kFF) cp_async_wait<0>();
       }
     } else {
-      stage_y_tile<A>(buf0, W, m0, m1, klist, p0, kk);
+      stage_y_tile<A>(buf0, W + (size_t)comp * wcs, m0, m1, klist, p0, kk);
       if constexpr (!A::kFF) cp_async_wait<0>();
     }
     __syncthreads();
@@ -240,8 +251,8 @@ __global__ void __launch_bounds__(256) k_partial_y(const double* __restrict__ W,
       if (r == 0 && jj < nout && p < m0) {
         const bool second = jj >= nsel;
         const int j = second ? jj - nsel : jj;
-        if (second) out2[(size_t)p + (size_t)m0 * (j + (size_t)nsel2 * kk)] = A::to(v);
-        else out[(size_t)p + (size_t)m0 * (j + (size_t)nsel * kk)] = A::to(v);
+        if (second) out2[comp * ocs2 + (size_t)p + (size_t)m0 * (j + (size_t)nsel2 * kk)] = A::to(v);
+        else out[comp * ocs + (size_t)p + (size_t)m0 * (j + (size_t)nsel * kk)] = A::to(v);
       }
     }
     __syncthreads();  // the tile's buffer is refilled next
@@ -252,8 +263,10 @@ __global__ void __launch_bounds__(256) k_partial_y(const double* __restrict__ W,
 // dst node (ia[a], ib[b], ic[c]) <- src[a + na*(b + nb*c)]; a null list means identity + off.
 __global__ void k_scatter3(const double* __restrict__ src, int na, int nb, int nc, const int* __restrict__ ia,
                            const int* __restrict__ ib, const int* __restrict__ ic, int off, double* __restrict__ dst,
-                           int dx, int dy) {
+                           int dx, int dy, size_t dcs) {
   const size_t n = (size_t)na * nb * nc;
+  src += blockIdx.y * n;  // component
+  dst += blockIdx.y * dcs;
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x) {
     const int a = (int)(t % na), b = (int)((t / na) % nb), c = (int)(t / ((size_t)na * nb));
     const int i = ia ? ia[a] : a + off, j = ib ? ib[b] : b + off, k = ic ? ic[c] : c + off;
@@ -268,44 +281,18 @@ __global__ void k_scatter3(const double* __restrict__ src, int na, int nb, int n
 // extractions below store the x and y pairs that way (the transforms along
 // the faces' own axes are linear): one FMA per axis and node in the sweep.
 //
-// Interior values of the six faces of the block: x pair (sum, difference)
-// [k][j], y pair [k][i], z faces [j][i].
-__global__ void k_extract_faces(const double* __restrict__ s, int NX, int NY, int NZ, double* __restrict__ fxs,
-                                double* __restrict__ fxd, double* __restrict__ fys, double* __restrict__ fyd,
-                                double* __restrict__ fz0, double* __restrict__ fzN) {
-  const int m0 = NX - 2, m1 = NY - 2, m2 = NZ - 2;
-  const size_t sy = NX, sz = (size_t)NX * NY;
-  const long nx = (long)m1 * m2, ny = (long)m0 * m2, nz = (long)m0 * m1;
-  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < nx + ny + nz; t += (long)gridDim.x * blockDim.x) {
-    if (t < nx) {
-      const int j = (int)(t % m1) + 1, k = (int)(t / m1) + 1;
-      const double a = s[sy * j + sz * k], b = s[(NX - 1) + sy * j + sz * k];
-      fxs[t] = a + b;
-      fxd[t] = a - b;
-    } else if (t < nx + ny) {
-      const long u = t - nx;
-      const int i = (int)(u % m0) + 1, k = (int)(u / m0) + 1;
-      const double a = s[i + sz * k], b = s[i + sy * (NY - 1) + sz * k];
-      fys[u] = a + b;
-      fyd[u] = a - b;
-    } else {
-      const long u = t - nx - ny;
-      const int i = (int)(u % m0) + 1, j = (int)(u / m0) + 1;
-      fz0[u] = s[i + sy * j];
-      fzN[u] = s[i + sy * j + sz * (NZ - 1)];
-    }
-  }
-}
-
 // The six faces of the box whose node (0,0,0) sits at (o0,o1,o2) of an
 // NX x NY x * array, interior m0 x m1 x m2: x pair (sum, difference) [k][j],
 // y pair [k][i], z faces [j][i].
 __global__ void k_extract_box_faces(const double* __restrict__ s, int NX, int NY, int o0, int o1, int o2, int m0,
                                     int m1, int m2, double* __restrict__ fxs, double* __restrict__ fxd,
                                     double* __restrict__ fys, double* __restrict__ fyd, double* __restrict__ fz0,
-                                    double* __restrict__ fzN) {
+                                    double* __restrict__ fzN, size_t scs, size_t fcs) {
   const size_t sy = NX, sz = (size_t)NX * NY;
   const long nx = (long)m1 * m2, ny = (long)m0 * m2, nz = (long)m0 * m1;
+  s += blockIdx.y * scs;  // component
+  fxs += blockIdx.y * fcs; fxd += blockIdx.y * fcs; fys += blockIdx.y * fcs;
+  fyd += blockIdx.y * fcs; fz0 += blockIdx.y * fcs; fzN += blockIdx.y * fcs;
   auto at = [&](int a, int b, int c) { return s[(size_t)(o0 + a) + sy * (o1 + b) + sz * (o2 + c)]; };
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < nx + ny + nz; t += (long)gridDim.x * blockDim.x) {
     if (t < nx) {
@@ -328,89 +315,132 @@ __global__ void k_extract_box_faces(const double* __restrict__ s, int NX, int NY
   }
 }
 
-struct FaceTerms {
-  const double *fxs, *fxd, *fys, *fyd, *fz0, *fzN;  // transforms: [k][q], [k][p], [q][p]
-  const double *ex1, *ey1;                          // sin(pi (p+1)/(m+1)) along x and y
-  double cx, cy, cz;                                // -scale / h^2
-};
-
-// Thomas sweep of -u[k-1] + d u[k] - u[k+1] = r[k] with the reciprocal pivot
-// table; r = ghat (+ the transformed Dirichlet face terms when bc).  The
-// recurrence stays in FP64: each line is a dependent chain and the lines
-// are too few to hide the longer chain of float-float operations.
-__global__ void k_thomas_faces(const double* __restrict__ g, double* __restrict__ out, const double* __restrict__ rinvt,
-                               int m0, int m1, int m2, int bc, FaceTerms F) {
+// The z pass: -u[k-1] + d u[k] - u[k+1] = r[k] per mode, r = g (+ the
+// transformed Dirichlet face terms), eliminated from both ends to the middle
+// and substituted back outwards ("burn at both ends"), with the reciprocal
+// pivots of k_pivots: the matrix is the same read from either end, so both
+// chains use one table of half the planes.  A thread owns one mode of NC
+// components: 2 NC independent chains of m2 / 2 steps each way, which share
+// the table's loads.  The recurrence stays in FP64 in both arithmetics.
+// Bound: HBM at large boxes (g read, the forward values written and read, u
+// written, half the table read twice: 32 + 8 / NC bytes per node); the
+// chains' latency at small ones, hence the U planes loaded ahead.
+template <int NC, bool BC>
+__global__ void __launch_bounds__(128) k_thomas_ends(const double* g, double* out, const double* __restrict__ rinv,
+                                                     int m0, int m1, int m2, size_t cs, const FaceTerms F) {
   const int pq = blockIdx.x * blockDim.x + threadIdx.x;
   if (pq >= m0 * m1) return;
   const int p = pq % m0, q = pq / m0;
   const size_t plane = (size_t)m0 * m1;
-  auto rinv = [&](size_t id) { return rinvt[id]; };
+  constexpr int U = NC == 1 ? 8 : 4;
   double ax = 0.0, ay = 0.0;
   const double *fx = nullptr, *fy = nullptr;
-  if (bc) {
+  if constexpr (BC) {
     ax = F.cx * F.ex1[p];
     ay = F.cy * F.ey1[q];
-    fx = (p & 1) ? F.fxd : F.fxs;  // the x pair's sum (p even) or difference
-    fy = (q & 1) ? F.fyd : F.fys;
+    fx = ((p & 1) ? F.fxd : F.fxs) + q;  // the x pair's sum (p even) or difference
+    fy = ((q & 1) ? F.fyd : F.fys) + p;
   }
-  auto rhs = [&](int k) -> double {
-    double r = g[pq + plane * k];
-    if (bc) {
-      r = fma(ay, fy[(size_t)k * m0 + p], fma(ax, fx[(size_t)k * m1 + q], r));
-      if (k == 0) r += F.cz * F.fz0[pq];
-      if (k == m2 - 1) r += F.cz * F.fzN[pq];
-    }
+  auto rhs = [&](int c, int k) -> double {
+    double r = g[c * cs + pq + plane * k];
+    if constexpr (BC) r = fma(ay, fy[c * F.cs + (size_t)k * m0], fma(ax, fx[c * F.cs + (size_t)k * m1], r));
     return r;
   };
-  // loads twelve planes ahead of the dependent chain (one thread per line
-  // leaves few warps per SM: the loads in flight set the speed); same
-  // arithmetic order
-  constexpr int U = 12;
-  double y = rhs(0);
-  out[pq] = y;
-  double ri = rinv(pq);
-  int k = 1;
-  for (; k + U - 1 < m2; k += U) {
-    const size_t id = pq + plane * k;
-    double qv[U], rv[U];
+  const int h = m2 >> 1;
+  double yt[NC], yb[NC];  // the two chains' values
+  if (h > 0) {
 #pragma unroll
-    for (int u = 0; u < U; ++u) qv[u] = rhs(k + u);
-#pragma unroll
-    for (int u = 0; u < U; ++u) rv[u] = rinv(id + plane * u);
+    for (int c = 0; c < NC; ++c) {
+      yt[c] = rhs(c, 0);
+      yb[c] = rhs(c, m2 - 1);
+      if constexpr (BC) {
+        yt[c] += F.cz * F.fz0[c * F.cs + pq];
+        yb[c] += F.cz * F.fzN[c * F.cs + pq];
+      }
+      out[c * cs + pq] = yt[c];
+      out[c * cs + pq + plane * (m2 - 1)] = yb[c];
+    }
+  }
+  auto fwd = [&](int k, int n) {  // planes k .. k+n-1 from both ends
+    double rt[U][NC], rb[U][NC], rv[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      y = fma(y, u ? rv[u - 1] : ri, qv[u]);
-      out[id + plane * u] = y;
+      if (u >= n) break;
+      rv[u] = rinv[pq + plane * (k + u - 1)];
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        rt[u][c] = rhs(c, k + u);
+        rb[u][c] = rhs(c, m2 - 1 - (k + u));
+      }
     }
-    ri = rv[U - 1];
-  }
-  for (; k < m2; ++k) {
-    const size_t id = pq + plane * k;
-    y = fma(y, ri, rhs(k));
-    out[id] = y;
-    ri = rinv(id);
-  }
-  double u = y * ri;
-  out[pq + plane * (m2 - 1)] = u;
-  k = m2 - 2;
-  for (; k - (U - 1) >= 0; k -= U) {
-    const size_t id = pq + plane * k;
-    double ov[U], rv[U];
 #pragma unroll
-    for (int v = 0; v < U; ++v) ov[v] = out[id - plane * v];
+    for (int u = 0; u < U; ++u) {
+      if (u >= n) break;
 #pragma unroll
-    for (int v = 0; v < U; ++v) rv[v] = rinv(id - plane * v);
-#pragma unroll
-    for (int v = 0; v < U; ++v) {
-      u = (ov[v] + u) * rv[v];
-      out[id - plane * v] = u;
+      for (int c = 0; c < NC; ++c) {
+        yt[c] = fma(yt[c], rv[u], rt[u][c]);
+        yb[c] = fma(yb[c], rv[u], rb[u][c]);
+        out[c * cs + pq + plane * (k + u)] = yt[c];
+        out[c * cs + pq + plane * (m2 - 1 - (k + u))] = yb[c];
+      }
     }
+  };
+  int k = 1;
+  for (; k + U <= h; k += U) fwd(k, U);
+  for (; k < h; ++k) fwd(k, 1);
+  const double mid = rinv[pq + plane * h];
+  const double rl = h > 0 ? rinv[pq + plane * (h - 1)] : 0.0;
+  if (m2 & 1) {
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      double r = rhs(c, h);
+      if (h > 0) {
+        r = fma(rl, yt[c] + yb[c], r);
+      } else if constexpr (BC) {
+        r += F.cz * F.fz0[c * F.cs + pq];
+        r += F.cz * F.fzN[c * F.cs + pq];
+      }
+      yt[c] = yb[c] = mid * r;
+      out[c * cs + pq + plane * h] = yt[c];
+    }
+    k = h - 1;
+  } else {
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const double a = yt[c], b = yb[c];
+      yt[c] = mid * fma(rl, b, a);
+      yb[c] = mid * fma(rl, a, b);
+      out[c * cs + pq + plane * (h - 1)] = yt[c];
+      out[c * cs + pq + plane * h] = yb[c];
+    }
+    k = h - 2;
   }
-  for (; k >= 0; --k) {
-    const size_t id = pq + plane * k;
-    u = (out[id] + u) * rinv(id);
-    out[id] = u;
-  }
+  auto bwd = [&](int kk, int n) {  // planes kk, kk-1, .. kk-n+1 outwards
+    double ot[U][NC], ob[U][NC], rv[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (u >= n) break;
+      rv[u] = rinv[pq + plane * (kk - u)];
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        ot[u][c] = out[c * cs + pq + plane * (kk - u)];
+        ob[u][c] = out[c * cs + pq + plane * (m2 - 1 - (kk - u))];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (u >= n) break;
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        yt[c] = (ot[u][c] + yt[c]) * rv[u];
+        yb[c] = (ob[u][c] + yb[c]) * rv[u];
+        out[c * cs + pq + plane * (kk - u)] = yt[c];
+        out[c * cs + pq + plane * (m2 - 1 - (kk - u))] = yb[c];
+      }
+    }
+  };
+  for (; k - U + 1 >= 0; k -= U) bwd(k, U);
+  for (; k >= 0; --k) bwd(k, 1);
 }
 
 // sin(pi (i+1)(p+1)/N) of the selected rows, one 8-byte word each: the
@@ -485,20 +515,21 @@ void partial_x_reserve(int m0, int nsel) {
 }
 
 void partial_x(int arith, const double* W, int m0, int m1, int nk, const int* klist, const double* S, int nsel,
-               double* out, cudaStream_t s) {
+               double* out, cudaStream_t s, int nc, size_t wcs) {
   const int nlines = m1 * nk;
   const bool dbl = arith != VPMG_ARITH_FF48;
   const int lines = partial_x_lines(m0, nsel, dbl);
   const size_t sm = partial_x_smem(m0, nsel, lines, dbl);
   VPMG_CHECK(sm <= granted(g_partial_smem), VPMG_ERR_STATE, "k_partial_x shared memory not reserved");
   // persistent CTAs: as many as fit on the SMs at this shared-memory size
-  const unsigned ntiles = (nlines + lines - 1) / lines;
+  const unsigned ntiles = (unsigned)nc * ((nlines + lines - 1) / lines);
   const unsigned per_sm = (unsigned)std::max<size_t>(1, std::min<size_t>(8, (227 * 1024) / (sm + 1024)));
   const unsigned g = std::min(ntiles, 152u * per_sm);
   if (arith == VPMG_ARITH_FF48)
-    k_partial_x<FF><<<g, 128, sm, s>>>(W, m0, m1, nk, klist, reinterpret_cast<const float2*>(S), nsel, out, lines, 0);
+    k_partial_x<FF><<<g, 128, sm, s>>>(W, m0, m1, nk, klist, reinterpret_cast<const float2*>(S), nsel, out, lines, 0,
+                                       nc, wcs);
   else
-    k_partial_x<F64><<<g, 128, sm, s>>>(W, m0, m1, nk, klist, S, nsel, out, lines, 1);
+    k_partial_x<F64><<<g, 128, sm, s>>>(W, m0, m1, nk, klist, S, nsel, out, lines, 1, nc, wcs);
   VPMG_LAUNCHED();
 }
 
@@ -519,31 +550,99 @@ void partial_y_reserve(int m1) {
 }
 
 void partial_y(int arith, const double* W, int m0, int m1, int nk, const int* klist, const double* S, int nsel,
-               double* out, cudaStream_t s, const double* S2 = nullptr, int nsel2 = 0, double* out2 = nullptr) {
+               double* out, cudaStream_t s, int nc, size_t wcs, const double* S2 = nullptr, int nsel2 = 0,
+               double* out2 = nullptr) {
   const int dbl = (arith != VPMG_ARITH_FF48 && partial_y_dbl(m1)) ? 1 : 0;
   const size_t sm = partial_y_smem(m1, dbl);  // tiles + partial sums of 8 rows
   VPMG_CHECK(sm <= granted(g_partial_y_smem), VPMG_ERR_STATE, "k_partial_y shared memory not reserved");
   // persistent CTAs: as many as fit on the SMs at this shared-memory size
-  const unsigned ntiles = (unsigned)(((m0 + kColTile - 1) / kColTile) * nk);
+  const unsigned ntiles = (unsigned)nc * (unsigned)(((m0 + kColTile - 1) / kColTile) * nk);
   const unsigned per_sm = (unsigned)std::max<size_t>(1, std::min<size_t>(8, (227 * 1024) / (sm + 1024)));
   const unsigned g = std::min(ntiles, 152u * per_sm);
   if (arith == VPMG_ARITH_FF48)
     k_partial_y<FF><<<g, 256, sm, s>>>(W, m0, m1, nk, klist, reinterpret_cast<const float2*>(S), nsel, out,
-                                      reinterpret_cast<const float2*>(S2), nsel2, out2, dbl);
+                                      reinterpret_cast<const float2*>(S2), nsel2, out2, dbl, nc, wcs);
   else
-    k_partial_y<F64><<<g, 256, sm, s>>>(W, m0, m1, nk, klist, S, nsel, out, S2, nsel2, out2, dbl);
+    k_partial_y<F64><<<g, 256, sm, s>>>(W, m0, m1, nk, klist, S, nsel, out, S2, nsel2, out2, dbl, nc,
+                                       wcs);
   VPMG_LAUNCHED();
 }
 
 void scatter3(const double* src, int na, int nb, int nc, const int* ia, const int* ib, const int* ic, int off,
-              double* dst, const int dims[3], cudaStream_t s) {
+              double* dst, const int dims[3], cudaStream_t s, int ncomp, size_t dcs) {
   const size_t n = (size_t)na * nb * nc;
-  k_scatter3<<<(unsigned)std::min<size_t>((n + 255) / 256, 152 * 16), 256, 0, s>>>(src, na, nb, nc, ia, ib, ic, off,
-                                                                                   dst, dims[0], dims[1]);
+  k_scatter3<<<dim3((unsigned)std::min<size_t>((n + 255) / 256, 152 * 16), ncomp), 256, 0, s>>>(
+      src, na, nb, nc, ia, ib, ic, off, dst, dims[0], dims[1], dcs);
   VPMG_LAUNCHED();
 }
 
+// The six faces of a box of sol as FaceTerms arrays of nc components in
+// buf, transformed along their own axes (two launches of job lists).
+FaceTerms face_terms(const DirichletPlan& P, double* buf, const double* ex1, const double* ey1, const double* sol,
+                     size_t scs, int nc, cudaStream_t s) {
+  const int m0 = P.m[0], m1 = P.m[1], m2 = P.m[2];
+  FaceTerms F;
+  double* fxs = buf;
+  double* fxd = fxs + (size_t)m1 * m2;
+  double* fys = fxd + (size_t)m1 * m2;
+  double* fyd = fys + (size_t)m0 * m2;
+  double* fz0 = fyd + (size_t)m0 * m2;
+  double* fzN = fz0 + (size_t)m0 * m1;
+  F.cs = face_doubles(P);
+  F.fxs = fxs; F.fxd = fxd; F.fys = fys; F.fyd = fyd; F.fz0 = fz0; F.fzN = fzN;
+  F.ex1 = ex1;
+  F.ey1 = ey1;
+  const double scale = dirichlet_scale(P);
+  F.cx = -scale / (P.h[0] * P.h[0]);
+  F.cy = -scale / (P.h[1] * P.h[1]);
+  F.cz = -scale / (P.h[2] * P.h[2]);
+  k_extract_box_faces<<<dim3(256, nc), 256, 0, s>>>(sol, P.dims[0], P.dims[1], P.box[0], P.box[1], P.box[2], m0, m1, m2,
+                                                    fxs, fxd, fys, fyd, fz0, fzN, scs, F.cs);
+  VPMG_LAUNCHED();
+  // rows over j -> q (x faces), over i -> p (y faces, and the z faces' rows)
+  // in one launch; then the z faces' columns over j
+  const DstYLines rows[6] = {{&P.fy, fxs, 1, m1, m2, F.cs}, {&P.fy, fxd, 1, m1, m2, F.cs},
+                             {&P.fx, fys, 1, m0, m2, F.cs}, {&P.fx, fyd, 1, m0, m2, F.cs},
+                             {&P.fx, fz0, 1, m0, m1, F.cs}, {&P.fx, fzN, 1, m0, m1, F.cs}};
+  dst_lines_y_jobs(rows, 6, s, nc);
+  const DstYLines cols[2] = {{&P.fy, fz0, m0, m1, 1, F.cs}, {&P.fy, fzN, m0, m1, 1, F.cs}};
+  dst_lines_y_jobs(cols, 2, s, nc);
+  return F;
+}
+
 }  // namespace
+
+size_t face_doubles(const DirichletPlan& P) {
+  const size_t m0 = P.m[0], m1 = P.m[1], m2 = P.m[2];
+  return 2 * (m1 * m2 + m0 * m2 + m0 * m1);
+}
+
+void thomas_launch(const double* g, double* out, const double* rinv, const int m[3], int nc, size_t cs,
+                   const FaceTerms* F, cudaStream_t s) {
+  const unsigned nb = (unsigned)(((size_t)m[0] * m[1] + 127) / 128);
+  const FaceTerms none{};
+  if (nc == 3) {
+    if (F) k_thomas_ends<3, true><<<nb, 128, 0, s>>>(g, out, rinv, m[0], m[1], m[2], cs, *F);
+    else k_thomas_ends<3, false><<<nb, 128, 0, s>>>(g, out, rinv, m[0], m[1], m[2], cs, none);
+  } else {
+    for (int c = 0; c < nc; ++c) {
+      if (F) {
+        FaceTerms f = *F;
+        f.fxs += c * F->cs; f.fxd += c * F->cs; f.fys += c * F->cs;
+        f.fyd += c * F->cs; f.fz0 += c * F->cs; f.fzN += c * F->cs;
+        k_thomas_ends<1, true><<<nb, 128, 0, s>>>(g + c * cs, out + c * cs, rinv, m[0], m[1], m[2], cs, f);
+      } else {
+        k_thomas_ends<1, false><<<nb, 128, 0, s>>>(g + c * cs, out + c * cs, rinv, m[0], m[1], m[2], cs, none);
+      }
+    }
+  }
+}
+void thomas_sweep(const double* g, double* out, const double* rinv, const int m[3], int nc, size_t cs,
+                  const FaceTerms* F, cudaStream_t s) {
+  thomas_launch(g, out, rinv, m, nc, cs, F, s);
+  count_launch(nc == 3 ? 1 : nc);
+  VPMG_CUDA(cudaGetLastError());
+}
 
 void BlockSolve::prepare(const DirichletPlan& P, const int nnbl_bl[6], int ncoarse) {
   arith = P.arith;
@@ -551,7 +650,7 @@ void BlockSolve::prepare(const DirichletPlan& P, const int nnbl_bl[6], int ncoar
   VPMG_CHECK(m[0] >= 8 && m[1] >= 8 && m[2] >= 8, VPMG_ERR_UNSUPPORTED, "block too small for the partial solve");
   const size_t nint = (size_t)m[0] * m[1] * m[2];
   ghat.ensure(3 * nint);
-  W.ensure(nint);
+  W.ensure(3 * nint);
   // normal-derivative layers: interior indices 0..3 and m-4..m-1
   std::vector<int> fx = {0, 1, 2, 3, m[0] - 4, m[0] - 3, m[0] - 2, m[0] - 1};
   std::vector<int> fylo = {0, 1, 2, 3}, fyhi = {m[1] - 4, m[1] - 3, m[1] - 2, m[1] - 1};
@@ -597,109 +696,87 @@ void BlockSolve::prepare(const DirichletPlan& P, const int nnbl_bl[6], int ncoar
   up(e_y1, edge(m[1]));
   partial_x_reserve(m[0], std::max(8, nsx));
   partial_y_reserve(m[1]);
-  X8.ensure((size_t)8 * m[1] * m[2]);
-  Y4.ensure((size_t)m[0] * 8 * m[2]);  // low and high face rows
-  X2.ensure((size_t)2 * m[1] * m[2]);
-  Y1.ensure((size_t)m[0] * 2 * m[2]);
-  Ys.ensure((size_t)m[0] * nsy * nsz);
-  XS.ensure((size_t)nsx * nsy * nsz);
-  fxs.ensure((size_t)m[1] * m[2]); fxd.ensure((size_t)m[1] * m[2]);
-  fys.ensure((size_t)m[0] * m[2]); fyd.ensure((size_t)m[0] * m[2]);
-  fz0.ensure((size_t)m[0] * m[1]); fzN.ensure((size_t)m[0] * m[1]);
+  X8.ensure((size_t)3 * 8 * m[1] * m[2]);
+  Y4.ensure((size_t)3 * m[0] * 8 * m[2]);  // low and high face rows
+  X2.ensure((size_t)3 * 2 * m[1] * m[2]);
+  Y1.ensure((size_t)3 * m[0] * 2 * m[2]);
+  Ys.ensure((size_t)3 * m[0] * nsy * nsz);
+  XS.ensure((size_t)3 * nsx * nsy * nsz);
+  f.ensure(3 * face_doubles(P));
   ready = true;
 }
 
-void block_solve_zero_bc(BlockSolve& B, DirichletPlan& P, const double* rhs_c, int c, double* sol0, cudaStream_t s) {
+void block_solve_zero_bc(BlockSolve& B, DirichletPlan& P, const double* rhs, size_t rcs, double* sol0, size_t scs,
+                         int nc, cudaStream_t s) {
   const int m0 = B.m[0], m1 = B.m[1], m2 = B.m[2];
   const size_t nint = (size_t)m0 * m1 * m2, plane = (size_t)m0 * m1;
-  double* g = B.ghat.p + (size_t)c * nint;
-  dst_forward_xy(P, rhs_c, nullptr, true, g, s);
-  FaceTerms F{};
-  k_thomas_faces<<<(int)((plane + 127) / 128), 128, 0, s>>>(g, B.W.p, P.rinvd.p, m0, m1, m2, 0, F);
-  VPMG_LAUNCHED();
+  dst_forward_xy(P, rhs, nullptr, true, B.ghat.p, s, nc, rcs, 0);
+  thomas_sweep(B.ghat.p, B.W.p, P.rinvd.p, B.m, nc, nint, nullptr, s);
   // x faces: 8 layers by dot products along x; y faces: 4 + 4 rows by dot products along y
-  partial_x(B.arith, B.W.p, m0, m1, m2, nullptr, B.S_fx.p, 8, B.X8.p, s);
-  double* Y4b = B.Y4.p + (size_t)m0 * 4 * m2;
-  partial_y(B.arith, B.W.p, m0, m1, m2, nullptr, B.S_fy_lo.p, 4, B.Y4.p, s, B.S_fy_hi.p, 4, Y4b);
+  partial_x(B.arith, B.W.p, m0, m1, m2, nullptr, B.S_fx.p, 8, B.X8.p, s, nc, nint);
+  const size_t xcs = (size_t)8 * m1 * m2, ycs = (size_t)m0 * 4 * m2;
+  double* Y4b = B.Y4.p + 3 * ycs;
+  partial_y(B.arith, B.W.p, m0, m1, m2, nullptr, B.S_fy_lo.p, 4, B.Y4.p, s, nc, nint, B.S_fy_hi.p, 4, Y4b);
   // one launch of inverse y transforms: the x-face layers and the first and
   // last 4 planes (z faces, in place on W after the dots) ...
   double* top = B.W.p + plane * (m2 - 4);
-  const DstYLines ys[3] = {{&P.fy, B.X8.p, 8, m1, m2}, {&P.fy, B.W.p, m0, m1, 4}, {&P.fy, top, m0, m1, 4}};
-  dst_lines_y_jobs(ys, 3, s);
-  scatter3(B.X8.p, 8, m1, m2, B.l_fx.p, nullptr, nullptr, 1, sol0, B.dims, s);
+  const DstYLines ys[3] = {{&P.fy, B.X8.p, 8, m1, m2, xcs}, {&P.fy, B.W.p, m0, m1, 4, nint}, {&P.fy, top, m0, m1, 4, nint}};
+  dst_lines_y_jobs(ys, 3, s, nc);
+  scatter3(B.X8.p, 8, m1, m2, B.l_fx.p, nullptr, nullptr, 1, sol0, B.dims, s, nc, scs);
   // ... then inverse x transforms into sol0: the y-face rows, then the z
   // planes.  Jobs of one launch write disjoint nodes; where the rows and the
   // planes meet (box edges) the planes' launch writes last, every run.
   const DstXInvLines xr[2] = {
-      {&P.fx, B.Y4.p, sol0, {B.dims[0], B.dims[1], B.dims[2]}, {1, 1, 1}, {m0, 4, m2}},
-      {&P.fx, Y4b, sol0, {B.dims[0], B.dims[1], B.dims[2]}, {1, 1 + m1 - 4, 1}, {m0, 4, m2}}};
-  dst_x_inv_jobs(xr, 2, s);
+      {&P.fx, B.Y4.p, sol0, {B.dims[0], B.dims[1], B.dims[2]}, {1, 1, 1}, {m0, 4, m2}, ycs, scs},
+      {&P.fx, Y4b, sol0, {B.dims[0], B.dims[1], B.dims[2]}, {1, 1 + m1 - 4, 1}, {m0, 4, m2}, ycs, scs}};
+  dst_x_inv_jobs(xr, 2, s, nc);
   const DstXInvLines xz[2] = {
-      {&P.fx, B.W.p, sol0, {B.dims[0], B.dims[1], B.dims[2]}, {1, 1, 1}, {m0, m1, 4}},
-      {&P.fx, top, sol0, {B.dims[0], B.dims[1], B.dims[2]}, {1, 1, 1 + m2 - 4}, {m0, m1, 4}}};
-  dst_x_inv_jobs(xz, 2, s);
+      {&P.fx, B.W.p, sol0, {B.dims[0], B.dims[1], B.dims[2]}, {1, 1, 1}, {m0, m1, 4}, nint, scs},
+      {&P.fx, top, sol0, {B.dims[0], B.dims[1], B.dims[2]}, {1, 1, 1 + m2 - 4}, {m0, m1, 4}, nint, scs}};
+  dst_x_inv_jobs(xz, 2, s, nc);
   VPMG_CUDA(cudaGetLastError());
 }
 
-void block_solve_bc(BlockSolve& B, DirichletPlan& P, int c, double* sol_c, cudaStream_t s) {
+void block_solve_bc(BlockSolve& B, DirichletPlan& P, double* sol, size_t scs, int nc, cudaStream_t s) {
   const int m0 = B.m[0], m1 = B.m[1], m2 = B.m[2];
   const size_t nint = (size_t)m0 * m1 * m2, plane = (size_t)m0 * m1;
   // boundary values of the faces, transformed along the face's axes
-  k_extract_faces<<<256, 256, 0, s>>>(sol_c, B.dims[0], B.dims[1], B.dims[2], B.fxs.p, B.fxd.p, B.fys.p, B.fyd.p,
-                                      B.fz0.p, B.fzN.p);
-  VPMG_LAUNCHED();
-  // transformed along the face's axes: rows over j -> q (x faces), over i ->
-  // p (y faces, and the z faces' rows), in one launch; then the z faces'
-  // columns over j
-  const DstYLines rows[6] = {{&P.fy, B.fxs.p, 1, m1, m2}, {&P.fy, B.fxd.p, 1, m1, m2},
-                             {&P.fx, B.fys.p, 1, m0, m2}, {&P.fx, B.fyd.p, 1, m0, m2},
-                             {&P.fx, B.fz0.p, 1, m0, m1}, {&P.fx, B.fzN.p, 1, m0, m1}};
-  dst_lines_y_jobs(rows, 6, s);
-  const DstYLines cols[2] = {{&P.fy, B.fz0.p, m0, m1, 1}, {&P.fy, B.fzN.p, m0, m1, 1}};
-  dst_lines_y_jobs(cols, 2, s);
-  const double scale = dirichlet_scale(P);
-  FaceTerms F;
-  F.fxs = B.fxs.p; F.fxd = B.fxd.p; F.fys = B.fys.p; F.fyd = B.fyd.p; F.fz0 = B.fz0.p; F.fzN = B.fzN.p;
-  F.ex1 = B.e_x1.p; F.ey1 = B.e_y1.p;
-  F.cx = -scale / (P.h[0] * P.h[0]);
-  F.cy = -scale / (P.h[1] * P.h[1]);
-  F.cz = -scale / (P.h[2] * P.h[2]);
-  const double* g = B.ghat.p + (size_t)c * nint;
-  k_thomas_faces<<<(int)((plane + 127) / 128), 128, 0, s>>>(g, B.W.p, P.rinvd.p, m0, m1, m2, 1, F);
-  VPMG_LAUNCHED();
+  const FaceTerms F = face_terms(P, B.f.p, B.e_x1.p, B.e_y1.p, sol, scs, nc, s);
+  thomas_sweep(B.ghat.p, B.W.p, P.rinvd.p, B.m, nc, nint, &F, s);
   // dot products: the inner-box x faces along x, its y faces along y, and
   // the interior samples along y then x
-  partial_x(B.arith, B.W.p, m0, m1, m2, nullptr, B.S_ix.p, 2, B.X2.p, s);
-  double* Y1b = B.Y1.p + (size_t)m0 * m2;
-  partial_y(B.arith, B.W.p, m0, m1, m2, nullptr, B.S_iy_lo.p, 1, B.Y1.p, s, B.S_iy_hi.p, 1, Y1b);
-  partial_y(B.arith, B.W.p, m0, m1, B.nsz, B.l_sz.p, B.S_sy.p, B.nsy, B.Ys.p, s);
-  partial_x(B.arith, B.Ys.p, m0, B.nsy, B.nsz, nullptr, B.S_sx.p, B.nsx, B.XS.p, s);
-  scatter3(B.XS.p, B.nsx, B.nsy, B.nsz, B.l_sx.p, B.l_sy.p, B.l_idz.p, 0, sol_c, B.dims, s);
+  partial_x(B.arith, B.W.p, m0, m1, m2, nullptr, B.S_ix.p, 2, B.X2.p, s, nc, nint);
+  const size_t xcs = (size_t)2 * m1 * m2, ycs = (size_t)m0 * m2;
+  double* Y1b = B.Y1.p + 3 * ycs;
+  partial_y(B.arith, B.W.p, m0, m1, m2, nullptr, B.S_iy_lo.p, 1, B.Y1.p, s, nc, nint, B.S_iy_hi.p, 1, Y1b);
+  partial_y(B.arith, B.W.p, m0, m1, B.nsz, B.l_sz.p, B.S_sy.p, B.nsy, B.Ys.p, s, nc, nint);
+  partial_x(B.arith, B.Ys.p, m0, B.nsy, B.nsz, nullptr, B.S_sx.p, B.nsx, B.XS.p, s, nc, (size_t)m0 * B.nsy * B.nsz);
+  scatter3(B.XS.p, B.nsx, B.nsy, B.nsz, B.l_sx.p, B.l_sy.p, B.l_idz.p, 0, sol, B.dims, s, nc, scs);
   // one launch of inverse y transforms: the x-face layers and the inner-box
   // z planes (in place on W, after the dots) ...
   double* pl0 = B.W.p + plane * B.inner_lo[2];
   double* pl1 = B.W.p + plane * B.inner_hi[2];
-  const DstYLines ys[3] = {{&P.fy, B.X2.p, 2, m1, m2}, {&P.fy, pl0, m0, m1, 1}, {&P.fy, pl1, m0, m1, 1}};
-  dst_lines_y_jobs(ys, 3, s);
-  scatter3(B.X2.p, 2, m1, m2, B.l_ix.p, nullptr, nullptr, 1, sol_c, B.dims, s);
-  // ... then inverse x transforms into sol_c: the y-face rows, then the z
+  const DstYLines ys[3] = {{&P.fy, B.X2.p, 2, m1, m2, xcs}, {&P.fy, pl0, m0, m1, 1, nint}, {&P.fy, pl1, m0, m1, 1, nint}};
+  dst_lines_y_jobs(ys, 3, s, nc);
+  scatter3(B.X2.p, 2, m1, m2, B.l_ix.p, nullptr, nullptr, 1, sol, B.dims, s, nc, scs);
+  // ... then inverse x transforms into sol: the y-face rows, then the z
   // planes (jobs of one launch write disjoint nodes; at the box edges the
   // planes' launch writes last, every run)
   const int dm[3] = {B.dims[0], B.dims[1], B.dims[2]};
   const DstXInvLines xr[2] = {
-      {&P.fx, B.Y1.p, sol_c, {dm[0], dm[1], dm[2]}, {1, B.inner_lo[1] + 1, 1}, {m0, 1, m2}},
-      {&P.fx, Y1b, sol_c, {dm[0], dm[1], dm[2]}, {1, B.inner_hi[1] + 1, 1}, {m0, 1, m2}}};
-  dst_x_inv_jobs(xr, 2, s);
+      {&P.fx, B.Y1.p, sol, {dm[0], dm[1], dm[2]}, {1, B.inner_lo[1] + 1, 1}, {m0, 1, m2}, ycs, scs},
+      {&P.fx, Y1b, sol, {dm[0], dm[1], dm[2]}, {1, B.inner_hi[1] + 1, 1}, {m0, 1, m2}, ycs, scs}};
+  dst_x_inv_jobs(xr, 2, s, nc);
   const DstXInvLines xz[2] = {
-      {&P.fx, pl0, sol_c, {dm[0], dm[1], dm[2]}, {1, 1, B.inner_lo[2] + 1}, {m0, m1, 1}},
-      {&P.fx, pl1, sol_c, {dm[0], dm[1], dm[2]}, {1, 1, B.inner_hi[2] + 1}, {m0, m1, 1}}};
-  dst_x_inv_jobs(xz, 2, s);
+      {&P.fx, pl0, sol, {dm[0], dm[1], dm[2]}, {1, 1, B.inner_lo[2] + 1}, {m0, m1, 1}, nint, scs},
+      {&P.fx, pl1, sol, {dm[0], dm[1], dm[2]}, {1, 1, B.inner_hi[2] + 1}, {m0, m1, 1}, nint, scs}};
+  dst_x_inv_jobs(xz, 2, s, nc);
   VPMG_CUDA(cudaGetLastError());
 }
 
 void FaceSolve::prepare(const DirichletPlan& P) {
-  const int m0 = P.m[0], m1 = P.m[1], m2 = P.m[2];
-  f.ensure(2 * ((size_t)m1 * m2 + (size_t)m0 * m2 + (size_t)m0 * m1));
+  const int m0 = P.m[0], m1 = P.m[1];
+  f.ensure(3 * face_doubles(P));
   std::vector<double> e((size_t)m0 + (size_t)m1);
   for (int p = 0; p < m0; ++p) e[p] = std::sin(kPI * (double)(p + 1) / (double)(m0 + 1));
   for (int q = 0; q < m1; ++q) e[m0 + q] = std::sin(kPI * (double)(q + 1) / (double)(m1 + 1));
@@ -708,41 +785,20 @@ void FaceSolve::prepare(const DirichletPlan& P) {
   ready = true;
 }
 
-void dirichlet_solve_faces(DirichletPlan& P, FaceSolve& FS, const double* rhs, double* sol, double* work,
-                           double* out, cudaStream_t s) {
-  VPMG_CHECK(FS.ready, VPMG_ERR_STATE, "face solve not prepared");
+void dirichlet_solve_faces(DirichletPlan& P, FaceSolve& FS, const double* rhs, size_t rcs, double* sol, size_t scs,
+                           int nc, double* work, double* out, cudaStream_t s) {
+  VPMG_CHECK(FS.ready && nc >= 1 && nc <= 3, VPMG_ERR_STATE, "face solve not prepared");
   const int m0 = P.m[0], m1 = P.m[1], m2 = P.m[2];
-  const size_t plane = (size_t)m0 * m1;
+  const size_t nint = (size_t)m0 * m1 * m2;
   // forward transforms of the RHS alone (zero tiles skip their FFTs)
-  dst_forward_xy(P, rhs, nullptr, true, work, s);
-  // the faces' values, transformed along their own axes
-  double* fxs = FS.f.p;
-  double* fxd = fxs + (size_t)m1 * m2;
-  double* fys = fxd + (size_t)m1 * m2;
-  double* fyd = fys + (size_t)m0 * m2;
-  double* fz0 = fyd + (size_t)m0 * m2;
-  double* fzN = fz0 + (size_t)m0 * m1;
-  k_extract_box_faces<<<256, 256, 0, s>>>(sol, P.dims[0], P.dims[1], P.box[0], P.box[1], P.box[2], m0, m1, m2, fxs,
-                                          fxd, fys, fyd, fz0, fzN);
-  VPMG_LAUNCHED();
-  const DstYLines rows[6] = {{&P.fy, fxs, 1, m1, m2}, {&P.fy, fxd, 1, m1, m2}, {&P.fx, fys, 1, m0, m2},
-                             {&P.fx, fyd, 1, m0, m2}, {&P.fx, fz0, 1, m0, m1}, {&P.fx, fzN, 1, m0, m1}};
-  dst_lines_y_jobs(rows, 6, s);
-  const DstYLines cols[2] = {{&P.fy, fz0, m0, m1, 1}, {&P.fy, fzN, m0, m1, 1}};
-  dst_lines_y_jobs(cols, 2, s);
-  // the sweep with the face terms, then the full inverse transforms
-  const double scale = dirichlet_scale(P);
-  FaceTerms F;
-  F.fxs = fxs; F.fxd = fxd; F.fys = fys; F.fyd = fyd; F.fz0 = fz0; F.fzN = fzN;
-  F.ex1 = FS.e.p; F.ey1 = FS.e.p + m0;
-  F.cx = -scale / (P.h[0] * P.h[0]);
-  F.cy = -scale / (P.h[1] * P.h[1]);
-  F.cz = -scale / (P.h[2] * P.h[2]);
-  k_thomas_faces<<<(int)((plane + 127) / 128), 128, 0, s>>>(work, out, P.rinvd.p, m0, m1, m2, 1, F);
-  VPMG_LAUNCHED();
-  dst_lines_y(P.fy, out, m0, m1, m2, s);
+  dst_forward_xy(P, rhs, nullptr, true, work, s, nc, rcs, 0);
+  // the faces' values, transformed along their own axes; the sweep with
+  // them, then the full inverse transforms
+  const FaceTerms F = face_terms(P, FS.f.p, FS.e.p, FS.e.p + m0, sol, scs, nc, s);
+  thomas_sweep(work, out, P.rinvd.p, P.m, nc, nint, &F, s);
+  dst_lines_y(P.fy, out, m0, m1, m2, s, nc, nint);
   const int o[3] = {P.box[0] + 1, P.box[1] + 1, P.box[2] + 1};
-  dst_x_inv_to_box(P.fx, out, sol, P.dims, o, P.m, s);
+  dst_x_inv_to_box(P.fx, out, sol, P.dims, o, P.m, s, nc, nint, scs);
   VPMG_CUDA(cudaGetLastError());
 }
 

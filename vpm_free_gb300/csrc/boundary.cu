@@ -718,12 +718,15 @@ __global__ void k_apply_corr(const int* __restrict__ rows, const long long* __re
   }
 }
 
-// calc_normalderiv_3d: one thread per panel.
+// calc_normalderiv_3d: one thread per panel, blockIdx.y = component.
 __global__ void k_normal_deriv(const double* __restrict__ sol0, int NX, int NY, int NZ, const int* __restrict__ face,
                                const int* __restrict__ pi, const int* __restrict__ pj, const int* __restrict__ pk,
-                               int nbound, double invx, double invy, double invz, double* __restrict__ src) {
+                               int nbound, double invx, double invy, double invz, double* __restrict__ src,
+                               size_t scs, size_t dcs) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= nbound) return;
+  sol0 += blockIdx.y * scs;
+  src += blockIdx.y * dcs;
   const double a1 = 25.0 / 12.0, a2 = -4.0, a3 = 3.0, a4 = -4.0 / 3.0, a5 = 0.25;
   const int f = face[p];
   const int i = pi[p] - 1, j = pj[p] - 1, k = pk[p] - 1;  // 0-based
@@ -986,11 +989,10 @@ void boundary_prepare(BoundaryOp& B, const Grid& g, int levmax, long long budget
   farfield_prepare(B, g, s);
 }
 
-void boundary_panels(BoundaryOp& B, const Grid& g, const double* sol0, int comp, cudaStream_t s) {
-  double* dst = B.csrc.p + (size_t)comp * B.ncell_total;  // level-0 part = panels
-  k_normal_deriv<<<(B.nbound + 255) / 256, 256, 0, s>>>(sol0, g.n[0], g.n[1], g.n[2], B.pan_face.p, B.pan_i.p,
-                                                        B.pan_j.p, B.pan_k.p, B.nbound, 1.0 / g.d[0], 1.0 / g.d[1],
-                                                        1.0 / g.d[2], dst);
+void boundary_panels(BoundaryOp& B, const Grid& g, const double* sol0, size_t scs, cudaStream_t s) {
+  k_normal_deriv<<<dim3((B.nbound + 255) / 256, 3), 256, 0, s>>>(
+      sol0, g.n[0], g.n[1], g.n[2], B.pan_face.p, B.pan_i.p, B.pan_j.p, B.pan_k.p, B.nbound, 1.0 / g.d[0],
+      1.0 / g.d[1], 1.0 / g.d[2], B.csrc.p, scs, (size_t)B.ncell_total);  // level-0 part = panels
   VPMG_LAUNCHED();
   VPMG_CUDA(cudaGetLastError());
 }

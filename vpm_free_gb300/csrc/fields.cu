@@ -17,10 +17,13 @@ namespace {
 // plane run over its e0 x e1 nodes without gaps (one 32-bit division per
 // node, no partly filled CTA per row).
 __global__ void k_box_copy(const double* __restrict__ src, int sx, int sy, int so0, int so1, int so2,
-                           double* __restrict__ dst, int dx, int dy, int do0, int do1, int do2, int e0, int e1) {
+                           double* __restrict__ dst, int dx, int dy, int do0, int do1, int do2, int e0, int e1,
+                           size_t scs, size_t dcs) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= e0 * e1) return;
   const int j = t / e0, i = t - j * e0, k = blockIdx.y;
+  src += blockIdx.z * scs;  // component
+  dst += blockIdx.z * dcs;
   dst[(size_t)(do0 + i) + (size_t)dx * ((do1 + j) + (size_t)dy * (do2 + k))] =
       src[(size_t)(so0 + i) + (size_t)sx * ((so1 + j) + (size_t)sy * (so2 + k))];
 }
@@ -35,8 +38,17 @@ __global__ void k_sample(const double* __restrict__ a0, const double* __restrict
   c2[dst[t]] = a2[src[t]];
 }
 
-__global__ void k_coarse_lap(const double* __restrict__ s, double* __restrict__ r, int CX, int CY, int lo0, int lo1,
-                             int lo2, int e0, int e1, int e2, double ih0, double ih1, double ih2) {
+struct In3 {
+  const double* p[3];
+};
+struct Out3 {
+  double* p[3];
+};
+// blockIdx.y = component (this kernel and k_face_interp)
+__global__ void k_coarse_lap(In3 s3, Out3 r3, int CX, int CY, int lo0, int lo1, int lo2, int e0, int e1, int e2,
+                             double ih0, double ih1, double ih2) {
+  const double* __restrict__ s = s3.p[blockIdx.y];
+  double* __restrict__ r = r3.p[blockIdx.y];
   const size_t n = (size_t)e0 * e1 * e2;
   const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (t >= n) return;
@@ -52,10 +64,12 @@ __global__ void k_coarse_lap(const double* __restrict__ s, double* __restrict__ 
 
 __global__ void k_face_interp(const long long* __restrict__ node, const long long* __restrict__ cbase,
                               const double* __restrict__ w, const int* __restrict__ flagged, int n,
-                              const double* __restrict__ csol, const double* __restrict__ samp, int CX, int CY,
-                              double* __restrict__ sol) {
+                              In3 csol3, In3 samp3, int CX, int CY, Out3 sol3) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
+  const double* __restrict__ csol = csol3.p[blockIdx.y];
+  const double* __restrict__ samp = samp3.p[blockIdx.y];
+  double* __restrict__ sol = sol3.p[blockIdx.y];
   const double* wt = w + 9 * (size_t)t;
   const size_t b = cbase[t];
   const size_t sy = CX, sz = (size_t)CX * CY;
@@ -213,14 +227,14 @@ unsigned grid_for(size_t n, int threads) { return (unsigned)std::max<size_t>(1, 
 }  // namespace
 
 void box_copy(const double* src, const int sdims[3], const int so[3], double* dst, const int ddims[3], const int dof[3],
-              const int ext[3], cudaStream_t s) {
+              const int ext[3], cudaStream_t s, int nc, size_t scs, size_t dcs) {
   const size_t n = (size_t)ext[0] * ext[1] * ext[2];
   if (!n) return;
   VPMG_CHECK(ext[2] <= 65535 && (size_t)ext[0] * ext[1] <= (size_t)INT32_MAX, VPMG_ERR_UNSUPPORTED,
              "box copy extent above the grid limit");
-  const dim3 grid((unsigned)(((size_t)ext[0] * ext[1] + 255) / 256), (unsigned)ext[2]);
+  const dim3 grid((unsigned)(((size_t)ext[0] * ext[1] + 255) / 256), (unsigned)ext[2], nc);
   k_box_copy<<<grid, 256, 0, s>>>(src, sdims[0], sdims[1], so[0], so[1], so[2], dst, ddims[0], ddims[1], dof[0], dof[1],
-                                  dof[2], ext[0], ext[1]);
+                                  dof[2], ext[0], ext[1], scs, dcs);
   VPMG_LAUNCHED();
   VPMG_CUDA(cudaGetLastError());
 }
@@ -259,22 +273,20 @@ void yaps_coarse_rhs(const YapsDev& Y, const int cdims[3], const double dc[3], c
   const int e[3] = {Y.map[3] - Y.map[0] - 1, Y.map[4] - Y.map[1] - 1, Y.map[5] - Y.map[2] - 1};
   if (e[0] <= 0 || e[1] <= 0 || e[2] <= 0) return;
   const size_t n = (size_t)e[0] * e[1] * e[2];
-  for (int c = 0; c < 3; ++c) {
-    k_coarse_lap<<<grid_for(n, 256), 256, 0, s>>>(samp[c], crhs[c], cdims[0], cdims[1], lo[0], lo[1], lo[2], e[0], e[1],
-                                                  e[2], 1.0 / (dc[0] * dc[0]), 1.0 / (dc[1] * dc[1]),
-                                                  1.0 / (dc[2] * dc[2]));
-    VPMG_LAUNCHED();
-  }
+  k_coarse_lap<<<dim3(grid_for(n, 256), 3), 256, 0, s>>>(In3{{samp[0], samp[1], samp[2]}},
+                                                         Out3{{crhs[0], crhs[1], crhs[2]}}, cdims[0], cdims[1], lo[0],
+                                                         lo[1], lo[2], e[0], e[1], e[2], 1.0 / (dc[0] * dc[0]),
+                                                         1.0 / (dc[1] * dc[1]), 1.0 / (dc[2] * dc[2]));
+  VPMG_LAUNCHED();
   VPMG_CUDA(cudaGetLastError());
 }
 
 void yaps_face_interp(const YapsDev& Y, const int cdims[3], const double* const csol[3], const double* const samp[3],
                       double* const sbl[3], cudaStream_t s) {
-  for (int c = 0; c < 3; ++c) {
-    k_face_interp<<<grid_for(Y.nface, 128), 128, 0, s>>>(Y.face_node.p, Y.face_cbase.p, Y.face_w.p, Y.face_flag.p,
-                                                         Y.nface, csol[c], samp[c], cdims[0], cdims[1], sbl[c]);
-    VPMG_LAUNCHED();
-  }
+  k_face_interp<<<dim3(grid_for(Y.nface, 128), 3), 128, 0, s>>>(
+      Y.face_node.p, Y.face_cbase.p, Y.face_w.p, Y.face_flag.p, Y.nface, In3{{csol[0], csol[1], csol[2]}},
+      In3{{samp[0], samp[1], samp[2]}}, cdims[0], cdims[1], Out3{{sbl[0], sbl[1], sbl[2]}});
+  VPMG_LAUNCHED();
   VPMG_CUDA(cudaGetLastError());
 }
 

@@ -15,7 +15,7 @@ struct YapsDev {
 };
 
 void box_copy(const double* src, const int sdims[3], const int so[3], double* dst, const int ddims[3], const int dof[3],
-              const int ext[3], cudaStream_t s);
+              const int ext[3], cudaStream_t s, int nc = 1, size_t scs = 0, size_t dcs = 0);
 void yaps_sample(const YapsDev& Y, const double* const sbl[3], double* const samp[3], cudaStream_t s);
 void yaps_coarse_rhs(const YapsDev& Y, const int cdims[3], const double dc[3], const double* const samp[3],
                      double* const crhs[3], cudaStream_t s);

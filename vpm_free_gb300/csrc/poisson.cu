@@ -15,9 +15,9 @@
 //      extension (two lines in one complex FFT of length 2N);
 //   2. y pass: the same DST-I along y, in place;
 //   3. z pass: per (p,q) mode the constant-coefficient tridiagonal system
-//      -u[k-1] + d_pq u[k] - u[k+1] = r[k] by a Thomas sweep whose
-//      reciprocal pivots come from a table built once per grid (no FP64
-//      divisions per step);
+//      -u[k-1] + d_pq u[k] - u[k+1] = r[k], eliminated from both ends to the
+//      middle with reciprocal pivots from a table built once per grid (no
+//      FP64 divisions per step; thomas_sweep in block_solve.cu);
 //   4. inverse y and x passes (DST-I is its own inverse up to 2/N).
 // FFTs run in shared memory as mixed-radix Stockham stages (radix 2,4,8
 // and odd primes up to 17 through the symmetric direct DFT), instantiated
@@ -362,6 +362,12 @@ __device__ __forceinline__ double dst_out(const typename A::C* O, const FFTDev& 
 }
 
 // ------------------------------------------------------------ passes ----
+// blockIdx.y = component of the solve: the three components of a vector
+// potential go through each pass in one launch.
+struct CompStride {
+  int n;                    // components
+  size_t rhs, sol, work;    // doubles between them
+};
 struct Box {
   int dims[3];  // node array dims
   int o[3];     // node offset of interior (a,b,c) = (0,0,0)
@@ -372,7 +378,11 @@ struct Box {
 template <class Ar, bool ODD, int PAIRS>
 __global__ void __launch_bounds__(kThreads) k_dst_x_fwd(const double* __restrict__ rhs, const double* __restrict__ sol,
                                                         int zero_bc, double* __restrict__ work, Box b, FFTDev p,
-                                                        double ihx2, double ihy2, double ihz2, double scale) {
+                                                        double ihx2, double ihy2, double ihz2, double scale,
+                                                        CompStride cs) {
+  rhs += blockIdx.y * cs.rhs;
+  sol += blockIdx.y * cs.sol;
+  work += blockIdx.y * cs.work;
   extern __shared__ double2 smem[];
   double2* A = smem;
   double2* B = smem + PAIRS * p.M;
@@ -459,8 +469,9 @@ __device__ __forceinline__ void y_body(double* __restrict__ work, int m0, int m1
   }
 }
 template <class Ar, bool ODD, int PAIRS>
-__global__ void __launch_bounds__(kThreads) k_dst_y(double* __restrict__ work, int m0, int m1, int m2, FFTDev p) {
-  y_body<Ar, ODD, PAIRS>(work, m0, m1, m2, p, blockIdx.x);
+__global__ void __launch_bounds__(kThreads) k_dst_y(double* __restrict__ work, int m0, int m1, int m2, FFTDev p,
+                                                    size_t cs) {
+  y_body<Ar, ODD, PAIRS>(work + blockIdx.y * cs, m0, m1, m2, p, blockIdx.x);
 }
 
 // x pass, inverse: work -> interior of sol.
@@ -493,8 +504,8 @@ __device__ __forceinline__ void xinv_body(const double* __restrict__ work, doubl
 }
 template <class Ar, bool ODD, int PAIRS>
 __global__ void __launch_bounds__(kThreads) k_dst_x_inv(const double* __restrict__ work, double* __restrict__ sol, Box b,
-                                                        FFTDev p) {
-  xinv_body<Ar, ODD, PAIRS>(work, sol, b, p, blockIdx.x);
+                                                        FFTDev p, CompStride cs) {
+  xinv_body<Ar, ODD, PAIRS>(work + blockIdx.y * cs.work, sol + blockIdx.y * cs.sol, b, p, blockIdx.x);
 }
 
 // Several small transforms of one solve in one launch (the partially
@@ -508,6 +519,7 @@ struct YJobs {
   int n;
   int tile0[kMaxJobs + 1];
   double* data[kMaxJobs];
+  size_t cs[kMaxJobs];  // doubles between components (blockIdx.y)
   int m0[kMaxJobs], m1[kMaxJobs], m2[kMaxJobs];
   FFTDev p[kMaxJobs];
 };
@@ -516,6 +528,7 @@ struct XJobs {
   int tile0[kMaxJobs + 1];
   const double* work[kMaxJobs];
   double* sol[kMaxJobs];
+  size_t wcs[kMaxJobs], scs[kMaxJobs];
   Box b[kMaxJobs];
   FFTDev p[kMaxJobs];
 };
@@ -527,22 +540,24 @@ __device__ __forceinline__ int job_of(const int* tile0, int n) {
 template <class Ar, bool ODD>
 __global__ void __launch_bounds__(kThreads) k_dst_y_jobs(const __grid_constant__ YJobs J) {
   const int j = job_of(J.tile0, J.n);
-  y_body<Ar, ODD, kJobPairs>(J.data[j], J.m0[j], J.m1[j], J.m2[j], J.p[j], blockIdx.x - J.tile0[j]);
+  y_body<Ar, ODD, kJobPairs>(J.data[j] + blockIdx.y * J.cs[j], J.m0[j], J.m1[j], J.m2[j], J.p[j], blockIdx.x - J.tile0[j]);
 }
 template <class Ar, bool ODD>
 __global__ void __launch_bounds__(kThreads) k_dst_x_inv_jobs(const __grid_constant__ XJobs J) {
   const int j = job_of(J.tile0, J.n);
-  xinv_body<Ar, ODD, kJobPairs>(J.work[j], J.sol[j], J.b[j], J.p[j], blockIdx.x - J.tile0[j]);
+  xinv_body<Ar, ODD, kJobPairs>(J.work[j] + blockIdx.y * J.wcs[j], J.sol[j] + blockIdx.y * J.scs[j], J.b[j], J.p[j],
+                                blockIdx.x - J.tile0[j]);
 }
 
-// z pass: Thomas sweep per (p,q) with the reciprocal pivot table (FP64:
-// rinvd, float-float: rinvf), in the policy's arithmetic: the forward
-// sweep leaves its values in place in that arithmetic, the backward sweep
-// writes the doubles.  The column's loads are issued four planes ahead of
-// the dependent chain (the sweep is latency-bound otherwise).
-template <class A>
-__global__ void k_thomas(double* __restrict__ g, const typename A::R* __restrict__ rinv, int m0, int m1, int m2) {
-  using R = typename A::R;
+// z pass in float-float: Thomas sweep per (p,q) with the reciprocal pivot
+// table rinvf; the forward sweep leaves its values in place as float-float
+// pairs, the backward sweep writes the doubles.  The column's loads are
+// issued four planes ahead of the dependent chain.  (FP64: thomas_sweep.)
+__global__ void k_thomas_ff(double* __restrict__ g, const float2* __restrict__ rinv, int m0, int m1, int m2,
+                            size_t cs) {
+  using A = FF;
+  using R = A::R;
+  g += blockIdx.y * cs;
   const int pq = blockIdx.x * blockDim.x + threadIdx.x;
   if (pq >= m0 * m1) return;
   const size_t plane = (size_t)m0 * m1;
@@ -594,34 +609,37 @@ __global__ void k_thomas(double* __restrict__ g, const typename A::R* __restrict
   }
 }
 
-// Reciprocal pivots 1/d, 1/(d - r), ... in FP64, stored as doubles (rinvd)
-// and as float-float pairs (rinvf); either may be null.
+// Reciprocal pivots of -u[k-1] + d u[k] - u[k+1], d = 2 + e:
+//   rinv_0 = 1 / d,  rinv_k = 1 / (d - rinv_{k-1}).
+// rinv tends to 1 for the smooth modes, so its complement s_k = 1 - rinv_k is
+// what the recurrence carries: t = e + s_{k-1}, rinv_k = 1 / (1 + t),
+// s_k = t / (1 + t) has no cancellation.  FP64 (rinvd): the elimination runs
+// from both ends, so rows 0..h-1 (h = m2 / 2) hold rinv_k and row h the
+// middle's constant, rinv / (1 - rinv^2) for even m2 and 1 / (d - 2 rinv)
+// for odd m2.  Float-float (rinvf): all m2 rows, as pairs.  Either may be null.
 __global__ void k_pivots(float2* __restrict__ rinvf, double* __restrict__ rinvd, const double* __restrict__ mux,
                          const double* __restrict__ muy, int m0, int m1, int m2, double cx, double cy) {
   const int pq = blockIdx.x * blockDim.x + threadIdx.x;
   if (pq >= m0 * m1) return;
   const int p = pq % m0, q = pq / m0;
-  const double d = 2.0 + (mux[p] * cx + muy[q] * cy);
+  const double e = mux[p] * cx + muy[q] * cy;
   const size_t plane = (size_t)m0 * m1;
-  double r = 1.0 / d;
-  if (rinvf) rinvf[pq] = ff::split(r);
-  if (rinvd) rinvd[pq] = r;
-  for (int c = 1; c < m2; ++c) {
-    r = 1.0 / (d - r);
-    if (rinvf) rinvf[pq + plane * c] = ff::split(r);
-    if (rinvd) rinvd[pq + plane * c] = r;
+  const int h = m2 / 2, rows = rinvf ? m2 : h;
+  double s = 1.0, sm = 1.0;  // s_{-1} = 1 (rinv_{-1} = 0); sm = s_{h-1}
+  for (int k = 0; k < rows; ++k) {
+    const double t = e + s;
+    const double r = 1.0 / (1.0 + t);
+    s = t * r;
+    if (k == h - 1) sm = s;
+    if (rinvf) rinvf[pq + plane * k] = ff::split(r);
+    if (rinvd && k < h) rinvd[pq + plane * k] = r;
   }
+  // 1 - rinv^2 = s (2 - s) and d - 2 rinv = e + 2 s
+  if (rinvd) rinvd[pq + plane * h] = (m2 & 1) ? 1.0 / (e + 2.0 * sm) : (1.0 - sm) / (sm * (2.0 - sm));
 }
 
-void launch_thomas(cudaStream_t s, double* work, const DirichletPlan& P, int arith) {
-  const int nl = P.m[0] * P.m[1];
-  if (arith == VPMG_ARITH_FF48)
-    k_thomas<FF><<<(nl + 127) / 128, 128, 0, s>>>(work, P.rinv.p, P.m[0], P.m[1], P.m[2]);
-  else
-    k_thomas<F64><<<(nl + 127) / 128, 128, 0, s>>>(work, P.rinvd.p, P.m[0], P.m[1], P.m[2]);
-}
-
-__global__ void k_zero_box_faces(double* __restrict__ sol, Box b) {
+__global__ void k_zero_box_faces(double* __restrict__ sol, Box b, size_t cs) {
+  sol += blockIdx.y * cs;
   // faces of the box [o-1, o+m] in each direction
   const int ex = b.m[0] + 2, ey = b.m[1] + 2, ez = b.m[2] + 2;
   const long total = 2L * ey * ez + 2L * ex * ez + 2L * ex * ey;
@@ -654,56 +672,56 @@ unsigned tile_grid(int lines, const FFTDev& p) { return (unsigned)((lines + 2 * 
 
 template <class A, int PAIRS>
 void x_fwd_t(cudaStream_t s, const double* rhs, const double* sol, int zbc, double* work, Box b, FFTDev p,
-             double ihx2, double ihy2, double ihz2, double scale) {
-  const unsigned g = tile_grid(b.m[1] * b.m[2], p);
+             double ihx2, double ihy2, double ihz2, double scale, CompStride cs) {
+  const dim3 g(tile_grid(b.m[1] * b.m[2], p), cs.n);
   if (p.odd)
-    k_dst_x_fwd<A, true, PAIRS><<<g, kThreads, tile_smem(p), s>>>(rhs, sol, zbc, work, b, p, ihx2, ihy2, ihz2, scale);
+    k_dst_x_fwd<A, true, PAIRS><<<g, kThreads, tile_smem(p), s>>>(rhs, sol, zbc, work, b, p, ihx2, ihy2, ihz2, scale, cs);
   else
-    k_dst_x_fwd<A, false, PAIRS><<<g, kThreads, tile_smem(p), s>>>(rhs, sol, zbc, work, b, p, ihx2, ihy2, ihz2, scale);
+    k_dst_x_fwd<A, false, PAIRS><<<g, kThreads, tile_smem(p), s>>>(rhs, sol, zbc, work, b, p, ihx2, ihy2, ihz2, scale, cs);
 }
 template <class A, int PAIRS>
-void y_t(cudaStream_t s, double* work, int m0, int m1, int m2, FFTDev p) {
-  const unsigned g = tile_grid(m0 * m2, p);
-  if (p.odd) k_dst_y<A, true, PAIRS><<<g, kThreads, tile_smem(p), s>>>(work, m0, m1, m2, p);
-  else k_dst_y<A, false, PAIRS><<<g, kThreads, tile_smem(p), s>>>(work, m0, m1, m2, p);
+void y_t(cudaStream_t s, double* work, int m0, int m1, int m2, FFTDev p, int nc, size_t cs) {
+  const dim3 g(tile_grid(m0 * m2, p), nc);
+  if (p.odd) k_dst_y<A, true, PAIRS><<<g, kThreads, tile_smem(p), s>>>(work, m0, m1, m2, p, cs);
+  else k_dst_y<A, false, PAIRS><<<g, kThreads, tile_smem(p), s>>>(work, m0, m1, m2, p, cs);
 }
 template <class A, int PAIRS>
-void x_inv_t(cudaStream_t s, const double* work, double* sol, Box b, FFTDev p) {
-  const unsigned g = tile_grid(b.m[1] * b.m[2], p);
-  if (p.odd) k_dst_x_inv<A, true, PAIRS><<<g, kThreads, tile_smem(p), s>>>(work, sol, b, p);
-  else k_dst_x_inv<A, false, PAIRS><<<g, kThreads, tile_smem(p), s>>>(work, sol, b, p);
+void x_inv_t(cudaStream_t s, const double* work, double* sol, Box b, FFTDev p, CompStride cs) {
+  const dim3 g(tile_grid(b.m[1] * b.m[2], p), cs.n);
+  if (p.odd) k_dst_x_inv<A, true, PAIRS><<<g, kThreads, tile_smem(p), s>>>(work, sol, b, p, cs);
+  else k_dst_x_inv<A, false, PAIRS><<<g, kThreads, tile_smem(p), s>>>(work, sol, b, p, cs);
 }
 template <class A>
 void launch_x_fwd_a(cudaStream_t s, const double* rhs, const double* sol, int zbc, double* work, Box b, FFTDev p,
-                    double ihx2, double ihy2, double ihz2, double scale) {
-  if (p.pairs == 2) x_fwd_t<A, 2>(s, rhs, sol, zbc, work, b, p, ihx2, ihy2, ihz2, scale);
-  else if (p.pairs == 8) x_fwd_t<A, 8>(s, rhs, sol, zbc, work, b, p, ihx2, ihy2, ihz2, scale);
-  else x_fwd_t<A, 4>(s, rhs, sol, zbc, work, b, p, ihx2, ihy2, ihz2, scale);
+                    double ihx2, double ihy2, double ihz2, double scale, CompStride cs) {
+  if (p.pairs == 2) x_fwd_t<A, 2>(s, rhs, sol, zbc, work, b, p, ihx2, ihy2, ihz2, scale, cs);
+  else if (p.pairs == 8) x_fwd_t<A, 8>(s, rhs, sol, zbc, work, b, p, ihx2, ihy2, ihz2, scale, cs);
+  else x_fwd_t<A, 4>(s, rhs, sol, zbc, work, b, p, ihx2, ihy2, ihz2, scale, cs);
 }
 template <class A>
-void launch_y_a(cudaStream_t s, double* work, int m0, int m1, int m2, FFTDev p) {
-  if (p.pairs == 2) y_t<A, 2>(s, work, m0, m1, m2, p);
-  else if (p.pairs == 8) y_t<A, 8>(s, work, m0, m1, m2, p);
-  else y_t<A, 4>(s, work, m0, m1, m2, p);
+void launch_y_a(cudaStream_t s, double* work, int m0, int m1, int m2, FFTDev p, int nc, size_t cs) {
+  if (p.pairs == 2) y_t<A, 2>(s, work, m0, m1, m2, p, nc, cs);
+  else if (p.pairs == 8) y_t<A, 8>(s, work, m0, m1, m2, p, nc, cs);
+  else y_t<A, 4>(s, work, m0, m1, m2, p, nc, cs);
 }
 template <class A>
-void launch_x_inv_a(cudaStream_t s, const double* work, double* sol, Box b, FFTDev p) {
-  if (p.pairs == 2) x_inv_t<A, 2>(s, work, sol, b, p);
-  else if (p.pairs == 8) x_inv_t<A, 8>(s, work, sol, b, p);
-  else x_inv_t<A, 4>(s, work, sol, b, p);
+void launch_x_inv_a(cudaStream_t s, const double* work, double* sol, Box b, FFTDev p, CompStride cs) {
+  if (p.pairs == 2) x_inv_t<A, 2>(s, work, sol, b, p, cs);
+  else if (p.pairs == 8) x_inv_t<A, 8>(s, work, sol, b, p, cs);
+  else x_inv_t<A, 4>(s, work, sol, b, p, cs);
 }
 void launch_x_fwd(cudaStream_t s, const double* rhs, const double* sol, int zbc, double* work, Box b, FFTDev p,
-                  double ihx2, double ihy2, double ihz2, double scale) {
-  if (p.arith == VPMG_ARITH_FF48) launch_x_fwd_a<FF>(s, rhs, sol, zbc, work, b, p, ihx2, ihy2, ihz2, scale);
-  else launch_x_fwd_a<F64>(s, rhs, sol, zbc, work, b, p, ihx2, ihy2, ihz2, scale);
+                  double ihx2, double ihy2, double ihz2, double scale, CompStride cs) {
+  if (p.arith == VPMG_ARITH_FF48) launch_x_fwd_a<FF>(s, rhs, sol, zbc, work, b, p, ihx2, ihy2, ihz2, scale, cs);
+  else launch_x_fwd_a<F64>(s, rhs, sol, zbc, work, b, p, ihx2, ihy2, ihz2, scale, cs);
 }
-void launch_y(cudaStream_t s, double* work, int m0, int m1, int m2, FFTDev p) {
-  if (p.arith == VPMG_ARITH_FF48) launch_y_a<FF>(s, work, m0, m1, m2, p);
-  else launch_y_a<F64>(s, work, m0, m1, m2, p);
+void launch_y(cudaStream_t s, double* work, int m0, int m1, int m2, FFTDev p, int nc = 1, size_t cs = 0) {
+  if (p.arith == VPMG_ARITH_FF48) launch_y_a<FF>(s, work, m0, m1, m2, p, nc, cs);
+  else launch_y_a<F64>(s, work, m0, m1, m2, p, nc, cs);
 }
-void launch_x_inv(cudaStream_t s, const double* work, double* sol, Box b, FFTDev p) {
-  if (p.arith == VPMG_ARITH_FF48) launch_x_inv_a<FF>(s, work, sol, b, p);
-  else launch_x_inv_a<F64>(s, work, sol, b, p);
+void launch_x_inv(cudaStream_t s, const double* work, double* sol, Box b, FFTDev p, CompStride cs) {
+  if (p.arith == VPMG_ARITH_FF48) launch_x_inv_a<FF>(s, work, sol, b, p, cs);
+  else launch_x_inv_a<F64>(s, work, sol, b, p, cs);
 }
 template <class A, int PAIRS>
 cudaError_t set_smem_t(int smax) {
@@ -941,11 +959,13 @@ void dirichlet_prepare(DirichletPlan& P, const int dims[3], const int box[6], co
   dmy.ensure(P.m[1]);
   VPMG_CUDA(cudaMemcpy(dmx.p, mux.data(), sizeof(double) * P.m[0], cudaMemcpyHostToDevice));
   VPMG_CUDA(cudaMemcpy(dmy.p, muy.data(), sizeof(double) * P.m[1], cudaMemcpyHostToDevice));
-  P.rinv.ensure((size_t)P.m[0] * P.m[1] * P.m[2]);
-  P.rinvd.ensure((size_t)P.m[0] * P.m[1] * P.m[2]);
+  const bool ffp = arith == VPMG_ARITH_FF48;  // the float-float sweep's table
+  if (ffp) P.rinv.ensure((size_t)P.m[0] * P.m[1] * P.m[2]);
+  else P.rinv.release();
+  P.rinvd.ensure((size_t)P.m[0] * P.m[1] * (P.m[2] / 2 + 1));
   const double hz2 = h[2] * h[2];
   const int nl = P.m[0] * P.m[1];
-  k_pivots<<<(nl + 255) / 256, 256, 0, s>>>(P.rinv.p, P.rinvd.p, dmx.p, dmy.p, P.m[0], P.m[1], P.m[2], hz2 / (h[0] * h[0]),
+  k_pivots<<<(nl + 255) / 256, 256, 0, s>>>(ffp ? P.rinv.p : nullptr, P.rinvd.p, dmx.p, dmy.p, P.m[0], P.m[1], P.m[2], hz2 / (h[0] * h[0]),
                                             hz2 / (h[1] * h[1]));
   VPMG_LAUNCHED();
   VPMG_CUDA(cudaGetLastError());
@@ -953,21 +973,29 @@ void dirichlet_prepare(DirichletPlan& P, const int dims[3], const int box[6], co
   P.ready = true;
 }
 
-void dirichlet_solve(DirichletPlan& P, const double* rhs, double* sol, bool zero_bc, double* work, cudaStream_t s) {
+void dirichlet_solve(DirichletPlan& P, const double* rhs, double* sol, bool zero_bc, double* work, cudaStream_t s,
+                     int nc, size_t rcs, size_t scs) {
   Box b;
   for (int d = 0; d < 3; ++d) { b.dims[d] = P.dims[d]; b.o[d] = P.box[d] + 1; b.m[d] = P.m[d]; }
   const FFTDev px = dev_plan(P.fx), py = dev_plan(P.fy);
   const double hx2 = P.h[0] * P.h[0], hy2 = P.h[1] * P.h[1], hz2 = P.h[2] * P.h[2];
   // Thomas RHS r = -hz^2 * ghat, with the inverse DST normalisation 4/(Nx Ny).
-  const double scale = -hz2 * 4.0 / ((double)(P.m[0] + 1) * (double)(P.m[1] + 1));
-  launch_x_fwd(s, rhs, sol, zero_bc ? 1 : 0, work, b, px, 1.0 / hx2, 1.0 / hy2, 1.0 / hz2, scale);
-  launch_y(s, work, P.m[0], P.m[1], P.m[2], py);
-  launch_thomas(s, work, P, P.arith);
-  launch_y(s, work, P.m[0], P.m[1], P.m[2], py);
-  launch_x_inv(s, work, sol, b, px);
-  count_launch(5);
+  const double scale = dirichlet_scale(P);
+  const size_t wcs = (size_t)P.m[0] * P.m[1] * P.m[2];
+  const CompStride cs{nc, rcs, scs, wcs};
+  launch_x_fwd(s, rhs, sol, zero_bc ? 1 : 0, work, b, px, 1.0 / hx2, 1.0 / hy2, 1.0 / hz2, scale, cs);
+  launch_y(s, work, P.m[0], P.m[1], P.m[2], py, nc, wcs);
+  if (P.arith == VPMG_ARITH_FF48) {
+    const int nl = P.m[0] * P.m[1];
+    k_thomas_ff<<<dim3((nl + 127) / 128, nc), 128, 0, s>>>(work, P.rinv.p, P.m[0], P.m[1], P.m[2], wcs);
+  } else {
+    thomas_sweep(work, work, P.rinvd.p, P.m, nc, wcs, nullptr, s);
+  }
+  launch_y(s, work, P.m[0], P.m[1], P.m[2], py, nc, wcs);
+  launch_x_inv(s, work, sol, b, px, cs);
+  count_launch(P.arith == VPMG_ARITH_FF48 ? 5 : 4);
   if (zero_bc) {
-    k_zero_box_faces<<<256, 256, 0, s>>>(sol, b);
+    k_zero_box_faces<<<dim3(256, nc), 256, 0, s>>>(sol, b, scs);
     VPMG_LAUNCHED();
   }
   VPMG_CUDA(cudaGetLastError());
@@ -977,14 +1005,16 @@ void dirichlet_solve(DirichletPlan& P, const double* rhs, double* sol, bool zero
 // Forward x and y passes only: ghat = scale * DST_y DST_x (rhs - folded
 // boundary values), the input of the Thomas sweep.
 void dst_forward_xy(DirichletPlan& P, const double* rhs, const double* sol, bool zero_bc, double* ghat,
-                    cudaStream_t s) {
+                    cudaStream_t s, int nc, size_t rcs, size_t scs) {
   Box b;
   for (int d = 0; d < 3; ++d) { b.dims[d] = P.dims[d]; b.o[d] = P.box[d] + 1; b.m[d] = P.m[d]; }
   const FFTDev px = dev_plan(P.fx), py = dev_plan(P.fy);
   const double hx2 = P.h[0] * P.h[0], hy2 = P.h[1] * P.h[1], hz2 = P.h[2] * P.h[2];
   const double scale = dirichlet_scale(P);
-  launch_x_fwd(s, rhs, sol, zero_bc ? 1 : 0, ghat, b, px, 1.0 / hx2, 1.0 / hy2, 1.0 / hz2, scale);
-  launch_y(s, ghat, P.m[0], P.m[1], P.m[2], py);
+  const size_t wcs = (size_t)P.m[0] * P.m[1] * P.m[2];
+  const CompStride cs{nc, rcs, scs, wcs};
+  launch_x_fwd(s, rhs, sol, zero_bc ? 1 : 0, ghat, b, px, 1.0 / hx2, 1.0 / hy2, 1.0 / hz2, scale, cs);
+  launch_y(s, ghat, P.m[0], P.m[1], P.m[2], py, nc, wcs);
   count_launch(2);
   VPMG_CUDA(cudaGetLastError());
 }
@@ -996,10 +1026,10 @@ double dirichlet_scale(const DirichletPlan& P) {
 
 // In-place DST-I along the middle axis of an m0 x m1 x m2 array (m1 = p.n).
 // With m0 = 1 it transforms contiguous rows.
-void dst_lines_y(const FFTPlan& p, double* data, int m0, int m1, int m2, cudaStream_t s) {
+void dst_lines_y(const FFTPlan& p, double* data, int m0, int m1, int m2, cudaStream_t s, int nc, size_t cs) {
   if (m0 <= 0 || m2 <= 0) return;
   VPMG_CHECK(m1 == p.n, VPMG_ERR_ARG, "dst_lines_y: line length differs from the plan");
-  launch_y(s, data, m0, m1, m2, dev_plan(p));
+  launch_y(s, data, m0, m1, m2, dev_plan(p), nc, cs);
   VPMG_LAUNCHED();
   VPMG_CUDA(cudaGetLastError());
 }
@@ -1007,19 +1037,19 @@ void dst_lines_y(const FFTPlan& p, double* data, int m0, int m1, int m2, cudaStr
 // Inverse DST-I along x of the m[0] x m[1] x m[2] array `data`; line (q, c)
 // lands on nodes (o0 + k, o1 + q, o2 + c) of the node array sol (dims).
 void dst_x_inv_to_box(const FFTPlan& p, const double* data, double* sol, const int dims[3], const int o[3],
-                      const int m[3], cudaStream_t s) {
+                      const int m[3], cudaStream_t s, int nc, size_t wcs, size_t scs) {
   if (m[1] <= 0 || m[2] <= 0) return;
   VPMG_CHECK(m[0] == p.n, VPMG_ERR_ARG, "dst_x_inv_to_box: line length differs from the plan");
   Box b;
   for (int d = 0; d < 3; ++d) { b.dims[d] = dims[d]; b.o[d] = o[d]; b.m[d] = m[d]; }
-  launch_x_inv(s, data, sol, b, dev_plan(p));
+  launch_x_inv(s, data, sol, b, dev_plan(p), CompStride{nc, 0, scs, wcs});
   VPMG_LAUNCHED();
   VPMG_CUDA(cudaGetLastError());
 }
 
 // Job lists: several small transforms in one launch (tiles of kJobPairs line
 // pairs; all jobs in the plans' common arithmetic).
-void dst_lines_y_jobs(const DstYLines* jobs, int n, cudaStream_t s) {
+void dst_lines_y_jobs(const DstYLines* jobs, int n, cudaStream_t s, int nc) {
   VPMG_CHECK(n >= 1 && n <= kMaxJobs, VPMG_ERR_ARG, "dst_lines_y_jobs: 1..8 jobs");
   YJobs J{};
   J.n = n;
@@ -1029,7 +1059,7 @@ void dst_lines_y_jobs(const DstYLines* jobs, int n, cudaStream_t s) {
     const DstYLines& q = jobs[j];
     VPMG_CHECK(q.m1 == q.plan->n && q.plan->arith == arith, VPMG_ERR_ARG, "dst_lines_y_jobs: plan mismatch");
     J.tile0[j] = tiles;
-    J.data[j] = q.data; J.m0[j] = q.m0; J.m1[j] = q.m1; J.m2[j] = q.m2;
+    J.data[j] = q.data; J.cs[j] = q.cs; J.m0[j] = q.m0; J.m1[j] = q.m1; J.m2[j] = q.m2;
     J.p[j] = dev_plan(*q.plan);
     J.p[j].pairs = kJobPairs;
     odd |= J.p[j].odd;
@@ -1039,17 +1069,17 @@ void dst_lines_y_jobs(const DstYLines* jobs, int n, cudaStream_t s) {
   J.tile0[n] = tiles;
   if (tiles == 0) return;
   if (arith == VPMG_ARITH_FF48) {
-    if (odd) k_dst_y_jobs<FF, true><<<tiles, kThreads, smem, s>>>(J);
-    else k_dst_y_jobs<FF, false><<<tiles, kThreads, smem, s>>>(J);
+    if (odd) k_dst_y_jobs<FF, true><<<dim3(tiles, nc), kThreads, smem, s>>>(J);
+    else k_dst_y_jobs<FF, false><<<dim3(tiles, nc), kThreads, smem, s>>>(J);
   } else {
-    if (odd) k_dst_y_jobs<F64, true><<<tiles, kThreads, smem, s>>>(J);
-    else k_dst_y_jobs<F64, false><<<tiles, kThreads, smem, s>>>(J);
+    if (odd) k_dst_y_jobs<F64, true><<<dim3(tiles, nc), kThreads, smem, s>>>(J);
+    else k_dst_y_jobs<F64, false><<<dim3(tiles, nc), kThreads, smem, s>>>(J);
   }
   VPMG_LAUNCHED();
   VPMG_CUDA(cudaGetLastError());
 }
 
-void dst_x_inv_jobs(const DstXInvLines* jobs, int n, cudaStream_t s) {
+void dst_x_inv_jobs(const DstXInvLines* jobs, int n, cudaStream_t s, int nc) {
   VPMG_CHECK(n >= 1 && n <= kMaxJobs, VPMG_ERR_ARG, "dst_x_inv_jobs: 1..8 jobs");
   XJobs J{};
   J.n = n;
@@ -1061,6 +1091,8 @@ void dst_x_inv_jobs(const DstXInvLines* jobs, int n, cudaStream_t s) {
     J.tile0[j] = tiles;
     J.work[j] = q.data;
     J.sol[j] = q.sol;
+    J.wcs[j] = q.wcs;
+    J.scs[j] = q.scs;
     for (int d = 0; d < 3; ++d) { J.b[j].dims[d] = q.dims[d]; J.b[j].o[d] = q.o[d]; J.b[j].m[d] = q.m[d]; }
     J.p[j] = dev_plan(*q.plan);
     J.p[j].pairs = kJobPairs;
@@ -1071,11 +1103,11 @@ void dst_x_inv_jobs(const DstXInvLines* jobs, int n, cudaStream_t s) {
   J.tile0[n] = tiles;
   if (tiles == 0) return;
   if (arith == VPMG_ARITH_FF48) {
-    if (odd) k_dst_x_inv_jobs<FF, true><<<tiles, kThreads, smem, s>>>(J);
-    else k_dst_x_inv_jobs<FF, false><<<tiles, kThreads, smem, s>>>(J);
+    if (odd) k_dst_x_inv_jobs<FF, true><<<dim3(tiles, nc), kThreads, smem, s>>>(J);
+    else k_dst_x_inv_jobs<FF, false><<<dim3(tiles, nc), kThreads, smem, s>>>(J);
   } else {
-    if (odd) k_dst_x_inv_jobs<F64, true><<<tiles, kThreads, smem, s>>>(J);
-    else k_dst_x_inv_jobs<F64, false><<<tiles, kThreads, smem, s>>>(J);
+    if (odd) k_dst_x_inv_jobs<F64, true><<<dim3(tiles, nc), kThreads, smem, s>>>(J);
+    else k_dst_x_inv_jobs<F64, false><<<dim3(tiles, nc), kThreads, smem, s>>>(J);
   }
   VPMG_LAUNCHED();
   VPMG_CUDA(cudaGetLastError());
@@ -1219,12 +1251,13 @@ extern "C" int vpmg_dirichlet_static(const double* rhs, double* sol, const int d
   Box b;
   for (int d = 0; d < 3; ++d) { b.dims[d] = dims[d]; b.o[d] = box[d] + 1; b.m[d] = m[d]; }
   const double scale = -hz2 * 4.0 / ((double)(m[0] + 1) * (double)(m[1] + 1));
-  launch_x_fwd(s, rhs, sol, zero_bc ? 1 : 0, work, b, px, 1.0 / hx2, 1.0 / hy2, 1.0 / hz2, scale);
+  const CompStride cs{1, 0, 0, 0};
+  launch_x_fwd(s, rhs, sol, zero_bc ? 1 : 0, work, b, px, 1.0 / hx2, 1.0 / hy2, 1.0 / hz2, scale, cs);
   launch_y(s, work, m[0], m[1], m[2], py);
-  k_thomas<F64><<<(nl + 127) / 128, 128, 0, s>>>(work, rinv, m[0], m[1], m[2]);
+  thomas_launch(work, work, rinv, m, 1, 0, nullptr, s);
   launch_y(s, work, m[0], m[1], m[2], py);
-  launch_x_inv(s, work, sol, b, px);
-  if (zero_bc) k_zero_box_faces<<<256, 256, 0, s>>>(sol, b);
+  launch_x_inv(s, work, sol, b, px, cs);
+  if (zero_bc) k_zero_box_faces<<<256, 256, 0, s>>>(sol, b, 0);
   if (cudaGetLastError() != cudaSuccess) return VPMG_ERR_CUDA;
   return VPMG_OK;
 }

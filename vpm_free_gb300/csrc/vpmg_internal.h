@@ -99,8 +99,8 @@ struct DirichletPlan {
   double h[3] = {0, 0, 0};
   int arith = VPMG_ARITH_FP64;  // arithmetic of the transforms and sweeps
   FFTPlan fx, fy;
-  DBuf<float2> rinv;  // reciprocal Thomas pivots, [k][q][p], float-float pairs
-  DBuf<double> rinvd; // the same in FP64
+  DBuf<float2> rinv;  // float-float plans: reciprocal Thomas pivots, [k][q][p], float-float pairs
+  DBuf<double> rinvd; // FP64: rows 0..m2/2-1 of them and the middle's constant (thomas_sweep)
   bool ready = false;
 };
 void dirichlet_prepare(DirichletPlan& P, const int dims[3], const int box[6], const double h[3], cudaStream_t s,
@@ -108,29 +108,47 @@ void dirichlet_prepare(DirichletPlan& P, const int dims[3], const int box[6], co
 // Interior of sol <- solution of Lap_h u = rhs with the box faces of sol as
 // boundary values (zero_bc = false) or zero (true; then the box faces of
 // sol are zeroed).  work: >= m0*m1*m2 doubles.
-void dirichlet_solve(DirichletPlan& P, const double* rhs, double* sol, bool zero_bc, double* work, cudaStream_t s);
+// nc components in one pass: rhs and sol rcs and scs doubles apart, work
+// nc * m0*m1*m2 doubles.
+void dirichlet_solve(DirichletPlan& P, const double* rhs, double* sol, bool zero_bc, double* work, cudaStream_t s,
+                     int nc = 1, size_t rcs = 0, size_t scs = 0);
+// The z pass in FP64 (block_solve.cu): per mode (p,q) and component the
+// tridiagonal system -u[k-1] + d u[k] - u[k+1] = g[k] (+ face terms), from
+// g to out (may be the same array), components cs doubles apart.
+struct FaceTerms {
+  const double *fxs, *fxd, *fys, *fyd, *fz0, *fzN;  // transforms: [k][q], [k][p], [q][p]
+  size_t cs;                                        // doubles between components
+  const double *ex1, *ey1;                          // sin(pi (p+1)/(m+1)) along x and y
+  double cx, cy, cz;                                // -scale / h^2
+};
+void thomas_launch(const double* g, double* out, const double* rinv, const int m[3], int nc, size_t cs,
+                   const FaceTerms* F, cudaStream_t s);
+void thomas_sweep(const double* g, double* out, const double* rinv, const int m[3], int nc, size_t cs,
+                  const FaceTerms* F, cudaStream_t s);  // the same, counted
 // Pieces of a partially evaluated solve (block_solve.cu).
 double dirichlet_scale(const DirichletPlan& P);  // factor applied in the forward x pass
 void dst_forward_xy(DirichletPlan& P, const double* rhs, const double* sol, bool zero_bc, double* ghat,
-                    cudaStream_t s);
-void dst_lines_y(const FFTPlan& p, double* data, int m0, int m1, int m2, cudaStream_t s);
+                    cudaStream_t s, int nc = 1, size_t rcs = 0, size_t scs = 0);
+void dst_lines_y(const FFTPlan& p, double* data, int m0, int m1, int m2, cudaStream_t s, int nc = 1, size_t cs = 0);
 void dst_x_inv_to_box(const FFTPlan& p, const double* data, double* sol, const int dims[3], const int o[3],
-                      const int m[3], cudaStream_t s);
+                      const int m[3], cudaStream_t s, int nc = 1, size_t wcs = 0, size_t scs = 0);
 // Up to 8 of the above in one launch (each job with its own plan and arrays;
 // the plans share one arithmetic).  Results equal the single launches'.
 struct DstYLines {
   const FFTPlan* plan;
   double* data;
   int m0, m1, m2;
+  size_t cs;  // doubles between the nc components
 };
-void dst_lines_y_jobs(const DstYLines* jobs, int n, cudaStream_t s);
+void dst_lines_y_jobs(const DstYLines* jobs, int n, cudaStream_t s, int nc);
 struct DstXInvLines {
   const FFTPlan* plan;
   const double* data;
   double* sol;
   int dims[3], o[3], m[3];
+  size_t wcs, scs;
 };
-void dst_x_inv_jobs(const DstXInvLines* jobs, int n, cudaStream_t s);
+void dst_x_inv_jobs(const DstXInvLines* jobs, int n, cudaStream_t s, int nc);
 
 // ------------------------------------------------- boundary operator ----
 struct TreeGeom;  // host-built quadtree of one grid (tree_host.cpp)
@@ -232,9 +250,10 @@ void farfield_prepare(BoundaryOp& B, const Grid& g, cudaStream_t s);
 // dsum[comp][target] = sum over every coarsest cell of dS/r times its source.
 void farfield_apply(BoundaryOp& B, double* dsum, cudaStream_t s);
 void farfield_release(BoundaryOp& B);
-// Per component: normal-derivative panels from the zero-BC solution sol0,
-// aggregate, then add the boundary values into the faces of sol.
-void boundary_panels(BoundaryOp& B, const Grid& g, const double* sol0, int comp, cudaStream_t s);
+// Normal-derivative panels of the three components from their zero-BC
+// solutions (scs doubles apart); boundary_apply aggregates them and adds the
+// boundary values into the faces of sol.
+void boundary_panels(BoundaryOp& B, const Grid& g, const double* sol0, size_t scs, cudaStream_t s);
 void boundary_apply(BoundaryOp& B, const Grid& g, double* const sol[3], cudaStream_t s);
 // Problems that share one recorded operator (same index geometry, weights
 // in proportion to the mesh spacing): each problem's sources go to its slot
