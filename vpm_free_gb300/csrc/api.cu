@@ -1257,13 +1257,12 @@ int vpmg_bench_kernel(vpmg_handle* h, int which, int reps, double* ms, double* f
       // streamed bytes: 12 per row entry (cell id + weight pair), 8 per slot of the dense block
       by = bo->precomputed ? (double)bo->nnz * (sizeof(int) + sizeof(float2)) + (double)bo->wtop.bytes() : 0.0;
       if (bo->ff.on) {
-        // the coarsest level by FFT: the finer rows and the correction rows
-        // at three FMAs per entry, plus the transforms' flops; bytes: both
-        // row lists, the kernel spectra, and the transform arrays read and
-        // written once per pass
+        // the coarsest level by FFT and the correction rows (three FMAs per
+        // entry) in FP64; bytes: the tables, the kernel spectra, and the
+        // transform arrays read and written once per pass
         const FarField& F = bo->ff;
-        fl = 6.0 * ((double)bo->nnz + (double)F.ncorr) + F.flops;
-        by = 12.0 * ((double)bo->nnz + (double)F.ncorr) + (double)(F.kperp.bytes() + F.kpar.bytes()) +
+        fl = 6.0 * (double)F.ncorr + F.flops;
+        by = 12.0 * (double)F.ncorr + (double)(F.kperp.bytes() + F.kpar.bytes()) + (double)bo->near.bytes() +
              4.0 * (double)(F.S2.bytes() + F.X.bytes() + F.Z.bytes() + F.Sw.bytes() + F.T.bytes());
       }
     } else if (which == 1) {

@@ -718,18 +718,12 @@ __global__ void k_apply_corr(const int* __restrict__ rows, const long long* __re
   }
 }
 
-// calc_normalderiv_3d: one thread per panel, blockIdx.y = component.
-__global__ void k_normal_deriv(const double* __restrict__ sol0, int NX, int NY, int NZ, const int* __restrict__ face,
-                               const int* __restrict__ pi, const int* __restrict__ pj, const int* __restrict__ pk,
-                               int nbound, double invx, double invy, double invz, double* __restrict__ src,
-                               size_t scs, size_t dcs) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= nbound) return;
-  sol0 += blockIdx.y * scs;
-  src += blockIdx.y * dcs;
+// Panel of face f with lower-corner node (i, j, k) (0-based): its source into
+// *src; returns the high word of its magnitude.
+__device__ __forceinline__ unsigned normal_deriv(const double* __restrict__ sol0, int NX, int NY, int f, int i, int j,
+                                                 int k, double invx, double invy, double invz,
+                                                 double* __restrict__ src) {
   const double a1 = 25.0 / 12.0, a2 = -4.0, a3 = 3.0, a4 = -4.0 / 3.0, a5 = 0.25;
-  const int f = face[p];
-  const int i = pi[p] - 1, j = pj[p] - 1, k = pk[p] - 1;  // 0-based
   const long long sx = 1, sy = NX, sz = (long long)NX * NY;
   long long step, e1, e2;
   double inv;
@@ -747,10 +741,29 @@ __global__ void k_normal_deriv(const double* __restrict__ sol0, int NX, int NY, 
                  v4 = sol0[n0 + 4 * step];
     ps[m] = inv * ((((a1 * v0 + a2 * v1) + a3 * v2) + a4 * v3) + a5 * v4);
   }
-  src[p] = 0.25 * (((ps[0] + ps[1]) + ps[2]) + ps[3]);
+  const double v = 0.25 * (((ps[0] + ps[1]) + ps[2]) + ps[3]);
+  *src = v;
+  return (unsigned)__double2hiint(v) & 0x7FFFFFFFu;
 }
 
-// build_level_nbound_3d sources: area-weighted mean over the istep^2 leaves.
+// calc_normalderiv_3d: one thread per panel, blockIdx.y = component.
+__global__ void k_normal_deriv(const double* __restrict__ sol0, int NX, int NY, int NZ, const int* __restrict__ face,
+                               const int* __restrict__ pi, const int* __restrict__ pj, const int* __restrict__ pk,
+                               int nbound, double invx, double invy, double invz, double* __restrict__ src,
+                               size_t scs, size_t dcs, unsigned* __restrict__ smax) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  sol0 += blockIdx.y * scs;
+  src += blockIdx.y * dcs;
+  unsigned hi = 0;
+  if (p < nbound) hi = normal_deriv(sol0, NX, NY, face[p], pi[p] - 1, pj[p] - 1, pk[p] - 1, invx, invy, invz, &src[p]);
+  // the largest panel source of the component, as the high word of its
+  // magnitude: the scale of the near field's integers (levels are averages)
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  if ((threadIdx.x & 31) == 0 && hi) atomicMax(&smax[blockIdx.y], hi);
+}
+
+// build_level_nbound_3d sources: area-weighted mean over the istep^2 leaves,
+// every level at once (they all read the leaves).
 __global__ void k_aggregate(const int* __restrict__ leaf0, const int* __restrict__ rowlen, const int* __restrict__ istep,
                             const double* __restrict__ cds, int first, int ncell, double* __restrict__ s0,
                             double* __restrict__ s1, double* __restrict__ s2) {
@@ -838,7 +851,7 @@ PanelFrame make_frame(int iplane, const double d[3]) {
 long long BoundaryOp::bytes() const {
   return (long long)(rowptr.bytes() + col.bytes() + w.bytes() + colptr.bytes() + trow.bytes() + tw.bytes() +
                      cx.bytes() * 5 + child.bytes() + csrc.bytes() + wtop.bytes() + dsum.bytes()) +
-         ff.bytes();
+         ff.bytes() + near.bytes();
 }
 
 void boundary_prepare(BoundaryOp& B, const Grid& g, int levmax, long long budget_bytes, cudaStream_t s, int ibctyp,
@@ -903,6 +916,8 @@ void boundary_prepare(BoundaryOp& B, const Grid& g, int levmax, long long budget
   upload(B.child, child); upload(B.flags, flags); upload(B.agg_leaf0, leaf0); upload(B.agg_rowlen, rowlen);
   upload(B.agg_istep, istep);
   B.csrc.ensure(3 * (size_t)NC);
+  B.smax.ensure(3);
+  VPMG_CUDA(cudaMemsetAsync(B.smax.p, 0, 3 * sizeof(unsigned), s));
   std::vector<int> pf(B.nbound), pi(B.nbound), pj(B.nbound), pk(B.nbound);
   for (int p = 0; p < B.nbound; ++p) {
     pf[p] = T.panels[p].face; pi[p] = T.panels[p].i; pj[p] = T.panels[p].j; pk[p] = T.panels[p].k;
@@ -916,12 +931,21 @@ void boundary_prepare(BoundaryOp& B, const Grid& g, int levmax, long long budget
     tf[t] = frame_slot(T.targets[t].iplane);
   }
   upload(B.tgt_node, tn); upload(B.tx, tx); upload(B.ty, ty); upload(B.tz, tz); upload(B.tgt_frame, tf);
-  // ---- record the interaction lists if they fit --------------------------
-  B.precomputed = false;
-  B.nnz = 0;
-  B.rowptr.release(); B.col.release(); B.w.release(); B.wtop.release(); B.dsum.release();
-  B.ndense_acc = 0;
   B.ntopd = B.nbound_lev[B.levmax];
+  B.budget = budget_bytes;
+  B.precomputed = B.dense = B.transposed = false;
+  B.nnz = 0;
+  B.ndense_acc = 0;
+  B.rowptr.release(); B.col.release(); B.w.release(); B.wtop.release(); B.dsum.release();
+  // uniform lattices need no recorded rows (the reverse mode records them
+  // when it first needs their transpose)
+  if (!farfield_prepare(B, g, s)) boundary_record(B, s);
+}
+
+void boundary_record(BoundaryOp& B, cudaStream_t s) {
+  const long long budget_bytes = B.budget;
+  B.precomputed = false;
+  B.rowptr.release(); B.col.release(); B.w.release(); B.wtop.release();
   const int nchunk = (B.ntarget + 31) / 32;
   const long long ntop2 = (B.ntopd + 1) / 2;
   const long long dense_bytes =
@@ -970,7 +994,7 @@ void boundary_prepare(BoundaryOp& B, const Grid& g, int levmax, long long budget
         int seg = 1;
         while (seg < 8 && (long long)nchunk * seg < 3 * slots && B.ntopd / (2 * seg) >= 64) seg *= 2;
         B.dseg = seg;
-        B.dsum.ensure(3 * (size_t)B.ntarget * seg);
+        if (!B.ff.on) B.dsum.ensure(3 * (size_t)B.ntarget * seg);  // else only the transposes read the block
       }
       k_walk<kFill><<<blocks, 128, 0, s>>>(W, nullptr, nullptr, nullptr, nullptr, B.rowptr.p, B.col.p, B.w.p,
                                            B.dense ? B.wtop.p : nullptr, nullptr);
@@ -981,18 +1005,18 @@ void boundary_prepare(BoundaryOp& B, const Grid& g, int levmax, long long budget
       B.precomputed = true;
     } catch (const Error& e) {
       if (e.status != VPMG_ERR_NOMEM) throw;
-      B.rowptr.release(); B.col.release(); B.w.release(); B.wtop.release(); B.dsum.release();
+      B.rowptr.release(); B.col.release(); B.w.release(); B.wtop.release();
       B.precomputed = false;
     }
   }
   if (!B.precomputed) B.dense = false;  // the walk covers every level
-  farfield_prepare(B, g, s);
 }
 
 void boundary_panels(BoundaryOp& B, const Grid& g, const double* sol0, size_t scs, cudaStream_t s) {
+  VPMG_CUDA(cudaMemsetAsync(B.smax.p, 0, 3 * sizeof(unsigned), s));
   k_normal_deriv<<<dim3((B.nbound + 255) / 256, 3), 256, 0, s>>>(
       sol0, g.n[0], g.n[1], g.n[2], B.pan_face.p, B.pan_i.p, B.pan_j.p, B.pan_k.p, B.nbound, 1.0 / g.d[0],
-      1.0 / g.d[1], 1.0 / g.d[2], B.csrc.p, scs, (size_t)B.ncell_total);  // level-0 part = panels
+      1.0 / g.d[1], 1.0 / g.d[2], B.csrc.p, scs, (size_t)B.ncell_total, B.smax.p);  // level-0 part = panels
   VPMG_LAUNCHED();
   VPMG_CUDA(cudaGetLastError());
 }
@@ -1007,13 +1031,10 @@ static void aggregate_levels(BoundaryOp& B, cudaStream_t s) {
   double* s0 = B.csrc.p;
   double* s1 = B.csrc.p + B.ncell_total;
   double* s2 = B.csrc.p + 2 * (size_t)B.ncell_total;
-  for (int l = 1; l <= B.levmax; ++l) {
-    const int n = B.nbound_lev[l];
-    if (n <= 0) continue;
-    k_aggregate<<<(n + 255) / 256, 256, 0, s>>>(B.agg_leaf0.p, B.agg_rowlen.p, B.agg_istep.p, B.cds.p, B.lev_off[l], n,
-                                                s0, s1, s2);
-    VPMG_LAUNCHED();
-  }
+  const int first = B.lev_off[1], n = B.ncell_total - first;
+  if (B.levmax < 1 || n <= 0) return;
+  k_aggregate<<<(n + 127) / 128, 128, 0, s>>>(B.agg_leaf0.p, B.agg_rowlen.p, B.agg_istep.p, B.cds.p, first, n, s0, s1, s2);
+  VPMG_LAUNCHED();
 }
 
 template <class M>
@@ -1025,21 +1046,6 @@ static void apply_recorded(BoundaryOp& B, double* const sol[3], cudaStream_t s) 
   k_split<M><<<(unsigned)std::min<size_t>((nc4 + 255) / 256, 152 * 16), 256, 0, s>>>(B.csrc.p, B.ncell_total, src);
   VPMG_LAUNCHED();
   const H* src2 = reinterpret_cast<const H*>(src);
-  if (!M::kFF && B.ff.on) {
-    // the coarsest level by FFT over every cell into the partial sums, the
-    // finer rows on top, then the opened coarsest cells taken back out
-    farfield_apply(B, B.dsum.p, s);
-    const long long threads = (long long)B.ntarget * 32;
-    k_apply_csr<M><<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(
-        B.rowptr.p, B.col.p, reinterpret_cast<const typename M::W*>(B.w.p), src2, B.tgt_node.p, B.ntarget,
-        1.0 / (4.0 * kPI), sol[0], sol[1], sol[2], B.dsum.p, 1);
-    VPMG_LAUNCHED();
-    k_apply_csr<M><<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(
-        B.ff.crow.p, B.ff.ccol.p, reinterpret_cast<const typename M::W*>(B.ff.cw.p), src2, B.tgt_node.p, B.ntarget,
-        1.0 / (4.0 * kPI), sol[0], sol[1], sol[2], nullptr, 0);
-    VPMG_LAUNCHED();
-    return;
-  }
   if (B.dense) {
     const long long dthreads = (long long)((B.ntarget + 31) / 32) * 32;
     const int cseg = dense_cseg(B);
@@ -1059,7 +1065,10 @@ static void apply_recorded(BoundaryOp& B, double* const sol[3], cudaStream_t s) 
 void boundary_apply(BoundaryOp& B, const Grid& g, double* const sol[3], cudaStream_t s) {
   (void)g;
   aggregate_levels(B, s);
-  if (B.precomputed) {
+  if (B.ff.on) {  // the coarsest level by FFT, the opened cells by tables
+    near_apply(B, s);
+    farfield_apply(B, sol, s);
+  } else if (B.precomputed) {
     if (B.arith == VPMG_ARITH_FF48) apply_recorded<MacFF>(B, sol, s);
     else apply_recorded<Mac64>(B, sol, s);
   } else {
@@ -1391,6 +1400,7 @@ __global__ void k_normal_deriv_T(const double* __restrict__ panelbar, int NX, in
 }  // namespace
 
 void boundary_transpose_prepare(BoundaryOp& B, cudaStream_t s) {
+  if (B.ff.on && !B.precomputed) boundary_record(B, s);
   if (B.precomputed) {  // at set-up: the transposes may be captured in graphs
     B.vff.ensure((size_t)B.ntarget);
     if (B.dense) B.dpart.ensure((size_t)B.ntopd * (((B.ntarget + 31) / 32 + kDenseTGroup - 1) / kDenseTGroup));

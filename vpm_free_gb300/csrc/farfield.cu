@@ -3,9 +3,7 @@
 // In Bounds3d_lev / tree_calc_3d (source/pmbound.f90:980-1249) every
 // boundary node visits every cell of the coarsest level and accepts it
 // unless r < 10 sqrt(dS); accepted cells add -dS/(4 pi r) times their
-// source.  The recorded operator stores these weights as a dense block
-// (two thirds of all interactions at 256^3) and applies it with 3 FMA per
-// weight.  When the coarsest cells form a uniform lattice on every face
+// source.  When the coarsest cells form a uniform lattice on every face
 // (each face side a multiple of 2^levmax panels), cell centres and boundary
 // nodes are points of one node lattice, and dS/r depends only on their
 // index offsets:
@@ -17,8 +15,8 @@
 //     distance to the source plane and the cell's distance to the target
 //     plane) in the frequency domain.
 // Both are evaluated with FP64 FFTs over every coarsest cell; the cells a
-// node opened (the walk's zero slots of the dense block) are subtracted as
-// correction rows, so the result is the dense block's sum to rounding.
+// node opened are taken back out with the finer levels' accepted cells by
+// the near field's tables (nearfield.cu), which join in k_ff_gather.
 // The kernels are even in the lattice offsets, so their spectra are real.
 // Inverse transforms use IFFT(Y) = conj(FFT(conj(Y))) / P with the 1/P
 // folded into the stored kernel spectra.
@@ -37,6 +35,7 @@ namespace {
 
 constexpr int kFFThreads = 128;
 constexpr int kFFJobs = 24;
+constexpr int kMinTargets = 12000;
 constexpr int kFFSmem = 48 * 1024;  // dynamic shared memory of the line kernel
 
 // in-plane axes of face f (normal f / 2): the panels' fast and slow axes
@@ -231,16 +230,28 @@ __global__ void __launch_bounds__(128) k_ff_perp_mv(const __grid_constant__ Perp
   }
 }
 
-// Boundary node t: dsum[comp][t] = the parallel part (X of the node's face)
-// plus both perpendicular groups (Z), read at the node's lattice position.
+// Boundary node t: the parallel part (X of the node's face) plus both
+// perpendicular groups (Z), read at the node's lattice position, the near
+// field's sums there and the node's correction row; sol -= their sum / (4 pi).
 struct GatherDev {
   long long x[6][2];     // X offsets per face and field
   long long z[6][2];     // Z offsets per face and group
   int Pu[6], P01[6][2], Nn[6][2];
   int N[3];
+  long long acc[6];      // the near field's sums per face
+  int uc;                // their unit 2^uc, times the source scale
+  double inv_pi4;
+  double* sol[3];
+  const double* src;     // cell sources [comp][ncell]
+  int ncell;
+  const long long* crow;
+  const int* ccol;
+  const double* cw;
 };
 __global__ void k_ff_gather(const __grid_constant__ GatherDev D, const int* __restrict__ tgt_node, int ntarget,
-                            const double2* __restrict__ X, const double2* __restrict__ Z, double* __restrict__ dsum) {
+                            const double2* __restrict__ X, const double2* __restrict__ Z,
+                            const unsigned long long* __restrict__ acc, const unsigned* __restrict__ smax,
+                            const int* __restrict__ failed) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= ntarget) return;
   const int node = tgt_node[t];
@@ -252,13 +263,13 @@ __global__ void k_ff_gather(const __grid_constant__ GatherDev D, const int* __re
   else if (idx[1] == D.N[1] - 1) f = 3;
   else if (idx[2] == 0) f = 4;
   else f = 5;
-  const int u = idx[ax_u(f)], v = idx[ax_v(f)];
-  const double2 p01 = X[D.x[f][0] + (long long)v * D.Pu[f] + u];
-  const double2 p2 = X[D.x[f][1] + (long long)v * D.Pu[f] + u];
+  const int u = idx[ax_u(f)], w = idx[ax_v(f)];
+  const double2 p01 = X[D.x[f][0] + (long long)w * D.Pu[f] + u];
+  const double2 p2 = X[D.x[f][1] + (long long)w * D.Pu[f] + u];
   double c0 = p01.x, c1 = -p01.y, c2 = p2.x;
   // g = 0: rows along u, elements along v; g = 1: rows along v, elements along u
   for (int g = 0; g < 2; ++g) {
-    const int i = g ? v : u, j = g ? u : v;
+    const int i = g ? w : u, j = g ? u : w;
     const int P = D.P01[f][g], Nn = D.Nn[f][g];
     const double2* z01 = Z + D.z[f][g];
     const double2* z2 = z01 + (long long)Nn * P;
@@ -268,9 +279,20 @@ __global__ void k_ff_gather(const __grid_constant__ GatherDev D, const int* __re
     c1 -= q.y;
     c2 += (i & 1) ? -r.y : r.x;
   }
-  dsum[t] = c0;
-  dsum[ntarget + t] = c1;
-  dsum[2 * (size_t)ntarget + t] = c2;
+  double cs[3] = {c0, c1, c2};
+  const int Nu = D.N[ax_u(f)], Nv = D.N[ax_v(f)];
+  const long long kb = D.crow[6 * (size_t)t], ke = D.crow[6 * (size_t)t + 6];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    // sources that are not finite have no scale: as in FP64, no sum of theirs is finite
+    const int es = (int)(smax[c] >> 20);
+    const long long n = (long long)acc[D.acc[f] + ((long long)c * Nv + w) * Nu + u];
+    double near = scalbn((double)n, D.uc + max(es, 1) - 1077);
+    if (es >= 0x7FF || *failed) near = __longlong_as_double(0x7FF8000000000000ll);
+    double v = cs[c] + near;
+    for (long long k = kb; k < ke; ++k) v = fma(D.cw[k], D.src[(size_t)c * D.ncell + D.ccol[k]], v);
+    D.sol[c][node] += -v * D.inv_pi4;
+  }
 }
 
 // ---- set-up kernels -------------------------------------------------------
@@ -321,51 +343,6 @@ __global__ void k_ff_real(const double2* __restrict__ src, long long nlines, int
     const int e = (int)(i % keep);
     dst[i] = src[l * P + e].x * scale;
   }
-}
-
-// Correction rows: per boundary node, the coarsest cells whose dense-block
-// slot is zero (the walk opened them), weight -dS/r by the lattice formula.
-struct CorrDev {
-  int cell0[7], ma[6];
-  double dS[6], h[3];
-  int N[3], istep, ntop, top0;
-};
-__device__ __forceinline__ void cell_centre(const CorrDev& D, int c, int& f, int o[3]) {
-  f = 0;
-  while (f < 5 && c >= D.cell0[f + 1]) ++f;
-  const int k = c - D.cell0[f];
-  const int a = k % D.ma[f], b = k / D.ma[f];
-  const int n = f >> 1;
-  o[n] = (f & 1) ? D.N[n] - 1 : 0;
-  o[ax_u(f)] = a * D.istep + D.istep / 2;
-  o[ax_v(f)] = b * D.istep + D.istep / 2;
-}
-template <bool FILL>
-__global__ void k_ff_corr(const __grid_constant__ CorrDev D, const double* __restrict__ wtop,
-                          const int* __restrict__ tgt_node, int ntarget, int* __restrict__ counts,
-                          const long long* __restrict__ rowptr, int* __restrict__ col, double* __restrict__ wgt) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ntarget) return;
-  const long long ntop2 = (D.ntop + 1) / 2;
-  const double* row = wtop + (size_t)(t >> 5) * ntop2 * 64 + (t & 31) * 2;
-  int cnt = 0;
-  long long out = FILL ? rowptr[t] : 0;
-  const int node = tgt_node[t];
-  const int ti[3] = {node % D.N[0], (node / D.N[0]) % D.N[1], node / (D.N[0] * D.N[1])};
-  for (int c = 0; c < D.ntop; ++c) {
-    if (row[(size_t)(c >> 1) * 64 + (c & 1)] != 0.0) continue;
-    if (FILL) {
-      int f, o[3];
-      cell_centre(D, c, f, o);
-      col[out] = D.top0 + c;
-      wgt[out] = -ff_kern(D.dS[f], __dmul_rn((double)(ti[0] - o[0]), D.h[0]), __dmul_rn((double)(ti[1] - o[1]), D.h[1]),
-                          __dmul_rn((double)(ti[2] - o[2]), D.h[2]));
-      ++out;
-    } else {
-      ++cnt;
-    }
-  }
-  if (!FILL) counts[t] = cnt;
 }
 
 // ---- host helpers ---------------------------------------------------------
@@ -459,17 +436,23 @@ void farfield_release(BoundaryOp& B) {
   F.kpar.release(); F.kperp.release(); F.T.release(); F.S2.release(); F.X.release(); F.Sw.release(); F.Z.release();
   F.crow.release(); F.ccol.release(); F.cw.release();
   F.ncorr = 0;
+  near_release(B);
 }
 
-void farfield_prepare(BoundaryOp& B, const Grid& g, cudaStream_t s) {
+bool farfield_prepare(BoundaryOp& B, const Grid& g, cudaStream_t s) {
   farfield_release(B);
   FarField& F = B.ff;
   const char* env = std::getenv("VPMG_FARFIELD");
-  if (env && env[0] == '0') return;
-  if (B.arith != VPMG_ARITH_FP64 || B.ibctyp != 2 || !B.tree || B.levmax < 1 || !B.precomputed || !B.dense) return;
+  if (env && env[0] == '0') return false;
+  if (B.arith != VPMG_ARITH_FP64 || B.ibctyp != 2 || !B.tree || B.levmax < 1 || B.budget <= 0) return false;
+  // small operators (the coarse grids, up to 9.6 thousand nodes at 41^3) are
+  // faster as recorded rows, which take two launches instead of twelve: with
+  // the coarse grid recorded a 64^3 step takes 1.94 ms and a 32^3 driver call
+  // 1.23 ms, by FFT and tables 1.99 and 1.31 ms
+  if (B.ntarget < kMinTargets) return false;
   const int istep = 1 << B.levmax;
   for (int a = 0; a < 3; ++a)
-    if ((g.n[a] - 1) % istep != 0 || g.n[a] - 1 <= istep) return;  // dummy cells at the coarsest level
+    if ((g.n[a] - 1) % istep != 0 || g.n[a] - 1 <= istep) return false;  // dummy cells at the coarsest level
   // faces' coarsest lattices, in the tree's face order
   int ma[6], mb[6], cell0[7];
   cell0[0] = 0;
@@ -478,7 +461,7 @@ void farfield_prepare(BoundaryOp& B, const Grid& g, cudaStream_t s) {
     mb[f] = (g.n[ax_v(f)] - 1) / istep;
     cell0[f + 1] = cell0[f] + ma[f] * mb[f];
   }
-  if (cell0[6] != B.ntopd) return;
+  if (cell0[6] != B.ntopd) return false;
   // every coarsest centre on its lattice node and one area per face
   const int top0 = B.lev_off[B.levmax];
   std::vector<double> cx(B.ntopd), cy(B.ntopd), cz(B.ntopd), cds(B.ntopd);
@@ -492,7 +475,7 @@ void farfield_prepare(BoundaryOp& B, const Grid& g, cudaStream_t s) {
     const double ds0 = cds[cell0[f]];
     for (int k = 0; k < ma[f] * mb[f]; ++k) {
       const int c = cell0[f] + k;
-      if (fl[c] < 0 || std::fabs(cds[c] - ds0) > 1e-13 * ds0) return;
+      if (fl[c] < 0 || std::fabs(cds[c] - ds0) > 1e-13 * ds0) return false;
       int o[3];
       const int n = f >> 1;
       o[n] = (f & 1) ? g.n[n] - 1 : 0;
@@ -501,7 +484,7 @@ void farfield_prepare(BoundaryOp& B, const Grid& g, cudaStream_t s) {
       const double pc[3] = {cx[c], cy[c], cz[c]};
       for (int a = 0; a < 3; ++a) {
         const double want = g.xmin[a] + (double)o[a] * g.d[a];
-        if (std::fabs(pc[a] - want) > 1e-9 * g.d[a]) return;
+        if (std::fabs(pc[a] - want) > 1e-9 * g.d[a]) return false;
       }
     }
     F.dS[f] = ds0;
@@ -510,7 +493,7 @@ void farfield_prepare(BoundaryOp& B, const Grid& g, cudaStream_t s) {
     F.N[a] = g.n[a];
     F.h[a] = g.d[a];
     const int P = smooth_length(2 * g.n[a] - 1 - istep);
-    if (P > 3 * 512 || P < 8) return;
+    if (P > 3 * 512 || P < 8) return false;
     make_axis(F.ax[a], P);
   }
   F.istep = istep;
@@ -606,35 +589,11 @@ void farfield_prepare(BoundaryOp& B, const Grid& g, cudaStream_t s) {
       }
       VPMG_CUDA(cudaStreamSynchronize(s));
     }
-  // ---- correction rows: the opened coarsest cells --------------------------
-  CorrDev D{};
-  for (int f = 0; f < 7; ++f) D.cell0[f] = cell0[f];
-  for (int f = 0; f < 6; ++f) { D.ma[f] = ma[f]; D.dS[f] = F.dS[f]; }
-  for (int a = 0; a < 3; ++a) { D.h[a] = g.d[a]; D.N[a] = g.n[a]; }
-  D.istep = istep;
-  D.ntop = B.ntopd;
-  D.top0 = top0;
-  DBuf<int> counts;
-  counts.ensure(B.ntarget);
-  const double* wt = reinterpret_cast<const double*>(B.wtop.p);
-  k_ff_corr<false><<<(B.ntarget + 127) / 128, 128, 0, s>>>(D, wt, B.tgt_node.p, B.ntarget, counts.p, nullptr, nullptr,
-                                                           nullptr);
-  VPMG_LAUNCHED();
-  std::vector<int> hc(B.ntarget);
-  VPMG_CUDA(cudaMemcpyAsync(hc.data(), counts.p, sizeof(int) * B.ntarget, cudaMemcpyDeviceToHost, s));
-  VPMG_CUDA(cudaStreamSynchronize(s));
-  std::vector<long long> rp(B.ntarget + 1, 0);
-  for (int t = 0; t < B.ntarget; ++t) rp[t + 1] = rp[t] + hc[t];
-  F.ncorr = rp[B.ntarget];
-  F.crow.ensure(B.ntarget + 1);
-  VPMG_CUDA(cudaMemcpy(F.crow.p, rp.data(), sizeof(long long) * (B.ntarget + 1), cudaMemcpyHostToDevice));
-  F.ccol.ensure((size_t)std::max<long long>(F.ncorr, 1));
-  F.cw.ensure((size_t)std::max<long long>(F.ncorr, 1));
-  k_ff_corr<true><<<(B.ntarget + 127) / 128, 128, 0, s>>>(D, wt, B.tgt_node.p, B.ntarget, nullptr, F.crow.p, F.ccol.p,
-                                                          F.cw.p);
-  VPMG_LAUNCHED();
-  VPMG_CUDA(cudaGetLastError());
-  VPMG_CUDA(cudaStreamSynchronize(s));
+  // ---- the opened cells and what the walk decides otherwise ----------------
+  if (!near_prepare(B, g, B.budget, s)) {
+    farfield_release(B);
+    return false;
+  }
   // FP64 flops of one apply: 5 P log2 P per line transform, 4 FMA per
   // spectrum product, 2 FMA per kernel value, component and part
   auto fft = [&](int a) { return 5.0 * F.ax[a].P * std::log2((double)F.ax[a].P); };
@@ -654,9 +613,10 @@ void farfield_prepare(BoundaryOp& B, const Grid& g, cudaStream_t s) {
   }
   F.flops = flop;
   F.on = true;
+  return true;
 }
 
-void farfield_apply(BoundaryOp& B, double* dsum, cudaStream_t s) {
+void farfield_apply(BoundaryOp& B, double* const sol[3], cudaStream_t s) {
   FarField& F = B.ff;
   const int istep = F.istep, h2 = istep / 2;
   const int NC = B.ncell_total, top0 = B.lev_off[B.levmax];
@@ -786,7 +746,17 @@ void farfield_apply(BoundaryOp& B, double* dsum, cudaStream_t s) {
     }
   }
   for (int a = 0; a < 3; ++a) GD.N[a] = F.N[a];
-  k_ff_gather<<<(B.ntarget + 255) / 256, 256, 0, s>>>(GD, B.tgt_node.p, B.ntarget, F.X.p, F.Z.p, dsum);
+  for (int f = 0; f < 6; ++f) GD.acc[f] = B.near.abase[f];
+  GD.uc = B.near.uc;
+  GD.inv_pi4 = 1.0 / (4.0 * kPI);
+  for (int c = 0; c < 3; ++c) GD.sol[c] = sol[c];
+  GD.src = B.csrc.p;
+  GD.ncell = NC;
+  GD.crow = F.crow.p;
+  GD.ccol = F.ccol.p;
+  GD.cw = F.cw.p;
+  k_ff_gather<<<(B.ntarget + 255) / 256, 256, 0, s>>>(GD, B.tgt_node.p, B.ntarget, F.X.p, F.Z.p, B.near.acc.p, B.smax.p,
+                                                      reinterpret_cast<const int*>(B.near.acc.p + B.near.nacc) + 1);
   VPMG_LAUNCHED();
   VPMG_CUDA(cudaGetLastError());
 }

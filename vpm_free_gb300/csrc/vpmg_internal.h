@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "../../include/vpmg.h"
+#include "near_host.h"
 
 namespace vpmg {
 
@@ -184,10 +185,30 @@ struct FarField {
   DBuf<double> kpar, kperp;           // kernel spectra (real), the inverse scalings folded in
   DBuf<double2> T, S2, X, Sw, Z;      // transform work arrays
   double flops = 0.0;                 // FP64 flops of one apply (FFTs 5 P log2 P per line, products, sums)
-  long long ncorr = 0;                // correction rows: the opened coarsest cells, weight -dS/r
-  DBuf<long long> crow;
+  long long ncorr = 0;                // correction rows: cells the walk and the lattice rule take differently
+  DBuf<long long> crow;               // six pointers per boundary node (its rows by source face)
   DBuf<int> ccol;
   DBuf<double> cw;
+  long long bytes() const;
+};
+
+// The opened cells by weight tables on the tensor cores (nearfield.cu).
+struct NearUnit {            // a tile of 128 runs x 64 nodes over stages k0..k1 of a list
+  long long table;
+  int row0, nrun, klist, k0, k1, col0, TB, q, sh;
+};
+struct NearField {
+  bool on = false;
+  int cell0[kNearLevels][7], ma[kNearLevels][6], mb[kNearLevels][6], Wp[kNearLevels][2][6];
+  long long dbase[kNearLevels][2][6], abase[6];
+  long long nacc = 0, stages = 0;   // sums; K = 16 products of one apply (tiles of 128 x 64, 28 digit pairs)
+  int edge = 0, group = 0, uc = 0, nunit = 0, sms = 0;
+  DBuf<unsigned char> table;
+  DBuf<unsigned short> dig;
+  DBuf<unsigned long long> acc;
+  DBuf<NearRow> rows;
+  DBuf<NearUnit> units;
+  DBuf<unsigned> klist;
   long long bytes() const;
 };
 
@@ -209,6 +230,8 @@ struct BoundaryOp {
   DBuf<int> anc;                        // [(lev-1)*nbound + leaf]: flat ancestor cell or -1
   DBuf<double> csrc;                    // 3 * ncell_total aggregated sources
   DBuf<float2> csrc_ff;                 // the same packed [cell][s0 s1 s2 0] in 8-byte words (doubles or float-float pairs)
+  DBuf<unsigned> smax;                  // per component: high word of the largest panel source's magnitude
+  long long budget = 0;                 // bytes that a recorded operator may take
   // panels: face geometry for the normal derivative
   DBuf<int> pan_face, pan_i, pan_j, pan_k;  // lower-corner node (0-based) of each panel
   // targets
@@ -238,17 +261,24 @@ struct BoundaryOp {
   DBuf<float2> tw;                      // weight words of the transposed list
   DBuf<float2> vff;                     // per target: the boundary-value adjoint in the operator's arithmetic
   DBuf<double> dpart;                   // dense transpose: partial sums [chunk group][cell]
-  FarField ff;                          // the dense block's sums by FFT (FP64, uniform coarsest lattices)
+  FarField ff;                          // the coarsest level by FFT (FP64, uniform lattices) ...
+  NearField near;                       // ... with the opened cells of every level by tables
   long long bytes() const;
 };
 void boundary_prepare(BoundaryOp& B, const Grid& g, int levmax, long long budget_bytes, cudaStream_t s,
                       int ibctyp, bool tree, int arith);
-// Sets B.ff up when the recorded operator's coarsest level is a uniform
-// lattice on every face (FP64, ibctyp 2, tree, dense block recorded) and
-// VPMG_FARFIELD is not "0"; set-up time, outside stream capture.
-void farfield_prepare(BoundaryOp& B, const Grid& g, cudaStream_t s);
-// dsum[comp][target] = sum over every coarsest cell of dS/r times its source.
-void farfield_apply(BoundaryOp& B, double* dsum, cudaStream_t s);
+// Sets B.ff and B.near up (the operator needs no recorded rows then) when the
+// cells of every level form uniform lattices on every face (FP64, ibctyp 2,
+// tree) and VPMG_FARFIELD is not "0"; set-up time, outside stream capture.
+bool farfield_prepare(BoundaryOp& B, const Grid& g, cudaStream_t s);
+bool near_prepare(BoundaryOp& B, const Grid& g, long long budget_bytes, cudaStream_t s);
+void near_apply(BoundaryOp& B, cudaStream_t s);
+void near_release(BoundaryOp& B);
+// Records the interaction lists if they fit the budget (B.precomputed).
+void boundary_record(BoundaryOp& B, cudaStream_t s);
+// sol += the boundary values: every coarsest cell by FFT, the near field's
+// sums (near_apply first) and the correction rows.
+void farfield_apply(BoundaryOp& B, double* const sol[3], cudaStream_t s);
 void farfield_release(BoundaryOp& B);
 // Normal-derivative panels of the three components from their zero-BC
 // solutions (scs doubles apart); boundary_apply aggregates them and adds the
