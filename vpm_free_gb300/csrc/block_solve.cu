@@ -41,6 +41,12 @@ __device__ __forceinline__ float2 shfl_xor(float2 v, int m) {
 
 // out[i + nsel*(q + m1*kk)] = sum_p S[i][p] * W[p + m0*(q + m1*k)],  k = klist ? klist[kk] : kk,
 // for nc components of W (wcs doubles apart; their outputs follow each other).
+//
+// pair: the selected rows are nsel layers i and their mirrors m-1-i, whose
+// sines are (-1)^p times the layer's: with the sums over the even and the odd
+// p apart, E and O, the layer is E + O and its mirror E - O: half the FMAs
+// (both partial kernels were bound by them).  The mirrors' outputs follow in
+// reverse order, at 2 nsel - 1 - i.
 // Persistent CTAs walk tiles of up to kLines lines; the sine rows are
 // staged once per CTA.  In FP64 (dbl) the next tile is staged with
 // asynchronous copies (cp.async, 8 bytes each) while the current one is
@@ -81,7 +87,7 @@ template <class A>
 __global__ void __launch_bounds__(128) k_partial_x(const double* __restrict__ W, int m0, int m1, int nk,
                                                    const int* __restrict__ klist, const typename A::R* __restrict__ S,
                                                    int nsel, double* __restrict__ out, int lines, int dbl, int nc,
-                                                   size_t wcs) {
+                                                   size_t wcs, int pair) {
   using R = typename A::R;
   extern __shared__ double smx[];
   R* Ss = reinterpret_cast<R*>(smx);               // nsel x m0
@@ -89,7 +95,8 @@ __global__ void __launch_bounds__(128) k_partial_x(const double* __restrict__ W,
   R* const buf1 = buf0 + (size_t)lines * m0;
   const int nlines = m1 * nk;
   const int ntile1 = (nlines + lines - 1) / lines, ntiles = ntile1 * nc;
-  const size_t ocs = (size_t)nsel * nlines;
+  const int nw = pair ? 2 * nsel : nsel;  // rows written
+  const size_t ocs = (size_t)nw * nlines;
   for (int t = threadIdx.x; t < nsel * m0; t += blockDim.x) Ss[t] = S[t];
   int cur = 0;
   if (dbl && (int)blockIdx.x < ntiles)
@@ -137,13 +144,17 @@ __global__ void __launch_bounds__(128) k_partial_x(const double* __restrict__ W,
         for (; p < m0; p += Rs) a0 = A::fma(a[p], b[p], a0);
       }
       R v = A::add(A::add(a0, a1), A::add(a2, a3));
-      for (int m = 1; m < Rs; m <<= 1) {
+      for (int m = pair ? 2 : 1; m < Rs; m <<= 1) {
         const R w = shfl_xor(v, m);
         v = (r & m) ? A::add(w, v) : A::add(v, w);
       }
-      if (ok && r == 0) {
+      if (pair) {  // Rs is even: threads of even r hold E, of odd r O
+        const R w = shfl_xor(v, 1);
+        v = (r & 1) ? A::sub(w, v) : A::add(v, w);
+      }
+      if (ok && (r == 0 || (pair && r == 1))) {
         const int q = l % m1, kk = l / m1;
-        oc[i + (size_t)nsel * (q + (size_t)m1 * kk)] = A::to(v);
+        oc[(r ? nw - 1 - i : i) + (size_t)nw * (q + (size_t)m1 * kk)] = A::to(v);
       }
     }
     __syncthreads();  // the buffer is refilled next (one buffer) or two tiles on (dbl)
@@ -156,8 +167,6 @@ __global__ void __launch_bounds__(128) k_partial_x(const double* __restrict__ W,
 // shared memory with coalesced row loads -- W is read from HBM once -- and
 // its threads then form the nsel x 32 dot products from the tile.
 constexpr int kColTile = 32;
-// A second row set (S2, nsel2 -> out2, same layout) is served from the
-// same staged tile when given, so two face sets cost one pass over W.
 template <class A>
 __device__ __forceinline__ void stage_y_tile(typename A::R* tile, const double* __restrict__ W, int m0, int m1,
                                              const int* __restrict__ klist, int p0, int kk) {
@@ -182,9 +191,8 @@ __device__ __forceinline__ void stage_y_tile(typename A::R* tile, const double* 
 template <class A>
 __global__ void __launch_bounds__(256) k_partial_y(const double* __restrict__ W, int m0, int m1, int nk,
                                                    const int* __restrict__ klist, const typename A::R* __restrict__ S,
-                                                   int nsel, double* __restrict__ out,
-                                                   const typename A::R* __restrict__ S2, int nsel2,
-                                                   double* __restrict__ out2, int dbl, int nc, size_t wcs) {
+                                                   int nsel, double* __restrict__ out, double* __restrict__ out2,
+                                                   int dbl, int nc, size_t wcs, int pair) {
   using R = typename A::R;
   extern __shared__ double smy[];
   R* const buf0 = reinterpret_cast<R*>(smy);              // [q][lane], m1 x kColTile
@@ -192,12 +200,13 @@ __global__ void __launch_bounds__(256) k_partial_y(const double* __restrict__ W,
   R* const partial = (dbl ? buf1 : buf0) + (size_t)m1 * kColTile;  // partial sums [row][lane]
   const int nbx = (m0 + kColTile - 1) / kColTile;
   const int ntile1 = nbx * nk, ntiles = ntile1 * nc;
-  const size_t ocs = (size_t)m0 * nsel * nk, ocs2 = (size_t)m0 * nsel2 * nk;
+  // pair: out2 holds the mirrors' rows (nsel of them, in reverse order)
+  const size_t ocs = (size_t)m0 * nsel * nk, ocs2 = ocs;
   const int lane = threadIdx.x % kColTile, row = threadIdx.x / kColTile, rows = blockDim.x / kColTile;
   // R rows share one output row set when there are fewer outputs than rows
   // (R a power of two), each summing every R-th q; the partials are added
   // in row order through shared memory.
-  const int nout = nsel + nsel2;
+  const int nout = nsel;
   int Rs = 1;
   while (Rs < rows && nout * Rs * 2 <= rows) Rs *= 2;
   const int r = row % Rs;
@@ -228,9 +237,7 @@ __global__ void __launch_bounds__(256) k_partial_y(const double* __restrict__ W,
       const int jj = j0 + row / Rs;
       R a0 = A::zero(), a1 = a0, a2 = a0, a3 = a0;
       if (jj < nout && p < m0) {
-        const bool second = jj >= nsel;
-        const int j = second ? jj - nsel : jj;
-        const R* Sj = (second ? S2 : S) + (size_t)j * m1;
+        const R* Sj = S + (size_t)jj * m1;
         int q = r;
         for (; q + 3 * Rs < m1; q += 4 * Rs) {
           a0 = A::fma(__ldg(&Sj[q]), tl[q * kColTile + lane], a0);
@@ -244,15 +251,25 @@ __global__ void __launch_bounds__(256) k_partial_y(const double* __restrict__ W,
       if (Rs > 1) {
         partial[row * kColTile + lane] = v;
         __syncthreads();
-        if (r == 0)
+        if (pair) {  // Rs is even: rows of even r hold parts of E, of odd r of O
+          R O = A::zero();
+          if (r == 0) {
+            O = partial[(row + 1) * kColTile + lane];
+            for (int m = 2; m < Rs; m += 2) {
+              v = A::add(v, partial[(row + m) * kColTile + lane]);
+              O = A::add(O, partial[(row + m + 1) * kColTile + lane]);
+            }
+            if (jj < nout && p < m0)
+              out2[comp * ocs2 + (size_t)p + (size_t)m0 * (nsel - 1 - jj + (size_t)nsel * kk)] = A::to(A::sub(v, O));
+            v = A::add(v, O);
+          }
+        } else if (r == 0) {
           for (int m = 1; m < Rs; ++m) v = A::add(v, partial[(row + m) * kColTile + lane]);
+        }
         __syncthreads();
       }
       if (r == 0 && jj < nout && p < m0) {
-        const bool second = jj >= nsel;
-        const int j = second ? jj - nsel : jj;
-        if (second) out2[comp * ocs2 + (size_t)p + (size_t)m0 * (j + (size_t)nsel2 * kk)] = A::to(v);
-        else out[comp * ocs + (size_t)p + (size_t)m0 * (j + (size_t)nsel * kk)] = A::to(v);
+        out[comp * ocs + (size_t)p + (size_t)m0 * (jj + (size_t)nsel * kk)] = A::to(v);
       }
     }
     __syncthreads();  // the tile's buffer is refilled next
@@ -515,11 +532,12 @@ void partial_x_reserve(int m0, int nsel) {
 }
 
 void partial_x(int arith, const double* W, int m0, int m1, int nk, const int* klist, const double* S, int nsel,
-               double* out, cudaStream_t s, int nc, size_t wcs) {
+               double* out, cudaStream_t s, int nc, size_t wcs, bool pair = false) {
   const int nlines = m1 * nk;
   const bool dbl = arith != VPMG_ARITH_FF48;
   const int lines = partial_x_lines(m0, nsel, dbl);
   const size_t sm = partial_x_smem(m0, nsel, lines, dbl);
+  VPMG_CHECK(!pair || lines * nsel <= 64, VPMG_ERR_STATE, "paired rows need two threads per output");
   VPMG_CHECK(sm <= granted(g_partial_smem), VPMG_ERR_STATE, "k_partial_x shared memory not reserved");
   // persistent CTAs: as many as fit on the SMs at this shared-memory size
   const unsigned ntiles = (unsigned)nc * ((nlines + lines - 1) / lines);
@@ -527,9 +545,10 @@ void partial_x(int arith, const double* W, int m0, int m1, int nk, const int* kl
   const unsigned g = std::min(ntiles, 152u * per_sm);
   if (arith == VPMG_ARITH_FF48)
     k_partial_x<FF><<<g, 128, sm, s>>>(W, m0, m1, nk, klist, reinterpret_cast<const float2*>(S), nsel, out, lines, 0,
-                                       nc, wcs);
+                                       nc, wcs, pair ? 1 : 0);
   else
-    k_partial_x<F64><<<g, 128, sm, s>>>(W, m0, m1, nk, klist, S, nsel, out, lines, 1, nc, wcs);
+    k_partial_x<F64><<<g, 128, sm, s>>>(W, m0, m1, nk, klist, S, nsel, out, lines, 1, nc, wcs,
+                                        pair ? 1 : 0);
   VPMG_LAUNCHED();
 }
 
@@ -550,8 +569,8 @@ void partial_y_reserve(int m1) {
 }
 
 void partial_y(int arith, const double* W, int m0, int m1, int nk, const int* klist, const double* S, int nsel,
-               double* out, cudaStream_t s, int nc, size_t wcs, const double* S2 = nullptr, int nsel2 = 0,
-               double* out2 = nullptr) {
+               double* out, cudaStream_t s, int nc, size_t wcs, double* mirrors = nullptr) {
+  VPMG_CHECK(!mirrors || nsel <= 4, VPMG_ERR_STATE, "paired rows need two rows of threads per output");
   const int dbl = (arith != VPMG_ARITH_FF48 && partial_y_dbl(m1)) ? 1 : 0;
   const size_t sm = partial_y_smem(m1, dbl);  // tiles + partial sums of 8 rows
   VPMG_CHECK(sm <= granted(g_partial_y_smem), VPMG_ERR_STATE, "k_partial_y shared memory not reserved");
@@ -561,10 +580,10 @@ void partial_y(int arith, const double* W, int m0, int m1, int nk, const int* kl
   const unsigned g = std::min(ntiles, 152u * per_sm);
   if (arith == VPMG_ARITH_FF48)
     k_partial_y<FF><<<g, 256, sm, s>>>(W, m0, m1, nk, klist, reinterpret_cast<const float2*>(S), nsel, out,
-                                      reinterpret_cast<const float2*>(S2), nsel2, out2, dbl, nc, wcs);
+                                      mirrors, dbl, nc, wcs, mirrors ? 1 : 0);
   else
-    k_partial_y<F64><<<g, 256, sm, s>>>(W, m0, m1, nk, klist, S, nsel, out, S2, nsel2, out2, dbl, nc,
-                                       wcs);
+    k_partial_y<F64><<<g, 256, sm, s>>>(W, m0, m1, nk, klist, S, nsel, out, mirrors, dbl, nc, wcs,
+                                        mirrors ? 1 : 0);
   VPMG_LAUNCHED();
 }
 
@@ -653,10 +672,9 @@ void BlockSolve::prepare(const DirichletPlan& P, const int nnbl_bl[6], int ncoar
   W.ensure(3 * nint);
   // normal-derivative layers: interior indices 0..3 and m-4..m-1
   std::vector<int> fx = {0, 1, 2, 3, m[0] - 4, m[0] - 3, m[0] - 2, m[0] - 1};
-  std::vector<int> fylo = {0, 1, 2, 3}, fyhi = {m[1] - 4, m[1] - 3, m[1] - 2, m[1] - 1};
-  up(S_fx, sine_rows(fx, m[0], arith));
-  up(S_fy_lo, sine_rows(fylo, m[1], arith));
-  up(S_fy_hi, sine_rows(fyhi, m[1], arith));
+  // the first of each pair of mirrored layers
+  up(S_fx, sine_rows({0, 1, 2, 3}, m[0], arith));
+  up(S_fy_lo, sine_rows({0, 1, 2, 3}, m[1], arith));
   up(l_fx, plus1(fx));
   // inner-box faces: 1-based node nnbl_bl -> interior index nnbl_bl - 2
   for (int d = 0; d < 3; ++d) {
@@ -665,10 +683,11 @@ void BlockSolve::prepare(const DirichletPlan& P, const int nnbl_bl[6], int ncoar
     VPMG_CHECK(inner_lo[d] >= 0 && inner_hi[d] < m[d] && inner_lo[d] < inner_hi[d], VPMG_ERR_ARG,
                "inner block box outside the padded block");
   }
+  for (int d = 0; d < 2; ++d)
+    VPMG_CHECK(inner_hi[d] == m[d] - 1 - inner_lo[d], VPMG_ERR_UNSUPPORTED, "inner block box not centred in the block");
   std::vector<int> ix = {inner_lo[0], inner_hi[0]};
-  up(S_ix, sine_rows(ix, m[0], arith));
+  up(S_ix, sine_rows({inner_lo[0]}, m[0], arith));
   up(S_iy_lo, sine_rows({inner_lo[1]}, m[1], arith));
-  up(S_iy_hi, sine_rows({inner_hi[1]}, m[1], arith));
   up(l_ix, plus1(ix));
   // samples: 0-based nodes nc*t inside the block interior -> interior index nc*t - 1
   auto samples = [&](int d) {
@@ -713,10 +732,10 @@ void block_solve_zero_bc(BlockSolve& B, DirichletPlan& P, const double* rhs, siz
   dst_forward_xy(P, rhs, nullptr, true, B.ghat.p, s, nc, rcs, 0);
   thomas_sweep(B.ghat.p, B.W.p, P.rinvd.p, B.m, nc, nint, nullptr, s);
   // x faces: 8 layers by dot products along x; y faces: 4 + 4 rows by dot products along y
-  partial_x(B.arith, B.W.p, m0, m1, m2, nullptr, B.S_fx.p, 8, B.X8.p, s, nc, nint);
+  partial_x(B.arith, B.W.p, m0, m1, m2, nullptr, B.S_fx.p, 4, B.X8.p, s, nc, nint, true);
   const size_t xcs = (size_t)8 * m1 * m2, ycs = (size_t)m0 * 4 * m2;
   double* Y4b = B.Y4.p + 3 * ycs;
-  partial_y(B.arith, B.W.p, m0, m1, m2, nullptr, B.S_fy_lo.p, 4, B.Y4.p, s, nc, nint, B.S_fy_hi.p, 4, Y4b);
+  partial_y(B.arith, B.W.p, m0, m1, m2, nullptr, B.S_fy_lo.p, 4, B.Y4.p, s, nc, nint, Y4b);
   // one launch of inverse y transforms: the x-face layers and the first and
   // last 4 planes (z faces, in place on W after the dots) ...
   double* top = B.W.p + plane * (m2 - 4);
@@ -745,10 +764,10 @@ void block_solve_bc(BlockSolve& B, DirichletPlan& P, double* sol, size_t scs, in
   thomas_sweep(B.ghat.p, B.W.p, P.rinvd.p, B.m, nc, nint, &F, s);
   // dot products: the inner-box x faces along x, its y faces along y, and
   // the interior samples along y then x
-  partial_x(B.arith, B.W.p, m0, m1, m2, nullptr, B.S_ix.p, 2, B.X2.p, s, nc, nint);
+  partial_x(B.arith, B.W.p, m0, m1, m2, nullptr, B.S_ix.p, 1, B.X2.p, s, nc, nint, true);
   const size_t xcs = (size_t)2 * m1 * m2, ycs = (size_t)m0 * m2;
   double* Y1b = B.Y1.p + 3 * ycs;
-  partial_y(B.arith, B.W.p, m0, m1, m2, nullptr, B.S_iy_lo.p, 1, B.Y1.p, s, nc, nint, B.S_iy_hi.p, 1, Y1b);
+  partial_y(B.arith, B.W.p, m0, m1, m2, nullptr, B.S_iy_lo.p, 1, B.Y1.p, s, nc, nint, Y1b);
   partial_y(B.arith, B.W.p, m0, m1, B.nsz, B.l_sz.p, B.S_sy.p, B.nsy, B.Ys.p, s, nc, nint);
   partial_x(B.arith, B.Ys.p, m0, B.nsy, B.nsz, nullptr, B.S_sx.p, B.nsx, B.XS.p, s, nc, (size_t)m0 * B.nsy * B.nsz);
   scatter3(B.XS.p, B.nsx, B.nsy, B.nsz, B.l_sx.p, B.l_sy.p, B.l_idz.p, 0, sol, B.dims, s, nc, scs);

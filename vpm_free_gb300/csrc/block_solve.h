@@ -15,7 +15,7 @@ struct BlockSolve {
   int arith = VPMG_ARITH_FP64;  // the plan's arithmetic
   // sine rows sin(pi (i+1)(p+1)/N) of the selected interior indices, one
   // 8-byte word each: a double, or a float-float pair (arith)
-  DBuf<double> S_fx, S_fy_lo, S_fy_hi, S_ix, S_iy_lo, S_iy_hi, S_sx, S_sy;
+  DBuf<double> S_fx, S_fy_lo, S_ix, S_iy_lo, S_sx, S_sy;
   DBuf<double> e_x1, e_y1;  // sines of the first interior layer along x and y
   DBuf<int> l_fx, l_ix, l_sx, l_sy, l_sz, l_idy, l_idz;  // node lists for scatters / plane lists
   DBuf<double> X8, Y4, X2, Y1, Ys, XS;  // compact partial results
