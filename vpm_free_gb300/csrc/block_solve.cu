@@ -815,9 +815,7 @@ void dirichlet_solve_faces(DirichletPlan& P, FaceSolve& FS, const double* rhs, s
   // them, then the full inverse transforms
   const FaceTerms F = face_terms(P, FS.f.p, FS.e.p, FS.e.p + m0, sol, scs, nc, s);
   thomas_sweep(work, out, P.rinvd.p, P.m, nc, nint, &F, s);
-  dst_lines_y(P.fy, out, m0, m1, m2, s, nc, nint);
-  const int o[3] = {P.box[0] + 1, P.box[1] + 1, P.box[2] + 1};
-  dst_x_inv_to_box(P.fx, out, sol, P.dims, o, P.m, s, nc, nint, scs);
+  dst_inverse_xy(P, out, sol, s, nc, scs);
   VPMG_CUDA(cudaGetLastError());
 }
 

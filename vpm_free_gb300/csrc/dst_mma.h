@@ -1,0 +1,23 @@
+// dst_mma.h -- the DST-I passes of the FP64 Dirichlet solves as exact
+// products on the tensor cores (dst_mma.cu).
+#pragma once
+#include "vpmg_internal.h"
+
+namespace vpmg {
+
+// Tables of a line length's sine matrix, for plans with p.n points.
+bool dst_mma_wanted(int n, long long lines);
+void dst_mma_table(DBuf<unsigned char>& T, int n, double factor, cudaStream_t s);  // factor in [1, 2)
+// Passes: lines of n points; nc components (strides in doubles).
+struct DstBox {
+  int dims[3], o[3], m[3];
+};
+void dst_mma_x_fwd(const unsigned char* T, int shift, int neg, const double* rhs, const double* sol, bool zero_bc,
+                   double* out, const DstBox& b, double ihx2, double ihy2, double ihz2, int nc, size_t rcs, size_t scs,
+                   size_t ocs, cudaStream_t s);
+void dst_mma_y(const unsigned char* T, const double* in, double* out, int m0, int m1, int m2, int nc, size_t cs,
+               cudaStream_t s);
+void dst_mma_x_inv(const unsigned char* T, const double* in, double* sol, const DstBox& b, int nc, size_t ics,
+                   size_t scs, cudaStream_t s);
+
+}  // namespace vpmg

@@ -76,15 +76,18 @@ __device__ __forceinline__ void stage(const typename A::C* __restrict__ in, type
   using C = typename A::C;
   const int nbf = M / R;
   const int tws = M / (Ns * R);
-  for (int t = threadIdx.x; t < npair * nbf; t += blockDim.x) {
-    const int pr = t / nbf;
-    const int j = t - pr * nbf;
+  // transform and butterfly by counting, j % Ns by one high product (exact for
+  // j < 2^16): no integer divisions
+  const unsigned inv = 0xFFFFFFFFu / (unsigned)Ns + 1u;  // ceil(2^32 / Ns); 0 for Ns = 1
+  for (int pr = 0, j = threadIdx.x;; j += blockDim.x) {
+    while (j >= nbf) { j -= nbf; ++pr; }
+    if (pr >= npair) break;
     const C* src = in + pr * M;
     C* dst = out + pr * M;
     C v[R];
 #pragma unroll
     for (int m = 0; m < R; ++m) v[m] = src[j + m * nbf];
-    const int k = j % Ns;
+    const int k = Ns > 1 ? j - (int)__umulhi((unsigned)j, inv) * Ns : 0;
     if (Ns > 1) {
 #pragma unroll
       for (int m = 1; m < R; ++m) v[m] = A::cmul(v[m], __ldg(&tw[k * m * tws]));

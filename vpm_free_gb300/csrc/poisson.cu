@@ -27,6 +27,7 @@
 #include <cstdlib>
 
 #include "arith.cuh"
+#include "dst_mma.h"
 #include "fft_stages.cuh"
 #include "vpmg_internal.h"
 
@@ -226,8 +227,9 @@ __device__ __forceinline__ void to_arith(double2* z, int n) {
 
 // Odd extension of the loaded real pairs: z[0] = z[N] = 0, z[M-j] = -z[j].
 __device__ __forceinline__ void odd_extend(double2* z, const FFTDev& p, int npair) {
-  for (int t = threadIdx.x; t < npair * p.N; t += blockDim.x) {
-    const int pr = t / p.N, j = t - pr * p.N;
+  for (int pr = 0, j = threadIdx.x;; j += blockDim.x) {
+    while (j >= p.N) { j -= p.N; ++pr; }
+    if (pr >= npair) break;
     double2* zz = z + pr * p.M;
     if (j == 0) {
       zz[0] = make_double2(0.0, 0.0);
@@ -247,8 +249,9 @@ __device__ __forceinline__ void rs_pre(const double2* __restrict__ L, typename A
                                        int npair) {
   using C = typename A::C;
   using R = typename A::R;
-  for (int t = threadIdx.x; t < npair * p.N; t += blockDim.x) {
-    const int pr = t / p.N, j = t - pr * p.N;
+  for (int pr = 0, j = threadIdx.x;; j += blockDim.x) {
+    while (j >= p.N) { j -= p.N; ++pr; }
+    if (pr >= npair) break;
     C z = A::cplx(A::zero(), A::zero());
     if (j > 0) {
       const C a = A::from2(L[pr * p.M + j]), b = A::from2(L[pr * p.M + p.N - j]);
@@ -275,8 +278,9 @@ __device__ __forceinline__ void rs_post(typename A::C* __restrict__ Z, typename 
   using C = typename A::C;
   using R = typename A::R;
   const int H = p.N >> 1;
-  for (int t = threadIdx.x; t < npair * H; t += blockDim.x) {
-    const int pr = t / H, m = t - pr * H;
+  for (int pr = 0, m = threadIdx.x;; m += blockDim.x) {
+    while (m >= H) { m -= H; ++pr; }
+    if (pr >= npair) break;
     const C u = Z[pr * p.M + m];
     if (m == 0) {
       O[pr * p.M + 1] = A::cplx(A::scale(A::re(u), 0.5f), A::scale(A::im(u), 0.5f));
@@ -390,44 +394,51 @@ __global__ void __launch_bounds__(kThreads) k_dst_x_fwd(const double* __restrict
   const int l0 = blockIdx.x * (2 * PAIRS);
   const int n = p.n;
   const size_t sy = b.dims[0], sz = (size_t)b.dims[0] * b.dims[1];
+  // a warp per line: no index division per value
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int nz = 0;
-  for (int t = threadIdx.x; t < 2 * PAIRS * n; t += blockDim.x) {
-    const int li = t / n, a = t - li * n;
+  for (int li = warp; li < 2 * PAIRS; li += kThreads / 32) {
     const int l = l0 + li;
-    double v = 0.0;
-    if (l < nlines) {
-      const int q = l % b.m[1], c = l / b.m[1];
-      const size_t node = (size_t)(b.o[0] + a) + sy * (b.o[1] + q) + sz * (b.o[2] + c);
-      v = rhs[node];
+    double* zp = reinterpret_cast<double*>(staging(A, B, p) + (li >> 1) * p.M + 1) + (li & 1);
+    if (l >= nlines) {
+      for (int a = lane; a < n; a += 32) zp[2 * a] = 0.0;
+      continue;
+    }
+    const int c = l / b.m[1], q = l - c * b.m[1];
+    const size_t line = (size_t)b.o[0] + sy * (b.o[1] + q) + sz * (b.o[2] + c);
+    const bool edge = !zero_bc && (q == 0 || q == b.m[1] - 1 || c == 0 || c == b.m[2] - 1);
+#pragma unroll 4
+    for (int a = lane; a < n; a += 32) {
+      const size_t node = line + a;
+      double v = rhs[node];
       if (!zero_bc) {
         if (a == 0) v -= sol[node - 1] * ihx2;
         if (a == b.m[0] - 1) v -= sol[node + 1] * ihx2;
-        if (q == 0) v -= sol[node - sy] * ihy2;
-        if (q == b.m[1] - 1) v -= sol[node + sy] * ihy2;
-        if (c == 0) v -= sol[node - sz] * ihz2;
-        if (c == b.m[2] - 1) v -= sol[node + sz] * ihz2;
+        if (edge) {
+          if (q == 0) v -= sol[node - sy] * ihy2;
+          if (q == b.m[1] - 1) v -= sol[node + sy] * ihy2;
+          if (c == 0) v -= sol[node - sz] * ihz2;
+          if (c == b.m[2] - 1) v -= sol[node + sz] * ihz2;
+        }
       }
       v *= scale;
+      nz |= v != 0.0;
+      zp[2 * a] = v;
     }
-    nz |= v != 0.0;
-    double* zp = reinterpret_cast<double*>(staging(A, B, p) + (li >> 1) * p.M + (a + 1));
-    zp[li & 1] = v;
   }
   if (!__syncthreads_or(nz)) {
     // a tile of zero lines (a vorticity-free part of the box): its
     // transform is zero, no FFT needed
-    for (int t = threadIdx.x; t < 2 * PAIRS * n; t += blockDim.x) {
-      const int l = l0 + t / n;
-      if (l < nlines) work[(size_t)l * n + (t - (t / n) * n)] = 0.0;
-    }
+    const size_t cnt = (size_t)min(2 * PAIRS, nlines - l0) * n;
+    for (size_t t = threadIdx.x; t < cnt; t += blockDim.x) work[(size_t)l0 * n + t] = 0.0;
     return;
   }
   const typename Ar::C* R = dst_pairs<Ar, ODD, PAIRS>(A, B, p);
-  for (int t = threadIdx.x; t < 2 * PAIRS * n; t += blockDim.x) {
-    const int li = t / n, k = t - li * n;
+  for (int li = warp; li < 2 * PAIRS; li += kThreads / 32) {
     const int l = l0 + li;
-    if (l >= nlines) continue;
-    work[(size_t)l * n + k] = dst_out<Ar>(R, p, li, k);
+    if (l >= nlines) break;
+#pragma unroll 4
+    for (int k = lane; k < n; k += 32) work[(size_t)l * n + k] = dst_out<Ar>(R, p, li, k);
   }
 }
 
@@ -444,29 +455,25 @@ __device__ __forceinline__ void y_body(double* __restrict__ work, int m0, int m1
   const int n = p.n;  // == m1
   const size_t plane = (size_t)m0 * m1;
   int nz = 0;
-  for (int t = threadIdx.x; t < 2 * PAIRS * n; t += blockDim.x) {
-    const int li = t % (2 * PAIRS), e = t / (2 * PAIRS);
-    const int l = l0 + li;
-    double v = 0.0;
-    if (l < nlines) {
-      const int a = l % m0, c = l / m0;
-      v = work[(size_t)a + (size_t)m0 * e + plane * c];
-    }
+  // a thread's line is the same in every trip
+  const int li = threadIdx.x % (2 * PAIRS), e0 = threadIdx.x / (2 * PAIRS);
+  constexpr int estep = kThreads / (2 * PAIRS);
+  const int l = l0 + li;
+  double* const wl = work + (l < nlines ? (size_t)(l % m0) + plane * (l / m0) : 0);
+  double* const zl = reinterpret_cast<double*>(staging(A, B, p) + (li >> 1) * p.M + 1) + (li & 1);
+#pragma unroll 4
+  for (int e = e0; e < n; e += estep) {
+    const double v = l < nlines ? wl[(size_t)m0 * e] : 0.0;
     nz |= v != 0.0;
-    double* zp = reinterpret_cast<double*>(staging(A, B, p) + (li >> 1) * p.M + (e + 1));
-    zp[li & 1] = v;
+    zl[2 * e] = v;
   }
   // zero lines (planes of the box without vorticity) transform to zero,
   // and the pass is in place: nothing to do
   if (!__syncthreads_or(nz)) return;
   const typename Ar::C* R = dst_pairs<Ar, ODD, PAIRS>(A, B, p);
-  for (int t = threadIdx.x; t < 2 * PAIRS * n; t += blockDim.x) {
-    const int li = t % (2 * PAIRS), k = t / (2 * PAIRS);
-    const int l = l0 + li;
-    if (l >= nlines) continue;
-    const int a = l % m0, c = l / m0;
-    work[(size_t)a + (size_t)m0 * k + plane * c] = dst_out<Ar>(R, p, li, k);
-  }
+  if (l >= nlines) return;
+#pragma unroll 4
+  for (int k = e0; k < n; k += estep) wl[(size_t)m0 * k] = dst_out<Ar>(R, p, li, k);
 }
 template <class Ar, bool ODD, int PAIRS>
 __global__ void __launch_bounds__(kThreads) k_dst_y(double* __restrict__ work, int m0, int m1, int m2, FFTDev p,
@@ -484,22 +491,23 @@ __device__ __forceinline__ void xinv_body(const double* __restrict__ work, doubl
   const int nlines = b.m[1] * b.m[2];
   const int l0 = tile * (2 * PAIRS);
   const int n = p.n;
-  for (int t = threadIdx.x; t < 2 * PAIRS * n; t += blockDim.x) {
-    const int li = t / n, a = t - li * n;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int li = warp; li < 2 * PAIRS; li += kThreads / 32) {
     const int l = l0 + li;
-    const double v = (l < nlines) ? work[(size_t)l * n + a] : 0.0;
-    double* zp = reinterpret_cast<double*>(staging(A, B, p) + (li >> 1) * p.M + (a + 1));
-    zp[li & 1] = v;
+    double* zp = reinterpret_cast<double*>(staging(A, B, p) + (li >> 1) * p.M + 1) + (li & 1);
+#pragma unroll 4
+    for (int a = lane; a < n; a += 32) zp[2 * a] = l < nlines ? work[(size_t)l * n + a] : 0.0;
   }
   __syncthreads();
   const typename Ar::C* R = dst_pairs<Ar, ODD, PAIRS>(A, B, p);
   const size_t sy = b.dims[0], sz = (size_t)b.dims[0] * b.dims[1];
-  for (int t = threadIdx.x; t < 2 * PAIRS * n; t += blockDim.x) {
-    const int li = t / n, k = t - li * n;
+  for (int li = warp; li < 2 * PAIRS; li += kThreads / 32) {
     const int l = l0 + li;
-    if (l >= nlines) continue;
-    const int q = l % b.m[1], c = l / b.m[1];
-    sol[(size_t)(b.o[0] + k) + sy * (b.o[1] + q) + sz * (b.o[2] + c)] = dst_out<Ar>(R, p, li, k);
+    if (l >= nlines) break;
+    const int c = l / b.m[1], q = l - c * b.m[1];
+    double* const out = sol + (size_t)b.o[0] + sy * (b.o[1] + q) + sz * (b.o[2] + c);
+#pragma unroll 4
+    for (int k = lane; k < n; k += 32) out[k] = dst_out<Ar>(R, p, li, k);
   }
 }
 template <class Ar, bool ODD, int PAIRS>
@@ -948,8 +956,25 @@ void dirichlet_prepare(DirichletPlan& P, const int dims[3], const int box[6], co
   make_fft_plan(P.fy, P.m[1], arith);
   VPMG_CHECK(std::max(smem_bytes(P.fx, 2), smem_bytes(P.fy, 2)) <= kMaxDstSmem, VPMG_ERR_UNSUPPORTED,
              "mesh too large for the shared-memory DST");
-  tune_pairs(P.fx, P.m[1] * P.m[2], 1, P.m[0], P.m[1] * P.m[2], s);  // rows along x
-  tune_pairs(P.fy, P.m[0] * P.m[2], P.m[0], P.m[1], P.m[2], s);      // columns along y
+  raise_dst_smem(std::max(smem_bytes(P.fx, kJobPairs), smem_bytes(P.fy, kJobPairs)));  // the job lists' tiles
+  P.mma_x = arith == VPMG_ARITH_FP64 && dst_mma_wanted(P.m[0], (long long)P.m[1] * P.m[2]);
+  P.mma_y = arith == VPMG_ARITH_FP64 && dst_mma_wanted(P.m[1], (long long)P.m[0] * P.m[2]);
+  if (P.mma_x) {
+    int e = 0;
+    const double f = std::frexp(std::fabs(dirichlet_scale(P)), &e);  // factor = 2 f 2^(e-1)
+    P.xf_shift = e - 1;
+    P.xf_neg = dirichlet_scale(P) < 0.0 ? 1 : 0;
+    dst_mma_table(P.tx, P.m[0], 1.0, s);
+    dst_mma_table(P.txf, P.m[0], 2.0 * f, s);
+  } else {
+    tune_pairs(P.fx, P.m[1] * P.m[2], 1, P.m[0], P.m[1] * P.m[2], s);  // rows along x
+  }
+  if (P.mma_y) {
+    dst_mma_table(P.ty, P.m[1], 1.0, s);
+    P.tmp.ensure(3 * (size_t)P.m[0] * P.m[1] * P.m[2]);
+  } else {
+    tune_pairs(P.fy, P.m[0] * P.m[2], P.m[0], P.m[1], P.m[2], s);      // columns along y
+  }
   // eigenvalues mu_p = 4 sin^2(pi p / 2N), pivots for d = 2 + hz^2 (mu_p/hx^2 + mu_q/hy^2)
   std::vector<double> mux(P.m[0]), muy(P.m[1]);
   for (int p = 0; p < P.m[0]; ++p) { const double sn = std::sin(kPI * (p + 1) / (2.0 * (P.m[0] + 1))); mux[p] = 4.0 * sn * sn; }
@@ -973,29 +998,69 @@ void dirichlet_prepare(DirichletPlan& P, const int dims[3], const int box[6], co
   P.ready = true;
 }
 
-void dirichlet_solve(DirichletPlan& P, const double* rhs, double* sol, bool zero_bc, double* work, cudaStream_t s,
-                     int nc, size_t rcs, size_t scs) {
+namespace {
+Box plan_box(const DirichletPlan& P) {
   Box b;
   for (int d = 0; d < 3; ++d) { b.dims[d] = P.dims[d]; b.o[d] = P.box[d] + 1; b.m[d] = P.m[d]; }
-  const FFTDev px = dev_plan(P.fx), py = dev_plan(P.fy);
-  const double hx2 = P.h[0] * P.h[0], hy2 = P.h[1] * P.h[1], hz2 = P.h[2] * P.h[2];
-  // Thomas RHS r = -hz^2 * ghat, with the inverse DST normalisation 4/(Nx Ny).
-  const double scale = dirichlet_scale(P);
+  return b;
+}
+DstBox mma_box(const DirichletPlan& P) {
+  DstBox b;
+  for (int d = 0; d < 3; ++d) { b.dims[d] = P.dims[d]; b.o[d] = P.box[d] + 1; b.m[d] = P.m[d]; }
+  return b;
+}
+void x_forward(DirichletPlan& P, const double* rhs, const double* sol, bool zero_bc, double* out, cudaStream_t s, int nc,
+               size_t rcs, size_t scs) {
+  const double ix = 1.0 / (P.h[0] * P.h[0]), iy = 1.0 / (P.h[1] * P.h[1]), iz = 1.0 / (P.h[2] * P.h[2]);
   const size_t wcs = (size_t)P.m[0] * P.m[1] * P.m[2];
-  const CompStride cs{nc, rcs, scs, wcs};
-  launch_x_fwd(s, rhs, sol, zero_bc ? 1 : 0, work, b, px, 1.0 / hx2, 1.0 / hy2, 1.0 / hz2, scale, cs);
-  launch_y(s, work, P.m[0], P.m[1], P.m[2], py, nc, wcs);
+  if (P.mma_x) {
+    dst_mma_x_fwd(P.txf.p, P.xf_shift, P.xf_neg, rhs, sol, zero_bc, out, mma_box(P), ix, iy, iz, nc, rcs, scs, wcs, s);
+    return;
+  }
+  launch_x_fwd(s, rhs, sol, zero_bc ? 1 : 0, out, plan_box(P), dev_plan(P.fx), ix, iy, iz, dirichlet_scale(P),
+               CompStride{nc, rcs, scs, wcs});
+  VPMG_LAUNCHED();
+}
+// y pass: returns the array that holds the result, data itself or (not in
+// place) other
+double* y_pass(DirichletPlan& P, double* data, double* other, cudaStream_t s, int nc) {
+  const size_t wcs = (size_t)P.m[0] * P.m[1] * P.m[2];
+  if (P.mma_y) {
+    dst_mma_y(P.ty.p, data, other, P.m[0], P.m[1], P.m[2], nc, wcs, s);
+    return other;
+  }
+  launch_y(s, data, P.m[0], P.m[1], P.m[2], dev_plan(P.fy), nc, wcs);
+  VPMG_LAUNCHED();
+  return data;
+}
+void x_inverse(DirichletPlan& P, const double* data, double* sol, cudaStream_t s, int nc, size_t scs) {
+  const size_t wcs = (size_t)P.m[0] * P.m[1] * P.m[2];
+  if (P.mma_x) {
+    dst_mma_x_inv(P.tx.p, data, sol, mma_box(P), nc, wcs, scs, s);
+    return;
+  }
+  launch_x_inv(s, data, sol, plan_box(P), dev_plan(P.fx), CompStride{nc, 0, scs, wcs});
+  VPMG_LAUNCHED();
+}
+}  // namespace
+
+void dirichlet_solve(DirichletPlan& P, const double* rhs, double* sol, bool zero_bc, double* work, cudaStream_t s,
+                     int nc, size_t rcs, size_t scs) {
+  // Thomas RHS r = -hz^2 * ghat, with the inverse DST normalisation 4/(Nx Ny).
+  const size_t wcs = (size_t)P.m[0] * P.m[1] * P.m[2];
+  x_forward(P, rhs, sol, zero_bc, work, s, nc, rcs, scs);
+  double* g = y_pass(P, work, P.tmp.p, s, nc);
   if (P.arith == VPMG_ARITH_FF48) {
     const int nl = P.m[0] * P.m[1];
-    k_thomas_ff<<<dim3((nl + 127) / 128, nc), 128, 0, s>>>(work, P.rinv.p, P.m[0], P.m[1], P.m[2], wcs);
+    k_thomas_ff<<<dim3((nl + 127) / 128, nc), 128, 0, s>>>(g, P.rinv.p, P.m[0], P.m[1], P.m[2], wcs);
+    VPMG_LAUNCHED();
   } else {
-    thomas_sweep(work, work, P.rinvd.p, P.m, nc, wcs, nullptr, s);
+    thomas_sweep(g, g, P.rinvd.p, P.m, nc, wcs, nullptr, s);
   }
-  launch_y(s, work, P.m[0], P.m[1], P.m[2], py, nc, wcs);
-  launch_x_inv(s, work, sol, b, px, cs);
-  count_launch(P.arith == VPMG_ARITH_FF48 ? 5 : 4);
+  g = y_pass(P, g, work, s, nc);
+  x_inverse(P, g, sol, s, nc, scs);
   if (zero_bc) {
-    k_zero_box_faces<<<dim3(256, nc), 256, 0, s>>>(sol, b, scs);
+    k_zero_box_faces<<<dim3(256, nc), 256, 0, s>>>(sol, plan_box(P), scs);
     VPMG_LAUNCHED();
   }
   VPMG_CUDA(cudaGetLastError());
@@ -1006,45 +1071,20 @@ void dirichlet_solve(DirichletPlan& P, const double* rhs, double* sol, bool zero
 // boundary values), the input of the Thomas sweep.
 void dst_forward_xy(DirichletPlan& P, const double* rhs, const double* sol, bool zero_bc, double* ghat,
                     cudaStream_t s, int nc, size_t rcs, size_t scs) {
-  Box b;
-  for (int d = 0; d < 3; ++d) { b.dims[d] = P.dims[d]; b.o[d] = P.box[d] + 1; b.m[d] = P.m[d]; }
-  const FFTDev px = dev_plan(P.fx), py = dev_plan(P.fy);
-  const double hx2 = P.h[0] * P.h[0], hy2 = P.h[1] * P.h[1], hz2 = P.h[2] * P.h[2];
-  const double scale = dirichlet_scale(P);
-  const size_t wcs = (size_t)P.m[0] * P.m[1] * P.m[2];
-  const CompStride cs{nc, rcs, scs, wcs};
-  launch_x_fwd(s, rhs, sol, zero_bc ? 1 : 0, ghat, b, px, 1.0 / hx2, 1.0 / hy2, 1.0 / hz2, scale, cs);
-  launch_y(s, ghat, P.m[0], P.m[1], P.m[2], py, nc, wcs);
-  count_launch(2);
+  double* x = P.mma_y ? P.tmp.p : ghat;
+  x_forward(P, rhs, sol, zero_bc, x, s, nc, rcs, scs);
+  y_pass(P, x, ghat, s, nc);
+  VPMG_CUDA(cudaGetLastError());
+}
+
+void dst_inverse_xy(DirichletPlan& P, double* data, double* sol, cudaStream_t s, int nc, size_t scs) {
+  x_inverse(P, y_pass(P, data, P.tmp.p, s, nc), sol, s, nc, scs);
   VPMG_CUDA(cudaGetLastError());
 }
 
 double dirichlet_scale(const DirichletPlan& P) {
   const double hz2 = P.h[2] * P.h[2];
   return -hz2 * 4.0 / ((double)(P.m[0] + 1) * (double)(P.m[1] + 1));
-}
-
-// In-place DST-I along the middle axis of an m0 x m1 x m2 array (m1 = p.n).
-// With m0 = 1 it transforms contiguous rows.
-void dst_lines_y(const FFTPlan& p, double* data, int m0, int m1, int m2, cudaStream_t s, int nc, size_t cs) {
-  if (m0 <= 0 || m2 <= 0) return;
-  VPMG_CHECK(m1 == p.n, VPMG_ERR_ARG, "dst_lines_y: line length differs from the plan");
-  launch_y(s, data, m0, m1, m2, dev_plan(p), nc, cs);
-  VPMG_LAUNCHED();
-  VPMG_CUDA(cudaGetLastError());
-}
-
-// Inverse DST-I along x of the m[0] x m[1] x m[2] array `data`; line (q, c)
-// lands on nodes (o0 + k, o1 + q, o2 + c) of the node array sol (dims).
-void dst_x_inv_to_box(const FFTPlan& p, const double* data, double* sol, const int dims[3], const int o[3],
-                      const int m[3], cudaStream_t s, int nc, size_t wcs, size_t scs) {
-  if (m[1] <= 0 || m[2] <= 0) return;
-  VPMG_CHECK(m[0] == p.n, VPMG_ERR_ARG, "dst_x_inv_to_box: line length differs from the plan");
-  Box b;
-  for (int d = 0; d < 3; ++d) { b.dims[d] = dims[d]; b.o[d] = o[d]; b.m[d] = m[d]; }
-  launch_x_inv(s, data, sol, b, dev_plan(p), CompStride{nc, 0, scs, wcs});
-  VPMG_LAUNCHED();
-  VPMG_CUDA(cudaGetLastError());
 }
 
 // Job lists: several small transforms in one launch (tiles of kJobPairs line

@@ -114,27 +114,40 @@ __device__ __forceinline__ long long fixed55(double v, int emax) {
   const unsigned long long m = ((b & 0xFFFFFFFFFFFFFull) | (e ? 0x10000000000000ull : 0ull)) << 2;
   const int sh = emax - (e ? e : 1);
   unsigned long long u = 0;
-  if (sh <= 0) u = m;
+  if (sh <= 0) u = m << min(-sh, 1);  // an average of a list may round to one step above its maximum
   else if (sh < 57) u = (m + (1ull << (sh - 1))) >> sh;
   return (long long)b < 0 ? -(long long)u : (long long)u;
 }
 // Biased exponent that scales a list whose largest magnitude has this high word.
 __device__ __forceinline__ int scale_exp(unsigned hi) { return max((int)(hi >> 20), 1); }
 
-// The seven balanced base-256 digits of |x| <= 2^55, x = sum_j d_j 256^(6-j),
-// |d_j| <= 128, as FP16 bits.  A biased digit u in 0..256 becomes the FP16
-// 1024 + u by bits, and 1152 is taken off exactly.
+// The seven balanced base-256 digits of two integers |x| <= 2^56 each,
+// x = sum_j d_j 256^(6-j), |d_j| <= 128 but for the top one (<= 256), as FP16
+// pairs (the first integer's digit in the low half).  A biased digit u < 1024
+// or-ed into the FP16 1024 is 1024 + u; 1024 + bias is taken off exactly.
+__device__ __forceinline__ unsigned hadd2(unsigned a, unsigned b) {
+  unsigned r;
+  asm("add.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+__device__ __forceinline__ void digits256x2(long long x0, long long x1, unsigned d[7]) {
+  const unsigned long long y0 = (unsigned long long)(x0 + 0x0200808080808080ll);  // + 512 on top, 128 below
+  const unsigned long long y1 = (unsigned long long)(x1 + 0x0200808080808080ll);
+  const unsigned l0 = (unsigned)y0, h0 = (unsigned)(y0 >> 32), l1 = (unsigned)y1, h1 = (unsigned)(y1 >> 32);
+  d[0] = hadd2(__byte_perm(h0, h1, 0x7632) | 0x64006400u, 0xE600E600u);                    // bits 48.., - 1536
+  d[1] = hadd2((__byte_perm(h0, h1, 0x0501) & 0x00FF00FFu) | 0x64006400u, 0xE480E480u);    // - 1152
+  d[2] = hadd2((__byte_perm(h0, h1, 0x0400) & 0x00FF00FFu) | 0x64006400u, 0xE480E480u);
+  d[3] = hadd2((__byte_perm(l0, l1, 0x0703) & 0x00FF00FFu) | 0x64006400u, 0xE480E480u);
+  d[4] = hadd2((__byte_perm(l0, l1, 0x0602) & 0x00FF00FFu) | 0x64006400u, 0xE480E480u);
+  d[5] = hadd2((__byte_perm(l0, l1, 0x0501) & 0x00FF00FFu) | 0x64006400u, 0xE480E480u);
+  d[6] = hadd2((__byte_perm(l0, l1, 0x0400) & 0x00FF00FFu) | 0x64006400u, 0xE480E480u);
+}
+// one integer's digits
 __device__ __forceinline__ void digits256(long long x, unsigned short d[7]) {
-  const unsigned long long y = (unsigned long long)(x + 0x0080808080808080ll);  // + 128 in every digit
+  unsigned p[7];
+  digits256x2(x, 0, p);
 #pragma unroll
-  for (int j = 0; j < 7; ++j) {
-    // byte 6 - j; the top digit's runs from 0 to 256
-    const unsigned w = j ? (unsigned)(y >> (8 * (6 - j))) & 0xFFu : (unsigned)(y >> 48);
-    const unsigned short bits = (unsigned short)(0x6400u + w);
-    unsigned short r;
-    asm("{\n.reg .b16 t;\nmov.b16 t, 0xE480;\nadd.rn.f16 %0, %1, t;\n}\n" : "=h"(r) : "h"(bits));  // - 1152
-    d[j] = r;
-  }
+  for (int j = 0; j < 7; ++j) d[j] = (unsigned short)p[j];
 }
 
 }  // namespace tc05

@@ -100,6 +100,13 @@ struct DirichletPlan {
   double h[3] = {0, 0, 0};
   int arith = VPMG_ARITH_FP64;  // arithmetic of the transforms and sweeps
   FFTPlan fx, fy;
+  // FP64 lines long and many enough: the passes as products (dst_mma.cu),
+  // with the sine matrices (xf: x forward, times the solve's factor) and a
+  // second array for 3 components, as those passes are not in place
+  bool mma_x = false, mma_y = false;
+  DBuf<unsigned char> tx, txf, ty;
+  int xf_shift = 0, xf_neg = 0;
+  DBuf<double> tmp;
   DBuf<float2> rinv;  // float-float plans: reciprocal Thomas pivots, [k][q][p], float-float pairs
   DBuf<double> rinvd; // FP64: rows 0..m2/2-1 of them and the middle's constant (thomas_sweep)
   bool ready = false;
@@ -130,9 +137,8 @@ void thomas_sweep(const double* g, double* out, const double* rinv, const int m[
 double dirichlet_scale(const DirichletPlan& P);  // factor applied in the forward x pass
 void dst_forward_xy(DirichletPlan& P, const double* rhs, const double* sol, bool zero_bc, double* ghat,
                     cudaStream_t s, int nc = 1, size_t rcs = 0, size_t scs = 0);
-void dst_lines_y(const FFTPlan& p, double* data, int m0, int m1, int m2, cudaStream_t s, int nc = 1, size_t cs = 0);
-void dst_x_inv_to_box(const FFTPlan& p, const double* data, double* sol, const int dims[3], const int o[3],
-                      const int m[3], cudaStream_t s, int nc = 1, size_t wcs = 0, size_t scs = 0);
+// data (overwritten) -> interior of the box of sol
+void dst_inverse_xy(DirichletPlan& P, double* data, double* sol, cudaStream_t s, int nc, size_t scs);
 // Up to 8 of the above in one launch (each job with its own plan and arrays;
 // the plans share one arithmetic).  Results equal the single launches'.
 struct DstYLines {
