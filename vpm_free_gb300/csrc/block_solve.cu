@@ -344,7 +344,15 @@ __global__ void k_extract_box_faces(const double* __restrict__ s, int NX, int NY
 // chains' latency at small ones, hence the U planes loaded ahead.
 template <int NC, bool BC>
 __global__ void __launch_bounds__(128) k_thomas_ends(const double* g, double* out, const double* __restrict__ rinv,
-                                                     int m0, int m1, int m2, size_t cs, const FaceTerms F) {
+                                                     int m0, int m1, int m2, size_t cs, FaceTerms F) {
+  if (NC == 1) {  // blockIdx.y = component
+    g += blockIdx.y * cs;
+    out += blockIdx.y * cs;
+    if constexpr (BC) {
+      const size_t f = blockIdx.y * F.cs;
+      F.fxs += f; F.fxd += f; F.fys += f; F.fyd += f; F.fz0 += f; F.fzN += f;
+    }
+  }
   const int pq = blockIdx.x * blockDim.x + threadIdx.x;
   if (pq >= m0 * m1) return;
   const int p = pq % m0, q = pq / m0;
@@ -638,28 +646,29 @@ size_t face_doubles(const DirichletPlan& P) {
 
 void thomas_launch(const double* g, double* out, const double* rinv, const int m[3], int nc, size_t cs,
                    const FaceTerms* F, cudaStream_t s) {
-  const unsigned nb = (unsigned)(((size_t)m[0] * m[1] + 127) / 128);
-  const FaceTerms none{};
-  if (nc == 3) {
-    if (F) k_thomas_ends<3, true><<<nb, 128, 0, s>>>(g, out, rinv, m[0], m[1], m[2], cs, *F);
-    else k_thomas_ends<3, false><<<nb, 128, 0, s>>>(g, out, rinv, m[0], m[1], m[2], cs, none);
+  const size_t modes = (size_t)m[0] * m[1];
+  const FaceTerms f = F ? *F : FaceTerms{};
+  // Three components per thread where the modes alone fill the GPU (they share
+  // the pivot loads); fewer modes as one component per thread in CTAs of one
+  // warp, for as many SMs as possible: at 79 x 79 modes 49 CTAs of 128 threads
+  // held the sweep with faces to a third of the FP64 units (two sweeps of a
+  // 64^3 step 130 -> 65 us, the three without faces 60 -> 40 us; at 255 x 255
+  // modes both forms keep the FP64 units busy and the shared pivots win).
+  if (nc == 3 && modes >= 152 * 256) {
+    const unsigned nb = (unsigned)((modes + 127) / 128);
+    if (F) k_thomas_ends<3, true><<<nb, 128, 0, s>>>(g, out, rinv, m[0], m[1], m[2], cs, f);
+    else k_thomas_ends<3, false><<<nb, 128, 0, s>>>(g, out, rinv, m[0], m[1], m[2], cs, f);
   } else {
-    for (int c = 0; c < nc; ++c) {
-      if (F) {
-        FaceTerms f = *F;
-        f.fxs += c * F->cs; f.fxd += c * F->cs; f.fys += c * F->cs;
-        f.fyd += c * F->cs; f.fz0 += c * F->cs; f.fzN += c * F->cs;
-        k_thomas_ends<1, true><<<nb, 128, 0, s>>>(g + c * cs, out + c * cs, rinv, m[0], m[1], m[2], cs, f);
-      } else {
-        k_thomas_ends<1, false><<<nb, 128, 0, s>>>(g + c * cs, out + c * cs, rinv, m[0], m[1], m[2], cs, none);
-      }
-    }
+    const int th = modes * nc >= 152 * 256 ? 128 : 32;
+    const dim3 nb((unsigned)((modes + th - 1) / th), nc);
+    if (F) k_thomas_ends<1, true><<<nb, th, 0, s>>>(g, out, rinv, m[0], m[1], m[2], cs, f);
+    else k_thomas_ends<1, false><<<nb, th, 0, s>>>(g, out, rinv, m[0], m[1], m[2], cs, f);
   }
 }
 void thomas_sweep(const double* g, double* out, const double* rinv, const int m[3], int nc, size_t cs,
                   const FaceTerms* F, cudaStream_t s) {
   thomas_launch(g, out, rinv, m, nc, cs, F, s);
-  count_launch(nc == 3 ? 1 : nc);
+  count_launch();
   VPMG_CUDA(cudaGetLastError());
 }
 
