@@ -1639,7 +1639,8 @@ int vpmg_pmesh(vpmg_handle* h, double* const sol[3], const double* const rhs[3],
       w.ensure(3 * (size_t)dp.m[0] * dp.m[1] * dp.m[2]);
       fill_zero(s0.p, 3 * n, h->stream);
       BoundaryOp bo;
-      boundary_prepare(bo, g, itree == 1 ? levmax : 0, h->op_budget, h->stream, h->cfg.ibctyp, itree == 1, h->arith);
+      boundary_prepare(bo, g, itree == 1 ? levmax : 0, h->op_budget, h->stream, h->cfg.ibctyp, itree == 1, h->arith,
+                       true);
       dirichlet_solve(dp, r.p, s0.p, true, w.p, h->stream, 3, n, n);
       boundary_panels(bo, g, s0.p, n, h->stream);
       double* sp[3] = {s.p, s.p + n, s.p + 2 * n};

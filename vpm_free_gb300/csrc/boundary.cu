@@ -26,7 +26,9 @@
 // reduction.  The relative error stays near 1e-14, and the product is
 // bound by the 12 bytes per interaction it streams from HBM.
 #include <algorithm>
+#include <climits>
 #include <cmath>
+#include <cstring>
 
 #include "ff.cuh"
 #include "tree_host.h"
@@ -37,26 +39,36 @@ namespace vpmg {
 namespace {
 
 constexpr int kMaxLev = 16;
+constexpr int kOnceTargets = 100000;  // one application walks below this
 
 struct WalkDev {
-  const double *cx, *cy, *cz, *cds, *cthr;
-  const int* child;
-  const int* flags;
-  const double* s0;
-  const double* s1;
-  const double* s2;
+  const WalkNode* nodes;  // the cells in the walk's order
+  const int* toppos;      // [ntop + 1] the coarsest cells' places in it
+  const double *s0, *s1, *s2;
   const int* tgt_node;
   const double *tx, *ty, *tz;
-  int top0, ntop, levmax, ntarget;
+  int ntop, ntarget, seg, cseg;  // segments of cseg coarsest cells each
   double lg;      // log((sqrt2-1)/(sqrt2+1))
   double inv_pi4, pi4;
-  int bctype;     // 2 or 3
+  long long tiny2;  // bits of the smallest d^2 with sqrt(d^2) > 1e-5
   int tree;       // 1: Bounds3d_lev walk; 0: untreed sum (levmax = 0)
   int dense;      // 1: the coarsest level goes to the dense block (count / fill)
   int ff;         // 1: recorded weights as float-float pairs, 0: as doubles
   const int* tgt_frame;
   PanelFrame frame[6];
 };
+
+// 1 / sqrt(d2) for the weights: CUDA's single-precision estimate and one step
+// of Householder's third-order iteration, y (1 + e/2 + 3 e^2/8) with
+// e = 1 - d2 y^2, whose remainder (5/16) e^3 is below 2^-60 for a 22-bit
+// estimate.  Five FP64 operations where a rounded root and a rounded division
+// take over twenty; squares outside the floats' range take rsqrt().
+__device__ __forceinline__ double inv_root(double d2) {
+  if (!(d2 > 1e-30 && d2 < 1e30)) return rsqrt(d2);
+  const double y = (double)rsqrtf((float)d2);
+  const double e = fma(-d2 * y, y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
 
 // FSOUR_A4 (source/pmbound.f90:1540-1620) with NSIDE = 0, ISING = 0,
 // EPSS = 1e-14: potential at XO of a flat quadrilateral of unit constant
@@ -114,84 +126,80 @@ __device__ double fsour_a4(const double XO[3], const double RG[3], const PanelFr
 
 enum { kAccum = 0, kCount = 1, kFill = 2, kTranspose = 3 };
 
+// One thread walks the tree for one target, over the cells in preorder: an
+// opened cell is followed by its children, an accepted one by its `skip`.
+// There is no stack, and the opening test r < 10 sqrt(dS) is the integer
+// comparison of d^2's bits with the cell's threshold (the smallest d^2 whose
+// rounded root is not below it), so it decides as the reference's expressions
+// do without a root.  A visit is bound by the FP64 units (two lanes per clock
+// and SM): 8 operations to decide, 6 for the weight, one per component.
+// kAccum and kTranspose split the coarsest cells into segments (blockIdx.y):
+// the 22 thousand targets of a 61 x 53 x 70 mesh alone are 4.6 warps per SM.
+// Its walk took 13.9 ms per pass, and as many for each of count and fill, with
+// roots, divisions and per-level stacks in local memory; kAccum takes 6.5 ms.  A
+// warp that keeps its lanes on one cell (least place first) takes 7.8: the
+// union of 32 targets' cells is more work than their separate paths.
 // With W.dense, kCount counts only the finer levels (and adds the coarsest
 // level's accepted cells to *dcount) and kFill writes the coarsest level
 // into the dense block wtop.
-template <int MODE>
-__global__ void k_walk(WalkDev W, double* __restrict__ o0, double* __restrict__ o1, double* __restrict__ o2,
-                       int* __restrict__ counts, const long long* __restrict__ rowptr, int* __restrict__ col,
-                       float2* __restrict__ wgt, float2* __restrict__ wtop = nullptr,
-                       unsigned long long* __restrict__ dcount = nullptr) {
+template <int MODE, bool BC3>
+__global__ void __launch_bounds__(64) k_walk(WalkDev W, double* __restrict__ o0, double* __restrict__ o1,
+                                             double* __restrict__ o2, int* __restrict__ counts,
+                                             const long long* __restrict__ rowptr, int* __restrict__ col,
+                                             float2* __restrict__ wgt, float2* __restrict__ wtop = nullptr,
+                                             unsigned long long* __restrict__ dcount = nullptr) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= W.ntarget) return;
   const double X = W.tx[t], Y = W.ty[t], Z = W.tz[t];
-  int parent[kMaxLev], pos[kMaxLev], cnt[kMaxLev];
-  int L = W.levmax;
-  pos[L] = 0;
   double a0 = 0.0, a1 = 0.0, a2 = 0.0;
   int ni = 0, nd = 0;
   long long out = 0;
   if (MODE == kFill) out = rowptr[t];
   double bcv = 0.0;  // transpose: o1 is the adjoint of the boundary values, o0 the cell adjoints
   if (MODE == kTranspose) bcv = -W.inv_pi4 * o1[W.tgt_node[t]];
-  while (true) {
-    int c;
-    if (L == W.levmax) {
-      if (pos[L] >= W.ntop) break;
-      c = W.top0 + pos[L]++;
-    } else {
-      if (pos[L] >= cnt[L]) {
-        ++L;
-        continue;
-      }
-      c = W.child[4 * parent[L] + pos[L]++];
-    }
-    const double XR = __dsub_rn(W.cx[c], X), YR = __dsub_rn(W.cy[c], Y), ZR = __dsub_rn(W.cz[c], Z);
-    const double r = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(XR, XR), __dmul_rn(YR, YR)), __dmul_rn(ZR, ZR)));
-    const int fl = W.flags[c];
-    // ibctyp 3 (tree_calc_3d_s) tests r / sqrt(dS) < 10 and always opens
-    // only the -1 dummies; a -2 dummy has dS = 0 and is never opened.
-    const bool open = (W.bctype == 3) ? ((__ddiv_rn(r, __dsqrt_rn(W.cds[c])) < 10.0 && L > 0) || fl == -1)
-                                      : ((r < W.cthr[c] && L > 0) || fl < 0);
-    if (open) {
-      parent[L - 1] = c;
-      cnt[L - 1] = (fl < 0) ? 2 : 4;
-      pos[L - 1] = 0;
-      --L;
+  int v = W.toppos[min((int)blockIdx.y * W.cseg, W.ntop)];
+  const int vend = W.toppos[min(((int)blockIdx.y + 1) * W.cseg, W.ntop)];
+  while (v < vend) {
+    const WalkNode N = W.nodes[v];
+    const double XR = __dsub_rn(N.x, X), YR = __dsub_rn(N.y, Y), ZR = __dsub_rn(N.z, Z);
+    const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(XR, XR), __dmul_rn(YR, YR)), __dmul_rn(ZR, ZR));
+    if (__double_as_longlong(d2) < N.open2) {
+      ++v;
       continue;
     }
+    v = N.skip & 0x7fffffff;
+    const bool top = N.skip < 0;  // a cell of the coarsest level
     if (MODE == kCount) {
-      if (W.dense && L == W.levmax) ++nd;
+      if (W.dense && top) ++nd;
       else ++ni;
       continue;
     }
-    const double DS = W.cds[c];
     double w;
-    int cc = c;
-    if (W.bctype == 3) {
-      if (L == W.levmax) {
+    int cc = N.cell;
+    if (BC3) {
+      if (top) {
         // coarsest level: FSOUR_A4 of the cell (area dS in the tree, the
         // target plane's cell area in the untreed sum), weighting the
         // source of the walk's start cell nv = 1 in the tree
         // (pmbound.f90:1492-1496) and the cell's own in the untreed sum
         const PanelFrame& F = W.frame[W.tgt_frame[t]];
-        const double XO[3] = {X, Y, Z}, RG[3] = {W.cx[c], W.cy[c], W.cz[c]};
-        const double fis = fsour_a4(XO, RG, F, W.tree ? DS : F.area, W.pi4);
+        const double XO[3] = {X, Y, Z}, RG[3] = {N.x, N.y, N.z};
+        const double fis = fsour_a4(XO, RG, F, W.tree ? N.ds : F.area, W.pi4);
         w = -fis * W.pi4;
-        if (W.tree) cc = W.top0;
+        if (W.tree) cc = W.nodes[0].cell;
       } else {
-        w = __ddiv_rn(DS, r);
+        w = N.ds * inv_root(d2);
       }
     } else {
-      w = (r > 1e-05) ? __ddiv_rn(DS, r) : -2.0 * __dsqrt_rn(DS) * W.lg;
+      w = (__double_as_longlong(d2) >= W.tiny2) ? N.ds * inv_root(d2) : -2.0 * __dsqrt_rn(N.ds) * W.lg;
     }
     if (MODE == kFill) {
       // the weight word: the double itself, or its float-float pair
       const float hi = __double2float_rn(w);
       const float2 wf = make_float2(hi, __double2float_rn(w - (double)hi));
       const double word = W.ff ? *reinterpret_cast<const double*>(&wf) : w;
-      if (W.dense && L == W.levmax) {
-        const int cc2 = c - W.top0;  // [chunk][cell pair][lane][2]
+      if (W.dense && top) {
+        const int cc2 = N.cell - W.nodes[0].cell;  // [chunk][cell pair][lane][2]
         reinterpret_cast<double*>(wtop)[(((size_t)(t >> 5) * ((W.ntop + 1) >> 1) + (cc2 >> 1)) * 32 + (t & 31)) * 2 +
                                          (cc2 & 1)] = word;
       } else {
@@ -211,11 +219,31 @@ __global__ void k_walk(WalkDev W, double* __restrict__ o0, double* __restrict__ 
     counts[t] = ni;
     if (nd) atomicAdd(dcount, (unsigned long long)nd);
   } else if (MODE == kAccum) {
-    const int node = W.tgt_node[t];
-    o0[node] += a0 * W.inv_pi4;
-    o1[node] += a1 * W.inv_pi4;
-    o2[node] += a2 * W.inv_pi4;
+    // one segment: onto the boundary node; several: partial sums in o0
+    if (W.seg == 1) {
+      const int node = W.tgt_node[t];
+      o0[node] += a0 * W.inv_pi4;
+      o1[node] += a1 * W.inv_pi4;
+      o2[node] += a2 * W.inv_pi4;
+    } else {
+      double* p = o0 + (size_t)blockIdx.y * 3 * W.ntarget + t;
+      p[0] = a0;
+      p[W.ntarget] = a1;
+      p[2 * (size_t)W.ntarget] = a2;
+    }
   }
+}
+
+// Adds the segments' partial sums, in order, to the boundary nodes.
+__global__ void k_walk_sum(const double* __restrict__ part, const int* __restrict__ tgt_node, int ntarget, int seg,
+                           double inv_pi4, double* __restrict__ o0, double* __restrict__ o1,
+                           double* __restrict__ o2) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= ntarget) return;
+  double* const o = blockIdx.y == 0 ? o0 : blockIdx.y == 1 ? o1 : o2;
+  double a = 0.0;
+  for (int g = 0; g < seg; ++g) a += part[((size_t)g * 3 + blockIdx.y) * ntarget + t];
+  o[tgt_node[t]] += a * inv_pi4;
 }
 
 // Float-float accumulate acc += w * s: the hi product and its exact error
@@ -793,26 +821,113 @@ void upload(DBuf<T>& b, const std::vector<T>& h) {
   if (!h.empty()) VPMG_CUDA(cudaMemcpy(b.p, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice));
 }
 
-WalkDev walk_dev(const BoundaryOp& B) {
+// The smallest d2 >= 0 (as bits) for which below(d2) fails; below() holds for
+// a prefix of the doubles and `t` is within a few units of its end.
+template <class P>
+long long root_bits(double t, P below) {
+  while (below(t)) t = std::nextafter(t, HUGE_VAL);
+  while (t > 0.0) {
+    const double p = std::nextafter(t, 0.0);
+    if (below(p)) break;
+    t = p;
+  }
+  long long b;
+  std::memcpy(&b, &t, sizeof b);
+  return b;
+}
+
+// Cells in the order of the walk (each coarsest cell, then the children of an
+// opened one), with the opening test as a threshold on d^2.
+void walk_prepare(BoundaryOp& B) {
+  if (B.wnodes.p) return;
+  const int NC = B.ncell_total;
+  std::vector<double> cx(NC), cy(NC), cz(NC), cds(NC), thr(NC);
+  std::vector<int> child(4 * (size_t)NC), flags(NC);
+  const auto get = [](auto& h, const auto& d) {
+    VPMG_CUDA(cudaMemcpy(h.data(), d.p, sizeof(h[0]) * h.size(), cudaMemcpyDeviceToHost));
+  };
+  get(cx, B.cx); get(cy, B.cy); get(cz, B.cz); get(cds, B.cds); get(thr, B.cthr); get(child, B.child);
+  get(flags, B.flags);
+  const int ntop = B.nbound_lev[B.levmax], top0 = B.lev_off[B.levmax];
+  std::vector<WalkNode> nodes;
+  nodes.reserve(NC);
+  std::vector<int> toppos(ntop + 1);
+  double last = -1.0;  // cells of one size follow one another
+  long long lastbits = 0;
+  const auto open2 = [&](int c, int L) -> long long {
+    const bool point = B.ibctyp == 2;
+    if (point ? flags[c] < 0 : flags[c] == -1) return LLONG_MAX;
+    if (L == 0) return 0;
+    // ibctyp 3 (tree_calc_3d_s) tests r / sqrt(dS) < 10 and always opens
+    // only the -1 dummies; a -2 dummy has dS = 0 and is never opened.
+    if (!point && !(cds[c] > 0.0)) return 0;
+    if (cds[c] == last) return lastbits;
+    last = cds[c];
+    const double h = thr[c], q = std::sqrt(cds[c]);
+    return lastbits = point ? root_bits(h * h, [h](double d2) { return std::sqrt(d2) < h; })
+                            : root_bits(100.0 * cds[c], [q](double d2) { return std::sqrt(d2) / q < 10.0; });
+  };
+  const auto visit = [&](auto& self, int c, int L) -> void {
+    const size_t at = nodes.size();
+    nodes.push_back(WalkNode{cx[c], cy[c], cz[c], cds[c], open2(c, L), c, 0});
+    if (L > 0) {
+      const int nch = flags[c] < 0 ? 2 : 4;
+      for (int m = 0; m < nch; ++m) self(self, child[4 * (size_t)c + m], L - 1);
+    }
+    VPMG_CHECK(nodes.size() < 0x7fffffff, VPMG_ERR_TREE, "too many cells");
+    nodes[at].skip = (int)((unsigned)nodes.size() | (L == B.levmax ? 0x80000000u : 0u));
+  };
+  for (int k = 0; k < ntop; ++k) {
+    toppos[k] = (int)nodes.size();
+    visit(visit, top0 + k, B.levmax);
+  }
+  toppos[ntop] = (int)nodes.size();
+  upload(B.toppos, toppos);
+  upload(B.wnodes, nodes);
+}
+
+// Segments of the coarsest cells for kAccum and kTranspose: 24 warps per SM,
+// at least 8 coarsest cells each.
+int walk_segments(const BoundaryOp& B) {
+  const int ntop = B.nbound_lev[B.levmax];
+  const long long want = (152LL * 24 * 32 + B.ntarget - 1) / B.ntarget;
+  return (int)std::max(1LL, std::min({want, 16LL, (long long)ntop / 8}));
+}
+
+// seg: segments of the coarsest cells (the launch's grid y).
+WalkDev walk_dev(const BoundaryOp& B, int seg) {
   WalkDev W;
-  W.cx = B.cx.p; W.cy = B.cy.p; W.cz = B.cz.p; W.cds = B.cds.p; W.cthr = B.cthr.p;
-  W.child = B.child.p; W.flags = B.flags.p;
+  W.nodes = B.wnodes.p;
+  W.toppos = B.toppos.p;
   W.s0 = B.csrc.p; W.s1 = B.csrc.p + B.ncell_total; W.s2 = B.csrc.p + 2 * (size_t)B.ncell_total;
   W.tgt_node = B.tgt_node.p; W.tx = B.tx.p; W.ty = B.ty.p; W.tz = B.tz.p;
-  W.top0 = B.lev_off[B.levmax];
   W.ntop = B.nbound_lev[B.levmax];
-  W.levmax = B.levmax;
   W.ntarget = B.ntarget;
+  W.seg = seg;
+  W.cseg = (W.ntop + seg - 1) / seg;
   W.lg = std::log((std::sqrt(2.0) - 1.0) / (std::sqrt(2.0) + 1.0));
   W.inv_pi4 = 1.0 / (4.0 * kPI);
   W.pi4 = 4.0 * kPI;
-  W.bctype = B.ibctyp;
+  W.tiny2 = root_bits(1e-05 * 1e-05, [](double d2) { return !(std::sqrt(d2) > 1e-05); });
   W.tree = B.tree ? 1 : 0;
   W.tgt_frame = B.tgt_frame.p;
   W.dense = B.dense ? 1 : 0;
   W.ff = B.arith == VPMG_ARITH_FF48 ? 1 : 0;
   for (int f = 0; f < 6; ++f) W.frame[f] = B.frame[f];
   return W;
+}
+
+template <int MODE>
+void walk_launch(const BoundaryOp& B, const WalkDev& W, double* o0, double* o1, double* o2, int* counts,
+                 const long long* rowptr, int* col, float2* wgt, float2* wtop, unsigned long long* dcount,
+                 cudaStream_t s) {
+  const dim3 grid((B.ntarget + 63) / 64, W.seg);
+  if (B.ibctyp == 3)
+    k_walk<MODE, true><<<grid, 64, 0, s>>>(W, o0, o1, o2, counts, rowptr, col, wgt, wtop, dcount);
+  else
+    k_walk<MODE, false><<<grid, 64, 0, s>>>(W, o0, o1, o2, counts, rowptr, col, wgt, wtop, dcount);
+  VPMG_LAUNCHED();
+  VPMG_CUDA(cudaGetLastError());
 }
 
 // Slot of Bounds3d_lev's plane argument: 2/-2 X min/max, 1/-1 Y, 3/-3 Z.
@@ -851,11 +966,23 @@ PanelFrame make_frame(int iplane, const double d[3]) {
 long long BoundaryOp::bytes() const {
   return (long long)(rowptr.bytes() + col.bytes() + w.bytes() + colptr.bytes() + trow.bytes() + tw.bytes() +
                      cx.bytes() * 5 + child.bytes() + csrc.bytes() + wtop.bytes() + dsum.bytes()) +
-         ff.bytes() + near.bytes();
+         wnodes.bytes() + toppos.bytes() + walkpart.bytes() + ff.bytes() + near.bytes();
+}
+
+// Buffers of an apply by the walk, ahead of it: steps may be captured.
+static void walk_ready(BoundaryOp& B) {
+  walk_prepare(B);
+  B.walkseg = walk_segments(B);
+  try {
+    if (B.walkseg > 1) B.walkpart.ensure(3 * (size_t)B.walkseg * B.ntarget);
+  } catch (const Error& e) {
+    if (e.status != VPMG_ERR_NOMEM) throw;
+    B.walkseg = 1;  // straight onto the nodes
+  }
 }
 
 void boundary_prepare(BoundaryOp& B, const Grid& g, int levmax, long long budget_bytes, cudaStream_t s, int ibctyp,
-                      bool tree, int arith) {
+                      bool tree, int arith, bool once) {
   VPMG_CHECK(arith == VPMG_ARITH_FP64 || arith == VPMG_ARITH_FF48, VPMG_ERR_ARG, "unknown arithmetic");
   B.arith = arith;
   VPMG_CHECK(levmax >= 0 && levmax < kMaxLev - 1, VPMG_ERR_ARG, "levmax out of range");
@@ -937,9 +1064,19 @@ void boundary_prepare(BoundaryOp& B, const Grid& g, int levmax, long long budget
   B.nnz = 0;
   B.ndense_acc = 0;
   B.rowptr.release(); B.col.release(); B.w.release(); B.wtop.release(); B.dsum.release();
+  B.wnodes.release(); B.toppos.release(); B.walkpart.release();
   // uniform lattices need no recorded rows (the reverse mode records them
   // when it first needs their transpose)
-  if (!farfield_prepare(B, g, s)) boundary_record(B, s);
+  // One application of a small operator walks once.  Recording walks twice and
+  // then reads the lists (pmesh of 61 x 53 x 70 nodes 32.2 ms, by one walk
+  // 10.9), and the transforms and tables of a uniform lattice take longer to
+  // set up than the walk: 65^3 nodes 16.6 against 11.3 ms, 97^3 27.2 against
+  // 23.3, 129^3 (97 thousand targets) 40.5 against 39.2, 161^3 57.5 against 62.6.
+  const bool walk_once = once && B.ntarget < kOnceTargets;
+  if (!walk_once && farfield_prepare(B, g, s)) return;
+  if (walk_once) farfield_release(B);
+  if (!once) boundary_record(B, s);
+  if (!B.precomputed) walk_ready(B);
 }
 
 void boundary_record(BoundaryOp& B, cudaStream_t s) {
@@ -953,16 +1090,13 @@ void boundary_record(BoundaryOp& B, cudaStream_t s) {
   // the dense block needs a tree (levmax >= 1), the cells' own columns (not
   // ibctyp 3's start-cell column) and at most half of the budget
   B.dense = B.levmax >= 1 && !(B.ibctyp == 3 && B.tree) && budget_bytes > 0 && dense_bytes <= budget_bytes / 2;
-  const WalkDev W = walk_dev(B);
-  const int blocks = (B.ntarget + 127) / 128;
+  walk_prepare(B);
+  const WalkDev W = walk_dev(B, 1);
   DBuf<int> counts;
   counts.ensure(B.ntarget);
   B.dcount.ensure(1);
   VPMG_CUDA(cudaMemsetAsync(B.dcount.p, 0, sizeof(unsigned long long), s));
-  k_walk<kCount><<<blocks, 128, 0, s>>>(W, nullptr, nullptr, nullptr, counts.p, nullptr, nullptr, nullptr, nullptr,
-                                        B.dcount.p);
-  VPMG_LAUNCHED();
-  VPMG_CUDA(cudaGetLastError());
+  walk_launch<kCount>(B, W, nullptr, nullptr, nullptr, counts.p, nullptr, nullptr, nullptr, nullptr, B.dcount.p, s);
   std::vector<int> hc(B.ntarget);
   unsigned long long nd = 0;
   VPMG_CUDA(cudaMemcpyAsync(hc.data(), counts.p, sizeof(int) * B.ntarget, cudaMemcpyDeviceToHost, s));
@@ -996,10 +1130,8 @@ void boundary_record(BoundaryOp& B, cudaStream_t s) {
         B.dseg = seg;
         if (!B.ff.on) B.dsum.ensure(3 * (size_t)B.ntarget * seg);  // else only the transposes read the block
       }
-      k_walk<kFill><<<blocks, 128, 0, s>>>(W, nullptr, nullptr, nullptr, nullptr, B.rowptr.p, B.col.p, B.w.p,
-                                           B.dense ? B.wtop.p : nullptr, nullptr);
-      VPMG_LAUNCHED();
-      VPMG_CUDA(cudaGetLastError());
+      walk_launch<kFill>(B, W, nullptr, nullptr, nullptr, nullptr, B.rowptr.p, B.col.p, B.w.p,
+                         B.dense ? B.wtop.p : nullptr, nullptr, s);
       VPMG_CUDA(cudaStreamSynchronize(s));
       B.csrc_ff.ensure(4 * (size_t)B.ncell_total);  // here, not in the apply: steps may be captured in graphs
       B.precomputed = true;
@@ -1010,6 +1142,7 @@ void boundary_record(BoundaryOp& B, cudaStream_t s) {
     }
   }
   if (!B.precomputed) B.dense = false;  // the walk covers every level
+  else B.wnodes.release();              // synchronised above
 }
 
 void boundary_panels(BoundaryOp& B, const Grid& g, const double* sol0, size_t scs, cudaStream_t s) {
@@ -1072,9 +1205,17 @@ void boundary_apply(BoundaryOp& B, const Grid& g, double* const sol[3], cudaStre
     if (B.arith == VPMG_ARITH_FF48) apply_recorded<MacFF>(B, sol, s);
     else apply_recorded<Mac64>(B, sol, s);
   } else {
-    const WalkDev W = walk_dev(B);
-    k_walk<kAccum><<<(B.ntarget + 127) / 128, 128, 0, s>>>(W, sol[0], sol[1], sol[2], nullptr, nullptr, nullptr, nullptr);
-    VPMG_LAUNCHED();
+    VPMG_CHECK(B.wnodes.p, VPMG_ERR_STATE, "boundary operator without its walk order");
+    const int seg = B.walkseg;
+    const WalkDev W = walk_dev(B, seg);
+    if (seg == 1) {
+      walk_launch<kAccum>(B, W, sol[0], sol[1], sol[2], nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, s);
+    } else {
+      walk_launch<kAccum>(B, W, B.walkpart.p, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, s);
+      k_walk_sum<<<dim3((B.ntarget + 127) / 128, 3), 128, 0, s>>>(B.walkpart.p, B.tgt_node.p, B.ntarget, seg,
+                                                                  W.inv_pi4, sol[0], sol[1], sol[2]);
+      VPMG_LAUNCHED();
+    }
   }
   VPMG_CUDA(cudaGetLastError());
 }
@@ -1178,6 +1319,7 @@ void boundary_release_recorded(BoundaryOp& B) {
   B.transposed = false;
   B.nnz = 0;
   B.ndense_acc = 0;
+  walk_ready(B);  // later applies walk
 }
 
 void boundary_group_correct(const BoundaryOp& F, const GroupCorrection& C, double* const sol[3], cudaStream_t s) {
@@ -1489,10 +1631,10 @@ void boundary_apply_T(BoundaryOp& B, const double* bcbar, double* cellbar, cudaS
     else apply_T_recorded<Mac64>(B, bcbar, cellbar, s);
   } else {
     VPMG_CUDA(cudaMemsetAsync(cellbar, 0, sizeof(double) * B.ncell_total, s));
-    const WalkDev W = walk_dev(B);
-    k_walk<kTranspose><<<(B.ntarget + 127) / 128, 128, 0, s>>>(W, cellbar, const_cast<double*>(bcbar), nullptr,
-                                                               nullptr, nullptr, nullptr, nullptr);
-    VPMG_LAUNCHED();
+    VPMG_CHECK(B.wnodes.p, VPMG_ERR_STATE, "boundary operator without its walk order");
+    const WalkDev W = walk_dev(B, walk_segments(B));
+    walk_launch<kTranspose>(B, W, cellbar, const_cast<double*>(bcbar), nullptr, nullptr, nullptr, nullptr, nullptr,
+                            nullptr, nullptr, s);
   }
   VPMG_CUDA(cudaGetLastError());
 }

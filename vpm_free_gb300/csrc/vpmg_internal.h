@@ -218,6 +218,14 @@ struct NearField {
   long long bytes() const;
 };
 
+// A cell of the tree walk, in the walk's order.
+struct alignas(16) WalkNode {
+  double x, y, z, ds;
+  long long open2;  // opened where the bits of d^2 are below this
+  int cell;         // flat cell
+  int skip;         // the next cell when this one is not opened; sign: a coarsest cell
+};
+
 struct BoundaryOp {
   // panels (level 0) and aggregated levels, device copies
   int nbound = 0, levmax = 0, ncell_total = 0, ntarget = 0;
@@ -267,12 +275,17 @@ struct BoundaryOp {
   DBuf<float2> tw;                      // weight words of the transposed list
   DBuf<float2> vff;                     // per target: the boundary-value adjoint in the operator's arithmetic
   DBuf<double> dpart;                   // dense transpose: partial sums [chunk group][cell]
+  // apply by the walk (not recorded)
+  DBuf<WalkNode> wnodes;
+  DBuf<int> toppos;
+  int walkseg = 1;
+  DBuf<double> walkpart;                // [segment][3][ntarget] partial sums
   FarField ff;                          // the coarsest level by FFT (FP64, uniform lattices) ...
   NearField near;                       // ... with the opened cells of every level by tables
   long long bytes() const;
 };
 void boundary_prepare(BoundaryOp& B, const Grid& g, int levmax, long long budget_bytes, cudaStream_t s,
-                      int ibctyp, bool tree, int arith);
+                      int ibctyp, bool tree, int arith, bool once = false);  // once: applied a single time
 // Sets B.ff and B.near up (the operator needs no recorded rows then) when the
 // cells of every level form uniform lattices on every face (FP64, ibctyp 2,
 // tree) and VPMG_FARFIELD is not "0"; set-up time, outside stream capture.
