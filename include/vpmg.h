@@ -148,7 +148,7 @@ double vpmg_projection_fun(int itype, double x);
  * the whole GPU to its own pool allocator, or one that runs inside a fixed
  * memory budget where an extra cudaMalloc would fail.  This call makes no
  * cudaMalloc, cudaFree or allocating library call: its temporaries live in
- * one static device array of 33.6 MB that every GPU which loads this
+ * one static device array of 53.2 MB that every GPU which loads this
  * library holds until the process exits.
  *   rhs, sol  device pointers to dims[0]*dims[1]*dims[2] doubles, x fastest;
  *             the interior of the 0-based inclusive node box `box` of sol

@@ -55,10 +55,18 @@ __device__ int g_dst_wait_failed;  // a bounded wait ran out (the pass then writ
 
 // Piece (par, mt, ks, digit) of the matrix times factor in [1, 2): rows m,
 // k positions 16 ks + 8 g' + i <-> j = 1 + g + G i with g = 2 ks + g'.
-__global__ void k_dst_table(unsigned char* __restrict__ T, int n, double factor) {
+struct DstTables {
+  DstTable t[3];
+  int block0[4];  // first block of each
+};
+__global__ void k_dst_table(const DstTables A) {
+  const int bx = (int)blockIdx.x, job = bx >= A.block0[2] ? 2 : bx >= A.block0[1] ? 1 : 0;
+  unsigned char* const T = A.t[job].T;
+  const int n = A.t[job].n;
+  const double factor = A.t[job].factor;
   const int N = n + 1, kp = dst_kp(n), G = kp / 8, nks = kp / 16;
   const int mt0 = dst_mtiles(n, 0), mts = mt0 + dst_mtiles(n, 1);
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;  // (mt, ks, g', m)
+  const int t = (bx - A.block0[job]) * (int)blockDim.x + threadIdx.x;  // (mt, ks, g', m)
   if (t >= mts * nks * 2 * kRows) return;
   const int m = t % kRows, gg = (t / kRows) & 1, ks = (t / (2 * kRows)) % nks, mt = t / (2 * kRows * nks);
   const int par = mt >= mt0 ? 1 : 0;
@@ -70,7 +78,7 @@ __global__ void k_dst_table(unsigned char* __restrict__ T, int n, double factor)
   for (int i = 0; i < 8; ++i) {
     const int j = 1 + (2 * ks + gg) + G * i;
     double s = 0.0;
-    if (k <= n && j <= N / 2) s = sinpi((double)((long long)j * k % (2 * N)) / N) * factor;
+    if (k <= n && j <= N / 2) s = sinpi((double)((unsigned)j * k % (2u * N)) / N) * factor;
     x[i] = (long long)rint(s * 36028797018963968.0);  // 2^55
   }
 #pragma unroll
@@ -174,19 +182,20 @@ __global__ void __launch_bounds__(kThreads, 1) k_dst_mma(const __grid_constant__
     emax[q][tid] = 0;
     if (tid == 0) some[q] = 0;
   };
-  // value j = 1..n of a line at `at`, with flags fl (x forward: the boundary values folded in)
-  auto value = [&](const double* in, const double* sol, long long at, int fl, int j) -> double {
-    double v = in[at];
-    if (MODE == 0 && !P.zero_bc) {
-      if (j == 1) v -= sol[at - 1] * P.ihx2;
-      if (j == n) v -= sol[at + 1] * P.ihx2;
-      if (fl & 2) v -= sol[at - P.sy] * P.ihy2;
-      if (fl & 4) v -= sol[at + P.sy] * P.ihy2;
-      if (fl & 8) v -= sol[at - P.sz] * P.ihz2;
-      if (fl & 16) v -= sol[at + P.sz] * P.ihz2;
-    }
+  // x forward: the boundary values that fold into value v = line[j] at `at`.
+  // Few values have any; callers load plainly and correct those (tests beside
+  // every load held the pass with given faces to twice the other passes' time).
+  auto ends = [&](const double* sol, double v, long long at, int j) {
+    if (j == 1) v -= sol[at - 1] * P.ihx2;
+    if (j == n) v -= sol[at + 1] * P.ihx2;
     return v;
   };
+  // nodes beyond the y and z faces next to a line: offset and factor of flag bit 1 + f
+  auto side = [&](int f, double& h) -> long long {
+    h = f < 2 ? P.ihy2 : P.ihz2;
+    return f == 0 ? -P.sy : f == 1 ? P.sy : f == 2 ? -P.sz : P.sz;
+  };
+  const bool faces = MODE == 0 && !P.zero_bc;
   // the largest magnitude of each line of `tile`, by the warps from w0 on
   auto magnitudes = [&](int tile, int q, int w0) {
     const double* in = in_of(tile);
@@ -203,7 +212,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_dst_mma(const __grid_constant__
           double v[U];
 #pragma unroll
           for (int u = 0; u < U; ++u)
-            v[u] = j0 + u * step <= n ? value(in, sol, at + estr * (j0 + u * step - 1), fl, j0 + u * step) : 0.0;
+            v[u] = j0 + u * step <= n ? in[at + estr * (j0 + u * step - 1)] : 0.0;
 #pragma unroll
           for (int u = 0; u < U; ++u) {
             m = max(m, (unsigned)__double2hiint(v[u]) & 0x7FFFFFFFu);
@@ -221,7 +230,23 @@ __global__ void __launch_bounds__(kThreads, 1) k_dst_mma(const __grid_constant__
             double v[U];
 #pragma unroll
             for (int u = 0; u < U; ++u)
-              v[u] = j0 + u * 32 <= n ? value(in, sol, at + j0 + u * 32 - 1, fl, j0 + u * 32) : 0.0;
+              v[u] = j0 + u * 32 <= n ? in[at + j0 + u * 32 - 1] : 0.0;
+            if (faces) {
+#pragma unroll
+              for (int u = 0; u < U; ++u) {
+                const int j = j0 + u * 32;
+                if (j == 1 || j == n) v[u] = ends(sol, v[u], at + j - 1, j);
+              }
+              for (int f = 0; f < 4; ++f)
+                if (fl >> (f + 1) & 1) {
+                  double h, q[U];
+                  const double* const p = sol + at + side(f, h) - 1;
+#pragma unroll
+                  for (int u = 0; u < U; ++u) q[u] = j0 + u * 32 <= n ? p[j0 + u * 32] : 0.0;
+#pragma unroll
+                  for (int u = 0; u < U; ++u) v[u] -= q[u] * h;
+                }
+            }
 #pragma unroll
             for (int u = 0; u < U; ++u) {
               m = max(m, (unsigned)__double2hiint(v[u]) & 0x7FFFFFFFu);
@@ -266,8 +291,30 @@ __global__ void __launch_bounds__(kThreads, 1) k_dst_mma(const __grid_constant__
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int j = 1 + g + G * i;
-        a[i] = (fl & 1) && j <= J ? value(in, sol, at + estr * j, fl, j) : 0.0;
-        b[i] = (fl & 1) && j <= J && N - j != j ? value(in, sol, at + estr * (N - j), fl, N - j) : 0.0;
+        a[i] = (fl & 1) && j <= J ? in[at + estr * j] : 0.0;
+        b[i] = (fl & 1) && j <= J && N - j != j ? in[at + estr * (N - j)] : 0.0;
+      }
+      if (faces && (fl & 1)) {
+        if (g == 0) {  // j = 1 and n
+          a[0] = ends(sol, a[0], at + 1, 1);
+          if (n > 1) b[0] = ends(sol, b[0], at + n, n);
+        }
+        for (int f = 0; f < 4; ++f)
+          if (fl >> (f + 1) & 1) {
+            double h, qa[8], qb[8];
+            const double* const p = sol + at + side(f, h);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const int j = 1 + g + G * i;
+              qa[i] = j <= J ? p[j] : 0.0;
+              qb[i] = j <= J && N - j != j ? p[N - j] : 0.0;
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              a[i] -= qa[i] * h;
+              b[i] -= qb[i] * h;
+            }
+          }
       }
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -432,27 +479,44 @@ void launch(DstArgs& A, cudaStream_t s) {
 // (N <= 416), 1024 of them or more.  Below, the FFT passes are faster: a 64^3
 // step (N = 64 and 80) took 1.91 ms with them and 1.96 ms with products; at
 // N = 128 and 144 the two are level (a 64 x 128 x 96 solve 3.79 against
-// 3.84 ms), and at N = 256 and 272 three components' pass takes 0.90 and
+// 3.84 ms; one component of 119 x 134 x 110 nodes, N = 120 and 135, 0.37 with
+// its tables made on the way against 0.53 ms), and at N = 256 and 272 three components' pass takes 0.90 and
 // 1.85 ms, the FFT's dense pass 1.88 ms at N = 256.
 bool dst_mma_wanted(int n, long long lines) {
   return n + 1 >= 100 && pieces_for(n) && lines >= 1024;
 }
 
-void dst_mma_table(DBuf<unsigned char>& T, int n, double factor, cudaStream_t s) {
+size_t dst_mma_table_bytes(int n) {
+  return (size_t)(dst_mtiles(n, 0) + dst_mtiles(n, 1)) * (dst_kp(n) / 16) * kDigits * kPiece;
+}
+
+void dst_mma_setup() {
   int dev = 0;
   VPMG_CUDA(cudaGetDevice(&dev));
   VPMG_CHECK(dev >= 0 && dev < kMaxDev, VPMG_ERR_UNSUPPORTED, "device index beyond the per-device tables");
-  if (!g_attr[dev]) {  // set-up time, outside any stream capture
+  if (!g_attr[dev]) {
     const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
     VPMG_CUDA(cudaFuncSetAttribute(k_dst_mma<0>, a, kSmemMax));
     VPMG_CUDA(cudaFuncSetAttribute(k_dst_mma<1>, a, kSmemMax));
     VPMG_CUDA(cudaFuncSetAttribute(k_dst_mma<2>, a, kSmemMax));
     g_attr[dev] = true;
   }
-  const int nks = dst_kp(n) / 16, mts = dst_mtiles(n, 0) + dst_mtiles(n, 1);
-  T.ensure((size_t)mts * nks * kDigits * kPiece);
-  const int t = mts * nks * 2 * kRows;
-  k_dst_table<<<(t + 127) / 128, 128, 0, s>>>(T.p, n, factor);
+}
+
+void dst_mma_tables(const DstTable* t, int count, cudaStream_t s) {
+  VPMG_CHECK(count >= 1 && count <= 3, VPMG_ERR_ARG, "dst_mma_tables: 1..3 tables");
+  DstTables A{};
+  int blocks = 0;
+  for (int i = 0; i < 3; ++i) {
+    A.block0[i] = blocks;
+    if (i >= count) continue;
+    A.t[i] = t[i];
+    const int n = t[i].n;
+    blocks += ((dst_mtiles(n, 0) + dst_mtiles(n, 1)) * (dst_kp(n) / 16) * 2 * kRows + 127) / 128;
+  }
+  A.block0[3] = blocks;
+  for (int i = count; i < 3; ++i) A.block0[i] = blocks;
+  k_dst_table<<<blocks, 128, 0, s>>>(A);
   VPMG_LAUNCHED();
   VPMG_CUDA(cudaGetLastError());
 }

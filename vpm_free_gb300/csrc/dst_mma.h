@@ -7,7 +7,14 @@ namespace vpmg {
 
 // Tables of a line length's sine matrix, for plans with p.n points.
 bool dst_mma_wanted(int n, long long lines);
-void dst_mma_table(DBuf<unsigned char>& T, int n, double factor, cudaStream_t s);  // factor in [1, 2)
+size_t dst_mma_table_bytes(int n);
+struct DstTable {
+  unsigned char* T;
+  int n;
+  double factor;  // in [1, 2)
+};
+void dst_mma_setup();  // once per device, outside stream capture
+void dst_mma_tables(const DstTable* t, int count, cudaStream_t s);  // up to three, one launch
 // Passes: lines of n points; nc components (strides in doubles).
 struct DstBox {
   int dims[3], o[3], m[3];

@@ -964,13 +964,19 @@ void dirichlet_prepare(DirichletPlan& P, const int dims[3], const int box[6], co
     const double f = std::frexp(std::fabs(dirichlet_scale(P)), &e);  // factor = 2 f 2^(e-1)
     P.xf_shift = e - 1;
     P.xf_neg = dirichlet_scale(P) < 0.0 ? 1 : 0;
-    dst_mma_table(P.tx, P.m[0], 1.0, s);
-    dst_mma_table(P.txf, P.m[0], 2.0 * f, s);
+    P.tx.ensure(dst_mma_table_bytes(P.m[0]));
+    P.txf.ensure(dst_mma_table_bytes(P.m[0]));
+    const DstTable t[2] = {{P.tx.p, P.m[0], 1.0}, {P.txf.p, P.m[0], 2.0 * f}};
+    dst_mma_setup();
+    dst_mma_tables(t, 2, s);
   } else {
     tune_pairs(P.fx, P.m[1] * P.m[2], 1, P.m[0], P.m[1] * P.m[2], s);  // rows along x
   }
   if (P.mma_y) {
-    dst_mma_table(P.ty, P.m[1], 1.0, s);
+    P.ty.ensure(dst_mma_table_bytes(P.m[1]));
+    const DstTable t{P.ty.p, P.m[1], 1.0};
+    dst_mma_setup();
+    dst_mma_tables(&t, 1, s);
     P.tmp.ensure(3 * (size_t)P.m[0] * P.m[1] * P.m[2]);
   } else {
     tune_pairs(P.fy, P.m[0] * P.m[2], P.m[0], P.m[1], P.m[2], s);      // columns along y
@@ -990,7 +996,7 @@ void dirichlet_prepare(DirichletPlan& P, const int dims[3], const int box[6], co
   P.rinvd.ensure((size_t)P.m[0] * P.m[1] * (P.m[2] / 2 + 1));
   const double hz2 = h[2] * h[2];
   const int nl = P.m[0] * P.m[1];
-  k_pivots<<<(nl + 255) / 256, 256, 0, s>>>(ffp ? P.rinv.p : nullptr, P.rinvd.p, dmx.p, dmy.p, P.m[0], P.m[1], P.m[2], hz2 / (h[0] * h[0]),
+  k_pivots<<<(nl + 63) / 64, 64, 0, s>>>(ffp ? P.rinv.p : nullptr, P.rinvd.p, dmx.p, dmy.p, P.m[0], P.m[1], P.m[2], hz2 / (h[0] * h[0]),
                                             hz2 / (h[1] * h[1]));
   VPMG_LAUNCHED();
   VPMG_CUDA(cudaGetLastError());
@@ -1155,18 +1161,26 @@ void dst_x_inv_jobs(const DstXInvLines* jobs, int n, cudaStream_t s, int nc) {
 
 // ------------------------------------------ allocation-free variant -----
 // vpmg_dirichlet_static: the same five-kernel solve, with every temporary
-// (DST work array, reciprocal pivot table, twiddles, eigenvalues) carved
-// out of one file-scope device array instead of cudaMalloc'd buffers.
+// (DST work arrays, reciprocal pivot table, twiddles, eigenvalues, sine
+// matrices) carved out of one file-scope device array instead of cudaMalloc'd
+// buffers.  The tables are made on every call.  119 x 134 x 110 nodes took
+// 0.62 ms with FFT passes (the odd extension along y 0.31 of it) and one
+// pivot kernel of 63 CTAs; with products where the handle-based solves take
+// them 0.37 ms (x 0.10 and 0.07, y 0.15, pivots and tables 0.04).
 namespace {
 
 constexpr size_t kStaticMaxInterior = (size_t)1 << 21;  // interior nodes (e.g. 128 x 128 x 128)
 constexpr int kStaticMaxLine = 900;                     // interior nodes along x and along y
 constexpr size_t kStaticTw = 2 * (kStaticMaxLine + 1);  // complex FFT length bound
 constexpr size_t kStaticSn = kStaticMaxLine + 1;         // sin(pi j / N) table bound
-// doubles: work | pivots | twiddles x (2 per complex) | twiddles y | mu x | mu y | sin x | sin y
-constexpr size_t kStaticDoubles = 2 * kStaticMaxInterior + 4 * kStaticTw + 2 * kStaticMaxLine + 2 * kStaticSn;
+constexpr size_t kStaticPivots = kStaticMaxInterior / 2 + (size_t)kStaticMaxLine * kStaticMaxLine;  // (m2 / 2 + 1) planes
+constexpr size_t kStaticTable = 190 * 1024;  // one sine matrix as digits: 1.49 MB at the longest line of the product form
+// doubles: work | second work array | pivots | sine matrices | twiddles x (2 per complex) | twiddles y | mu x | mu y |
+// sin x | sin y
+constexpr size_t kStaticDoubles = 2 * kStaticMaxInterior + kStaticPivots + 3 * kStaticTable + 4 * kStaticTw +
+                                  2 * kStaticMaxLine + 2 * kStaticSn;
 
-// 33.6 MB per GPU that loads the library, held until the process exits.
+// 53.2 MB per GPU that loads the library, held until the process exits.
 __device__ __align__(256) double g_static_scratch[kStaticDoubles];
 
 constexpr int kStaticMaxDevices = 64;
@@ -1263,8 +1277,10 @@ extern "C" int vpmg_dirichlet_static(const double* rhs, double* sol, const int d
   // FP64 throughout, as the handle-based solves by default
   double* base = g_static_base[dev];
   double* work = base;
-  double* rinv = base + kStaticMaxInterior;                                  // reciprocal pivots
-  double2* twx = reinterpret_cast<double2*>(base + 2 * kStaticMaxInterior);  // twiddles, 16 B each
+  double* work2 = base + kStaticMaxInterior;
+  double* rinv = base + 2 * kStaticMaxInterior;  // reciprocal pivots
+  unsigned char* mtab = reinterpret_cast<unsigned char*>(rinv + kStaticPivots);
+  double2* twx = reinterpret_cast<double2*>(rinv + kStaticPivots + 3 * kStaticTable);  // twiddles, 16 B each
   double2* twy = twx + kStaticTw;
   double* mux = reinterpret_cast<double*>(twy + kStaticTw);
   double* muy = mux + kStaticMaxLine;
@@ -1280,23 +1296,56 @@ extern "C" int vpmg_dirichlet_static(const double* rhs, double* sol, const int d
     return VPMG_ERR_CUDA;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  // the passes as products by the rule of the handle-based solves
+  constexpr size_t tb = kStaticTable * sizeof(double);
+  const bool mx = dst_mma_wanted(m[0], (long long)m[1] * m[2]) && dst_mma_table_bytes(m[0]) <= tb;
+  const bool my = dst_mma_wanted(m[1], (long long)m[0] * m[2]) && dst_mma_table_bytes(m[1]) <= tb;
   // tables and pivots are rebuilt on every call: the array keeps whatever the
   // previous call (possibly another grid) left in it
-  const int nt = std::max(std::max(px.M, py.M), std::max(px.N, py.N));
-  k_static_tables<<<(nt + 255) / 256, 256, 0, s>>>(twx, px.M, twy, py.M, mux, m[0], muy, m[1], snx,
-                                                   px.rs ? px.N : 0, sny, py.rs ? py.N : 0);
+  const int nt = std::max(std::max(mx ? 0 : px.M, my ? 0 : py.M), std::max(px.N, py.N));
+  k_static_tables<<<(nt + 255) / 256, 256, 0, s>>>(twx, mx ? 0 : px.M, twy, my ? 0 : py.M, mux, m[0], muy, m[1], snx,
+                                                   !mx && px.rs ? px.N : 0, sny, !my && py.rs ? py.N : 0);
   const double hz2 = h[2] * h[2], hx2 = h[0] * h[0], hy2 = h[1] * h[1];
   const int nl = m[0] * m[1];
-  k_pivots<<<(nl + 255) / 256, 256, 0, s>>>(nullptr, rinv, mux, muy, m[0], m[1], m[2], hz2 / hx2, hz2 / hy2);
+  k_pivots<<<(nl + 63) / 64, 64, 0, s>>>(nullptr, rinv, mux, muy, m[0], m[1], m[2], hz2 / hx2, hz2 / hy2);
   Box b;
-  for (int d = 0; d < 3; ++d) { b.dims[d] = dims[d]; b.o[d] = box[d] + 1; b.m[d] = m[d]; }
+  DstBox db;
+  for (int d = 0; d < 3; ++d) {
+    b.dims[d] = db.dims[d] = dims[d];
+    b.o[d] = db.o[d] = box[d] + 1;
+    b.m[d] = db.m[d] = m[d];
+  }
   const double scale = -hz2 * 4.0 / ((double)(m[0] + 1) * (double)(m[1] + 1));
   const CompStride cs{1, 0, 0, 0};
-  launch_x_fwd(s, rhs, sol, zero_bc ? 1 : 0, work, b, px, 1.0 / hx2, 1.0 / hy2, 1.0 / hz2, scale, cs);
-  launch_y(s, work, m[0], m[1], m[2], py);
-  thomas_launch(work, work, rinv, m, 1, 0, nullptr, s);
-  launch_y(s, work, m[0], m[1], m[2], py);
-  launch_x_inv(s, work, sol, b, px, cs);
+  try {
+    int e = 0;
+    const double f = std::frexp(-scale, &e);  // -scale = 2 f 2^(e - 1)
+    if (mx || my) {
+      DstTable t[3];
+      int c = 0;
+      if (mx) {
+        t[c++] = {mtab, m[0], 1.0};
+        t[c++] = {mtab + tb, m[0], 2.0 * f};
+      }
+      if (my) t[c++] = {mtab + 2 * tb, m[1], 1.0};
+      dst_mma_setup();
+      dst_mma_tables(t, c, s);
+    }
+    if (mx)
+      dst_mma_x_fwd(mtab + tb, e - 1, 1, rhs, sol, zero_bc != 0, work, db, 1.0 / hx2, 1.0 / hy2, 1.0 / hz2, 1, 0, 0, 0, s);
+    else
+      launch_x_fwd(s, rhs, sol, zero_bc ? 1 : 0, work, b, px, 1.0 / hx2, 1.0 / hy2, 1.0 / hz2, scale, cs);
+    double* g = my ? work2 : work;
+    if (my) dst_mma_y(mtab + 2 * tb, work, g, m[0], m[1], m[2], 1, 0, s);
+    else launch_y(s, work, m[0], m[1], m[2], py);
+    thomas_launch(g, g, rinv, m, 1, 0, nullptr, s);
+    if (my) dst_mma_y(mtab + 2 * tb, g, work, m[0], m[1], m[2], 1, 0, s);
+    else launch_y(s, work, m[0], m[1], m[2], py);
+    if (mx) dst_mma_x_inv(mtab, work, sol, db, 1, 0, 0, s);
+    else launch_x_inv(s, work, sol, b, px, cs);
+  } catch (const Error& err) {
+    return err.status;
+  }
   if (zero_bc) k_zero_box_faces<<<256, 256, 0, s>>>(sol, b, 0);
   if (cudaGetLastError() != cudaSuccess) return VPMG_ERR_CUDA;
   return VPMG_OK;
