@@ -32,11 +32,11 @@ struct AdjointState {
   vpmg::DBuf<double> xq1;   // X', Q' after the Euler push: 6 x cap
   vpmg::DBuf<double> pbar;  // xbar qbar upbar gpbar qnew xb1 qb1: 21 x cap
   vpmg::DBuf<double> rbar, psibar, ubar, gbar, nodeA;  // 3 x N each
-  vpmg::DBuf<double> blA, blB, blC, blD;               // block arrays (NB)
-  vpmg::DBuf<double> cA, cB, cC;                       // coarse arrays (NC)
+  vpmg::DBuf<double> blA, blB, blC, blD;               // block arrays (3 NB)
+  vpmg::DBuf<double> cA, cB, cC;                       // coarse arrays (3 NC)
   vpmg::DBuf<double> cellbar, panelbar;
-  vpmg::DBuf<double> sampbar, crhsbar, csolbar;  // NC each
-  vpmg::DBuf<double> rhsbarbl;                   // NB
+  vpmg::DBuf<double> sampbar, crhsbar, csolbar;  // 3 NC each
+  vpmg::DBuf<double> rhsbarbl;                   // 3 NB
   vpmg::DBuf<double> probes, uprobe;             // 3 x nprobe each (component-major)
   vpmg::DBuf<double> lossv;                      // block partial sums
   vpmg::DBuf<double> out;                        // AoS gradients for the host copy
@@ -258,7 +258,10 @@ __global__ void k_curl_T(const double* __restrict__ ubar, int NX, int NY, int NZ
 // bbar = ubar - fbar(interior neighbour) / h^2, on box edges bbar = ubar.
 __global__ void k_face_bc_T(const double* __restrict__ ubar, const double* __restrict__ fbar, int NX, int NY, int lo0,
                             int lo1, int lo2, int hi0, int hi1, int hi2, double ihx2, double ihy2, double ihz2,
-                            double* __restrict__ bbar) {
+                            double* __restrict__ bbar, size_t cs) {
+  ubar += blockIdx.y * cs;  // component
+  fbar += blockIdx.y * cs;
+  bbar += blockIdx.y * cs;
   const int ex = hi0 - lo0 + 1, ey = hi1 - lo1 + 1, ez = hi2 - lo2 + 1;
   const long long total = (long long)ex * ey * ez;
   const size_t sy = NX, sz = (size_t)NX * NY;
@@ -287,7 +290,10 @@ __global__ void k_axpy(double* __restrict__ y, const double* __restrict__ x, dou
 }
 // dst(box at dof) += src(box at so), box extent e.
 __global__ void k_box_add(const double* __restrict__ src, int sx, int sy, int so0, int so1, int so2,
-                          double* __restrict__ dst, int dx, int dy, int do0, int do1, int do2, int e0, int e1, int e2) {
+                          double* __restrict__ dst, int dx, int dy, int do0, int do1, int do2, int e0, int e1, int e2,
+                          size_t scs, size_t dcs) {
+  src += blockIdx.y * scs;  // component
+  dst += blockIdx.y * dcs;
   const size_t n = (size_t)e0 * e1 * e2;
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x) {
     const int i = (int)(t % e0), j = (int)((t / e0) % e1), k = (int)(t / ((size_t)e0 * e1));
@@ -300,7 +306,10 @@ __global__ void k_box_add(const double* __restrict__ src, int sx, int sy, int so
 __global__ void k_face_interp_T(const long long* __restrict__ node, const long long* __restrict__ cbase,
                                 const double* __restrict__ w, const int* __restrict__ flagged, int n, int CX, int CY,
                                 const double* __restrict__ fbar, double* __restrict__ csolbar,
-                                double* __restrict__ sampbar) {
+                                double* __restrict__ sampbar, size_t fcs, size_t ccs) {
+  fbar += blockIdx.y * fcs;  // component
+  csolbar += blockIdx.y * ccs;
+  sampbar += blockIdx.y * ccs;
   const size_t sy = CX, sz = (size_t)CX * CY;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
     const double F = fbar[node[t]];
@@ -323,6 +332,8 @@ __global__ void k_face_interp_T(const long long* __restrict__ node, const long l
 __global__ void k_coarse_lap_T(const double* __restrict__ cr, double* __restrict__ sb, int CX, int CY, int CZ, int lo0,
                                int lo1, int lo2, int e0, int e1, int e2, double ih0, double ih1, double ih2) {
   const size_t N = (size_t)CX * CY * CZ;
+  cr += blockIdx.y * N;  // component
+  sb += blockIdx.y * N;
   for (size_t id = blockIdx.x * (size_t)blockDim.x + threadIdx.x; id < N; id += (size_t)gridDim.x * blockDim.x) {
     int i, j, k;
     unflatten(id, CX, CY, i, j, k);
@@ -337,7 +348,9 @@ __global__ void k_coarse_lap_T(const double* __restrict__ cr, double* __restrict
 }
 
 __global__ void k_sample_T(const long long* __restrict__ src, const long long* __restrict__ dst, int n,
-                           const double* __restrict__ sampbar, double* __restrict__ ubl) {
+                           const double* __restrict__ sampbar, double* __restrict__ ubl, size_t ccs, size_t fcs) {
+  sampbar += blockIdx.y * ccs;  // component
+  ubl += blockIdx.y * fcs;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
     atomicAdd(&ubl[src[t]], sampbar[dst[t]]);
 }
@@ -478,27 +491,32 @@ __global__ void k_from_aos(int n, const double* __restrict__ o, int cap, double*
 unsigned grid(size_t n, int t = 256) { return (unsigned)std::max<size_t>(1, std::min<size_t>((n + t - 1) / t, 152 * 16)); }
 
 // ----------------------------------------------------------- L^T ---------
+// All three components in every launch (their arrays follow one another): a
+// 64^3 step back is launches of a few microseconds, and one component filled
+// a fraction of the GPU.  The ten-step gradient took 84.6 ms component by
+// component, 73.5 together.
+
 // Transposed Dirichlet solve with the box faces of the output as boundary
 // values (dirichlet_solve with zero_bc = false).  ubar: adjoint of the
 // output, zero outside the box.  rhsbar += A^-1 ubar (interior; the 7-point
 // Laplacian is symmetric), bbar <- adjoint of the boundary values (box faces,
-// zero elsewhere).  fbar: scratch of the array's size.
+// zero elsewhere).  fbar: scratch of the arrays' size (3 n).
 void dirichlet_T(vpmg_handle* h, DirichletPlan& dp, const double* ubar, double* rhsbar, double* bbar, double* fbar,
                  size_t n) {
   cudaStream_t st = h->stream;
-  k_zero<<<grid(n), 256, 0, st>>>(fbar, n);
+  k_zero<<<grid(3 * n), 256, 0, st>>>(fbar, 3 * n);
   VPMG_LAUNCHED();
-  dirichlet_solve(dp, ubar, fbar, true, h->work.p, st);
-  k_axpy<<<grid(n), 256, 0, st>>>(rhsbar, fbar, 1.0, n);
-  k_zero<<<grid(n), 256, 0, st>>>(bbar, n);
-  k_face_bc_T<<<grid((size_t)(dp.m[0] + 2) * (dp.m[1] + 2) * (dp.m[2] + 2)), 256, 0, st>>>(
+  dirichlet_solve(dp, ubar, fbar, true, h->work.p, st, 3, n, n);
+  k_axpy<<<grid(3 * n), 256, 0, st>>>(rhsbar, fbar, 1.0, 3 * n);
+  k_zero<<<grid(3 * n), 256, 0, st>>>(bbar, 3 * n);
+  k_face_bc_T<<<dim3(grid((size_t)(dp.m[0] + 2) * (dp.m[1] + 2) * (dp.m[2] + 2)), 3), 256, 0, st>>>(
       ubar, fbar, dp.dims[0], dp.dims[1], dp.box[0], dp.box[1], dp.box[2], dp.box[3], dp.box[4], dp.box[5],
-      1.0 / (dp.h[0] * dp.h[0]), 1.0 / (dp.h[1] * dp.h[1]), 1.0 / (dp.h[2] * dp.h[2]), bbar);
+      1.0 / (dp.h[0] * dp.h[0]), 1.0 / (dp.h[1] * dp.h[1]), 1.0 / (dp.h[2] * dp.h[2]), bbar, n);
   count_launch(3);
   VPMG_CUDA(cudaGetLastError());
 }
 
-// Transposed infinite-domain solve of one component (pmesh, iynbc = 1):
+// Transposed infinite-domain solve (pmesh, iynbc = 1):
 // sol = D2(rhs, bc),  bc = -(1/4pi) T agg N D0(rhs).  rhsbar += ...
 void infinite_domain_T(vpmg_handle* h, DirichletPlan& dp, BoundaryOp& bo, const Grid& g, const double* solbar,
                        double* rhsbar, double* A, double* B, double* C) {
@@ -506,13 +524,13 @@ void infinite_domain_T(vpmg_handle* h, DirichletPlan& dp, BoundaryOp& bo, const 
   cudaStream_t st = h->stream;
   const size_t n = g.count();
   dirichlet_T(h, dp, solbar, rhsbar, A, B, n);  // A = boundary-value adjoint
-  boundary_apply_T(bo, A, S.cellbar.p, st);
+  boundary_apply_T(bo, A, n, S.cellbar.p, st);
   boundary_agg_T(bo, S.cellbar.p, S.panelbar.p, st);
-  k_zero<<<grid(n), 256, 0, st>>>(C, n);
+  k_zero<<<grid(3 * n), 256, 0, st>>>(C, 3 * n);
   VPMG_LAUNCHED();
-  boundary_panels_T(bo, g, S.panelbar.p, C, st);   // C = adjoint of the zero-BC solution
-  dirichlet_solve(dp, C, B, true, h->work.p, st);  // D0^T (interior of B; B spans the whole box)
-  k_axpy<<<grid(n), 256, 0, st>>>(rhsbar, B, 1.0, n);
+  boundary_panels_T(bo, g, S.panelbar.p, C, n, st);         // C = adjoint of the zero-BC solution
+  dirichlet_solve(dp, C, B, true, h->work.p, st, 3, n, n);  // D0^T (interior of B; B spans the whole box)
+  k_axpy<<<grid(3 * n), 256, 0, st>>>(rhsbar, B, 1.0, 3 * n);
   VPMG_LAUNCHED();
 }
 
@@ -526,46 +544,44 @@ void poisson_T(vpmg_handle* h, const double* psibar, double* rbar) {
   const YapsDev& Y = h->yaps;
   const int lo[3] = {Y.map[0], Y.map[1], Y.map[2]};
   const int e[3] = {Y.map[3] - Y.map[0] - 1, Y.map[4] - Y.map[1] - 1, Y.map[5] - Y.map[2] - 1};
-  for (int c = 0; c < 3; ++c) {
-    double* ubl = S.blA.p;  // adjoint of the block solution
-    double* rbl = S.rhsbarbl.p;
-    fill_zero(ubl, NB, st);
-    fill_zero(rbl, NB, st);
-    // solget^T
-    box_copy(psibar + (size_t)c * N, s.nn, go, ubl, s.nnbl, h->inner_lo, h->inner_ext, st);
-    // final solve on the inner box: rhs part -> rbl, face values -> blB
-    dirichlet_T(h, h->dp_inner, ubl, rbl, S.blB.p, S.blC.p, NB);
-    // face interpolation: the faces kept their values and received the coarse correction
-    fill_zero(S.csolbar.p, NC, st);
-    fill_zero(S.sampbar.p, NC, st);
-    k_face_interp_T<<<grid(Y.nface, 128), 128, 0, st>>>(Y.face_node.p, Y.face_cbase.p, Y.face_w.p, Y.face_flag.p,
-                                                         Y.nface, s.nn_coarse[0], s.nn_coarse[1], S.blB.p,
-                                                         S.csolbar.p, S.sampbar.p);
+  double* ubl = S.blA.p;  // adjoint of the block solution
+  double* rbl = S.rhsbarbl.p;
+  fill_zero(ubl, 3 * NB, st);
+  fill_zero(rbl, 3 * NB, st);
+  // solget^T
+  box_copy(psibar, s.nn, go, ubl, s.nnbl, h->inner_lo, h->inner_ext, st, 3, N, NB);
+  // final solve on the inner box: rhs part -> rbl, face values -> blB
+  dirichlet_T(h, h->dp_inner, ubl, rbl, S.blB.p, S.blC.p, NB);
+  // face interpolation: the faces kept their values and received the coarse correction
+  fill_zero(S.csolbar.p, 3 * NC, st);
+  fill_zero(S.sampbar.p, 3 * NC, st);
+  k_face_interp_T<<<dim3(grid(Y.nface, 128), 3), 128, 0, st>>>(Y.face_node.p, Y.face_cbase.p, Y.face_w.p,
+                                                               Y.face_flag.p, Y.nface, s.nn_coarse[0], s.nn_coarse[1],
+                                                               S.blB.p, S.csolbar.p, S.sampbar.p, NB, NC);
+  VPMG_LAUNCHED();
+  VPMG_CUDA(cudaMemcpyAsync(ubl, S.blB.p, 3 * sizeof(double) * NB, cudaMemcpyDeviceToDevice, st));
+  // coarse infinite-domain solve, then the coarse Laplacian of the samples
+  fill_zero(S.crhsbar.p, 3 * NC, st);
+  infinite_domain_T(h, h->dp_c, h->bo_c, h->gco, S.csolbar.p, S.crhsbar.p, S.cA.p, S.cB.p, S.cC.p);
+  if (e[0] > 0 && e[1] > 0 && e[2] > 0) {
+    k_coarse_lap_T<<<dim3(grid(NC), 3), 256, 0, st>>>(S.crhsbar.p, S.sampbar.p, s.nn_coarse[0], s.nn_coarse[1],
+                                                      s.nn_coarse[2], lo[0], lo[1], lo[2], e[0], e[1], e[2],
+                                                      1.0 / (s.dpm_coarse[0] * s.dpm_coarse[0]),
+                                                      1.0 / (s.dpm_coarse[1] * s.dpm_coarse[1]),
+                                                      1.0 / (s.dpm_coarse[2] * s.dpm_coarse[2]));
     VPMG_LAUNCHED();
-    VPMG_CUDA(cudaMemcpyAsync(ubl, S.blB.p, sizeof(double) * NB, cudaMemcpyDeviceToDevice, st));
-    // coarse infinite-domain solve, then the coarse Laplacian of the samples
-    fill_zero(S.crhsbar.p, NC, st);
-    infinite_domain_T(h, h->dp_c, h->bo_c, h->gco, S.csolbar.p, S.crhsbar.p, S.cA.p, S.cB.p, S.cC.p);
-    if (e[0] > 0 && e[1] > 0 && e[2] > 0) {
-      k_coarse_lap_T<<<grid(NC), 256, 0, st>>>(S.crhsbar.p, S.sampbar.p, s.nn_coarse[0], s.nn_coarse[1],
-                                               s.nn_coarse[2], lo[0], lo[1], lo[2], e[0], e[1], e[2],
-                                               1.0 / (s.dpm_coarse[0] * s.dpm_coarse[0]),
-                                               1.0 / (s.dpm_coarse[1] * s.dpm_coarse[1]),
-                                               1.0 / (s.dpm_coarse[2] * s.dpm_coarse[2]));
-      VPMG_LAUNCHED();
-    }
-    // sampling of the fine block solution
-    k_sample_T<<<grid(Y.nsamp), 256, 0, st>>>(Y.samp_src.p, Y.samp_dst.p, Y.nsamp, S.sampbar.p, ubl);
-    VPMG_LAUNCHED();
-    // fine infinite-domain solve on the padded block
-    infinite_domain_T(h, h->dp_bl, h->bo_bl, h->gbl, ubl, rbl, S.blB.p, S.blC.p, S.blD.p);
-    // rhsscat^T: the block RHS holds the global RHS on the inner box
-    k_box_add<<<grid((size_t)h->inner_ext[0] * h->inner_ext[1] * h->inner_ext[2]), 256, 0, st>>>(
-        rbl, s.nnbl[0], s.nnbl[1], h->inner_lo[0], h->inner_lo[1], h->inner_lo[2], rbar + (size_t)c * N, s.nn[0],
-        s.nn[1], go[0], go[1], go[2], h->inner_ext[0], h->inner_ext[1], h->inner_ext[2]);
-    VPMG_LAUNCHED();
-    VPMG_CUDA(cudaGetLastError());
   }
+  // sampling of the fine block solution
+  k_sample_T<<<dim3(grid(Y.nsamp), 3), 256, 0, st>>>(Y.samp_src.p, Y.samp_dst.p, Y.nsamp, S.sampbar.p, ubl, NC, NB);
+  VPMG_LAUNCHED();
+  // fine infinite-domain solve on the padded block
+  infinite_domain_T(h, h->dp_bl, h->bo_bl, h->gbl, ubl, rbl, S.blB.p, S.blC.p, S.blD.p);
+  // rhsscat^T: the block RHS holds the global RHS on the inner box
+  k_box_add<<<dim3(grid((size_t)h->inner_ext[0] * h->inner_ext[1] * h->inner_ext[2]), 3), 256, 0, st>>>(
+      rbl, s.nnbl[0], s.nnbl[1], h->inner_lo[0], h->inner_lo[1], h->inner_lo[2], rbar, s.nn[0], s.nn[1], go[0], go[1],
+      go[2], h->inner_ext[0], h->inner_ext[1], h->inner_ext[2], NB, N);
+  VPMG_LAUNCHED();
+  VPMG_CUDA(cudaGetLastError());
 }
 
 // ------------------------------------------------------------ steps ------
@@ -594,10 +610,10 @@ void ensure_state(vpmg_handle* h, int K, int nprobe) {
   S.xq1.ensure(6 * (size_t)S.cap);
   S.pbar.ensure(21 * (size_t)S.cap);
   for (DBuf<double>* b : {&S.rbar, &S.psibar, &S.ubar, &S.gbar, &S.nodeA}) b->ensure(3 * N);
-  for (DBuf<double>* b : {&S.blA, &S.blB, &S.blC, &S.blD, &S.rhsbarbl}) b->ensure(NB);
-  for (DBuf<double>* b : {&S.cA, &S.cB, &S.cC, &S.sampbar, &S.crhsbar, &S.csolbar}) b->ensure(NC);
-  S.cellbar.ensure(std::max(h->bo_bl.ncell_total, h->bo_c.ncell_total));
-  S.panelbar.ensure(std::max(h->bo_bl.nbound, h->bo_c.nbound));
+  for (DBuf<double>* b : {&S.blA, &S.blB, &S.blC, &S.blD, &S.rhsbarbl}) b->ensure(3 * NB);
+  for (DBuf<double>* b : {&S.cA, &S.cB, &S.cC, &S.sampbar, &S.crhsbar, &S.csolbar}) b->ensure(3 * NC);
+  S.cellbar.ensure(3 * (size_t)std::max(h->bo_bl.ncell_total, h->bo_c.ncell_total));
+  S.panelbar.ensure(3 * (size_t)std::max(h->bo_bl.nbound, h->bo_c.nbound));
   S.probes.ensure(3 * (size_t)std::max(nprobe, 1));
   S.uprobe.ensure(3 * (size_t)std::max(nprobe, 1));
   S.lossv.ensure(2 * kSumBlocks);

@@ -1439,41 +1439,60 @@ __global__ void k_col_fill(const long long* __restrict__ rowptr, const int* __re
     tw[slot] = wgt[k];  // the 8-byte weight word, either arithmetic
   }
 }
-// The boundary-value adjoint of each target in the policy's arithmetic, once per call.
+// The boundary-value adjoints of each target in the policy's arithmetic, once
+// per call, packed as the sources are: (v0, v1, v2, 0).
 template <class M>
-__global__ void k_split_bc(const double* __restrict__ bcbar, const int* __restrict__ tgt_node, int ntarget,
+__global__ void k_split_bc(const double* __restrict__ bcbar, size_t cs, const int* __restrict__ tgt_node, int ntarget,
                            typename M::V* __restrict__ v) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < ntarget) v[t] = M::vsplit(bcbar[tgt_node[t]]);
+  if (t >= ntarget) return;
+  const int node = tgt_node[t];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) v[4 * (size_t)t + c] = M::vsplit(c < 3 ? bcbar[c * cs + node] : 0.0);
 }
 
-// cellbar[c] = scale * sum over the cell's targets of w * bcbar(target node);
-// warp per cell, products and sums in the policy's arithmetic.
+// cellbar[c] = scale * sum over the cell's targets of w * bcbar(target node),
+// for the three components at once: the list (12 bytes an entry) is read once
+// and a target's adjoints are one 32-byte sector.  Warp per cell, products and
+// sums in the policy's arithmetic.  Bound by the FP64 units: the list of the
+// 81^3 block takes 1.04 ms for the three components (1.2 ms one by one); lists
+// in target order, whose gathers share sectors, change nothing.
 template <class M>
 __global__ void __launch_bounds__(256) k_csc_T(const long long* __restrict__ colptr, const int* __restrict__ trow,
                                                const typename M::W* __restrict__ tw,
-                                               const typename M::V* __restrict__ v, int ncell, double scale,
+                                               const typename M::H* __restrict__ v, int ncell, double scale,
                                                double* __restrict__ cellbar) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= ncell) return;
-  typename M::Acc f;
-  for (long long k = colptr[warp] + lane; k < colptr[warp + 1]; k += 32)
-    M::mac(f, __ldg(&tw[k]), __ldg(&v[__ldg(&trow[k])]));
-  double a = M::fin(f);
+  typename M::Acc f0, f1, f2;
+  const long long end = colptr[warp + 1];
+#pragma unroll 2
+  for (long long k = colptr[warp] + lane; k < end; k += 32) {
+    const typename M::W w = __ldg(&tw[k]);
+    const size_t t = (size_t)__ldg(&trow[k]);
+    const typename M::H h0 = __ldg(&v[2 * t]), h1 = __ldg(&v[2 * t + 1]);
+    M::mac(f0, w, M::v0(h0));
+    M::mac(f1, w, M::v1(h0));
+    M::mac(f2, w, M::v0(h1));
+  }
+  double a[3] = {M::fin(f0), M::fin(f1), M::fin(f2)};
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-  if (lane == 0) cellbar[warp] = scale * a;
+  for (int c = 0; c < 3; ++c) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a[c] += __shfl_xor_sync(0xffffffffu, a[c], o);
+    if (lane == 0) cellbar[(size_t)c * ncell + warp] = scale * a[c];
+  }
 }
 
 // Transpose of the dense block: cellbar[top0 + c] += scale * sum_t w(t, c) bcbar(node t).
-// A warp per (cell, group of kDenseTGroup target chunks) forms a partial sum
-// (each chunk's 32 weights are one coalesced row), then k_dense_T_sum adds
-// a cell's groups in order (deterministic).
+// A warp per (cell, group of kDenseTGroup target chunks) forms the partial
+// sums of the three components (each chunk's 32 weights are one coalesced
+// row), then k_dense_T_sum adds a cell's groups in order (deterministic).
 constexpr int kDenseTGroup = 64;
 template <class M>
 __global__ void __launch_bounds__(256) k_dense_T(const typename M::W* __restrict__ wtop,
-                                                 const typename M::V* __restrict__ v, int ntop, int ntarget,
+                                                 const typename M::H* __restrict__ v, int ntop, int ntarget,
                                                  double* __restrict__ part) {
   const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -1482,33 +1501,43 @@ __global__ void __launch_bounds__(256) k_dense_T(const typename M::W* __restrict
   if (wid >= (long long)ntop * ngroup) return;
   const int c = (int)(wid % ntop), grp = (int)(wid / ntop);
   const int g1 = min(nchunk, (grp + 1) * kDenseTGroup);
-  typename M::Acc f;
+  typename M::Acc f0, f1, f2;
+#pragma unroll 2
   for (int g = grp * kDenseTGroup; g < g1; ++g) {
     const int t = g * 32 + lane;
     if (t >= ntarget) continue;
     const typename M::W w = __ldg(&wtop[(((size_t)g * ((ntop + 1) >> 1) + (c >> 1)) * 32 + lane) * 2 + (c & 1)]);
-    M::mac(f, w, __ldg(&v[t]));
+    const typename M::H h0 = __ldg(&v[2 * (size_t)t]), h1 = __ldg(&v[2 * (size_t)t + 1]);
+    M::mac(f0, w, M::v0(h0));
+    M::mac(f1, w, M::v1(h0));
+    M::mac(f2, w, M::v0(h1));
   }
-  double a = M::fin(f);
+  double a[3] = {M::fin(f0), M::fin(f1), M::fin(f2)};
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-  if (lane == 0) part[(size_t)grp * ntop + c] = a;
+  for (int d = 0; d < 3; ++d) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a[d] += __shfl_xor_sync(0xffffffffu, a[d], o);
+    if (lane == 0) part[((size_t)d * ngroup + grp) * ntop + c] = a[d];
+  }
 }
 
 __global__ void k_dense_T_sum(const double* __restrict__ part, int ntop, int ngroup, int top0, double scale,
-                              double* __restrict__ cellbar) {
+                              double* __restrict__ cellbar, size_t cs) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ntop) return;
+  part += (size_t)blockIdx.y * ngroup * ntop;
   double a = 0.0;
   for (int grp = 0; grp < ngroup; ++grp) a += part[(size_t)grp * ntop + c];
-  cellbar[top0 + c] += scale * a;
+  cellbar[blockIdx.y * cs + top0 + c] += scale * a;
 }
 
 // leaf adjoint = its own level-0 adjoint + sum over ancestors of ds_leaf / ds_cell * cell adjoint
 __global__ void k_agg_T(const int* __restrict__ anc, const double* __restrict__ cds, int nbound, int levmax,
-                        const double* __restrict__ cellbar, double* __restrict__ panelbar) {
+                        const double* __restrict__ cellbar, double* __restrict__ panelbar, size_t cs) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= nbound) return;
+  cellbar += blockIdx.y * cs;  // component
+  panelbar += (size_t)blockIdx.y * nbound;
   double v = cellbar[p];
   const double ds = cds[p];
   for (int l = 1; l <= levmax; ++l) {
@@ -1520,10 +1549,12 @@ __global__ void k_agg_T(const int* __restrict__ anc, const double* __restrict__ 
 
 __global__ void k_normal_deriv_T(const double* __restrict__ panelbar, int NX, int NY, const int* __restrict__ face,
                                  const int* __restrict__ pi, const int* __restrict__ pj, const int* __restrict__ pk,
-                                 int nbound, double invx, double invy, double invz, double* __restrict__ sol0bar) {
+                                 int nbound, double invx, double invy, double invz, double* __restrict__ sol0bar,
+                                 size_t scs) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= nbound) return;
-  const double g = 0.25 * panelbar[p];
+  sol0bar += blockIdx.y * scs;  // component
+  const double g = 0.25 * panelbar[(size_t)blockIdx.y * nbound + p];
   if (g == 0.0) return;
   const double a[5] = {25.0 / 12.0, -4.0, 3.0, -4.0 / 3.0, 0.25};
   const int f = face[p];
@@ -1544,8 +1575,8 @@ __global__ void k_normal_deriv_T(const double* __restrict__ panelbar, int NX, in
 void boundary_transpose_prepare(BoundaryOp& B, cudaStream_t s) {
   if (B.ff.on && !B.precomputed) boundary_record(B, s);
   if (B.precomputed) {  // at set-up: the transposes may be captured in graphs
-    B.vff.ensure((size_t)B.ntarget);
-    if (B.dense) B.dpart.ensure((size_t)B.ntopd * (((B.ntarget + 31) / 32 + kDenseTGroup - 1) / kDenseTGroup));
+    B.vff.ensure(4 * (size_t)B.ntarget);
+    if (B.dense) B.dpart.ensure(3 * (size_t)B.ntopd * (((B.ntarget + 31) / 32 + kDenseTGroup - 1) / kDenseTGroup));
   }
   if (!B.precomputed || B.transposed || B.nnz == 0) return;
   const long long need = B.nnz * (long long)(sizeof(int) + sizeof(float2)) + 8LL * (B.ncell_total + 1);
@@ -1584,71 +1615,72 @@ void boundary_transpose_prepare(BoundaryOp& B, cudaStream_t s) {
 }
 
 template <class M>
-static void apply_T_recorded(BoundaryOp& B, const double* bcbar, double* cellbar, cudaStream_t s) {
+static void apply_T_recorded(BoundaryOp& B, const double* bcbar, size_t bcs, double* cellbar, cudaStream_t s) {
   using V = typename M::V;
+  using H = typename M::H;
   using W = typename M::W;
   const double scale = -1.0 / (4.0 * kPI);
   V* vv = reinterpret_cast<V*>(B.vff.p);
+  const H* vh = reinterpret_cast<const H*>(B.vff.p);
   if (B.transposed || B.dense) {
-    VPMG_CHECK(B.vff.n >= (size_t)B.ntarget, VPMG_ERR_STATE, "boundary transpose not prepared");
-    k_split_bc<M><<<(B.ntarget + 255) / 256, 256, 0, s>>>(bcbar, B.tgt_node.p, B.ntarget, vv);
+    VPMG_CHECK(B.vff.n >= 4 * (size_t)B.ntarget, VPMG_ERR_STATE, "boundary transpose not prepared");
+    k_split_bc<M><<<(B.ntarget + 255) / 256, 256, 0, s>>>(bcbar, bcs, B.tgt_node.p, B.ntarget, vv);
     VPMG_LAUNCHED();
   }
-  auto dense_T = [&] {
-    if (!B.dense) return;
-    const int ngroup = ((B.ntarget + 31) / 32 + kDenseTGroup - 1) / kDenseTGroup;
-    VPMG_CHECK(B.dpart.n >= (size_t)ngroup * B.ntopd, VPMG_ERR_STATE, "boundary transpose not prepared");
-    const long long threads = (long long)B.ntopd * ngroup * 32;
-    k_dense_T<M><<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(reinterpret_cast<const W*>(B.wtop.p), vv, B.ntopd,
-                                                                  B.ntarget, B.dpart.p);
-    VPMG_LAUNCHED();
-    k_dense_T_sum<<<(B.ntopd + 255) / 256, 256, 0, s>>>(B.dpart.p, B.ntopd, ngroup, B.lev_off[B.levmax], scale,
-                                                         cellbar);
-    VPMG_LAUNCHED();
-  };
   if (B.transposed) {
     const long long threads = (long long)B.ncell_total * 32;
-    k_csc_T<M><<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(B.colptr.p, B.trow.p,
-                                                                 reinterpret_cast<const W*>(B.tw.p), vv,
-                                                                 B.ncell_total, scale, cellbar);
+    k_csc_T<M><<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(
+        B.colptr.p, B.trow.p, reinterpret_cast<const W*>(B.tw.p), vh, B.ncell_total, scale, cellbar);
     VPMG_LAUNCHED();
-    dense_T();
-    return;
+  } else {
+    VPMG_CUDA(cudaMemsetAsync(cellbar, 0, 3 * sizeof(double) * B.ncell_total, s));
+    const long long threads = (long long)B.ntarget * 32;
+    for (int c = 0; c < 3; ++c) {
+      k_csr_T<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(
+          B.rowptr.p, B.col.p, reinterpret_cast<const double*>(B.w.p), M::kFF ? 1 : 0, B.tgt_node.p, B.ntarget, scale,
+          bcbar + c * bcs, cellbar + (size_t)c * B.ncell_total);
+      VPMG_LAUNCHED();
+    }
   }
-  VPMG_CUDA(cudaMemsetAsync(cellbar, 0, sizeof(double) * B.ncell_total, s));
-  const long long threads = (long long)B.ntarget * 32;
-  k_csr_T<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(B.rowptr.p, B.col.p,
-                                                            reinterpret_cast<const double*>(B.w.p),
-                                                            M::kFF ? 1 : 0, B.tgt_node.p, B.ntarget, scale, bcbar,
-                                                            cellbar);
+  if (!B.dense) return;
+  const int ngroup = ((B.ntarget + 31) / 32 + kDenseTGroup - 1) / kDenseTGroup;
+  VPMG_CHECK(B.dpart.n >= 3 * (size_t)ngroup * B.ntopd, VPMG_ERR_STATE, "boundary transpose not prepared");
+  const long long threads = (long long)B.ntopd * ngroup * 32;
+  k_dense_T<M><<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(reinterpret_cast<const W*>(B.wtop.p), vh, B.ntopd,
+                                                                B.ntarget, B.dpart.p);
   VPMG_LAUNCHED();
-  dense_T();
+  k_dense_T_sum<<<dim3((B.ntopd + 255) / 256, 3), 256, 0, s>>>(B.dpart.p, B.ntopd, ngroup, B.lev_off[B.levmax], scale,
+                                                               cellbar, (size_t)B.ncell_total);
+  VPMG_LAUNCHED();
 }
 
-void boundary_apply_T(BoundaryOp& B, const double* bcbar, double* cellbar, cudaStream_t s) {
+void boundary_apply_T(BoundaryOp& B, const double* bcbar, size_t bcs, double* cellbar, cudaStream_t s) {
   if (B.precomputed) {
-    if (B.arith == VPMG_ARITH_FF48) apply_T_recorded<MacFF>(B, bcbar, cellbar, s);
-    else apply_T_recorded<Mac64>(B, bcbar, cellbar, s);
+    if (B.arith == VPMG_ARITH_FF48) apply_T_recorded<MacFF>(B, bcbar, bcs, cellbar, s);
+    else apply_T_recorded<Mac64>(B, bcbar, bcs, cellbar, s);
   } else {
-    VPMG_CUDA(cudaMemsetAsync(cellbar, 0, sizeof(double) * B.ncell_total, s));
+    VPMG_CUDA(cudaMemsetAsync(cellbar, 0, 3 * sizeof(double) * B.ncell_total, s));
     VPMG_CHECK(B.wnodes.p, VPMG_ERR_STATE, "boundary operator without its walk order");
     const WalkDev W = walk_dev(B, walk_segments(B));
-    walk_launch<kTranspose>(B, W, cellbar, const_cast<double*>(bcbar), nullptr, nullptr, nullptr, nullptr, nullptr,
-                            nullptr, nullptr, s);
+    for (int c = 0; c < 3; ++c)
+      walk_launch<kTranspose>(B, W, cellbar + (size_t)c * B.ncell_total, const_cast<double*>(bcbar + c * bcs), nullptr,
+                              nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, s);
   }
   VPMG_CUDA(cudaGetLastError());
 }
 
 void boundary_agg_T(BoundaryOp& B, const double* cellbar, double* panelbar, cudaStream_t s) {
-  k_agg_T<<<(B.nbound + 255) / 256, 256, 0, s>>>(B.anc.p, B.cds.p, B.nbound, B.levmax, cellbar, panelbar);
+  k_agg_T<<<dim3((B.nbound + 255) / 256, 3), 256, 0, s>>>(B.anc.p, B.cds.p, B.nbound, B.levmax, cellbar, panelbar,
+                                                          (size_t)B.ncell_total);
   VPMG_LAUNCHED();
   VPMG_CUDA(cudaGetLastError());
 }
 
-void boundary_panels_T(BoundaryOp& B, const Grid& g, const double* panelbar, double* sol0bar, cudaStream_t s) {
-  k_normal_deriv_T<<<(B.nbound + 255) / 256, 256, 0, s>>>(panelbar, g.n[0], g.n[1], B.pan_face.p, B.pan_i.p, B.pan_j.p,
-                                                          B.pan_k.p, B.nbound, 1.0 / g.d[0], 1.0 / g.d[1],
-                                                          1.0 / g.d[2], sol0bar);
+void boundary_panels_T(BoundaryOp& B, const Grid& g, const double* panelbar, double* sol0bar, size_t scs,
+                       cudaStream_t s) {
+  k_normal_deriv_T<<<dim3((B.nbound + 255) / 256, 3), 256, 0, s>>>(
+      panelbar, g.n[0], g.n[1], B.pan_face.p, B.pan_i.p, B.pan_j.p, B.pan_k.p, B.nbound, 1.0 / g.d[0], 1.0 / g.d[1],
+      1.0 / g.d[2], sol0bar, scs);
   VPMG_LAUNCHED();
   VPMG_CUDA(cudaGetLastError());
 }

@@ -340,14 +340,14 @@ void boundary_group_apply(const BoundaryOp& L, const float2* gsrc, int nprob, do
                           cudaStream_t s);
 // Transposes (one component): boundary-value adjoint (grid node array) ->
 // cell adjoints -> panel adjoints -> accumulated into the sol0 adjoint.
-void boundary_apply_T(BoundaryOp& B, const double* bcbar, double* cellbar, cudaStream_t s);
+void boundary_apply_T(BoundaryOp& B, const double* bcbar, size_t bcs, double* cellbar, cudaStream_t s);
 // Builds the transposed interaction list when the operator is recorded and
 // the copy fits in half of the free device memory (set-up time, outside
 // stream capture); boundary_apply_T then gathers per cell instead of
 // scattering with atomics.
 void boundary_transpose_prepare(BoundaryOp& B, cudaStream_t s);
 void boundary_agg_T(BoundaryOp& B, const double* cellbar, double* panelbar, cudaStream_t s);
-void boundary_panels_T(BoundaryOp& B, const Grid& g, const double* panelbar, double* sol0bar, cudaStream_t s);
+void boundary_panels_T(BoundaryOp& B, const Grid& g, const double* panelbar, double* sol0bar, size_t scs, cudaStream_t s);
 
 // ---------------------------------------------------- small kernels ----
 void fill_zero(double* p, size_t n, cudaStream_t s);
