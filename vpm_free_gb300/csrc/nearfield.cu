@@ -37,8 +37,13 @@
 // Tile: M = 128 runs, N = 64 nodes: seven 64-column accumulators fill 448 of
 // the 512 tensor-memory columns.  K = 16 per stage (43 KB: 28 KB of source
 // digits gathered by 16-byte asynchronous copies, 14 KB of table by one bulk
-// copy), four stages.  Bound: the issue of 28 products per stage (about 50
-// clocks each at N = 64) with the L2 reads of the digits close behind.
+// copy), five stages.  The products alone take about 53 clocks each at N = 64
+// (their operands' shared-memory reads), 1480 a stage; reading the sums every
+// 16 stages, when the tensor core waits, 400 more (57 thousand conversions to
+// integers at 16 per clock).  One warp each for the products and the tables
+// beside the gathering ones took the 81^3 block of a 64^3 step from 358 to
+// 283 us and the 273^3 block of a 256^3 step from 1.50 to 1.21 ms; with one
+// barrier of all threads per stage the next gather waited for the products.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -51,8 +56,10 @@ namespace vpmg {
 
 namespace {
 
-constexpr int kThreads = 256;
-constexpr int kStages = 4;
+constexpr int kWorkers = 256;               // threads that gather the sources and read the sums
+constexpr int kThreads = kWorkers + 64;     // and a warp each for the tables and the products
+constexpr int kStages = 5;
+constexpr int kLag = 3;                     // stages whose copies a worker has in flight
 constexpr int kDigits = kNearDigits;
 constexpr int kRunsM = 128;   // runs per tile
 constexpr int kCols = kNearCols;  // nodes per tile
@@ -180,127 +187,186 @@ struct MmaArgs {
   const unsigned char* table;
   const unsigned short* dig;
   unsigned long long* acc;
-  int* counter;   // next unit; counter[1]: a wait ran out
+  int* failed;   // a wait ran out
 };
 
+// Units are dealt longest first, forth and back over the CTAs.  Warps 0..7
+// gather the sources' digits and, at the end of a group of stages, read the
+// sums; warp 8 loads the tables, warp 9 issues the products.  They meet in
+// mbarriers only, and the gathers run ahead of the products across the ends of
+// groups and units.
 __global__ void __launch_bounds__(kThreads, 1) k_near_mma(const __grid_constant__ MmaArgs P) {
   extern __shared__ unsigned char near_sm[];
-  __shared__ __align__(8) uint64_t bars[2 * kStages];
+  __shared__ __align__(8) uint64_t bars[2 * kStages + 2];
   __shared__ uint32_t tslot;
-  __shared__ int next_unit;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t sm = (tc05::smem_u32(near_sm) + 1023u) & ~1023u;
-  const uint32_t full = tc05::smem_u32(bars), empty = full + 8 * kStages;
+  const uint32_t full = tc05::smem_u32(bars), empty = full + 8 * kStages, done = full + 16 * kStages, unread = done + 8;
   if (warp == 0) tc05::tmem_alloc(tc05::smem_u32(&tslot), 512);
   if (tid == 0) {
-    for (int i = 0; i < 2 * kStages; ++i) tc05::bar_init(full + 8 * i, 1);
+    for (int i = 0; i < kStages; ++i) {
+      tc05::bar_init(full + 8 * i, kWorkers / 32 + 1);  // the gathering warps and the table's copy
+      tc05::bar_init(empty + 8 * i, 1);
+    }
+    tc05::bar_init(done, 1);
+    tc05::bar_init(unread, kWorkers / 32);
     tc05::bar_init_fence();
   }
   tc05::fence_before();
   __syncthreads();
   tc05::fence_after();
   const uint32_t tb = tslot;
-  bool dead = false;
-  uint32_t g0 = 0;  // stages used by earlier units
-  const int r = tid >> 1, kg = tid & 1;  // this thread's run and 8-cell group of a stage
-  const uint32_t adst = (uint32_t)((kg * kRunsM + r) * 16);
   constexpr uint32_t idesc = tc05::idesc_f16(kRunsM, kCols);
-  for (;;) {
-    __syncthreads();
-    if (tid == 0) next_unit = atomicAdd(P.counter, 1);
-    __syncthreads();
-    const int u = next_unit;
-    if (u >= P.nunit) break;
-    const NearUnit U = P.units[u];
-    const bool live = r < U.nrun;
-    NearRow R{};
-    if (live) R = P.rows[U.row0 + r];
-    const int nst = U.k1 - U.k0;
-    auto issue = [&](int k) {  // copies of stage k of this unit
-      const uint32_t g = g0 + (uint32_t)k, st = g % kStages;
-      if (g >= (uint32_t)kStages) tc05::bar_wait(empty + 8 * st, ((g / kStages) - 1) & 1, dead, P.counter + 1);
-      const uint32_t base = sm + st * kStageBytes;
-      if (tid == 0) {
-        tc05::bar_expect(full + 8 * st, kBytesB);
-        tc05::bulk_load(base + kBytesA, P.table + U.table + (size_t)(U.k0 + k) * kBytesB, kBytesB, full + 8 * st);
+  bool dead = false;
+  auto unit_of = [&](int i) {  // this CTA's i-th unit
+    const long long u = (long long)i * gridDim.x + ((i & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
+    return u < P.nunit ? (int)u : -1;
+  };
+  if (warp == kWorkers / 32) {
+    if (lane == 0) {  // the tables
+      uint32_t g = 0;
+      for (int i = 0, u; (u = unit_of(i)) >= 0; ++i) {
+        const NearUnit U = P.units[u];
+        const unsigned char* src = P.table + U.table + (size_t)U.k0 * kBytesB;
+        for (int k = U.k0; k < U.k1; ++k, ++g, src += kBytesB) {
+          const uint32_t st = g % kStages;
+          if (g >= (uint32_t)kStages) tc05::bar_wait(empty + 8 * st, ((g / kStages) - 1) & 1, dead, P.failed);
+          tc05::bar_expect(full + 8 * st, kBytesB);
+          tc05::bulk_load(sm + st * kStageBytes + kBytesA, src, kBytesB, full + 8 * st);
+        }
       }
-      const unsigned e = __ldg(&P.klist[U.klist + U.k0 + k]);
-      const int row = R.row0 + R.rs * (int)(e >> 8), cell = R.wst + 16 * (int)(e & 255u) + 8 * kg;
-      const bool ok = live && row >= 0 && row < R.nrow && cell >= 0 && cell < R.Wp;
-      const unsigned short* src = P.dig + (ok ? R.abase + (long long)row * R.Wp + cell : 0);
-      const long long ds = ok ? (long long)R.nrow * R.Wp : 0;
+    }
+    __syncwarp();
+  } else if (warp > kWorkers / 32) {
+    if (lane == 0) {  // the products
+      uint32_t g = 0, groups = 0;
+      for (int i = 0, u; (u = unit_of(i)) >= 0; ++i) {
+        const int nst = P.units[u].k1 - P.units[u].k0;
+        for (int k = 0; k < nst; ++k, ++g) {
+          const uint32_t st = g % kStages;
+          const int kin = k % P.group;
+          if (kin == 0 && groups > 0) tc05::bar_wait(unread, (groups - 1) & 1, dead, P.failed);
+          tc05::bar_wait(full + 8 * st, (g / kStages) & 1, dead, P.failed);
+          tc05::fence_after();
+          const uint32_t base = sm + st * kStageBytes;
+          const uint64_t da = tc05::desc(base, kRunsM * 16), db = tc05::desc(base + kBytesA, kCols * 16);
 #pragma unroll
-      for (int j = 0; j < kDigits; ++j) tc05::cp16(base + j * (2 * kRunsM * 16) + adst, src + j * ds, ok);
+          for (int w = 0; w < kDigits; ++w)
+#pragma unroll
+            for (int j = 0; j < kDigits - w; ++j)
+              tc05::mma(tb + (w + j) * kCols, da + (uint64_t)(j * (2 * kRunsM * 16 >> 4)),
+                        db + (uint64_t)(w * (2 * kCols * 16 >> 4)), idesc, (w > 0 || kin > 0) ? 1u : 0u);
+          tc05::commit(empty + 8 * st);
+          if (kin == P.group - 1 || k == nst - 1) {
+            tc05::commit(done);
+            ++groups;
+          }
+        }
+      }
+    }
+    __syncwarp();
+  } else {
+    // this thread's run and 8-cell group of a stage: eight neighbouring threads write 128 bytes
+    const int r = 16 * warp + (lane & 15), kg = lane >> 4;
+    const uint32_t adst = (uint32_t)((kg * kRunsM + r) * 16);
+    // the gathers' place: unit, its stages, its run
+    int ii = 0, iu = unit_of(0), ik = 0, in = 0;
+    NearRow R{};
+    const unsigned* kl = nullptr;
+    unsigned e = 0;
+    auto enter = [&] {
+      if (iu < 0) return;
+      const NearUnit U = P.units[iu];
+      ik = 0;
+      in = U.k1 - U.k0;
+      kl = P.klist + U.klist + U.k0;
+      e = __ldg(kl);
+      R = NearRow{};
+      if (r < U.nrun) R = P.rows[U.row0 + r];  // else no source row (nrow = 0)
     };
+    enter();
+    // the sums' place
+    int ai = 0, au = iu, ak = 0, an = in, q = au >= 0 ? P.units[au].q : 0;
+    uint32_t g = 0, ga = 0, groups = 0;
     long long sum[32];
 #pragma unroll
     for (int i = 0; i < 32; ++i) sum[i] = 0;
+    for (int step = 0; au >= 0; ++step) {
+      if (iu >= 0) {
+        const uint32_t st = g % kStages;
+        const int row = R.row0 + R.rs * (int)(e >> 8), cell = R.wst + 16 * (int)(e & 255u) + 8 * kg;
+        const bool ok = row >= 0 && row < R.nrow && cell >= 0 && cell < R.Wp;
+        const unsigned short* src = P.dig + (ok ? R.abase + (long long)row * R.Wp + cell : 0);
+        const long long ds = ok ? (long long)R.nrow * R.Wp : 0;
+        if (ik + 1 < in) e = __ldg(kl + ik + 1);
+        if (g >= (uint32_t)kStages) tc05::bar_wait(empty + 8 * st, ((g / kStages) - 1) & 1, dead, P.failed);
+        const uint32_t dst = sm + st * kStageBytes + adst;
 #pragma unroll
-    for (int k = 0; k < kStages - 1; ++k) {
-      if (k < nst) issue(k);
-      tc05::cp_commit();
-    }
-    for (int k = 0; k < nst; ++k) {
-      tc05::cp_wait<kStages - 2>();
-      tc05::fence_async();
-      __syncthreads();
-      const uint32_t g = g0 + (uint32_t)k, st = g % kStages;
-      const int kin = k % P.group;
-      if (tid == 0) {
-        tc05::bar_wait(full + 8 * st, (g / kStages) & 1, dead, P.counter + 1);
-        tc05::fence_after();
-        const uint32_t base = sm + st * kStageBytes;
-        const uint64_t da = tc05::desc(base, kRunsM * 16), db = tc05::desc(base + kBytesA, kCols * 16);
-#pragma unroll
-        for (int i = 0; i < kDigits; ++i)
-#pragma unroll
-          for (int j = 0; j < kDigits - i; ++j)
-            tc05::mma(tb + (i + j) * kCols, da + (uint64_t)(j * (2 * kRunsM * 16 >> 4)),
-                      db + (uint64_t)(i * (2 * kCols * 16 >> 4)), idesc, (i > 0 || kin > 0) ? 1u : 0u);
-        tc05::commit(empty + 8 * st);
-      }
-      if (kin == P.group - 1 || k == nst - 1) {
-        // the group's exact sums join the running integers
-        tc05::bar_wait(empty + 8 * st, (g / kStages) & 1, dead, P.counter + 1);
-        tc05::fence_after();
-        const uint32_t ta = tb + ((uint32_t)(32 * (warp & 3)) << 16) + 32 * (warp >> 2);
-        const int q = U.q;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          uint32_t v[kDigits][8];
-#pragma unroll
-          for (int d = 0; d < kDigits; ++d) tc05::ld8(ta + d * kCols + 8 * c, v[d]);
-          tc05::ld_wait();
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            auto n = [&](int d) { return (long long)__float2int_rn(__uint_as_float(v[d][i])); };
-            const long long hi = (n(0) << 32) + (n(1) << 24) + (n(2) << 16) + (n(3) << 8) + n(4);
-            const long long lo = (n(5) << 8) + n(6);
-            sum[8 * c + i] += (hi << (16 - q)) + ((lo + ((1ll << q) >> 1)) >> q);
-          }
+        for (int j = 0; j < kDigits; ++j) tc05::cp16(dst + j * (2 * kRunsM * 16), src + j * ds, ok);
+        ++g;
+        if (++ik == in) {
+          iu = unit_of(++ii);
+          enter();
         }
-        tc05::fence_before();
-        __syncthreads();  // every warp has read before the next products overwrite
-        tc05::fence_after();
       }
-      if (k + kStages - 1 < nst) issue(k + kStages - 1);
       tc05::cp_commit();
-    }
-    g0 += (uint32_t)nst;
-    // row `run` of the tile, columns 32 (warp / 4) ..
-    const int run = 32 * (warp & 3) + lane;
-    if (run < U.nrun) {
-      const NearRow O = P.rows[U.row0 + run];
-      const long long half = (1ll << U.sh) >> 1;
+      if (step < kLag) continue;
+      // the copies of kLag steps ago are in
+      tc05::cp_wait<kLag>();
+      tc05::fence_async();
+      __syncwarp();
+      if (lane == 0) tc05::bar_arrive(full + 8 * (ga % kStages));
+      ++ga;
+      ++ak;
+      if (ak % P.group != 0 && ak != an) continue;
+      // the group's exact sums join the running integers
+      tc05::bar_wait(done, groups & 1, dead, P.failed);
+      ++groups;
+      tc05::fence_after();
+      const uint32_t ta = tb + ((uint32_t)(32 * (warp & 3)) << 16) + 32 * (warp >> 2);
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const int n = U.col0 + 32 * (warp >> 2) + i;
-        const int tr = n / U.TB, tw = n - tr * U.TB;
-        if (tr < O.rlim && tw < O.wlim)
-          atomicAdd(&P.acc[O.obase + (long long)tr * O.ostr_r + (long long)tw * O.ostr_w],
-                    (unsigned long long)((sum[i] + half) >> U.sh));
+      for (int c = 0; c < 8; ++c) {
+        uint32_t v[kDigits][4];
+#pragma unroll
+        for (int d = 0; d < kDigits; ++d) tc05::ld4(ta + d * kCols + 4 * c, v[d]);
+        tc05::ld_wait();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          auto n = [&](int d) { return (long long)__float2int_rn(__uint_as_float(v[d][i])); };
+          const long long hi = (n(0) << 32) + (n(1) << 24) + (n(2) << 16) + (n(3) << 8) + n(4);
+          const long long lo = (n(5) << 8) + n(6);
+          sum[4 * c + i] += (hi << (16 - q)) + ((lo + ((1ll << q) >> 1)) >> q);
+        }
+      }
+      tc05::fence_before();
+      __syncwarp();
+      if (lane == 0) tc05::bar_arrive(unread);  // the next products may overwrite
+      if (ak != an) continue;
+      // row `run` of the tile, columns 32 (warp / 4) ..
+      const NearUnit U = P.units[au];
+      const int run = 32 * (warp & 3) + lane;
+      if (run < U.nrun) {
+        const NearRow O = P.rows[U.row0 + run];
+        const long long half = (1ll << U.sh) >> 1;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          const int n = U.col0 + 32 * (warp >> 2) + i;
+          const int tr = n / U.TB, tw = n - tr * U.TB;
+          if (tr < O.rlim && tw < O.wlim)
+            atomicAdd(&P.acc[O.obase + (long long)tr * O.ostr_r + (long long)tw * O.ostr_w],
+                      (unsigned long long)((sum[i] + half) >> U.sh));
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 32; ++i) sum[i] = 0;
+      au = unit_of(++ai);
+      ak = 0;
+      if (au >= 0) {
+        an = P.units[au].k1 - P.units[au].k0;
+        q = P.units[au].q;
       }
     }
+    tc05::cp_wait<0>();
   }
   __syncthreads();
   if (warp == 0) tc05::tmem_free(tb, 512);
@@ -522,7 +588,7 @@ bool near_prepare(BoundaryOp& B, const Grid& g, long long budget_bytes, cudaStre
   F.table.ensure(std::max<size_t>((size_t)tbytes, 16));
   F.dig.ensure((size_t)nd + 64);
   VPMG_CUDA(cudaMemsetAsync(F.dig.p, 0, F.dig.bytes(), s));
-  F.acc.ensure((size_t)na + 1);  // the sums, then the unit counter and the failure flag
+  F.acc.ensure((size_t)na + 1);  // the sums, then the failure flag (second int)
   std::vector<size_t> col0(nt + 1, 0);  // first node of each table in wsum
   for (int t = 0; t < nt; ++t) col0[t + 1] = col0[t] + (size_t)tabs[t].nchunk * kCols;
   DBuf<unsigned long long> wsum;
@@ -672,7 +738,7 @@ bool near_prepare(BoundaryOp& B, const Grid& g, long long budget_bytes, cudaStre
 // acc[face][component][v][u] = the near field's integers of every face node.
 void near_apply(BoundaryOp& B, cudaStream_t s) {
   NearField& F = B.near;
-  VPMG_CUDA(cudaMemsetAsync(F.acc.p, 0, F.acc.bytes(), s));  // and the two counters behind the sums
+  VPMG_CUDA(cudaMemsetAsync(F.acc.p, 0, F.acc.bytes(), s));  // and the flag behind the sums
   DigitsDev D{};
   for (int l = 0; l <= B.levmax; ++l) {
     D.lev[l] = B.lev_off[l];
@@ -700,7 +766,7 @@ void near_apply(BoundaryOp& B, cudaStream_t s) {
   A.table = F.table.p;
   A.dig = F.dig.p;
   A.acc = F.acc.p;
-  A.counter = reinterpret_cast<int*>(F.acc.p + F.nacc);
+  A.failed = reinterpret_cast<int*>(F.acc.p + F.nacc) + 1;
   k_near_mma<<<std::min(F.nunit, F.sms), kThreads, kSmem, s>>>(A);
   VPMG_LAUNCHED();
   VPMG_CUDA(cudaGetLastError());
