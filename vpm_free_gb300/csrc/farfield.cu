@@ -36,6 +36,7 @@ namespace {
 constexpr int kFFThreads = 128;
 constexpr int kFFJobs = 24;
 constexpr int kMinTargets = 12000;
+constexpr int kMinTargetsFF = 60000;
 constexpr int kFFSmem = 48 * 1024;  // dynamic shared memory of the line kernel
 
 // in-plane axes of face f (normal f / 2): the panels' fast and slow axes
@@ -444,12 +445,17 @@ bool farfield_prepare(BoundaryOp& B, const Grid& g, cudaStream_t s) {
   FarField& F = B.ff;
   const char* env = std::getenv("VPMG_FARFIELD");
   if (env && env[0] == '0') return false;
-  if (B.arith != VPMG_ARITH_FP64 || B.ibctyp != 2 || !B.tree || B.levmax < 1 || B.budget <= 0) return false;
+  if (B.ibctyp != 2 || !B.tree || B.levmax < 1 || B.budget <= 0) return false;
   // small operators (the coarse grids, up to 9.6 thousand nodes at 41^3) are
   // faster as recorded rows, which take two launches instead of twelve: with
   // the coarse grid recorded a 64^3 step takes 1.94 ms and a 32^3 driver call
-  // 1.23 ms, by FFT and tables 1.99 and 1.31 ms
-  if (B.ntarget < kMinTargets) return false;
+  // 1.23 ms, by FFT and tables 1.99 and 1.31 ms.  Float-float rows (their sums
+  // run on the FP32 units) hold out longer: a step of the ring takes 1.44 ms
+  // with them and 1.47 by FFT and tables at 64^3 (39 thousand nodes), 2.58 and
+  // 2.34 at 96^3 (86 thousand), and of the leapfrogging rings 23.3 and 17.7 at
+  // 256^3.  The transforms and tables are FP64 and 55-bit integers in either
+  // arithmetic.
+  if (B.ntarget < (B.arith == VPMG_ARITH_FF48 ? kMinTargetsFF : kMinTargets)) return false;
   const int istep = 1 << B.levmax;
   for (int a = 0; a < 3; ++a)
     if ((g.n[a] - 1) % istep != 0 || g.n[a] - 1 <= istep) return false;  // dummy cells at the coarsest level

@@ -280,14 +280,14 @@ struct BoundaryOp {
   DBuf<int> toppos;
   int walkseg = 1;
   DBuf<double> walkpart;                // [segment][3][ntarget] partial sums
-  FarField ff;                          // the coarsest level by FFT (FP64, uniform lattices) ...
+  FarField ff;                          // the coarsest level by FFT (uniform lattices) ...
   NearField near;                       // ... with the opened cells of every level by tables
   long long bytes() const;
 };
 void boundary_prepare(BoundaryOp& B, const Grid& g, int levmax, long long budget_bytes, cudaStream_t s,
                       int ibctyp, bool tree, int arith, bool once = false);  // once: applied a single time
 // Sets B.ff and B.near up (the operator needs no recorded rows then) when the
-// cells of every level form uniform lattices on every face (FP64, ibctyp 2,
+// cells of every level form uniform lattices on every face (ibctyp 2,
 // tree) and VPMG_FARFIELD is not "0"; set-up time, outside stream capture.
 bool farfield_prepare(BoundaryOp& B, const Grid& g, cudaStream_t s);
 bool near_prepare(BoundaryOp& B, const Grid& g, long long budget_bytes, cudaStream_t s);
