@@ -421,10 +421,10 @@ def run_dirichlet(args, local):
 
 
 KERNELS = (  # vpmg_bench_kernel ids: (id, name, launches per step); the first word keys profiles/traffic.json
-    (0, "boundary (the fine block's operator: coarsest level by FFT k_ff_* or the dense block k_apply_dense, "
-        "finer levels and corrections k_apply_csr)", 1),
-    (1, "inner-box Dirichlet solve (k_dst_x_fwd, k_dst_y x2, k_thomas, k_dst_x_inv)", 3),
-    (6, "padded-block zero-BC solve where read (k_dst_x_fwd, k_dst_y, k_thomas_faces, k_partial_x/y, "
+    (0, "boundary (the fine block's operator: coarsest level by FFT k_ff_*, opened cells by tables k_near_mma, or "
+        "recorded rows k_apply_dense, k_apply_csr)", 1),
+    (1, "inner-box Dirichlet solve (k_dst_mma or k_dst_x_fwd, k_dst_y, k_dst_x_inv; k_thomas_ends)", 3),
+    (6, "padded-block zero-BC solve where read (k_dst_mma or k_dst_*, k_thomas_ends, k_partial_x/y, "
         "partial inverses)", 3),
     (2, "k_deposit (M4' gather deposition; field step and remesh)", 2),
     (5, "k_m2p (mesh-to-particle gather + Euler)", 1),

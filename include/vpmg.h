@@ -203,14 +203,19 @@ long long vpmg_kernel_launches(const vpmg_handle* h);
  * [0] deposit, [1] fine zero-BC solve, [2] boundary values, [3] fine BC
  * solve, [4] coarse, [5] final solve, [6] FD, [7] M2P+Euler, [8] remesh. */
 int vpmg_phase_times(const vpmg_handle* h, double ms[9]);
-/* Boundary-operator statistics: interactions per fine solve, bytes held. */
+/* Boundary-operator statistics: interactions per fine solve, bytes held,
+ * and whether the interaction lists are recorded (0 while the operator goes
+ * by FFT and tables: the reverse mode records them on its first use; also 0
+ * when it walks the tree).                                              */
 int vpmg_tree_stats(const vpmg_handle* h, long long* interactions, long long* bytes, int* precomputed);
 /* Whether the fine block's operator evaluates its coarsest tree level by
- * FFT convolutions on the face lattices (FP64 handles whose coarsest cells
- * form uniform lattices; VPMG_FARFIELD=0 at set-up keeps the dense block),
- * its correction entries (the coarsest cells the walk opened) and the
- * FP64 flops of one apply of the FFT part.  Instrumentation; no counterpart
- * in the reference.                                                     */
+ * FFT convolutions on the face lattices and the opened cells by weight
+ * tables on the tensor cores (operators of 12 thousand boundary nodes or
+ * more, 60 thousand in float-float, whose cells form uniform lattices;
+ * VPMG_FARFIELD=0 at set-up records the lists instead), its correction
+ * entries (cells that the walk and the lattice rule take differently) and
+ * the FP64 flops of one apply of the FFT part.  Instrumentation; no
+ * counterpart in the reference.                                         */
 int vpmg_farfield_stats(const vpmg_handle* h, int* on, long long* corrections, double* flops);
 /* Per-phase event timing: 0 off (default), 1 on; 2 also keeps the
  * intermediate block fields readable by vpmg_get_field and evaluates the
@@ -296,8 +301,8 @@ int vpmg_fp64_peak(vpmg_handle* h, double* tflops);
  * or 8) of the padded block's x and y transforms, the inner box's and the
  * coarse grid's, in that order.                                         */
 int vpmg_dst_tiles(const vpmg_handle* h, int pairs[6]);
-/* Memory limit (bytes) for the precomputed boundary operator; 0 = never
- * precompute (walk the tree every step).  Default: 100 GiB.              */
+/* Memory limit (bytes) for the boundary operator's tables or recorded
+ * lists; 0 = neither (walk the tree every step).  Default: 100 GiB.      */
 int vpmg_set_operator_budget(vpmg_handle* h, long long bytes);
 
 /* ---- the reference's files ------------------------------------------- */

@@ -464,9 +464,10 @@ class VPM:
         return {"interactions": a.value, "bytes": b.value, "precomputed": bool(c.value)}
 
     def farfield_stats(self):
-        """{'on': the coarsest tree level goes by FFT convolutions, 'corrections':
-        opened coarsest cells subtracted as rows, 'flops': FP64 flops of one
-        apply of the FFT part}."""
+        """{'on': the coarsest tree level goes by FFT convolutions and the opened
+        cells by tables, 'corrections': cells that the walk and the lattice rule
+        take differently, kept as rows, 'flops': FP64 flops of one apply of the
+        FFT part}."""
         a, b, c = C.c_int(0), C.c_longlong(0), C.c_double(0.0)
         self._chk(self._L.vpmg_farfield_stats(self._h, C.byref(a), C.byref(b), C.byref(c)))
         return {"on": bool(a.value), "corrections": b.value, "flops": c.value}

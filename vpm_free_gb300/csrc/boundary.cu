@@ -13,18 +13,18 @@
 //     (pmbound.f90:1379-1501) and the untreed calc_boundinf_3d_s
 //     (pmbound.f90:520-648), whose unopened cells contribute the panel
 //     potential FSOUR_A4 (pmbound.f90:1540-1620) where the reference calls it.
-// The walk is evaluated with explicitly rounded operations so its opening
-// decisions are those of the reference's expressions.  Because the mesh is
-// frozen after the first step, the walk's interaction list (cell, dS/r) is
-// the same every step: when it fits the memory budget it is recorded once
-// (count + fill passes) and each step is a CSR product with the three
-// source components.  The product runs in float-float arithmetic: weights
-// and sources are stored as pairs of floats (hi + lo, a 48-bit mantissa),
-// products are split exactly with an FMA and sums are error-free
-// (two-sum), so the FP32 pipes, about thirty times GB300's FP64 rate, do
-// the work; each lane's partial sum is converted to FP64 before the warp
-// reduction.  The relative error stays near 1e-14, and the product is
-// bound by the 12 bytes per interaction it streams from HBM.
+// The walk's opening decisions are those of the reference's expressions.
+// Because the mesh is frozen after the first step, its interaction list
+// (cell, dS/r) is the same every step.  Operators on uniform lattices need no
+// list: every coarsest cell goes by FFT (farfield.cu) and the opened ones by
+// weight tables (nearfield.cu).  The others, small ones and the reverse mode's
+// transpose record it (count + fill passes) when it fits the memory budget:
+// each step is then a product with the three source components, the coarsest
+// level as a dense block and the finer ones as CSR rows, bound by the FP64
+// units (three FMAs per entry) or, in float-float (weights and sources as
+// pairs of floats, products split exactly with an FMA, error-free sums, relative
+// error near 1e-14), by the FP32 units and the 12 bytes per entry.  What does
+// not fit, or is applied once, walks.
 #include <algorithm>
 #include <climits>
 #include <cmath>
