@@ -15,7 +15,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 @pytest.fixture(scope="module")
-def checker(tmp_path_factory):
+def plan_program(tmp_path_factory):
     cxx = os.environ.get("CXX") or shutil.which("g++")
     if not cxx:
         pytest.skip("no C++ compiler")
@@ -34,13 +34,13 @@ def checker(tmp_path_factory):
     ((33, 25, 41), (0.1, 0.12, 0.09), 3),    # unequal spacings: tables of their own per pair of axes
     ((33, 65, 33), (0.05, 0.05, 0.07), 4),
 ])
-def test_plan_equals_the_direct_sum(checker, shape, h, levmax):
-    out = subprocess.run([checker, *map(str, shape), *map(str, h), str(levmax)], capture_output=True, text=True)
+def test_plan_equals_the_direct_sum(plan_program, shape, h, levmax):
+    out = subprocess.run([plan_program, *map(str, shape), *map(str, h), str(levmax)], capture_output=True, text=True)
     assert out.returncode == 0, out.stdout
     assert float(out.stdout) <= 1e-12
 
 
 @pytest.mark.parametrize("shape,levmax", [((27, 35, 30), 3), ((9, 17, 17), 3), ((18, 17, 17), 1)])
-def test_ragged_lattices_have_no_plan(checker, shape, levmax):
-    out = subprocess.run([checker, *map(str, shape), "0.1", "0.1", "0.1", str(levmax)], capture_output=True, text=True)
+def test_ragged_lattices_have_no_plan(plan_program, shape, levmax):
+    out = subprocess.run([plan_program, *map(str, shape), "0.1", "0.1", "0.1", str(levmax)], capture_output=True, text=True)
     assert out.returncode == 0 and out.stdout.strip() == "no plan"
