@@ -458,16 +458,8 @@ __global__ void __launch_bounds__(kDepWarps * 32) k_deposit64(const int* __restr
   r2[id] = b2 * inv_dv;
 }
 
-// Particles below which a particle takes four lanes: 16 warps per SM of one
-// particle per lane.
-constexpr int kFewParticles = 152 * 16 * 32;
-
 // FP64 mesh-to-particle over sorted slots: UP = sum W vel, GP = (sum W def)
 // * vol; optionally the forward Euler push.  6 DFMA per particle-node visit.
-// Fewer particles than kFewParticles leave SMs without the warps that hide
-// the gathers: four neighbouring lanes then share a particle, one z plane of
-// its nodes each, and add their sums (the 64^3 ring's 84 -> 73 us, the 32^3
-// ring's driver call 1148 -> 1123 us).
 __global__ void __launch_bounds__(128) k_m2p64(const int* __restrict__ perm, const int* __restrict__ nsorted_dev,
                                                const double* __restrict__ rec, size_t cs, MeshDev m,
                                                const double* __restrict__ v0, const double* __restrict__ v1,
@@ -480,10 +472,7 @@ __global__ void __launch_bounds__(128) k_m2p64(const int* __restrict__ perm, con
                                                const double* __restrict__ vol, int do_euler, double dt, double ux,
                                                double uy, double uz) {
   const int nsorted = *nsorted_dev;
-  const int sh = nsorted < kFewParticles ? 2 : 0, part = threadIdx.x & ((1 << sh) - 1);
-  const long long nt = (long long)nsorted << sh;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < nt; t += (long long)gridDim.x * blockDim.x) {
-    const int s = (int)(t >> sh);
+  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < nsorted; s += gridDim.x * blockDim.x) {
     const int p = perm[s];
     const double* r = rec + s;  // slot-major records (stride cs)
     double wx[4];
@@ -494,7 +483,7 @@ __global__ void __launch_bounds__(128) k_m2p64(const int* __restrict__ perm, con
     const int cj = (kk / m.n[0]) % m.n[1], ck = kk / (m.n[0] * m.n[1]);
     const int nw = m.ips + m.ipf + 1;
     double u[3] = {0.0, 0.0, 0.0}, gl[3] = {0.0, 0.0, 0.0};
-    for (int c = part; c < nw; c += 1 << sh) {
+    for (int c = 0; c < nw; ++c) {
       const int kk = ck - m.ips + c;
       for (int b = 0; b < nw; ++b) {
         const int jj = cj - m.ips + b;
@@ -513,17 +502,6 @@ __global__ void __launch_bounds__(128) k_m2p64(const int* __restrict__ perm, con
           gl[2] = fma(f, __ldg(&g2[id]), gl[2]);
         }
       }
-    }
-    if (sh) {
-      const unsigned mask = 0xFu << (threadIdx.x & 28);  // the particle's lanes
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        u[d] += __shfl_xor_sync(mask, u[d], 1);
-        u[d] += __shfl_xor_sync(mask, u[d], 2);
-        gl[d] += __shfl_xor_sync(mask, gl[d], 1);
-        gl[d] += __shfl_xor_sync(mask, gl[d], 2);
-      }
-      if (part) continue;
     }
     const double vp = vol[p];
     const double gg0 = gl[0] * vp, gg1 = gl[1] * vp, gg2 = gl[2] * vp;
