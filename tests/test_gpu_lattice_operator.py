@@ -1,0 +1,50 @@
+"""The boundary operator of uniform lattices, the coarsest level by FFT and the
+opened cells by weight tables (csrc/farfield.cu, csrc/nearfield.cu), against the
+recorded rows of the same operator (VPMG_FARFIELD=0), through a handle's
+vector-potential solve of seeded random right-hand sides.
+
+Both sum the same weights in another order and rounding: the tables hold them to
+2^-55 of the largest and the FFT adds a few units of 2^-53 per stage, so the
+solutions agree to 1e-13 in FP64; float-float rows keep 48 bits of each weight
+and source, 1e-12.
+"""
+import numpy as np
+import pytest
+
+from helpers import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+def _solve(V, monkeypatch, cells, h, tables, origin=(0.0, 0.0, 0.0), **cfg):
+    if tables:
+        monkeypatch.delenv("VPMG_FARFIELD", raising=False)
+    else:
+        monkeypatch.setenv("VPMG_FARFIELD", "0")
+    h = np.broadcast_to(np.asarray(h, dtype=np.float64), 3)
+    lo = np.asarray(origin, dtype=np.float64)
+    box = tuple(lo) + tuple(lo + np.asarray(cells) * h)
+    with V.VPM(V.VPMConfig.make(dpm=tuple(h), box=box, **cfg)) as H:
+        H.define_sizes(np.array([lo + 0.5 * np.asarray(cells) * h]))
+        r = np.random.default_rng(5).standard_normal(tuple(H._mesh_shape()))
+        return H.apply_poisson(r), H.farfield_stats()["on"]
+
+
+def _same(gpulib, monkeypatch, cells, h, **kw):
+    a, on = _solve(gpulib, monkeypatch, cells, h, True, **kw)
+    b, off = _solve(gpulib, monkeypatch, cells, h, False, **kw)
+    assert on and not off
+    for c in range(3):
+        assert rel_l2(a[c], b[c]) <= (1e-13 if gpulib.arith == "fp64" else 1e-12), (c, rel_l2(a[c], b[c]))
+
+
+# 48^3 cells: 25 thousand boundary nodes of the padded block; 96^3: 76 thousand,
+# where float-float handles take the tables too
+@pytest.mark.parametrize("h", [1.3e-5, 1e-5, 1e-6, 1.25e-7, 1e-8])
+def test_spacings_below_the_panel_distance(gpulib, monkeypatch, h):
+    """Cells within 1e-5 of a node weigh as a panel at its own centre: the nearest
+    leaf cells at 1.3e-5, whole levels below (distances of exactly 1e-5 among
+    them), and accepted coarsest cells at 1e-7 and less."""
+    if gpulib.arith != "fp64" and h != 1e-6:
+        pytest.skip("one spacing in float-float")
+    _same(gpulib, monkeypatch, (48,) * 3 if gpulib.arith == "fp64" else (96,) * 3, h)

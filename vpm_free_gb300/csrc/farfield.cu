@@ -50,13 +50,10 @@ struct AxisDev {
   const double2* tw;
 };
 
-// dS / r for the node-lattice offset (ex, ey, ez) = offset * spacing, with
-// every operation rounded explicitly so that all kernels (spectra and
-// correction rows) evaluate the same value; 0 at r = 0 (such a cell is
-// always opened, and its correction uses the same 0).
-__device__ __forceinline__ double ff_kern(double dS, double ex, double ey, double ez) {
-  const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(ex, ex), __dmul_rn(ey, ey)), __dmul_rn(ez, ez));
-  return r2 > 0.0 ? __ddiv_rn(dS, __dsqrt_rn(r2)) : 0.0;
+// Weight of a cell for the node-lattice offset o: that of the near field's
+// tables (lattice_weight), which take the opened cells back out.
+__device__ __forceinline__ double ff_kern(double dS, const int o[3], double hx, double hy, double hz) {
+  return lattice_weight(dS, (double)o[0], hx, (double)o[1], hy, (double)o[2], hz);
 }
 
 // signed offset of circular index e in a transform of length P
@@ -309,9 +306,7 @@ __global__ void k_ff_kpar_build(int Pu, int Pv, int axu, int axv, int axn, int d
     o[axu] = circ(u, Pu);
     o[axv] = circ(v, Pv);
     o[axn] = dn;
-    out[i] = make_double2(ff_kern(dS, __dmul_rn((double)o[0], hx), __dmul_rn((double)o[1], hy),
-                                  __dmul_rn((double)o[2], hz)),
-                          0.0);
+    out[i] = make_double2(ff_kern(dS, o, hx, hy, hz), 0.0);
   }
 }
 
@@ -329,9 +324,7 @@ __global__ void k_ff_kperp_build(int Nn, int Mc, int P, int ng, int nf, int w, i
     o[ng] = r - iG;
     o[nf] = iF - (c * istep + istep / 2);
     o[w] = circ(e, P);
-    out[i] = make_double2(ff_kern(dS, __dmul_rn((double)o[0], hx), __dmul_rn((double)o[1], hy),
-                                  __dmul_rn((double)o[2], hz)),
-                          0.0);
+    out[i] = make_double2(ff_kern(dS, o, hx, hy, hz), 0.0);
   }
 }
 

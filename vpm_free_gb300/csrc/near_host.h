@@ -78,6 +78,38 @@ VPMG_HD double lattice_weight(double ds, double r2) {
 #endif
 }
 
+// Whether an offset in nodes lies within 1e-5 of length, where the reference
+// takes a cell's potential at its own centre (tree_calc_3d, source/pmbound.f90:980-1249).
+// The squares are added by size, so that every order of the axes decides alike.
+VPMG_HD bool lattice_close(double a, double ha, double b, double hb, double n, double hn) {
+  const double x = rn_mul(a, ha), y = rn_mul(b, hb), z = rn_mul(n, hn);
+  const double u = rn_mul(x, x), v = rn_mul(y, y), w = rn_mul(z, z);
+  const double lo = u < v ? u : v, hi = u < v ? v : u;
+  const double mid = w < lo ? lo : (w < hi ? w : hi);
+  const double r2 = rn_add(rn_add(w < lo ? w : lo, mid), w < hi ? hi : w);
+#ifdef __CUDA_ARCH__
+  return !(__dsqrt_rn(r2) > 1e-05);
+#else
+  return !(std::sqrt(r2) > 1e-05);
+#endif
+}
+// log((sqrt 2 - 1) / (sqrt 2 + 1)): a square panel of area dS has the potential
+// -2 sqrt(dS) times it at its centre
+constexpr double kPanelLog = -1.7627471740390861;
+// Weight of a cell of area ds at an offset: ds / r, within 1e-5 the panel's own
+// potential, 0 at the cell's centre (such a cell is always opened).
+VPMG_HD double lattice_weight(double ds, double a, double ha, double b, double hb, double n, double hn) {
+  const double r2 = lattice_r2(a, ha, b, hb, n, hn);
+  if (r2 > 0.0 && r2 < 1.01e-10 && lattice_close(a, ha, b, hb, n, hn)) {
+#ifdef __CUDA_ARCH__
+    return rn_mul(rn_mul(-2.0, __dsqrt_rn(ds)), kPanelLog);
+#else
+    return -2.0 * std::sqrt(ds) * kPanelLog;
+#endif
+  }
+  return lattice_weight(ds, r2);
+}
+
 // Weight of (column, row, cell) of a table.
 VPMG_HD double near_weight(const NearTable& T, int n, int row, int cell) {
   const int tr = n / T.TB, tw = n - tr * T.TB;
@@ -88,13 +120,13 @@ VPMG_HD double near_weight(const NearTable& T, int n, int row, int cell) {
   const double orr = T.par ? s * ((double)cr + 0.5) - (double)tr : s * ((double)cr + 0.5);
   const double on = T.par ? (double)T.dn : (double)tr;
   const double r2 = lattice_r2(ow, T.hw, orr, T.hr, on, T.hn);
-  if (T.top) return r2 < T.thr2_own ? -lattice_weight(T.ds, r2) : 0.0;
+  if (T.top) return r2 < T.thr2_own ? -lattice_weight(T.ds, ow, T.hw, orr, T.hr, on, T.hn) : 0.0;
   const double pw = 2.0 * s * ((double)floor_half(cw) + 0.5) - (double)tw;
   const double pc = 2.0 * s * ((double)floor_half(cr) + 0.5);
   const double pr = T.par ? pc - (double)tr : pc;
   if (!(lattice_r2(pw, T.hw, pr, T.hr, on, T.hn) < T.thr2_out)) return 0.0;
   if (T.s > 1 && r2 < T.thr2_own) return 0.0;
-  return lattice_weight(T.ds, r2);
+  return lattice_weight(T.ds, ow, T.hw, orr, T.hr, on, T.hn);
 }
 
 }  // namespace vpmg

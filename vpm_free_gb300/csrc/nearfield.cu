@@ -385,9 +385,10 @@ struct DiffDev {
 };
 // Counts (FILL = false) or writes the cells that a node's walk and the
 // lattice rule take differently: the walk's with weight dS/r, the rule's
-// with -dS/r.  Decisions away from an opening radius are made in FP32 (both
-// sides agree there); within 1e-4 of one the walk's own expressions decide
-// for the walk and lattice_r2 for the rule.
+// with -dS/r, and both where only one sees the cell within the 1e-5 of length
+// at which the weight changes.  Decisions away from a radius are made in FP32
+// (both sides agree there); within 1e-4 of one the walk's own expressions
+// decide for the walk and lattice_r2 (lattice_close) for the rule.
 template <bool FILL>
 __global__ void k_near_diff(const __grid_constant__ DiffDev D, int* __restrict__ counts,
                             unsigned long long* __restrict__ accepted, const long long* __restrict__ rowptr,
@@ -443,19 +444,26 @@ __global__ void k_near_diff(const __grid_constant__ DiffDev D, int* __restrict__
       o2[fu] = 2 * a * s + s;
       o2[fv] = 2 * b * s + s;
       bool wo = false, ro = false;
+      const float ex = 0.5f * (float)(2 * ti[0] - o2[0]) * hf[0], ey = 0.5f * (float)(2 * ti[1] - o2[1]) * hf[1],
+                  ez = 0.5f * (float)(2 * ti[2] - o2[2]) * hf[2];
+      const float r2 = ex * ex + ey * ey + ez * ez;
+      const double ou = 0.5 * (double)(2 * ti[fu] - o2[fu]), ov = 0.5 * (double)(2 * ti[fv] - o2[fv]),
+                   on = 0.5 * (double)(2 * ti[fn] - o2[fn]);
+      auto walk_r = [&] {
+        const double XR = __dsub_rn(D.cx[c], X), YR = __dsub_rn(D.cy[c], Y), ZR = __dsub_rn(D.cz[c], Z);
+        return __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(XR, XR), __dmul_rn(YR, YR)), __dmul_rn(ZR, ZR)));
+      };
+      auto walk_weight = [&](double rr) {
+        return rr > 1e-05 ? __ddiv_rn(D.cds[c], rr) : -2.0 * __dsqrt_rn(D.cds[c]) * kPanelLog;
+      };
+      auto rule_weight = [&] { return lattice_weight(D.ds[l][fn], ou, D.h[fu], ov, D.h[fv], on, D.h[fn]); };
       if (l > 0) {
-        const float ex = 0.5f * (float)(2 * ti[0] - o2[0]) * hf[0], ey = 0.5f * (float)(2 * ti[1] - o2[1]) * hf[1],
-                    ez = 0.5f * (float)(2 * ti[2] - o2[2]) * hf[2];
-        const float r2 = ex * ex + ey * ey + ez * ez, th = (float)D.thr2[l][fn];
+        const float th = (float)D.thr2[l][fn];
         if (fabsf(r2 - th) > 1e-4f * th) {
           wo = ro = r2 < th;
         } else {
-          const double XR = __dsub_rn(D.cx[c], X), YR = __dsub_rn(D.cy[c], Y), ZR = __dsub_rn(D.cz[c], Z);
-          const double rr =
-              __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(XR, XR), __dmul_rn(YR, YR)), __dmul_rn(ZR, ZR)));
-          wo = rr < D.cthr[c];
-          ro = lattice_r2(0.5 * (double)(2 * ti[fu] - o2[fu]), D.h[fu], 0.5 * (double)(2 * ti[fv] - o2[fv]), D.h[fv],
-                          0.5 * (double)(2 * ti[fn] - o2[fn]), D.h[fn]) < D.thr2[l][fn];
+          wo = walk_r() < D.cthr[c];
+          ro = lattice_r2(ou, D.h[fu], ov, D.h[fv], on, D.h[fn]) < D.thr2[l][fn];
         }
       }
       const bool w = md & 1, g = md & 2;
@@ -465,17 +473,13 @@ __global__ void k_near_diff(const __grid_constant__ DiffDev D, int* __restrict__
         else ++na;
       }
       if (wa != ra) {
-        if (wa) {
-          const double XR = __dsub_rn(D.cx[c], X), YR = __dsub_rn(D.cy[c], Y), ZR = __dsub_rn(D.cz[c], Z);
-          const double rr =
-              __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(XR, XR), __dmul_rn(YR, YR)), __dmul_rn(ZR, ZR)));
-          emit(c, rr > 1e-05 ? __ddiv_rn(D.cds[c], rr)
-                             : -2.0 * __dsqrt_rn(D.cds[c]) * log((sqrt(2.0) - 1.0) / (sqrt(2.0) + 1.0)));
-        } else {
-          emit(c, -lattice_weight(D.ds[l][fn],
-                                  lattice_r2(0.5 * (double)(2 * ti[fu] - o2[fu]), D.h[fu],
-                                             0.5 * (double)(2 * ti[fv] - o2[fv]), D.h[fv],
-                                             0.5 * (double)(2 * ti[fn] - o2[fn]), D.h[fn])));
+        if (wa) emit(c, walk_weight(walk_r()));
+        else emit(c, -rule_weight());
+      } else if (wa && !(fabsf(r2 - 1e-10f) > 1e-14f)) {
+        const double rr = walk_r();
+        if ((rr > 1e-05) == lattice_close(ou, D.h[fu], ov, D.h[fv], on, D.h[fn])) {
+          emit(c, walk_weight(rr));
+          emit(c, -rule_weight());
         }
       }
       const int cm = ((w && wo) ? 1 : 0) | ((g && ro) ? 2 : 0);
