@@ -388,8 +388,10 @@ struct DiffDev {
 // with -dS/r, and both where only one sees the cell within the 1e-5 of length
 // at which the weight changes.  Decisions away from a radius are made in FP32
 // (both sides agree there); within 1e-4 of one the walk's own expressions
-// decide for the walk and lattice_r2 (lattice_close) for the rule.
-template <bool FILL>
+// decide for the walk and lattice_r2 (lattice_close) for the rule.  FINE: some
+// cell can lie that close (looking for them on every mesh doubled the set-up of
+// 256^3, 180 to 350 ms).
+template <bool FILL, bool FINE>
 __global__ void k_near_diff(const __grid_constant__ DiffDev D, int* __restrict__ counts,
                             unsigned long long* __restrict__ accepted, const long long* __restrict__ rowptr,
                             int* __restrict__ col, double* __restrict__ wgt) {
@@ -444,11 +446,8 @@ __global__ void k_near_diff(const __grid_constant__ DiffDev D, int* __restrict__
       o2[fu] = 2 * a * s + s;
       o2[fv] = 2 * b * s + s;
       bool wo = false, ro = false;
-      const float ex = 0.5f * (float)(2 * ti[0] - o2[0]) * hf[0], ey = 0.5f * (float)(2 * ti[1] - o2[1]) * hf[1],
-                  ez = 0.5f * (float)(2 * ti[2] - o2[2]) * hf[2];
-      const float r2 = ex * ex + ey * ey + ez * ez;
-      const double ou = 0.5 * (double)(2 * ti[fu] - o2[fu]), ov = 0.5 * (double)(2 * ti[fv] - o2[fv]),
-                   on = 0.5 * (double)(2 * ti[fn] - o2[fn]);
+      // FP64 only where a decision is close: these run for one pair in thousands
+      auto off = [&](int a) { return 0.5 * (double)(2 * ti[a] - o2[a]); };
       auto walk_r = [&] {
         const double XR = __dsub_rn(D.cx[c], X), YR = __dsub_rn(D.cy[c], Y), ZR = __dsub_rn(D.cz[c], Z);
         return __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(XR, XR), __dmul_rn(YR, YR)), __dmul_rn(ZR, ZR)));
@@ -456,14 +455,22 @@ __global__ void k_near_diff(const __grid_constant__ DiffDev D, int* __restrict__
       auto walk_weight = [&](double rr) {
         return rr > 1e-05 ? __ddiv_rn(D.cds[c], rr) : -2.0 * __dsqrt_rn(D.cds[c]) * kPanelLog;
       };
-      auto rule_weight = [&] { return lattice_weight(D.ds[l][fn], ou, D.h[fu], ov, D.h[fv], on, D.h[fn]); };
+      auto rule_weight = [&] {
+        return lattice_weight(D.ds[l][fn], off(fu), D.h[fu], off(fv), D.h[fv], off(fn), D.h[fn]);
+      };
+      float r2 = 0.f;
+      if (FINE || l > 0) {
+        const float ex = 0.5f * (float)(2 * ti[0] - o2[0]) * hf[0], ey = 0.5f * (float)(2 * ti[1] - o2[1]) * hf[1],
+                    ez = 0.5f * (float)(2 * ti[2] - o2[2]) * hf[2];
+        r2 = ex * ex + ey * ey + ez * ez;
+      }
       if (l > 0) {
         const float th = (float)D.thr2[l][fn];
         if (fabsf(r2 - th) > 1e-4f * th) {
           wo = ro = r2 < th;
         } else {
           wo = walk_r() < D.cthr[c];
-          ro = lattice_r2(ou, D.h[fu], ov, D.h[fv], on, D.h[fn]) < D.thr2[l][fn];
+          ro = lattice_r2(off(fu), D.h[fu], off(fv), D.h[fv], off(fn), D.h[fn]) < D.thr2[l][fn];
         }
       }
       const bool w = md & 1, g = md & 2;
@@ -475,9 +482,9 @@ __global__ void k_near_diff(const __grid_constant__ DiffDev D, int* __restrict__
       if (wa != ra) {
         if (wa) emit(c, walk_weight(walk_r()));
         else emit(c, -rule_weight());
-      } else if (wa && !(fabsf(r2 - 1e-10f) > 1e-14f)) {
+      } else if (FINE && wa && !(fabsf(r2 - 1e-10f) > 1e-14f)) {
         const double rr = walk_r();
-        if ((rr > 1e-05) == lattice_close(ou, D.h[fu], ov, D.h[fv], on, D.h[fn])) {
+        if ((rr > 1e-05) == lattice_close(off(fu), D.h[fu], off(fv), D.h[fv], off(fn), D.h[fn])) {
           emit(c, walk_weight(rr));
           emit(c, -rule_weight());
         }
@@ -707,7 +714,10 @@ bool near_prepare(BoundaryOp& B, const Grid& g, long long budget_bytes, cudaStre
   acc2.ensure(2);
   VPMG_CUDA(cudaMemsetAsync(acc2.p, 0, 2 * sizeof(unsigned long long), s));
   const dim3 blocks((unsigned)((B.ntarget + 127) / 128), 6);
-  k_near_diff<false><<<blocks, 128, 0, s>>>(D, counts.p, acc2.p, nullptr, nullptr, nullptr);
+  // leaf centres are at least half a diagonal from every node
+  const bool fine = std::min({g.d[0], g.d[1], g.d[2]}) < 2e-5;
+  if (fine) k_near_diff<false, true><<<blocks, 128, 0, s>>>(D, counts.p, acc2.p, nullptr, nullptr, nullptr);
+  else k_near_diff<false, false><<<blocks, 128, 0, s>>>(D, counts.p, acc2.p, nullptr, nullptr, nullptr);
   VPMG_LAUNCHED();
   const size_t nrow = 6 * (size_t)B.ntarget;  // a node's row: its six faces' in turn
   std::vector<int> hc(nrow);
@@ -723,7 +733,8 @@ bool near_prepare(BoundaryOp& B, const Grid& g, long long budget_bytes, cudaStre
   FF.ccol.ensure((size_t)std::max<long long>(FF.ncorr, 1));
   FF.cw.ensure((size_t)std::max<long long>(FF.ncorr, 1));
   if (FF.ncorr) {
-    k_near_diff<true><<<blocks, 128, 0, s>>>(D, nullptr, nullptr, FF.crow.p, FF.ccol.p, FF.cw.p);
+    if (fine) k_near_diff<true, true><<<blocks, 128, 0, s>>>(D, nullptr, nullptr, FF.crow.p, FF.ccol.p, FF.cw.p);
+    else k_near_diff<true, false><<<blocks, 128, 0, s>>>(D, nullptr, nullptr, FF.crow.p, FF.ccol.p, FF.cw.p);
     VPMG_LAUNCHED();
   }
   VPMG_CUDA(cudaGetLastError());
