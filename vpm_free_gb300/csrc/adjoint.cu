@@ -1032,7 +1032,7 @@ int vpmg_apply_poisson(vpmg_handle* h, const double* r, double* psi) {
     VPMG_CUDA(cudaMemcpyAsync(h->rhs.p, r, sizeof(double) * 3 * N, cudaMemcpyHostToDevice, h->stream));
     hx::poisson_part(h);
     VPMG_CUDA(cudaMemcpyAsync(psi, h->sol.p, sizeof(double) * 3 * N, cudaMemcpyDeviceToHost, h->stream));
-    VPMG_CUDA(cudaStreamSynchronize(h->stream));
+    check_wait_errors(h->bins, h->stream);
   });
 }
 
@@ -1047,7 +1047,7 @@ int vpmg_adjoint_poisson(vpmg_handle* h, const double* psibar, double* rbar) {
     fill_zero(S.rbar.p, 3 * N, h->stream);
     poisson_T(h, S.psibar.p, S.rbar.p);
     VPMG_CUDA(cudaMemcpyAsync(rbar, S.rbar.p, sizeof(double) * 3 * N, cudaMemcpyDeviceToHost, h->stream));
-    VPMG_CUDA(cudaStreamSynchronize(h->stream));
+    check_wait_errors(h->bins, h->stream);
   });
 }
 

@@ -158,9 +158,9 @@ void prepare(vpmg_handle* h) {
   const int bl_inner[6] = {s.nnbl_bl[0] - 1, s.nnbl_bl[1] - 1, s.nnbl_bl[2] - 1,
                            s.nnbl_bl[3] - 1, s.nnbl_bl[4] - 1, s.nnbl_bl[5] - 1};
   const int c_full[6] = {0, 0, 0, s.nn_coarse[0] - 1, s.nn_coarse[1] - 1, s.nn_coarse[2] - 1};
-  dirichlet_prepare(h->dp_bl, s.nnbl, bl_full, s.dpm, st, h->arith);
-  dirichlet_prepare(h->dp_inner, s.nnbl, bl_inner, s.dpm, st, h->arith);
-  dirichlet_prepare(h->dp_c, s.nn_coarse, c_full, s.dpm_coarse, st, h->arith);
+  dirichlet_prepare(h->dp_bl, s.nnbl, bl_full, s.dpm, st, h->arith, h->bins.err.p);
+  dirichlet_prepare(h->dp_inner, s.nnbl, bl_inner, s.dpm, st, h->arith, h->bins.err.p);
+  dirichlet_prepare(h->dp_c, s.nn_coarse, c_full, s.dpm_coarse, st, h->arith, h->bins.err.p);
   size_t wmax = 0;
   for (DirichletPlan* p : {&h->dp_bl, &h->dp_inner, &h->dp_c}) wmax = std::max(wmax, (size_t)p->m[0] * p->m[1] * p->m[2]);
   h->work.ensure(3 * wmax);
@@ -439,7 +439,7 @@ void remesh(vpmg_handle* h) {
 __global__ void k_set_int(int* __restrict__ d, int v) { *d = v; }
 
 // Host mirror of the device particle count, and the errors flagged since
-// the last sync (stencil outside the mesh, remesh over capacity).
+// the last sync (stencil outside the mesh, remesh over capacity, a wait that ran out).
 void sync_np(vpmg_handle* h) {
   check_particle_errors(h->bins, h->stream);
   h->np = read_count(h->parts.d_np.p, h->stream);
@@ -605,6 +605,8 @@ int vpmg_create(const vpmg_config* cfg, int device, vpmg_handle** out) {
   int rc = guarded(h, [&] {
     VPMG_CUDA(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
     for (int i = 0; i < 10; ++i) VPMG_CUDA(cudaEventCreate(&h->ev[i]));
+    h->bins.err.ensure(1);
+    VPMG_CUDA(cudaMemset(h->bins.err.p, 0, sizeof(int)));
     size_t fr = 0, tot = 0;
     VPMG_CUDA(cudaMemGetInfo(&fr, &tot));
     h->op_budget = std::min<long long>(100LL << 30, (long long)(0.6 * (double)fr));
@@ -1635,7 +1637,7 @@ int vpmg_pmesh(vpmg_handle* h, double* const sol[3], const double* const rhs[3],
     DirichletPlan dp;
     if (iynbc == 1) {
       const int full[6] = {0, 0, 0, nn[0] - 1, nn[1] - 1, nn[2] - 1};
-      dirichlet_prepare(dp, nn, full, dpm, h->stream, h->arith);
+      dirichlet_prepare(dp, nn, full, dpm, h->stream, h->arith, h->bins.err.p);
       w.ensure(3 * (size_t)dp.m[0] * dp.m[1] * dp.m[2]);
       fill_zero(s0.p, 3 * n, h->stream);
       BoundaryOp bo;
@@ -1646,16 +1648,16 @@ int vpmg_pmesh(vpmg_handle* h, double* const sol[3], const double* const rhs[3],
       double* sp[3] = {s.p, s.p + n, s.p + 2 * n};
       boundary_apply(bo, g, sp, h->stream);
       dirichlet_solve(dp, r.p, s.p, false, w.p, h->stream, 3, n, n);
-      VPMG_CUDA(cudaStreamSynchronize(h->stream));
+      VPMG_CUDA(cudaStreamSynchronize(h->stream));  // the operator's arrays end here
     } else {
       const int box[6] = {nn_bl[0] - 1, nn_bl[1] - 1, nn_bl[2] - 1, nn_bl[3] - 1, nn_bl[4] - 1, nn_bl[5] - 1};
-      dirichlet_prepare(dp, nn, box, dpm, h->stream, h->arith);
+      dirichlet_prepare(dp, nn, box, dpm, h->stream, h->arith, h->bins.err.p);
       w.ensure(3 * (size_t)dp.m[0] * dp.m[1] * dp.m[2]);
       dirichlet_solve(dp, r.p, s.p, false, w.p, h->stream, 3, n, n);
     }
     for (int c = 0; c < 3; ++c)
       VPMG_CUDA(cudaMemcpyAsync(sol[c], s.p + c * n, sizeof(double) * n, cudaMemcpyDeviceToHost, h->stream));
-    VPMG_CUDA(cudaStreamSynchronize(h->stream));
+    check_wait_errors(h->bins, h->stream);
   });
 }
 

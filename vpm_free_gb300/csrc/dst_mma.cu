@@ -26,6 +26,7 @@
 // outputs, 13 the scale before it moved beside the product.
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 
 #include "dst_mma.h"
 #include "tc05.cuh"
@@ -50,8 +51,6 @@ constexpr int kSlot[3] = {0, 7 * kPiece, 4 * kPiece};
 __host__ __device__ __forceinline__ int dst_kp(int n) { return (((n + 1) / 2) + 15) & ~15; }  // padded folded length
 __host__ __device__ __forceinline__ int dst_count(int n, int par) { return par ? n / 2 : (n + 1) / 2; }
 __host__ __device__ __forceinline__ int dst_mtiles(int n, int par) { return (dst_count(n, par) + kRows - 1) / kRows; }
-
-__device__ int g_dst_wait_failed;  // a bounded wait ran out (the pass then writes NaN)
 
 // Piece (par, mt, ks, digit) of the matrix times factor in [1, 2): rows m,
 // k positions 16 ks + 8 g' + i <-> j = 1 + g + G i with g = 2 ks + g'.
@@ -101,6 +100,8 @@ struct DstArgs {
   long long sy, sz, o;  // node strides and the offset of the first interior node (x passes)
   size_t ics, scs, ocs;
   double ihx2, ihy2, ihz2;
+  int polls;     // limit of every wait
+  int* status;   // null or the word that gets kErrWait when a wait runs out
 };
 
 // V 2^e as a double, rounded to nearest even.
@@ -122,10 +123,15 @@ __device__ __forceinline__ double to_double(long long V, int e) {
 }
 
 // MODE 0: x forward (node array -> lines), 1: y, 2: x inverse (lines -> node array)
+//
+// Every wait has a limit.  When one runs out, the thread that waited stops
+// loading or issuing; the barrier behind each product tells the whole CTA, which
+// waits for its own copies and products in flight, sets *status, writes NaN to
+// the outputs of this tile and of those it still had, and ends.
 template <int MODE>
 __global__ void __launch_bounds__(kThreads, 1) k_dst_mma(const __grid_constant__ DstArgs P) {
   extern __shared__ __align__(128) unsigned char dst_sm[];
-  __shared__ __align__(8) uint64_t bars[2 * kMaxSlots + 1];
+  __shared__ __align__(8) uint64_t bars[2 * kMaxSlots + 2];
   __shared__ uint32_t tslot;
   // the lines of this tile and of the next (its magnitudes are taken while this one's last product runs)
   __shared__ long long loff[2][kLines], ooff[2][kLines];  // first value of each line, read and written
@@ -138,9 +144,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_dst_mma(const __grid_constant__
   const uint32_t ring = dig + (uint32_t)(kDigits * G * kCol);
   unsigned char* const stage = dst_sm + (size_t)kDigits * G * kCol;
   const uint32_t full = tc05::smem_u32(bars), empty = full + 8 * kMaxSlots, done = full + 16 * kMaxSlots;
+  const uint32_t drained = done + 8;
   if (warp == 0) tc05::tmem_alloc(tc05::smem_u32(&tslot), 512);
   if (tid == 0) {
-    for (int i = 0; i < 2 * kMaxSlots + 1; ++i) tc05::bar_init(full + 8 * i, 1);
+    for (int i = 0; i < 2 * kMaxSlots + 2; ++i) tc05::bar_init(full + 8 * i, 1);
     tc05::bar_init_fence();
   }
   tc05::fence_before();
@@ -148,12 +155,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_dst_mma(const __grid_constant__
   tc05::fence_after();
   const uint32_t tb = tslot;
   constexpr uint32_t idesc = tc05::idesc_f16(kRows, kLines);
-  bool dead = false;
+  bool dead = false, failed = false;
   const int S = P.slots, np = P.np;
   const uint32_t sbytes = np == 1 ? 7 * kPiece : 4 * kPiece;
   // the loading thread's (warp 1) and the issuing thread's (warp 0) place in the ring
   int slot = 0;
   uint32_t phase = 0, wrapped = 0, ndone = 0;
+  uint32_t loads = 0;  // pieces loaded by this thread
   const long long estr = MODE == 1 ? P.m0 : 1;  // doubles between a line's values
   const int ntot = P.ntile * P.nc;
   auto in_of = [&](int tile) { return P.in + (size_t)(tile / P.ntile) * P.ics; };
@@ -263,7 +271,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_dst_mma(const __grid_constant__
   if (tile < ntot && tid < kLines) lines_of(tile, 0);
   __syncthreads();
   if (tile < ntot) magnitudes(tile, 0, 0);
-  for (; tile < ntot; tile += gridDim.x, cur ^= 1) {
+  for (; tile < ntot && !failed; tile += gridDim.x, cur ^= 1) {
     __syncthreads();
     const int next = tile + gridDim.x;
     if (next < ntot && tid < kLines) lines_of(next, cur ^ 1);
@@ -337,7 +345,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_dst_mma(const __grid_constant__
     };
     const int units = kLines * G;
     int mt = 0;
-    for (int par = 0; par < 2; ++par) {
+    for (int par = 0; par < 2 && !failed; ++par) {
       const int cnt = dst_count(n, par), mts = dst_mtiles(n, par);
       for (int u = tid; u < units; u += kThreads) {
         unsigned d[4][kDigits];
@@ -352,7 +360,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_dst_mma(const __grid_constant__
             const unsigned char* src = P.T + (size_t)mt * nks * kDigits * kPiece;
             for (int i = 0; i < nks * np; ++i) {
               const uint32_t bytes = np == 1 ? 7 * kPiece : (i & 1) ? 4 * kPiece : 3 * kPiece;
-              if (wrapped) tc05::bar_wait(empty + 8 * slot, phase ^ 1u, dead, &g_dst_wait_failed);
+              if (wrapped) tc05::bar_wait(empty + 8 * slot, phase ^ 1u, dead, P.polls);
+              if (dead) break;
+              ++loads;
               tc05::bar_expect(full + 8 * slot, bytes);
               tc05::bulk_load(ring + slot * sbytes, src, bytes, full + 8 * slot);
               src += bytes;
@@ -367,14 +377,15 @@ __global__ void __launch_bounds__(kThreads, 1) k_dst_mma(const __grid_constant__
         } else if (warp == 0) {  // the products
           if (lane == 0) {
             tc05::fence_after();
-            for (int ks = 0; ks < nks; ++ks) {
+            for (int ks = 0; ks < nks && !dead; ++ks) {
               const uint64_t db = tc05::desc(dig + (uint32_t)(2 * ks) * kCol, kCol);
               const uint64_t dj = (uint64_t)((uint32_t)(G * kCol) >> 4);
               uint64_t da = 0;
 #pragma unroll
               for (int w = 0; w < kDigits; ++w) {
                 if (w == 0 || (w == 3 && np == 2)) {  // the next piece
-                  tc05::bar_wait(full + 8 * slot, phase, dead, &g_dst_wait_failed);
+                  tc05::bar_wait(full + 8 * slot, phase, dead, P.polls);
+                  if (dead) break;
                   da = tc05::desc(ring + slot * sbytes, kRows * 16);
                 }
 #pragma unroll
@@ -396,8 +407,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_dst_mma(const __grid_constant__
         } else if (par == 1 && h == mts - 1 && next < ntot) {  // meanwhile: the next tile's magnitudes
           magnitudes(next, cur ^ 1, 2);
         }
-        tc05::bar_wait(done, ndone & 1, dead, &g_dst_wait_failed);
+        tc05::bar_wait(done, ndone & 1, dead, P.polls);
         ++ndone;
+        if (__syncthreads_or(dead)) {
+          failed = true;
+          break;
+        }
         tc05::fence_after();
         // outputs: row m of the tile in lane m, 16 lines per warp
         const int m = 32 * (warp & 3) + lane, cb = 16 * (warp >> 2);
@@ -424,7 +439,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_dst_mma(const __grid_constant__
             const long long V = (hi << 7) + ((lo + 256) >> 9);
             const int E = tc05::scale_exp(emax[cur][line]);
             double r = to_double(P.neg ? -V : V, 57 + E - 1077 - 55 + P.shift);
-            if (E >= 0x7FF || dead) r = __longlong_as_double(0x7FF8000000000000ll);
+            if (E >= 0x7FF) r = __longlong_as_double(0x7FF8000000000000ll);
             if (MODE == 1) {
               st[lane * 8 + (i ^ (lane & 7))] = r;
             } else if (o < cnt && (lflag[cur][line] & 1)) {
@@ -450,6 +465,30 @@ __global__ void __launch_bounds__(kThreads, 1) k_dst_mma(const __grid_constant__
     }
   }
   __syncthreads();
+  if (failed) {
+    bool late = false;  // these waits have the full limit
+    if (warp == 0 && lane == 0) {
+      tc05::commit(drained);
+      tc05::bar_wait(drained, 0, late, tc05::kPolls);
+    }
+    if (warp == 1 && lane == 0)
+      for (uint32_t i = 0; i < (uint32_t)S && i < loads; ++i)  // the last copy into each slot
+        tc05::bar_wait(full + 8 * i, ((loads - i - 1) / S) & 1, late, tc05::kPolls);
+    __syncwarp();
+    if (tid == 0 && P.status) atomicMax(P.status, kErrWait);
+    const double nan = __longlong_as_double(0x7FF8000000000000ll);
+    for (tile -= gridDim.x; tile < ntot; tile += gridDim.x) {  // from the tile that failed
+      __syncthreads();
+      if (tid < kLines) lines_of(tile, 0);
+      __syncthreads();
+      double* out = P.out + (size_t)(tile / P.ntile) * P.ocs;
+      for (int t = tid; t < kLines * n; t += kThreads) {
+        const int line = MODE == 1 ? t & (kLines - 1) : t / n, k = MODE == 1 ? t / kLines : t - line * n;
+        if (lflag[0][line] & 1) out[ooff[0][line] + estr * k] = nan;
+      }
+    }
+    __syncthreads();
+  }
   if (warp == 0) tc05::tmem_free(tb, 512);
 }
 
@@ -484,6 +523,11 @@ void launch(DstArgs& A, cudaStream_t s) {
 // 1.85 ms, the FFT's dense pass 1.88 ms at N = 256.
 bool dst_mma_wanted(int n, long long lines) {
   return n + 1 >= 100 && pieces_for(n) && lines >= 1024;
+}
+
+int wait_polls() {
+  const char* e = std::getenv("VPMG_WAIT_POLLS");
+  return e ? std::max(0, std::atoi(e)) : tc05::kPolls;
 }
 
 size_t dst_mma_table_bytes(int n) {
@@ -532,8 +576,9 @@ static void box_args(DstArgs& A, const DstBox& b) {
 
 void dst_mma_x_fwd(const unsigned char* T, int shift, int neg, const double* rhs, const double* sol, bool zero_bc,
                    double* out, const DstBox& b, double ihx2, double ihy2, double ihz2, int nc, size_t rcs, size_t scs,
-                   size_t ocs, cudaStream_t s) {
+                   size_t ocs, const DstWait& w, cudaStream_t s) {
   DstArgs A{};
+  A.polls = w.polls; A.status = w.status;
   box_args(A, b);
   A.T = T;
   A.in = rhs; A.sol = sol; A.out = out;
@@ -546,8 +591,9 @@ void dst_mma_x_fwd(const unsigned char* T, int shift, int neg, const double* rhs
 }
 
 void dst_mma_y(const unsigned char* T, const double* in, double* out, int m0, int m1, int m2, int nc, size_t cs,
-               cudaStream_t s) {
+               const DstWait& w, cudaStream_t s) {
   DstArgs A{};
+  A.polls = w.polls; A.status = w.status;
   A.T = T;
   A.n = m1;
   A.nlines = m0 * m2;
@@ -559,8 +605,9 @@ void dst_mma_y(const unsigned char* T, const double* in, double* out, int m0, in
 }
 
 void dst_mma_x_inv(const unsigned char* T, const double* in, double* sol, const DstBox& b, int nc, size_t ics,
-                   size_t scs, cudaStream_t s) {
+                   size_t scs, const DstWait& w, cudaStream_t s) {
   DstArgs A{};
+  A.polls = w.polls; A.status = w.status;
   box_args(A, b);
   A.T = T;
   A.in = in; A.out = sol;

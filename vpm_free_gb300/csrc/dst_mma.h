@@ -15,16 +15,21 @@ struct DstTable {
 };
 void dst_mma_setup();  // once per device, outside stream capture
 void dst_mma_tables(const DstTable* t, int count, cudaStream_t s);  // up to three, one launch
-// Passes: lines of n points; nc components (strides in doubles).
+// Passes: lines of n points; nc components (strides in doubles).  A wait that
+// runs out of polls makes the outputs NaN and *status (if any) kErrWait.
+struct DstWait {
+  int polls;
+  int* status;
+};
 struct DstBox {
   int dims[3], o[3], m[3];
 };
 void dst_mma_x_fwd(const unsigned char* T, int shift, int neg, const double* rhs, const double* sol, bool zero_bc,
                    double* out, const DstBox& b, double ihx2, double ihy2, double ihz2, int nc, size_t rcs, size_t scs,
-                   size_t ocs, cudaStream_t s);
+                   size_t ocs, const DstWait& w, cudaStream_t s);
 void dst_mma_y(const unsigned char* T, const double* in, double* out, int m0, int m1, int m2, int nc, size_t cs,
-               cudaStream_t s);
+               const DstWait& w, cudaStream_t s);
 void dst_mma_x_inv(const unsigned char* T, const double* in, double* sol, const DstBox& b, int nc, size_t ics,
-                   size_t scs, cudaStream_t s);
+                   size_t scs, const DstWait& w, cudaStream_t s);
 
 }  // namespace vpmg

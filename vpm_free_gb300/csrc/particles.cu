@@ -92,7 +92,7 @@ __global__ void k_keys(const double* __restrict__ x, const double* __restrict__ 
                   j0 + m.ipf < m.n[1] && k0 + m.ipf < m.n[2];
   if (!ok) {
     key[p] = -1;
-    atomicExch(err, 1);
+    atomicMax(err, kErrOutside);
     continue;
   }
   const int kk = i0 + m.n[0] * (j0 + m.n[1] * k0);
@@ -654,7 +654,7 @@ __global__ void k_set_count(int* __restrict__ np, const int* __restrict__ total,
   const int t = *total;
   if (t > capacity) {
     *np = capacity;
-    atomicExch(err, 2);
+    atomicMax(err, kErrCapacity);
   } else {
     *np = t;
   }
@@ -689,7 +689,7 @@ void Binning::ensure(size_t ncell) {
 
 // Sort by cell + records, all on the stream (no host round trip): the
 // particle count is read from P.d_np, the sorted count lands in starts[N].
-// Errors (stencil outside the mesh = 1, remesh overflow = 2) accumulate in
+// Errors (kErrOutside, kErrCapacity; kErrWait of the solves) accumulate in
 // B.err and are reported by check_particle_errors at the next host sync.
 void bin_particles(Particles& P, const MeshDev& m, Binning& B, cudaStream_t s) {
   const size_t N = (size_t)m.n[0] * m.n[1] * m.n[2];
@@ -724,8 +724,18 @@ void check_particle_errors(Binning& B, cudaStream_t s) {
   VPMG_CUDA(cudaMemcpyAsync(&e, B.err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
   VPMG_CUDA(cudaStreamSynchronize(s));
   if (e) VPMG_CUDA(cudaMemsetAsync(B.err.p, 0, sizeof(int), s));
-  VPMG_CHECK(e != 1, VPMG_ERR_OUTSIDE, "a particle's projection stencil leaves the mesh");
-  VPMG_CHECK(e != 2, VPMG_ERR_CAPACITY, "remesh produced more particles than the capacity");
+  VPMG_CHECK(e != kErrWait, VPMG_ERR_CUDA, "a wait inside a kernel ran out");
+  VPMG_CHECK(e != kErrOutside, VPMG_ERR_OUTSIDE, "a particle's projection stencil leaves the mesh");
+  VPMG_CHECK(e != kErrCapacity, VPMG_ERR_CAPACITY, "remesh produced more particles than the capacity");
+}
+
+void check_wait_errors(Binning& B, cudaStream_t s) {
+  int e = 0;
+  VPMG_CUDA(cudaMemcpyAsync(&e, B.err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+  VPMG_CUDA(cudaStreamSynchronize(s));
+  if (e != kErrWait) return;
+  VPMG_CUDA(cudaMemsetAsync(B.err.p, 0, sizeof(int), s));
+  throw Error{VPMG_ERR_CUDA, "a wait inside a kernel ran out"};
 }
 
 int read_count(const int* d, cudaStream_t s) {

@@ -71,6 +71,7 @@ void remesh_emit_masked(Particles& P, const MeshDev& m, Binning& B, const double
                         cudaStream_t s);
 // Host sync points.
 void check_particle_errors(Binning& B, cudaStream_t s);
+void check_wait_errors(Binning& B, cudaStream_t s);  // kErrWait alone, for calls without particles; others stay
 int read_count(const int* d, cudaStream_t s);
 
 }  // namespace vpmg

@@ -939,7 +939,9 @@ void make_fft_plan(FFTPlan& p, int n, int arith) {
 }
 
 void dirichlet_prepare(DirichletPlan& P, const int dims[3], const int box[6], const double h[3], cudaStream_t s,
-                       int arith) {
+                       int arith, int* status) {
+  P.status = status;
+  P.polls = wait_polls();
   VPMG_CHECK(arith == VPMG_ARITH_FP64 || arith == VPMG_ARITH_FF48, VPMG_ERR_ARG, "unknown arithmetic");
   bool same = P.ready && P.arith == arith;
   for (int d = 0; d < 3; ++d) same = same && P.dims[d] == dims[d] && P.h[d] == h[d];
@@ -1020,7 +1022,8 @@ void x_forward(DirichletPlan& P, const double* rhs, const double* sol, bool zero
   const double ix = 1.0 / (P.h[0] * P.h[0]), iy = 1.0 / (P.h[1] * P.h[1]), iz = 1.0 / (P.h[2] * P.h[2]);
   const size_t wcs = (size_t)P.m[0] * P.m[1] * P.m[2];
   if (P.mma_x) {
-    dst_mma_x_fwd(P.txf.p, P.xf_shift, P.xf_neg, rhs, sol, zero_bc, out, mma_box(P), ix, iy, iz, nc, rcs, scs, wcs, s);
+    dst_mma_x_fwd(P.txf.p, P.xf_shift, P.xf_neg, rhs, sol, zero_bc, out, mma_box(P), ix, iy, iz, nc, rcs, scs, wcs,
+                  DstWait{P.polls, P.status}, s);
     return;
   }
   launch_x_fwd(s, rhs, sol, zero_bc ? 1 : 0, out, plan_box(P), dev_plan(P.fx), ix, iy, iz, dirichlet_scale(P),
@@ -1032,7 +1035,7 @@ void x_forward(DirichletPlan& P, const double* rhs, const double* sol, bool zero
 double* y_pass(DirichletPlan& P, double* data, double* other, cudaStream_t s, int nc) {
   const size_t wcs = (size_t)P.m[0] * P.m[1] * P.m[2];
   if (P.mma_y) {
-    dst_mma_y(P.ty.p, data, other, P.m[0], P.m[1], P.m[2], nc, wcs, s);
+    dst_mma_y(P.ty.p, data, other, P.m[0], P.m[1], P.m[2], nc, wcs, DstWait{P.polls, P.status}, s);
     return other;
   }
   launch_y(s, data, P.m[0], P.m[1], P.m[2], dev_plan(P.fy), nc, wcs);
@@ -1042,7 +1045,7 @@ double* y_pass(DirichletPlan& P, double* data, double* other, cudaStream_t s, in
 void x_inverse(DirichletPlan& P, const double* data, double* sol, cudaStream_t s, int nc, size_t scs) {
   const size_t wcs = (size_t)P.m[0] * P.m[1] * P.m[2];
   if (P.mma_x) {
-    dst_mma_x_inv(P.tx.p, data, sol, mma_box(P), nc, wcs, scs, s);
+    dst_mma_x_inv(P.tx.p, data, sol, mma_box(P), nc, wcs, scs, DstWait{P.polls, P.status}, s);
     return;
   }
   launch_x_inv(s, data, sol, plan_box(P), dev_plan(P.fx), CompStride{nc, 0, scs, wcs});
@@ -1317,6 +1320,7 @@ extern "C" int vpmg_dirichlet_static(const double* rhs, double* sol, const int d
   }
   const double scale = -hz2 * 4.0 / ((double)(m[0] + 1) * (double)(m[1] + 1));
   const CompStride cs{1, 0, 0, 0};
+  const DstWait wait{wait_polls(), nullptr};  // no handle: a wait that runs out shows as NaN alone
   try {
     int e = 0;
     const double f = std::frexp(-scale, &e);  // -scale = 2 f 2^(e - 1)
@@ -1332,16 +1336,17 @@ extern "C" int vpmg_dirichlet_static(const double* rhs, double* sol, const int d
       dst_mma_tables(t, c, s);
     }
     if (mx)
-      dst_mma_x_fwd(mtab + tb, e - 1, 1, rhs, sol, zero_bc != 0, work, db, 1.0 / hx2, 1.0 / hy2, 1.0 / hz2, 1, 0, 0, 0, s);
+      dst_mma_x_fwd(mtab + tb, e - 1, 1, rhs, sol, zero_bc != 0, work, db, 1.0 / hx2, 1.0 / hy2, 1.0 / hz2, 1, 0, 0, 0,
+                    wait, s);
     else
       launch_x_fwd(s, rhs, sol, zero_bc ? 1 : 0, work, b, px, 1.0 / hx2, 1.0 / hy2, 1.0 / hz2, scale, cs);
     double* g = my ? work2 : work;
-    if (my) dst_mma_y(mtab + 2 * tb, work, g, m[0], m[1], m[2], 1, 0, s);
+    if (my) dst_mma_y(mtab + 2 * tb, work, g, m[0], m[1], m[2], 1, 0, wait, s);
     else launch_y(s, work, m[0], m[1], m[2], py);
     thomas_launch(g, g, rinv, m, 1, 0, nullptr, s);
-    if (my) dst_mma_y(mtab + 2 * tb, g, work, m[0], m[1], m[2], 1, 0, s);
+    if (my) dst_mma_y(mtab + 2 * tb, g, work, m[0], m[1], m[2], 1, 0, wait, s);
     else launch_y(s, work, m[0], m[1], m[2], py);
-    if (mx) dst_mma_x_inv(mtab, work, sol, db, 1, 0, 0, s);
+    if (mx) dst_mma_x_inv(mtab, work, sol, db, 1, 0, 0, wait, s);
     else launch_x_inv(s, work, sol, b, px, cs);
   } catch (const Error& err) {
     return err.status;

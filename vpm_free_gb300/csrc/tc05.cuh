@@ -52,6 +52,16 @@ __device__ __forceinline__ void bar_wait(uint32_t bar, uint32_t parity, bool& de
   atomicExch(err, 1);
 }
 
+// The same with the limit as an argument and no word to the host: the caller
+// spreads `dead` over its CTA, drains it and reports.
+__device__ __forceinline__ void bar_wait(uint32_t bar, uint32_t parity, bool& dead, int polls) {
+  if (dead) return;
+  for (int i = 0; i < polls; ++i)
+    if (bar_try(bar, parity)) return;
+  dead = true;
+}
+constexpr int kPolls = 1 << 20;  // about a second
+
 // 16 bytes, zero-filled when !ok (src is not read then)
 __device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool ok) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");

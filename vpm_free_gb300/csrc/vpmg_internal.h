@@ -65,6 +65,13 @@ struct DBuf {
   size_t bytes() const { return n * sizeof(T); }
 };
 
+// A handle's device error word holds the largest of these since the last host
+// sync, which turns it into a status (check_particle_errors).
+enum { kErrOutside = 1, kErrCapacity = 2, kErrWait = 3 };
+// Polls after which a wait inside a kernel gives up; VPMG_WAIT_POLLS sets it
+// for the plans and operators made from then on.
+int wait_polls();
+
 // ------------------------------------------------------------- grids ----
 // A node grid: origin, spacing and node counts (1-based node i sits at
 // xmin + (i-1)*d, as everywhere in the reference).
@@ -107,12 +114,14 @@ struct DirichletPlan {
   DBuf<unsigned char> tx, txf, ty;
   int xf_shift = 0, xf_neg = 0;
   DBuf<double> tmp;
+  int polls = 0;          // of those passes' waits (wait_polls),
+  int* status = nullptr;  // and the error word that one which runs out sets
   DBuf<float2> rinv;  // float-float plans: reciprocal Thomas pivots, [k][q][p], float-float pairs
   DBuf<double> rinvd; // FP64: rows 0..m2/2-1 of them and the middle's constant (thomas_sweep)
   bool ready = false;
 };
 void dirichlet_prepare(DirichletPlan& P, const int dims[3], const int box[6], const double h[3], cudaStream_t s,
-                       int arith);
+                       int arith, int* status);
 // Interior of sol <- solution of Lap_h u = rhs with the box faces of sol as
 // boundary values (zero_bc = false) or zero (true; then the box faces of
 // sol are zeroed).  work: >= m0*m1*m2 doubles.
