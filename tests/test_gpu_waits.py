@@ -91,3 +91,31 @@ def test_steps_report_waits_that_run_out(gpulib, monkeypatch):
         up, gp = np.zeros((n, 3)), np.zeros((n, 3))
         h.vpm(xp, qp, up, gp, n, WhatToDo=2)
         assert np.isfinite(up).all() and np.isfinite(gp).all()
+
+
+@pytest.mark.parametrize("polls", [0, 1, 3, 10])
+def test_boundary_operator_reports_waits_that_run_out(gpulib, monkeypatch, polls):
+    """The weight tables' products (81^3 block of the 64^3 ring, 113^3 in
+    float-float; the lines of the former go by FFT)."""
+    from vpm_free_gb300 import workloads as W
+    V = gpulib
+    xp, qp, w = W.ring64() if gpulib.arith == "fp64" else W.scaled_ring(96)
+    cfg = V.VPMConfig.make(dpm=w["dpm"], box=w["box"])
+    n = xp.shape[0]
+
+    def step():
+        with V.VPM(cfg) as h:
+            h.define_sizes(xp)
+            assert h.farfield_stats()["on"]
+            up, gp = np.zeros((n, 3)), np.zeros((n, 3))
+            h.vpm(xp, qp, up, gp, n, WhatToDo=2)
+            return up
+    good = step()
+    monkeypatch.setenv("VPMG_WAIT_POLLS", str(polls))
+    try:
+        got = step()
+        assert polls > 0 and np.array_equal(got, good)
+    except V.VPMError as e:
+        assert e.status == -2 and "wait" in str(e)
+    monkeypatch.delenv("VPMG_WAIT_POLLS")
+    assert np.array_equal(step(), good)

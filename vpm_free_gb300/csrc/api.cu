@@ -175,10 +175,10 @@ void prepare(vpmg_handle* h) {
   // boundary operators: fine block (levels ilevmax), coarse (ilevmax-1); iyntree = 0 -> untreed sum
   const bool tree = h->cfg.iyntree == 1;
   boundary_prepare(h->bo_c, h->gco, tree ? std::max(s.ilevmax - 1, 0) : 0, h->op_budget, st, h->cfg.ibctyp, tree,
-                   h->arith);
+                   h->arith, h->bins.err.p);
   if (h->nblk == 1) {
     boundary_prepare(h->bo_bl, h->gbl, tree ? std::max(s.ilevmax, 0) : 0, h->op_budget, st, h->cfg.ibctyp, tree,
-                     h->arith);
+                     h->arith, h->bins.err.p);
     // YAPS maps
     YapsGeom Y;
     try {
@@ -204,7 +204,7 @@ void prepare(vpmg_handle* h) {
       h->g_blk[b] = make_grid(&Y.xbl[6 * (size_t)b], s.dpm, s.nnbl);
       h->bo_blk.push_back(std::make_unique<BoundaryOp>());
       boundary_prepare(*h->bo_blk[b], h->g_blk[b], tree ? std::max(s.ilevmax, 0) : 0, h->op_budget / h->nblk, st,
-                       h->cfg.ibctyp, tree, h->arith);
+                       h->cfg.ibctyp, tree, h->arith, h->bins.err.p);
     }
     h->ym.prepare(Y);
   }
@@ -1642,7 +1642,7 @@ int vpmg_pmesh(vpmg_handle* h, double* const sol[3], const double* const rhs[3],
       fill_zero(s0.p, 3 * n, h->stream);
       BoundaryOp bo;
       boundary_prepare(bo, g, itree == 1 ? levmax : 0, h->op_budget, h->stream, h->cfg.ibctyp, itree == 1, h->arith,
-                       true);
+                       h->bins.err.p, true);
       dirichlet_solve(dp, r.p, s0.p, true, w.p, h->stream, 3, n, n);
       boundary_panels(bo, g, s0.p, n, h->stream);
       double* sp[3] = {s.p, s.p + n, s.p + 2 * n};

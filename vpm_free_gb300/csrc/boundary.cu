@@ -982,7 +982,8 @@ static void walk_ready(BoundaryOp& B) {
 }
 
 void boundary_prepare(BoundaryOp& B, const Grid& g, int levmax, long long budget_bytes, cudaStream_t s, int ibctyp,
-                      bool tree, int arith, bool once) {
+                      bool tree, int arith, int* status, bool once) {
+  B.status = status;
   VPMG_CHECK(arith == VPMG_ARITH_FP64 || arith == VPMG_ARITH_FF48, VPMG_ERR_ARG, "unknown arithmetic");
   B.arith = arith;
   VPMG_CHECK(levmax >= 0 && levmax < kMaxLev - 1, VPMG_ERR_ARG, "levmax out of range");

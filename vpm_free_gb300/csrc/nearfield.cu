@@ -187,29 +187,36 @@ struct MmaArgs {
   const unsigned char* table;
   const unsigned short* dig;
   unsigned long long* acc;
-  int* failed;   // a wait ran out
+  int polls;     // limit of every wait
+  int* failed;   // set when one runs out (the boundary values are NaN then),
+  int* status;   // and the handle's error word
 };
 
 // Units are dealt longest first, forth and back over the CTAs.  Warps 0..7
 // gather the sources' digits and, at the end of a group of stages, read the
 // sums; warp 8 loads the tables, warp 9 issues the products.  They meet in
 // mbarriers only, and the gathers run ahead of the products across the ends of
-// groups and units.
+// groups and units.  Every wait has a limit: whoever waited in vain stops, the
+// others then wait in vain too, and all meet at the end, where the copies and
+// products in flight are waited for before the CTA ends.
 __global__ void __launch_bounds__(kThreads, 1) k_near_mma(const __grid_constant__ MmaArgs P) {
   extern __shared__ unsigned char near_sm[];
-  __shared__ __align__(8) uint64_t bars[2 * kStages + 2];
+  __shared__ __align__(8) uint64_t bars[3 * kStages + 3];
   __shared__ uint32_t tslot;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t sm = (tc05::smem_u32(near_sm) + 1023u) & ~1023u;
-  const uint32_t full = tc05::smem_u32(bars), empty = full + 8 * kStages, done = full + 16 * kStages, unread = done + 8;
+  const uint32_t full = tc05::smem_u32(bars), empty = full + 8 * kStages, tabled = full + 16 * kStages,
+                 done = full + 24 * kStages, unread = done + 8, drained = done + 16;
   if (warp == 0) tc05::tmem_alloc(tc05::smem_u32(&tslot), 512);
   if (tid == 0) {
     for (int i = 0; i < kStages; ++i) {
-      tc05::bar_init(full + 8 * i, kWorkers / 32 + 1);  // the gathering warps and the table's copy
+      tc05::bar_init(full + 8 * i, kWorkers / 32);  // the gathering warps
+      tc05::bar_init(tabled + 8 * i, 1);            // the table's copy
       tc05::bar_init(empty + 8 * i, 1);
     }
     tc05::bar_init(done, 1);
     tc05::bar_init(unread, kWorkers / 32);
+    tc05::bar_init(drained, 1);
     tc05::bar_init_fence();
   }
   tc05::fence_before();
@@ -218,6 +225,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_near_mma(const __grid_constant_
   const uint32_t tb = tslot;
   constexpr uint32_t idesc = tc05::idesc_f16(kRunsM, kCols);
   bool dead = false;
+  uint32_t loads = 0;  // tables copied by this thread
   auto unit_of = [&](int i) {  // this CTA's i-th unit
     const long long u = (long long)i * gridDim.x + ((i & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
     return u < P.nunit ? (int)u : -1;
@@ -225,14 +233,16 @@ __global__ void __launch_bounds__(kThreads, 1) k_near_mma(const __grid_constant_
   if (warp == kWorkers / 32) {
     if (lane == 0) {  // the tables
       uint32_t g = 0;
-      for (int i = 0, u; (u = unit_of(i)) >= 0; ++i) {
+      for (int i = 0, u; !dead && (u = unit_of(i)) >= 0; ++i) {
         const NearUnit U = P.units[u];
         const unsigned char* src = P.table + U.table + (size_t)U.k0 * kBytesB;
         for (int k = U.k0; k < U.k1; ++k, ++g, src += kBytesB) {
           const uint32_t st = g % kStages;
-          if (g >= (uint32_t)kStages) tc05::bar_wait(empty + 8 * st, ((g / kStages) - 1) & 1, dead, P.failed);
-          tc05::bar_expect(full + 8 * st, kBytesB);
-          tc05::bulk_load(sm + st * kStageBytes + kBytesA, src, kBytesB, full + 8 * st);
+          if (g >= (uint32_t)kStages) tc05::bar_wait(empty + 8 * st, ((g / kStages) - 1) & 1, dead, P.polls);
+          if (dead) break;
+          tc05::bar_expect(tabled + 8 * st, kBytesB);
+          tc05::bulk_load(sm + st * kStageBytes + kBytesA, src, kBytesB, tabled + 8 * st);
+          ++loads;
         }
       }
     }
@@ -240,13 +250,15 @@ __global__ void __launch_bounds__(kThreads, 1) k_near_mma(const __grid_constant_
   } else if (warp > kWorkers / 32) {
     if (lane == 0) {  // the products
       uint32_t g = 0, groups = 0;
-      for (int i = 0, u; (u = unit_of(i)) >= 0; ++i) {
+      for (int i = 0, u; !dead && (u = unit_of(i)) >= 0; ++i) {
         const int nst = P.units[u].k1 - P.units[u].k0;
         for (int k = 0; k < nst; ++k, ++g) {
           const uint32_t st = g % kStages;
           const int kin = k % P.group;
-          if (kin == 0 && groups > 0) tc05::bar_wait(unread, (groups - 1) & 1, dead, P.failed);
-          tc05::bar_wait(full + 8 * st, (g / kStages) & 1, dead, P.failed);
+          if (kin == 0 && groups > 0) tc05::bar_wait(unread, (groups - 1) & 1, dead, P.polls);
+          tc05::bar_wait(full + 8 * st, (g / kStages) & 1, dead, P.polls);
+          tc05::bar_wait(tabled + 8 * st, (g / kStages) & 1, dead, P.polls);
+          if (dead) break;
           tc05::fence_after();
           const uint32_t base = sm + st * kStageBytes;
           const uint64_t da = tc05::desc(base, kRunsM * 16), db = tc05::desc(base + kBytesA, kCols * 16);
@@ -299,7 +311,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_near_mma(const __grid_constant_
         const unsigned short* src = P.dig + (ok ? R.abase + (long long)row * R.Wp + cell : 0);
         const long long ds = ok ? (long long)R.nrow * R.Wp : 0;
         if (ik + 1 < in) e = __ldg(kl + ik + 1);
-        if (g >= (uint32_t)kStages) tc05::bar_wait(empty + 8 * st, ((g / kStages) - 1) & 1, dead, P.failed);
+        if (g >= (uint32_t)kStages) tc05::bar_wait(empty + 8 * st, ((g / kStages) - 1) & 1, dead, P.polls);
+        if (__any_sync(0xffffffffu, dead)) {
+          dead = true;
+          break;
+        }
         const uint32_t dst = sm + st * kStageBytes + adst;
 #pragma unroll
         for (int j = 0; j < kDigits; ++j) tc05::cp16(dst + j * (2 * kRunsM * 16), src + j * ds, ok);
@@ -320,7 +336,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_near_mma(const __grid_constant_
       ++ak;
       if (ak % P.group != 0 && ak != an) continue;
       // the group's exact sums join the running integers
-      tc05::bar_wait(done, groups & 1, dead, P.failed);
+      tc05::bar_wait(done, groups & 1, dead, P.polls);
+      if (__any_sync(0xffffffffu, dead)) {
+        dead = true;
+        break;
+      }
       ++groups;
       tc05::fence_after();
       const uint32_t ta = tb + ((uint32_t)(32 * (warp & 3)) << 16) + 32 * (warp >> 2);
@@ -368,7 +388,21 @@ __global__ void __launch_bounds__(kThreads, 1) k_near_mma(const __grid_constant_
     }
     tc05::cp_wait<0>();
   }
-  __syncthreads();
+  if (__syncthreads_or(dead)) {
+    bool late = false;  // these waits have the full limit
+    if (warp == kWorkers / 32 && lane == 0)
+      for (uint32_t i = 0; i < (uint32_t)kStages && i < loads; ++i)  // the last copy into each stage
+        tc05::bar_wait(tabled + 8 * i, ((loads - i - 1) / kStages) & 1, late, tc05::kPolls);
+    if (warp == kWorkers / 32 + 1 && lane == 0) {
+      tc05::commit(drained);
+      tc05::bar_wait(drained, 0, late, tc05::kPolls);
+    }
+    if (tid == 0) {
+      atomicExch(P.failed, 1);
+      if (P.status) atomicMax(P.status, kErrWait);
+    }
+    __syncthreads();
+  }
   if (warp == 0) tc05::tmem_free(tb, 512);
 }
 
@@ -536,6 +570,7 @@ void near_release(BoundaryOp& B) {
 bool near_prepare(BoundaryOp& B, const Grid& g, long long budget_bytes, cudaStream_t s) {
   near_release(B);
   NearField& F = B.near;
+  F.polls = wait_polls();
   const int L = B.levmax;
   NearPlan P;
   if (!build_near_plan(g.n, g.d, L, P)) return false;
@@ -782,6 +817,8 @@ void near_apply(BoundaryOp& B, cudaStream_t s) {
   A.dig = F.dig.p;
   A.acc = F.acc.p;
   A.failed = reinterpret_cast<int*>(F.acc.p + F.nacc) + 1;
+  A.polls = F.polls;
+  A.status = B.status;
   k_near_mma<<<std::min(F.nunit, F.sms), kThreads, kSmem, s>>>(A);
   VPMG_LAUNCHED();
   VPMG_CUDA(cudaGetLastError());

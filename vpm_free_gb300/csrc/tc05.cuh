@@ -42,18 +42,9 @@ __device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Waits with a limit (about a second); once a wait has run out, `dead` stays
-// set, *err tells the host, and every later wait returns at once.
-__device__ __forceinline__ void bar_wait(uint32_t bar, uint32_t parity, bool& dead, int* err) {
-  if (dead) return;
-  for (int i = 0; i < (1 << 20); ++i)
-    if (bar_try(bar, parity)) return;
-  dead = true;
-  atomicExch(err, 1);
-}
-
-// The same with the limit as an argument and no word to the host: the caller
-// spreads `dead` over its CTA, drains it and reports.
+// Waits with a limit; once a wait has run out, `dead` stays set and every later
+// wait of the thread returns at once.  The caller spreads `dead` over its CTA,
+// waits for what is in flight and reports.
 __device__ __forceinline__ void bar_wait(uint32_t bar, uint32_t parity, bool& dead, int polls) {
   if (dead) return;
   for (int i = 0; i < polls; ++i)

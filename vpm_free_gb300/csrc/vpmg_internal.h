@@ -217,7 +217,7 @@ struct NearField {
   int cell0[kNearLevels][7], ma[kNearLevels][6], mb[kNearLevels][6], Wp[kNearLevels][2][6];
   long long dbase[kNearLevels][2][6], abase[6];
   long long nacc = 0, stages = 0;   // sums; K = 16 products of one apply (tiles of 128 x 64, 28 digit pairs)
-  int edge = 0, group = 0, uc = 0, nunit = 0, sms = 0;
+  int edge = 0, group = 0, uc = 0, nunit = 0, sms = 0, polls = 0;
   DBuf<unsigned char> table;
   DBuf<unsigned short> dig;
   DBuf<unsigned long long> acc;
@@ -255,6 +255,7 @@ struct BoundaryOp {
   DBuf<float2> csrc_ff;                 // the same packed [cell][s0 s1 s2 0] in 8-byte words (doubles or float-float pairs)
   DBuf<unsigned> smax;                  // per component: high word of the largest panel source's magnitude
   long long budget = 0;                 // bytes that a recorded operator may take
+  int* status = nullptr;                // the handle's error word
   // panels: face geometry for the normal derivative
   DBuf<int> pan_face, pan_i, pan_j, pan_k;  // lower-corner node (0-based) of each panel
   // targets
@@ -294,7 +295,7 @@ struct BoundaryOp {
   long long bytes() const;
 };
 void boundary_prepare(BoundaryOp& B, const Grid& g, int levmax, long long budget_bytes, cudaStream_t s,
-                      int ibctyp, bool tree, int arith, bool once = false);  // once: applied a single time
+                      int ibctyp, bool tree, int arith, int* status, bool once = false);  // once: applied a single time
 // Sets B.ff and B.near up (the operator needs no recorded rows then) when the
 // cells of every level form uniform lattices on every face (ibctyp 2,
 // tree) and VPMG_FARFIELD is not "0"; set-up time, outside stream capture.
