@@ -1061,7 +1061,7 @@ void boundary_prepare(BoundaryOp& B, const Grid& g, int levmax, long long budget
   upload(B.tgt_node, tn); upload(B.tx, tx); upload(B.ty, ty); upload(B.tz, tz); upload(B.tgt_frame, tf);
   B.ntopd = B.nbound_lev[B.levmax];
   B.budget = budget_bytes;
-  B.precomputed = B.dense = B.transposed = false;
+  B.precomputed = B.dense = B.transposed = B.refused = false;
   B.nnz = 0;
   B.ndense_acc = 0;
   B.rowptr.release(); B.col.release(); B.w.release(); B.wtop.release(); B.dsum.release();
@@ -1142,6 +1142,7 @@ void boundary_record(BoundaryOp& B, cudaStream_t s) {
       B.precomputed = false;
     }
   }
+  B.refused = !B.precomputed;
   if (!B.precomputed) B.dense = false;  // the walk covers every level
   else B.wnodes.release();              // synchronised above
 }
@@ -1573,7 +1574,7 @@ __global__ void k_normal_deriv_T(const double* __restrict__ panelbar, int NX, in
 }  // namespace
 
 void boundary_transpose_prepare(BoundaryOp& B, cudaStream_t s) {
-  if (B.ff.on && !B.precomputed) boundary_record(B, s);
+  if (B.ff.on && !B.precomputed && !B.refused) boundary_record(B, s);
   if (B.precomputed) {  // at set-up: the transposes may be captured in graphs
     B.vff.ensure(4 * (size_t)B.ntarget);
     if (B.dense) B.dpart.ensure(3 * (size_t)B.ntopd * (((B.ntarget + 31) / 32 + kDenseTGroup - 1) / kDenseTGroup));

@@ -255,6 +255,7 @@ struct BoundaryOp {
   DBuf<float2> csrc_ff;                 // the same packed [cell][s0 s1 s2 0] in 8-byte words (doubles or float-float pairs)
   DBuf<unsigned> smax;                  // per component: high word of the largest panel source's magnitude
   long long budget = 0;                 // bytes that a recorded operator may take
+  bool refused = false;                 // recording did not fit: not tried again (captured transposes walk by now)
   int* status = nullptr;                // the handle's error word
   // panels: face geometry for the normal derivative
   DBuf<int> pan_face, pan_i, pan_j, pan_k;  // lower-corner node (0-based) of each panel
