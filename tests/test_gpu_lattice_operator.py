@@ -48,3 +48,17 @@ def test_spacings_below_the_panel_distance(gpulib, monkeypatch, h):
     if gpulib.arith != "fp64" and h != 1e-6:
         pytest.skip("one spacing in float-float")
     _same(gpulib, monkeypatch, (48,) * 3 if gpulib.arith == "fp64" else (96,) * 3, h)
+
+
+@pytest.mark.parametrize("spacings,on", [(1e4, True), (1e6, False)])
+def test_boxes_far_from_the_origin(gpulib, monkeypatch, spacings, on):
+    """Coordinates rounded to 1e-10 of a spacing decide weights of their own: such
+    boxes keep the walk's (tests/test_lattice_origin.py has the limit)."""
+    if gpulib.arith != "fp64":
+        pytest.skip("float-float handles of this size record")
+    org = (0.05 * spacings * 1.0000001,) * 3
+    got, tables = _solve(gpulib, monkeypatch, (48, 48, 48), 0.05, True, origin=org)
+    assert tables == on
+    rows, _ = _solve(gpulib, monkeypatch, (48, 48, 48), 0.05, False, origin=org)
+    for c in range(3):
+        assert rel_l2(got[c], rows[c]) <= (1e-13 if on else 0.0), c

@@ -452,6 +452,7 @@ bool farfield_prepare(BoundaryOp& B, const Grid& g, cudaStream_t s) {
   const int istep = 1 << B.levmax;
   for (int a = 0; a < 3; ++a)
     if ((g.n[a] - 1) % istep != 0 || g.n[a] - 1 <= istep) return false;  // dummy cells at the coarsest level
+  if (!lattice_exact(g.xmin, g.d, g.n)) return false;
   // faces' coarsest lattices, in the tree's face order
   int ma[6], mb[6], cell0[7];
   cell0[0] = 0;

@@ -3,12 +3,29 @@
 // cells lie in the digit arrays and where its sums go (nearfield.cu).
 // Compiled with -ffp-contract=off, as the other mesh geometry.
 #include <algorithm>
+#include <cmath>
 #include <map>
 #include <tuple>
 
 #include "near_host.h"
 
 namespace vpmg {
+
+bool lattice_exact(const double xmin[3], const double d[3], const int n[3]) {
+  for (int a = 0; a < 3; ++a) {
+    double node = 0.0, leaf = 0.0;
+    for (int i = 0; i < n[a]; ++i) {
+      // the tree's coordinates (build_tree_geometry)
+      const double x0 = xmin[a] + (double)i * d[a], x1 = xmin[a] + (double)(i + 1) * d[a];
+      node = std::max(node, std::fabs((x0 - xmin[a]) - (double)i * d[a]));
+      if (i == n[a] - 1) continue;
+      for (double c : {0.25 * (((x0 + x0) + x1) + x1), 0.25 * (((x1 + x1) + x0) + x0), 0.25 * (((x0 + x1) + x1) + x0)})
+        leaf = std::max(leaf, std::fabs((c - xmin[a]) - ((double)i + 0.5) * d[a]));
+    }
+    if (!(node + leaf <= 4e-11 * d[a])) return false;
+  }
+  return true;
+}
 
 bool build_near_plan(const int n3[3], const double d3[3], int L, NearPlan& P) {
   if (L < 1 || L >= kNearLevels) return false;

@@ -40,6 +40,13 @@ struct NearPlan {
 // false where the cells of some level are not a uniform lattice on every face
 bool build_near_plan(const int n3[3], const double d3[3], int L, NearPlan& P);
 
+// Whether the rounded coordinates of nodes and leaf centres are those of the
+// lattice closely enough for the lattice's weights to stand for the walk's: a
+// leaf centre is h / sqrt 2 or more from a node, so offsets that are off by 4e-11 h
+// along each axis change a weight by less than 1e-10 of it.  An origin further
+// than some 2e5 spacings from zero fails (unless its nodes are exact).
+bool lattice_exact(const double xmin[3], const double d[3], const int n[3]);
+
 // in-plane axes of face f (normal f / 2): the panels' fast and slow axes
 VPMG_HD int face_u(int f) { return (f >> 1) == 0 ? 1 : 0; }
 VPMG_HD int face_v(int f) { return (f >> 1) == 2 ? 1 : 2; }
