@@ -62,3 +62,14 @@ def test_boxes_far_from_the_origin(gpulib, monkeypatch, spacings, on):
     rows, _ = _solve(gpulib, monkeypatch, (48, 48, 48), 0.05, False, origin=org)
     for c in range(3):
         assert rel_l2(got[c], rows[c]) <= (1e-13 if on else 0.0), c
+
+
+@pytest.mark.parametrize("cells,thin", [((64, 64, 64), 80), ((48, 24, 56), 40), ((64, 48, 32), 80)])
+def test_faces_exactly_an_opening_radius_apart(gpulib, monkeypatch, cells, thin):
+    """At a spacing of 1/64 the sides' distance (80 or 40 spacings of the padded
+    block) is exactly ten cell sides of some level: no cell is opened across,
+    and the table of that pair of faces is empty."""
+    if gpulib.arith != "fp64":
+        pytest.skip("float-float handles of this size record")
+    assert any(c + 16 == thin for c in cells)
+    _same(gpulib, monkeypatch, cells, 1.0 / 64)

@@ -696,6 +696,7 @@ bool near_prepare(BoundaryOp& B, const Grid& g, long long budget_bytes, cudaStre
   per = std::max<long long>(per, kGroup);
   for (int t = 0; t < nt; ++t) {
     const NearTable& T = tabs[t];
+    if (!hw[t]) continue;  // no weight: a face exactly an opening radius away
     const int ew = std::max((int)(hw[t] >> 20), 1);
     const int q = std::max(0, (int)std::ceil(std::log2(std::max(sumw[t], 1e-300))) - ew + 1022 + 1);
     const int sh = F.uc - 48 - q - ew + 1077;
