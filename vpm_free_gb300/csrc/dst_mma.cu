@@ -498,6 +498,20 @@ int pieces_for(int n) { return ring_bytes(n) >= 2 * kSlot[1] ? 1 : ring_bytes(n)
 
 constexpr int kMaxDev = 64;
 bool g_attr[kMaxDev] = {false};
+int g_sms[kMaxDev] = {0};
+int current_device() {
+  int dev = 0;
+  VPMG_CUDA(cudaGetDevice(&dev));
+  VPMG_CHECK(dev >= 0 && dev < kMaxDev, VPMG_ERR_UNSUPPORTED, "device index beyond the per-device tables");
+  return dev;
+}
+// One CTA fills an SM and the tiles are dealt by a fixed stride: more CTAs than
+// SMs would run after the others' whole share.
+int sm_count() {
+  int& n = g_sms[current_device()];
+  if (!n) VPMG_CUDA(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, current_device()));
+  return n;
+}
 template <int MODE>
 void launch(DstArgs& A, cudaStream_t s) {
   A.ntile = (A.nlines + kLines - 1) / kLines;
@@ -507,7 +521,7 @@ void launch(DstArgs& A, cudaStream_t s) {
   const size_t sm = (size_t)kDigits * (dst_kp(A.n) / 8) * kCol + (size_t)A.slots * kSlot[A.np];
   const int tiles = A.ntile * A.nc;
   if (tiles <= 0) return;
-  k_dst_mma<MODE><<<std::min(tiles, 152), kThreads, sm, s>>>(A);
+  k_dst_mma<MODE><<<std::min(tiles, sm_count()), kThreads, sm, s>>>(A);
   VPMG_LAUNCHED();
   VPMG_CUDA(cudaGetLastError());
 }
@@ -535,9 +549,7 @@ size_t dst_mma_table_bytes(int n) {
 }
 
 void dst_mma_setup() {
-  int dev = 0;
-  VPMG_CUDA(cudaGetDevice(&dev));
-  VPMG_CHECK(dev >= 0 && dev < kMaxDev, VPMG_ERR_UNSUPPORTED, "device index beyond the per-device tables");
+  const int dev = current_device();
   if (!g_attr[dev]) {
     const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
     VPMG_CUDA(cudaFuncSetAttribute(k_dst_mma<0>, a, kSmemMax));
