@@ -519,7 +519,7 @@ def run_ours(args, dist):
                            "HBM: MEASURED_PEAKS.json hbm_gbs (of measured)")
     roof["hbm_frac"] = dom["hbm_frac"]
     tree = h.tree_stats()
-    tiles = h.dst_tiles()
+    tiles = {k: v or "products" for k, v in h.dst_tiles().items()}
     sizes_bl = list(h.sizes().nnbl)
     sizes_nn = list(h.sizes().nn)
     np_end = h.num_particles()

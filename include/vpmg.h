@@ -299,7 +299,8 @@ int vpmg_bench_kernel(vpmg_handle* h, int which, int reps, double* ms, double* f
 int vpmg_fp64_peak(vpmg_handle* h, double* tflops);
 /* DST tile shapes chosen by the set-up autotuner (line pairs per CTA, 2, 4
  * or 8) of the padded block's x and y transforms, the inner box's and the
- * coarse grid's, in that order.                                         */
+ * coarse grid's, in that order; 0 where the passes go as products on the
+ * tensor cores instead.                                                 */
 int vpmg_dst_tiles(const vpmg_handle* h, int pairs[6]);
 /* Memory limit (bytes) for the boundary operator's tables or recorded
  * lists; 0 = neither (walk the tree every step).  Default: 100 GiB.      */

@@ -488,7 +488,8 @@ class VPM:
         self._chk(self._L.vpmg_set_output(self._h, d, (1 if solution else 0) | (2 if hist else 0)))
 
     def dst_tiles(self):
-        """Autotuned DST tile shapes (line pairs per CTA) of the block x/y, inner-box x/y and coarse x/y plans."""
+        """Autotuned DST tile shapes (line pairs per CTA) of the block x/y, inner-box x/y and coarse x/y plans;
+        0 where a pass goes as products on the tensor cores."""
         t = (C.c_int * 6)()
         self._chk(self._L.vpmg_dst_tiles(self._h, t))
         keys = ["block_x", "block_y", "inner_x", "inner_y", "coarse_x", "coarse_y"]

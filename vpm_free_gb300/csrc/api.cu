@@ -1746,8 +1746,11 @@ int vpmg_fp64_peak(vpmg_handle* h, double* tflops) {
 int vpmg_dst_tiles(const vpmg_handle* h, int pairs[6]) {
   if (!h || !pairs) return VPMG_ERR_ARG;
   if (!h->prepared) return VPMG_ERR_STATE;
-  const vpmg::FFTPlan* p[6] = {&h->dp_bl.fx, &h->dp_bl.fy, &h->dp_inner.fx, &h->dp_inner.fy, &h->dp_c.fx, &h->dp_c.fy};
-  for (int i = 0; i < 6; ++i) pairs[i] = p[i]->pairs;
+  const vpmg::DirichletPlan* p[3] = {&h->dp_bl, &h->dp_inner, &h->dp_c};
+  for (int i = 0; i < 3; ++i) {
+    pairs[2 * i] = p[i]->mma_x ? 0 : p[i]->fx.pairs;
+    pairs[2 * i + 1] = p[i]->mma_y ? 0 : p[i]->fy.pairs;
+  }
   return VPMG_OK;
 }
 
