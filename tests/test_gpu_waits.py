@@ -13,7 +13,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 D = (0.05, 0.06, 0.04)
-SHAPE = (26, 103, 101)  # products along x (N = 100) and y (N = 102)
+SHAPE = (82, 103, 101)  # products along x (N = 100) and y (N = 102), also for one component (126 and 124 tiles)
 
 
 def _pmesh(V, rhs, sol):

@@ -529,14 +529,27 @@ void launch(DstArgs& A, cudaStream_t s) {
 }  // namespace
 
 // Lines of N = n + 1 >= 100 intervals whose digits leave room for the ring
-// (N <= 416), 1024 of them or more.  Below, the FFT passes are faster: a 64^3
-// step (N = 64 and 80) took 1.91 ms with them and 1.96 ms with products; at
-// N = 128 and 144 the two are level (a 64 x 128 x 96 solve 3.79 against
-// 3.84 ms; one component of 119 x 134 x 110 nodes, N = 120 and 135, 0.37 with
-// its tables made on the way against 0.53 ms), and at N = 256 and 272 three components' pass takes 0.90 and
-// 1.85 ms, the FFT's dense pass 1.88 ms at N = 256.
-bool dst_mma_wanted(int n, long long lines) {
-  return n + 1 >= 100 && pieces_for(n) && lines >= 1024;
+// (N <= 416), where the tiles of 64 lines fill the SMs: a tile takes as long
+// alone as among one per SM, the FFT's time grows with the lines.  Measured on
+// the two x passes of a dense one-component solve, FFT over products, at 35, 66,
+// 79, 108, 142, 195 and 302 tiles on 152 SMs:
+//   N = 100  0.88 0.95 1.04 1.10 1.16 1.13 1.24    N = 135  0.86 1.09 1.24 1.36 1.49 1.46 1.59
+//   N = 160  0.78 0.99 1.10 1.19 1.30 1.18 1.35    N = 165  0.90 1.27 1.32 1.50 1.67 1.51 1.70
+//   N = 256  0.80 1.06 1.11 1.19 1.28 1.15 1.29    N = 320  0.65 0.92 0.97 1.10 1.20 1.04 1.23
+// (odd N go by FFTs of twice the length).  Hence from 0.55 tiles per SM and
+// round, odd N from 0.35.  Tables made for one call weigh as 26 tiles: the
+// allocation-free solve of N = 129 takes 0.185 ms with products and 0.132 with
+// FFTs at 36 tiles, 0.202 and 0.167 at 63, 0.291 and 0.315 at 143.  Lines of 64
+// to 96 intervals gain nothing (a 64^3 step, N = 64 and 80, 1.91 ms by FFT and
+// 1.96 by products).  Where most lines are zero, as the right-hand sides of few
+// particles in long boxes, the FFT skips more of them: steps on 256 x 48 x 48 and
+// 400 x 48 x 48 cells lose 3 and 5 %.
+bool dst_mma_wanted(int n, long long lines, int nc, bool once) {
+  if (n + 1 < 100 || !pieces_for(n)) return false;
+  const double sms = sm_count();
+  const double tiles = (double)((lines + kLines - 1) / kLines * nc);
+  const double fill = (tiles - (once ? 26.0 : 0.0)) / (std::ceil(tiles / sms) * sms);
+  return fill >= ((n + 1) & 1 ? 0.35 : 0.55);
 }
 
 int wait_polls() {

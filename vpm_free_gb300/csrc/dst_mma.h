@@ -5,8 +5,10 @@
 
 namespace vpmg {
 
+// Whether `lines` lines of n points each, in nc components, go as products; once:
+// with tables made for this call alone.
+bool dst_mma_wanted(int n, long long lines, int nc, bool once);
 // Tables of a line length's sine matrix, for plans with p.n points.
-bool dst_mma_wanted(int n, long long lines);
 size_t dst_mma_table_bytes(int n);
 struct DstTable {
   unsigned char* T;

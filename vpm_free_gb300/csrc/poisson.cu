@@ -959,8 +959,8 @@ void dirichlet_prepare(DirichletPlan& P, const int dims[3], const int box[6], co
   VPMG_CHECK(std::max(smem_bytes(P.fx, 2), smem_bytes(P.fy, 2)) <= kMaxDstSmem, VPMG_ERR_UNSUPPORTED,
              "mesh too large for the shared-memory DST");
   raise_dst_smem(std::max(smem_bytes(P.fx, kJobPairs), smem_bytes(P.fy, kJobPairs)));  // the job lists' tiles
-  P.mma_x = arith == VPMG_ARITH_FP64 && dst_mma_wanted(P.m[0], (long long)P.m[1] * P.m[2]);
-  P.mma_y = arith == VPMG_ARITH_FP64 && dst_mma_wanted(P.m[1], (long long)P.m[0] * P.m[2]);
+  P.mma_x = arith == VPMG_ARITH_FP64 && dst_mma_wanted(P.m[0], (long long)P.m[1] * P.m[2], 3, false);
+  P.mma_y = arith == VPMG_ARITH_FP64 && dst_mma_wanted(P.m[1], (long long)P.m[0] * P.m[2], 3, false);
   if (P.mma_x) {
     int e = 0;
     const double f = std::frexp(std::fabs(dirichlet_scale(P)), &e);  // factor = 2 f 2^(e-1)
@@ -1299,10 +1299,15 @@ extern "C" int vpmg_dirichlet_static(const double* rhs, double* sol, const int d
     return VPMG_ERR_CUDA;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // the passes as products by the rule of the handle-based solves
+  // the passes as products by the rule of the handle-based solves, tables included
   constexpr size_t tb = kStaticTable * sizeof(double);
-  const bool mx = dst_mma_wanted(m[0], (long long)m[1] * m[2]) && dst_mma_table_bytes(m[0]) <= tb;
-  const bool my = dst_mma_wanted(m[1], (long long)m[0] * m[2]) && dst_mma_table_bytes(m[1]) <= tb;
+  bool mx = false, my = false;
+  try {
+    mx = dst_mma_wanted(m[0], (long long)m[1] * m[2], 1, true) && dst_mma_table_bytes(m[0]) <= tb;
+    my = dst_mma_wanted(m[1], (long long)m[0] * m[2], 1, true) && dst_mma_table_bytes(m[1]) <= tb;
+  } catch (const Error& err) {
+    return err.status;
+  }
   // tables and pivots are rebuilt on every call: the array keeps whatever the
   // previous call (possibly another grid) left in it
   const int nt = std::max(std::max(mx ? 0 : px.M, my ? 0 : py.M), std::max(px.N, py.N));
