@@ -1074,8 +1074,14 @@ void boundary_prepare(BoundaryOp& B, const Grid& g, int levmax, long long budget
   // set up than the walk: 65^3 nodes 16.6 against 11.3 ms, 97^3 27.2 against
   // 23.3, 129^3 (97 thousand targets) 40.5 against 39.2, 161^3 57.5 against 62.6.
   const bool walk_once = once && B.ntarget < kOnceTargets;
-  if (!walk_once && farfield_prepare(B, g, s)) return;
-  if (walk_once) farfield_release(B);
+  bool lattice = false;
+  try {
+    lattice = !walk_once && farfield_prepare(B, g, s);
+  } catch (const Error& e) {
+    if (e.status != VPMG_ERR_NOMEM) throw;  // no room for its arrays: as without them
+  }
+  if (lattice) return;
+  farfield_release(B);
   if (!once) boundary_record(B, s);
   if (!B.precomputed) walk_ready(B);
 }
