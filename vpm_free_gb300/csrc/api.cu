@@ -132,6 +132,15 @@ Grid make_grid(const double xb[6], const double d[3], const int n[3]) {
 void prepare(vpmg_handle* h) {
   const vpmg_sizes& s = h->sz;
   cudaStream_t st = h->stream;
+  // captured steps hold the sizes and the arrays of the mesh that was
+  h->prepared = false;
+  ++h->prepares;
+  if (h->graph.exec) {
+    VPMG_CUDA(cudaStreamSynchronize(st));
+    VPMG_CUDA(cudaGraphExecDestroy(h->graph.exec));
+    h->graph.exec = nullptr;
+  }
+  vpmg::hx::destroy_adjoint(h);
   h->gglob = make_grid(s.xbound, s.dpm, s.nn);
   h->gbl = make_grid(s.xbound_bl, s.dpm, s.nnbl);
   h->gco = make_grid(s.xbound_coarse, s.dpm_coarse, s.nn_coarse);
@@ -911,6 +920,7 @@ struct vpmg_batch {
     int remesh = -1;
   };
   std::vector<vpmg_handle*> hs;
+  std::vector<unsigned long long> prepares;  // of each problem when the units were made
   std::vector<std::unique_ptr<Unit>> units;
   // replay order of the units within a step: 0 concurrent (each unit on its
   // leader's stream), 1 one after another on one stream, -1 chosen by timing
@@ -1106,6 +1116,7 @@ int vpmg_batch_create(vpmg_handle* const* hs, int n, int flags, vpmg_batch** out
     }
   });
   if (rc != VPMG_OK) return rc;
+  for (vpmg_handle* h : b->hs) b->prepares.push_back(h->prepares);
   *out = b.release();
   return VPMG_OK;
 }
@@ -1130,6 +1141,11 @@ int vpmg_batch_step(vpmg_batch* b, int nsteps, double dt, int do_remesh, double*
   vpmg_handle* h0 = b->hs[0];
   return guarded(h0, [&] {
     VPMG_CHECK(nsteps <= kHistCap, VPMG_ERR_ARG, "too many steps for one batched run");
+    for (auto& u : b->units)
+      if (u->m.size() > 1)
+        for (int i : u->m)
+          VPMG_CHECK(b->hs[i]->prepares == b->prepares[i], VPMG_ERR_STATE,
+                     "a problem of a group was sized anew: make the batch again");
     for (auto& u : b->units) {
       if (u->m.size() == 1) {
         vpmg_handle* h = b->hs[u->m[0]];

@@ -22,6 +22,7 @@ struct vpmg_handle {
   long long launches = 0;
   vpmg_sizes sz{};
   bool sized = false, prepared = false;
+  unsigned long long prepares = 0;  // how often the mesh's arrays and plans were made: graphs of an earlier time are stale
   long long op_budget = 100LL << 30;
   int arith = VPMG_ARITH_FP64;  // arithmetic of the heavy kernels (vpmg_set_arithmetic)
   // grids
