@@ -283,14 +283,16 @@ int vpmg_batch_destroy(vpmg_batch* b);
 /* Replays one kernel of the last step `reps` times between CUDA events on
  * the handle's stream (instrumentation for roofline figures).
  *   which = 0: boundary operator apply on the fine block (recorded operator
- *              or the tree walk), 1: one inner-box Dirichlet solve (5
- *              kernels), 2: deposition gather, 3: velocity curl, 4:
- *              stretching, 5: mesh-to-particle gather, 6: one component of
- *              the padded block's zero-BC solve evaluated where it is read,
- *              7: the remesh's |w| flags and their scan, 8: the sort by
- *              cell and the particle records on the global mesh.
- * Outputs: mean device ms per replay, algorithmic FP64 flops (an FMA
- * counts 2) and DRAM bytes per replay (figures of the algorithm, not
+ *              or the tree walk), 1: the inner-box Dirichlet solve of the
+ *              three components (5 kernels), 2: deposition gather, 3:
+ *              velocity curl, 4: stretching, 5: mesh-to-particle gather, 6:
+ *              the padded block's zero-BC solve of the three components
+ *              evaluated where it is read, 7: the remesh's |w| flags and
+ *              their scan, 8: the sort by cell and the particle records on
+ *              the global mesh.
+ * Outputs: mean device ms per replay, FP64 flops that run on the FP64
+ * units (an FMA counts 2; passes as products on the tensor cores count
+ * none) and DRAM bytes per replay (figures of the algorithm, not
  * counters).  The replay writes only scratch buffers, the particles'
  * UP/GP and the binning arrays, all rewritten by the next step.          */
 int vpmg_bench_kernel(vpmg_handle* h, int which, int reps, double* ms, double* flops, double* bytes);

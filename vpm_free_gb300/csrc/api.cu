@@ -1284,13 +1284,18 @@ int vpmg_bench_kernel(vpmg_handle* h, int which, int reps, double* ms, double* f
              4.0 * (double)(F.S2.bytes() + F.X.bytes() + F.Z.bytes() + F.Sw.bytes() + F.T.bytes());
       }
     } else if (which == 1) {
-      h->bench_scratch.ensure(NB);
+      // the inner box's solve of the three components, as the step runs it
+      h->bench_scratch.ensure(3 * NB);
       double* o = h->bench_scratch.p;
-      f = [h, o, st] { dirichlet_solve(h->dp_inner, h->rhs_bl.p, o, true, h->work.p, st); };
+      f = [h, o, NB, st] { dirichlet_solve(h->dp_inner, h->rhs_bl.p, o, true, h->work.p, st, 3, NB, NB); };
       const DirichletPlan& P = h->dp_inner;
       const double nint = (double)P.m[0] * P.m[1] * P.m[2];
-      fl = nint * (5.0 * std::log2(2.0 * (P.m[0] + 1)) + 5.0 * std::log2(2.0 * (P.m[1] + 1)) + 9.0);
-      by = 16.0 * (double)NB;
+      // FP64: the sweep, and both passes along an axis that goes by FFT (the
+      // products run on the tensor cores).  Every pass reads and writes its
+      // array, the sweep twice, with half a table of pivots each way.
+      fl = 3.0 * nint * ((P.mma_x ? 0.0 : 5.0 * std::log2(2.0 * (P.m[0] + 1))) +
+                         (P.mma_y ? 0.0 : 5.0 * std::log2(2.0 * (P.m[1] + 1))) + 4.0);
+      by = 8.0 * nint * (3.0 * (4 * 2 + 4) + 1.0);
     } else if (which == 2) {
       h->bench_scratch.ensure(3 * N);
       double* o[3] = {h->bench_scratch.p, h->bench_scratch.p + N, h->bench_scratch.p + 2 * N};
@@ -1344,16 +1349,19 @@ int vpmg_bench_kernel(vpmg_handle* h, int which, int reps, double* ms, double* f
       fl = P * w * w * w * 13.0;              // per visit: 1 multiply + 6 FMAs
       by = 80.0 * P + 48.0 * (double)N;        // X, vol read, UP/GP written; 6 fields read once
     } else if (which == 6) {
-      // one component of the padded block's zero-BC solve, evaluated where it is read
+      // the padded block's zero-BC solve of the three components, evaluated where it is read
       VPMG_CHECK(h->nblk == 1 && h->bsolve.ready, VPMG_ERR_UNSUPPORTED, "one-block handle needed");
-      h->bench_scratch.ensure(NB);
+      h->bench_scratch.ensure(3 * NB);
       double* o = h->bench_scratch.p;
-      f = [h, o, NB, st] { block_solve_zero_bc(h->bsolve, h->dp_bl, h->rhs_bl.p, NB, o, NB, 1, st); };
+      f = [h, o, NB, st] { block_solve_zero_bc(h->bsolve, h->dp_bl, h->rhs_bl.p, NB, o, NB, 3, st); };
       const DirichletPlan& P = h->dp_bl;
       const double nint = (double)P.m[0] * P.m[1] * P.m[2];
-      // forward x and y transforms, the Thomas sweep, 8 x-layer and 8 y-layer dot products
-      fl = nint * (2.5 * std::log2(2.0 * (P.m[0] + 1)) + 2.5 * std::log2(2.0 * (P.m[1] + 1)) + 4.0 + 32.0);
-      by = 8.0 * nint * 5.0;  // RHS read, transform written, sweep read + written, dots read
+      // FP64: forward passes that go by FFT, the sweep, four pairs of mirrored
+      // layers along x and along y (one FMA per pair and value).  Passes, sweep
+      // and pivots as above, the transform read for either set of layers.
+      fl = 3.0 * nint * ((P.mma_x ? 0.0 : 2.5 * std::log2(2.0 * (P.m[0] + 1))) +
+                         (P.mma_y ? 0.0 : 2.5 * std::log2(2.0 * (P.m[1] + 1))) + 4.0 + 16.0);
+      by = 8.0 * nint * (3.0 * (2 * 2 + 4 + 2) + 1.0);
     } else if (which == 7) {
       // the remesh's |w| flags and their exclusive scan on the remesh grid
       const Grid gr = hx::remesh_grid(h);
