@@ -38,7 +38,7 @@ def _same(gpulib, monkeypatch, cells, h, **kw):
         assert rel_l2(a[c], b[c]) <= (1e-13 if gpulib.arith == "fp64" else 1e-12), (c, rel_l2(a[c], b[c]))
 
 
-# 48^3 cells: 25 thousand boundary nodes of the padded block; 96^3: 76 thousand,
+# 48^3 cells: 25 thousand boundary nodes of the padded block; 96^3: 75 thousand,
 # where float-float handles take the tables too
 @pytest.mark.parametrize("h", [1.3e-5, 1e-5, 1e-6, 1.25e-7, 1e-8])
 def test_spacings_below_the_panel_distance(gpulib, monkeypatch, h):

@@ -8,10 +8,16 @@
 // product a value needs none.  The line becomes 55-bit integers at the scale
 // of its own largest magnitude, the folds are integer sums (no rounding), and
 // seven balanced base-256 digits of them and of the matrix, held as FP16, meet
-// in 28 digit products whose FP32 sums are exact (K <= 224: at most 224 x 128
-// x 75 on average per digit pair, six pairs below 2^24); the seven sums join
-// as one integer, rounded once to double.  The error is that of rounding the
-// line's values and the sines to 55 bits.
+// in the 28 of 49 digit products with i + j <= 6, accumulated in FP32 by i + j.
+// The six sums up to i + j = 5 are exact: with every digit of the line at its
+// largest (128, the top one 256) and the digits of the sine matrices as they
+// are, for all N up to 417 and factors in [1, 2), they stay below 0.91 2^24.
+// The seventh can reach 1.01 2^24; its rounding is below the nine bits that the
+// joined integer drops.  That integer is rounded once to double.  The error is
+// that of rounding the line's values and the sines to 55 bits and of the dropped
+// products, of which the six with i + j = 7 reach 2^-53.4 of a product's scale at
+// worst; as digits of either sign they are a seventh of that (root mean square)
+// and add up as the root of K.
 //
 // Tile: 64 lines (columns) x 128 outputs of one parity (rows), seven
 // accumulators of 64 columns in tensor memory; the lines' digits stay in
@@ -433,7 +439,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_dst_mma(const __grid_constant__
             const int line = cb + 8 * c8 + i;
             auto q = [&](int d) { return (long long)__float2int_rn(__uint_as_float(v[d][i])); };
             // integers: values 2^(1077 - E), sines 2^55, the sums in units of
-            // 2^48; |sum| < 224 2^56 2^56 / 2^48, so it fits with 9 bits dropped
+            // 2^48; |sum| < 208 2^56 2^56 / 2^48, so it fits with 9 bits dropped
             const long long hi = (q(0) << 32) + (q(1) << 24) + (q(2) << 16) + (q(3) << 8) + q(4);
             const long long lo = (q(5) << 8) + q(6);
             const long long V = (hi << 7) + ((lo + 256) >> 9);

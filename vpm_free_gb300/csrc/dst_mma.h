@@ -1,4 +1,4 @@
-// dst_mma.h -- the DST-I passes of the FP64 Dirichlet solves as exact
+// dst_mma.h -- the DST-I passes of the FP64 Dirichlet solves as integer
 // products on the tensor cores (dst_mma.cu).
 #pragma once
 #include "vpmg_internal.h"

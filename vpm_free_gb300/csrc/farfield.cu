@@ -444,9 +444,10 @@ bool farfield_prepare(BoundaryOp& B, const Grid& g, cudaStream_t s) {
   // the coarse grid recorded a 64^3 step takes 1.94 ms and a 32^3 driver call
   // 1.23 ms, by FFT and tables 1.99 and 1.31 ms.  Float-float rows (their sums
   // run on the FP32 units) hold out longer: a step of the ring takes 1.44 ms
-  // with them and 1.47 by FFT and tables at 64^3 (39 thousand nodes), 2.58 and
-  // 2.34 at 96^3 (86 thousand), and of the leapfrogging rings 23.3 and 17.7 at
-  // 256^3.  The transforms and tables are FP64 and 55-bit integers in either
+  // with them and 1.47 by FFT and tables at 64^3 (38 thousand nodes), 2.58 and
+  // 2.34 at 96^3 (75 thousand), and of the leapfrogging rings 23.3 and 17.7 at
+  // 256^3; between them, with the coarse grid by FFT and tables as well, 1.51 and
+  // 1.49 at 72^3 (46 thousand) and 1.68 and 1.59 at 80^3 (55 thousand).  The transforms and tables are FP64 and 55-bit integers in either
   // arithmetic.
   if (B.ntarget < (B.arith == VPMG_ARITH_FF48 ? kMinTargetsFF : kMinTargets)) return false;
   const int istep = 1 << B.levmax;

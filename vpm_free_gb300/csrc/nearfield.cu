@@ -29,8 +29,9 @@
 // FP16.  Digit products d_i e_j with i + j <= 6 (28 of 49) accumulate in
 // seven FP32 accumulators by i + j, exact while below 2^24, which 256 cells
 // guarantee (checked against the table's digits); then the seven sums join
-// as a 64-bit integer per node.  Dropped terms are below 2^-54 of a
-// product's scale, less than the rounding of an FP64 FMA chain.  Integer sums
+// as a 64-bit integer per node.  Of the dropped products the six with i + j = 7
+// reach 2^-53.4 of a product's scale at worst; as digits of either sign they are a
+// seventh of that (root mean square), below the rounding of an FP64 FMA chain.  Integer sums
 // do not depend on the order, so units of work are dealt dynamically and
 // added with 64-bit integer atomics, and results stay the same bits.
 //

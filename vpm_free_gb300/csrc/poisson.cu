@@ -5,6 +5,9 @@
 // discrete solution of  Lap_h u = RHS  on a node box with Dirichlet values.
 //
 // Method (GB300-first: FP64 is the scarce resource, ~1.2 TFLOP/s):
+// FP64 lines of 100 to 417 intervals, enough of them to fill the SMs, go through
+// passes 1, 2 and 4 as products on the tensor cores (dst_mma.cu; its y pass writes
+// to a second array).  The others, and float-float, by FFT:
 //   1. x pass: fold the boundary values into the RHS of the first/last
 //      interior layers, DST-I along x, scaled for the later inverse.  For
 //      even N = n+1 the DST-I is computed in its real-symmetric form: the

@@ -175,12 +175,12 @@ struct PanelFrame {
   double E1[3], E2[3], E3[3], S[4], T[4], D[4], diag, area;
 };
 
-// The coarsest tree level of a recorded operator evaluated as convolutions
-// on the face lattices (farfield.cu).  Every target sums every coarsest cell
+// The coarsest tree level of an operator on uniform lattices evaluated as
+// convolutions on them (farfield.cu).  Every target sums every coarsest cell
 // (the opened ones included) by FFTs: between parallel faces a 2-D
 // convolution, between perpendicular faces a 1-D convolution along their
-// shared axis and a dense sum over the other two; the cells each target
-// opened are then subtracted as sparse correction rows.
+// shared axis and a dense sum over the other two; the tables below take the
+// cells each target opened back out.
 struct FarFieldAxis {    // complex FFT of length P = 2^a 3^b along one axis
   int P = 0, nst = 0, npair = 1;
   int radix[16];
