@@ -78,22 +78,39 @@ __device__ double2* ff_fft(double2* a, double2* b, const AxisDev& p, int npair) 
   return a;
 }
 
+// Components 0 and 1 share complex transforms, where the larger one's rounding
+// would be the smaller one's error: component 1 enters times 2^pair_shift, at the
+// other's exponent, and comes out times its inverse (both exact).  A component
+// that is not finite enters as zero; k_ff_gather makes its sums NaN.
+__device__ __forceinline__ int pair_shift(const unsigned* smax) {
+  const int e0 = (int)(smax[0] >> 20), e1 = (int)(smax[1] >> 20);
+  if (!smax[0] || !smax[1] || e0 >= 0x7FF || e1 >= 0x7FF) return 0;
+  return max(-1000, min(1000, e0 - e1));
+}
+__device__ __forceinline__ double power_of_two(int k) { return __hiloint2double((1023 + k) << 20, 0); }
+__device__ __forceinline__ double enter(double v, int c, const unsigned* smax) {
+  if ((smax[c] >> 20) >= 0x7FF) return 0.0;
+  return c == 1 ? v * power_of_two(pair_shift(smax)) : v;
+}
+
 // One batch of line transforms.  Line l = q * nl2 + r (r < nl2) reads from
 // sbase + q * sqs + r * sls and writes to dbase + q * dqs + r * dls.
 // Element e of the transform: dense (sparse = 0): source index e * ses for
 // e < scnt, zero beyond; lattice (sparse = 1): nonzero only at
 // e = soff + b * sstep (b < scnt), from source index b * ses.  A real
-// source (real = 1) reads doubles: re at the index, im at index + ioff
-// (ioff < 0: im = 0).  The first nkeep outputs are written (stride des).
+// source (real = 1) reads doubles: re, of component comp + q, at the index, im,
+// of component 1, at index + ioff (ioff < 0: im = 0).  The first nkeep outputs
+// are written (stride des).
 struct FFJob {
   long long sbase, sqs, sls, ses, dbase, dqs, dls, des, ioff;
-  int nlines, nl2, nkeep, soff, sstep, scnt, sparse, real, axis;
+  int nlines, nl2, nkeep, soff, sstep, scnt, sparse, real, comp, axis;
 };
 struct FFJobs {
   FFJob j[kFFJobs];
   AxisDev ax[3];
   const double2* src;
   const double* srcr;
+  const unsigned* smax;  // of the real sources' components
   double2* dst;
 };
 
@@ -125,7 +142,9 @@ __global__ void __launch_bounds__(kFFThreads) k_ff_lines(const __grid_constant__
         const int l = l0 + li;
         const long long idx = jb.sbase + (long long)(l / jb.nl2) * jb.sqs + (long long)(l % jb.nl2) * jb.sls +
                               (long long)b * jb.ses;
-        if (jb.real) v = make_double2(J.srcr[idx], jb.ioff >= 0 ? J.srcr[idx + jb.ioff] : 0.0);
+        if (jb.real)
+          v = make_double2(enter(J.srcr[idx], jb.comp + l / jb.nl2, J.smax),
+                           jb.ioff >= 0 ? enter(J.srcr[idx + jb.ioff], 1, J.smax) : 0.0);
         else v = J.src[idx];
       }
     }
@@ -277,7 +296,7 @@ __global__ void k_ff_gather(const __grid_constant__ GatherDev D, const int* __re
     c1 -= q.y;
     c2 += (i & 1) ? -r.y : r.x;
   }
-  double cs[3] = {c0, c1, c2};
+  double cs[3] = {c0, c1 * power_of_two(-pair_shift(smax)), c2};
   const int Nu = D.N[ax_u(f)], Nv = D.N[ax_v(f)];
   const long long kb = D.crow[6 * (size_t)t], ke = D.crow[6 * (size_t)t + 6];
 #pragma unroll
@@ -287,7 +306,7 @@ __global__ void k_ff_gather(const __grid_constant__ GatherDev D, const int* __re
     const long long n = (long long)acc[D.acc[f] + ((long long)c * Nv + w) * Nu + u];
     double near = scalbn((double)n, D.uc + max(es, 1) - 1077);
     if (es >= 0x7FF || *failed) near = __longlong_as_double(0x7FF8000000000000ll);
-    double v = cs[c] + near;
+    double v = smax[c] ? cs[c] + near : 0.0;  // no source at all: not the other component's rounding
     for (long long k = kb; k < ke; ++k) v = fma(D.cw[k], D.src[(size_t)c * D.ncell + D.ccol[k]], v);
     D.sol[c][node] += -v * D.inv_pi4;
   }
@@ -383,7 +402,7 @@ AxisDev axis_dev(const FarFieldAxis& A) {
 
 // Runs a list of line-transform jobs, at most kFFJobs per launch.
 void run_jobs(const FarField& F, const std::vector<FFJob>& jobs, const double2* src, const double* srcr, double2* dst,
-              cudaStream_t s) {
+              cudaStream_t s, const unsigned* smax = nullptr) {
   for (size_t j0 = 0; j0 < jobs.size(); j0 += kFFJobs) {
     FFJobs J;
     const int nj = (int)std::min<size_t>(kFFJobs, jobs.size() - j0);
@@ -396,6 +415,7 @@ void run_jobs(const FarField& F, const std::vector<FFJob>& jobs, const double2* 
     for (int a = 0; a < 3; ++a) J.ax[a] = axis_dev(F.ax[a]);
     J.src = src;
     J.srcr = srcr;
+    J.smax = smax;
     J.dst = dst;
     k_ff_lines<<<dim3((unsigned)gx, (unsigned)nj), kFFThreads, kFFSmem, s>>>(J);
     VPMG_LAUNCHED();
@@ -636,13 +656,13 @@ void farfield_apply(BoundaryOp& B, double* const sol[3], cudaStream_t s) {
       j.axis = au;
       j.sbase = (long long)(phi ? 2 : 0) * NC + top0 + F.cell0[f];
       j.sqs = 0; j.sls = ma[f]; j.ses = 1;
-      j.real = 1; j.ioff = phi ? -1 : NC;
+      j.real = 1; j.ioff = phi ? -1 : NC; j.comp = phi ? 2 : 0;
       j.sparse = 1; j.soff = h2; j.sstep = istep; j.scnt = ma[f];
       j.dbase = F.t_off[f][phi]; j.dqs = 0; j.dls = Pu; j.des = 1;
       j.nlines = mb[f]; j.nl2 = mb[f]; j.nkeep = Pu;
       jobs.push_back(j);
     }
-  run_jobs(F, jobs, nullptr, B.csrc.p, F.T.p, s);
+  run_jobs(F, jobs, nullptr, B.csrc.p, F.T.p, s, B.smax.p);
   // 2. columns: column w_u of face f has the rows' values at v = b * istep + istep / 2
   jobs.clear();
   for (int f = 0; f < 6; ++f)
@@ -696,13 +716,13 @@ void farfield_apply(BoundaryOp& B, double* const sol[3], cudaStream_t s) {
       j.sbase = top0 + F.cell0[G]; j.sqs = NC;
       j.sls = ws ? 1 : ma[G];   // next cell across w
       j.ses = ws ? ma[G] : 1;   // next cell along w
-      j.real = 1; j.ioff = -1;
+      j.real = 1; j.ioff = -1; j.comp = 0;
       j.sparse = 1; j.soff = h2; j.sstep = istep; j.scnt = nalong;
       j.dbase = F.sw_off[G][ws]; j.dqs = (long long)nacross * Pw; j.dls = Pw; j.des = 1;
       j.nlines = 3 * nacross; j.nl2 = nacross; j.nkeep = Pw / 2 + 1;
       jobs.push_back(j);
     }
-  run_jobs(F, jobs, nullptr, B.csrc.p, F.Sw.p, s);
+  run_jobs(F, jobs, nullptr, B.csrc.p, F.Sw.p, s, B.smax.p);
   // 7. the dense sums per frequency, packed for the inverse transforms
   PerpDev QD{};
   long long maxthreads = 0;
