@@ -202,17 +202,17 @@ struct MmaArgs {
 // products in flight are waited for before the CTA ends.
 __global__ void __launch_bounds__(kThreads, 1) k_near_mma(const __grid_constant__ MmaArgs P) {
   extern __shared__ unsigned char near_sm[];
-  __shared__ __align__(8) uint64_t bars[3 * kStages + 3];
+  __shared__ __align__(8) uint64_t bars[2 * kStages + 3];
+  __shared__ uint32_t arrived[kWorkers / 32];  // stages that each gathering warp has filled
   __shared__ uint32_t tslot;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t sm = (tc05::smem_u32(near_sm) + 1023u) & ~1023u;
-  const uint32_t full = tc05::smem_u32(bars), empty = full + 8 * kStages, tabled = full + 16 * kStages,
-                 done = full + 24 * kStages, unread = done + 8, drained = done + 16;
+  const uint32_t full = tc05::smem_u32(bars), empty = full + 8 * kStages, done = full + 16 * kStages, unread = done + 8,
+                 drained = done + 16;
   if (warp == 0) tc05::tmem_alloc(tc05::smem_u32(&tslot), 512);
   if (tid == 0) {
     for (int i = 0; i < kStages; ++i) {
-      tc05::bar_init(full + 8 * i, kWorkers / 32);  // the gathering warps
-      tc05::bar_init(tabled + 8 * i, 1);            // the table's copy
+      tc05::bar_init(full + 8 * i, kWorkers / 32 + 1);  // the gathering warps and the table's copy
       tc05::bar_init(empty + 8 * i, 1);
     }
     tc05::bar_init(done, 1);
@@ -241,8 +241,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_near_mma(const __grid_constant_
           const uint32_t st = g % kStages;
           if (g >= (uint32_t)kStages) tc05::bar_wait(empty + 8 * st, ((g / kStages) - 1) & 1, dead, P.polls);
           if (dead) break;
-          tc05::bar_expect(tabled + 8 * st, kBytesB);
-          tc05::bulk_load(sm + st * kStageBytes + kBytesA, src, kBytesB, tabled + 8 * st);
+          tc05::bar_expect(full + 8 * st, kBytesB);
+          tc05::bulk_load(sm + st * kStageBytes + kBytesA, src, kBytesB, full + 8 * st);
           ++loads;
         }
       }
@@ -258,7 +258,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_near_mma(const __grid_constant_
           const int kin = k % P.group;
           if (kin == 0 && groups > 0) tc05::bar_wait(unread, (groups - 1) & 1, dead, P.polls);
           tc05::bar_wait(full + 8 * st, (g / kStages) & 1, dead, P.polls);
-          tc05::bar_wait(tabled + 8 * st, (g / kStages) & 1, dead, P.polls);
           if (dead) break;
           tc05::fence_after();
           const uint32_t base = sm + st * kStageBytes;
@@ -388,12 +387,20 @@ __global__ void __launch_bounds__(kThreads, 1) k_near_mma(const __grid_constant_
       }
     }
     tc05::cp_wait<0>();
+    if (lane == 0) arrived[warp] = ga;
   }
   if (__syncthreads_or(dead)) {
     bool late = false;  // these waits have the full limit
     if (warp == kWorkers / 32 && lane == 0)
-      for (uint32_t i = 0; i < (uint32_t)kStages && i < loads; ++i)  // the last copy into each stage
-        tc05::bar_wait(tabled + 8 * i, ((loads - i - 1) / kStages) & 1, late, tc05::kPolls);
+      // the last copy into each stage, with the arrivals of the gathering warps
+      // that stopped before it (one at most: a stage is loaded again only once
+      // all of them have filled it and its products are done)
+      for (uint32_t i = 0; i < (uint32_t)kStages && i < loads; ++i) {
+        const uint32_t last = (loads - i - 1) / kStages;
+        for (int w = 0; w < kWorkers / 32; ++w)
+          if (arrived[w] <= i + last * kStages) tc05::bar_arrive(full + 8 * i);
+        tc05::bar_wait(full + 8 * i, last & 1, late, tc05::kPolls);
+      }
     if (warp == kWorkers / 32 + 1 && lane == 0) {
       tc05::commit(drained);
       tc05::bar_wait(drained, 0, late, tc05::kPolls);
