@@ -88,10 +88,11 @@ __device__ __forceinline__ int pair_shift(const unsigned* smax) {
   return max(-1000, min(1000, e0 - e1));
 }
 __device__ __forceinline__ double power_of_two(int k) { return __hiloint2double((1023 + k) << 20, 0); }
-__device__ __forceinline__ double enter(double v, int c, const unsigned* smax) {
+__device__ __forceinline__ double enter_factor(int c, const unsigned* smax) {
   if ((smax[c] >> 20) >= 0x7FF) return 0.0;
-  return c == 1 ? v * power_of_two(pair_shift(smax)) : v;
+  return c == 1 ? power_of_two(pair_shift(smax)) : 1.0;
 }
+__device__ __forceinline__ double enter(double v, double factor) { return factor != 0.0 ? v * factor : 0.0; }
 
 // One batch of line transforms.  Line l = q * nl2 + r (r < nl2) reads from
 // sbase + q * sqs + r * sls and writes to dbase + q * dqs + r * dls.
@@ -127,6 +128,12 @@ __global__ void __launch_bounds__(kFFThreads) k_ff_lines(const __grid_constant__
   // consecutive threads: consecutive elements of a line when the source
   // elements are contiguous, else consecutive lines
   const bool along = jb.ses == 1;
+  double f0 = 1.0, f1 = 1.0, f2 = 1.0;
+  if (jb.real) {
+    f0 = enter_factor(0, J.smax);
+    f1 = enter_factor(1, J.smax);
+    f2 = enter_factor(2, J.smax);
+  }
   for (int t = threadIdx.x; t < npair * P; t += blockDim.x) {
     const int li = along ? t / P : t % npair, e = along ? t % P : t / npair;
     double2 v = make_double2(0.0, 0.0);
@@ -139,12 +146,11 @@ __global__ void __launch_bounds__(kFFThreads) k_ff_lines(const __grid_constant__
         b = e;
       }
       if (b >= 0) {
-        const int l = l0 + li;
-        const long long idx = jb.sbase + (long long)(l / jb.nl2) * jb.sqs + (long long)(l % jb.nl2) * jb.sls +
-                              (long long)b * jb.ses;
+        const int l = l0 + li, q = l / jb.nl2, c = jb.comp + q;
+        const long long idx = jb.sbase + (long long)q * jb.sqs + (long long)(l - q * jb.nl2) * jb.sls + (long long)b * jb.ses;
         if (jb.real)
-          v = make_double2(enter(J.srcr[idx], jb.comp + l / jb.nl2, J.smax),
-                           jb.ioff >= 0 ? enter(J.srcr[idx + jb.ioff], 1, J.smax) : 0.0);
+          v = make_double2(enter(J.srcr[idx], c == 0 ? f0 : c == 1 ? f1 : f2),
+                           jb.ioff >= 0 ? enter(J.srcr[idx + jb.ioff], f1) : 0.0);
         else v = J.src[idx];
       }
     }
