@@ -32,7 +32,8 @@ extern "C" {
 typedef enum vpmg_status {
   VPMG_OK = 0,
   VPMG_ERR_ARG = -1,          /* bad argument / size                              */
-  VPMG_ERR_CUDA = -2,         /* CUDA runtime error (message via vpmg_last_error) */
+  VPMG_ERR_CUDA = -2,         /* CUDA runtime error, or a bounded wait inside a
+                                 kernel that ran out (vpmg_last_error says which)  */
   VPMG_ERR_NOMEM = -3,        /* device allocation failed                          */
   VPMG_ERR_OUTSIDE = -4,      /* a particle stencil leaves the mesh                */
   VPMG_ERR_CAPACITY = -5,     /* remesh produced more particles than capacity      */
@@ -155,7 +156,8 @@ double vpmg_projection_fun(int itype, double x);
  *             receives the solution of Lap_h u = rhs; the box faces of sol
  *             are the Dirichlet values (zero_bc = 0) or are zeroed (1);
  *   h         mesh spacings;  stream: a cudaStream_t (NULL = default
- *             stream); the call is asynchronous on that stream.
+ *             stream); the call is asynchronous on that stream (should a
+ *             bounded wait inside a kernel run out, the interior is NaN).
  * Limits: at most 2^21 interior nodes and 900 along x and along y; larger
  * boxes return VPMG_ERR_ARG before any GPU work.  2*(cells) along x and y
  * must have no prime factor above 17 (else VPMG_ERR_UNSUPPORTED).
