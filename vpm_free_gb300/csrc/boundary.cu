@@ -1044,6 +1044,9 @@ void boundary_prepare(BoundaryOp& B, const Grid& g, int levmax, long long budget
   upload(B.child, child); upload(B.flags, flags); upload(B.agg_leaf0, leaf0); upload(B.agg_rowlen, rowlen);
   upload(B.agg_istep, istep);
   B.csrc.ensure(3 * (size_t)NC);
+  // dummy cells have no panels and are never written, but the dense block and the
+  // rows multiply them by their zero weights: whatever memory held may be no number
+  VPMG_CUDA(cudaMemsetAsync(B.csrc.p, 0, B.csrc.bytes(), s));
   B.smax.ensure(3);
   VPMG_CUDA(cudaMemsetAsync(B.smax.p, 0, 3 * sizeof(unsigned), s));
   std::vector<int> pf(B.nbound), pi(B.nbound), pj(B.nbound), pk(B.nbound);
