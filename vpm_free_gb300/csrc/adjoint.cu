@@ -85,7 +85,7 @@ __device__ __forceinline__ bool stencil(const MeshDev& m, double px, double py, 
   for (int d = 0; d < 3; ++d) {
     if (!(p[d] - m.xmin[d] >= 0.0)) return false;
     S.c0[d] = cell_of(p[d], m.xmin[d], m.d[d]);
-    if (S.c0[d] - 1 < 0 || S.c0[d] + 2 >= m.n[d]) return false;
+    if (S.c0[d] < 1 || S.c0[d] >= m.n[d] - 2) return false;  // nothing is added to the largest int
     const double inv = 1.0 / m.d[d];
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
@@ -631,8 +631,8 @@ void check_probes(const vpmg_handle* h, const double* pr, int n) {
     for (int d = 0; d < 3; ++d) {
       const double x = pr[3 * (size_t)p + d];
       VPMG_CHECK(std::isfinite(x) && x - g.xmin[d] >= 0.0, VPMG_ERR_ARG, "a probe lies outside the mesh");
-      const int c = (int)((x - g.xmin[d]) / g.d[d]);
-      VPMG_CHECK(c - 1 >= 0 && c + 2 < g.n[d], VPMG_ERR_ARG, "a probe's M4' stencil leaves the mesh");
+      const double c = (x - g.xmin[d]) / g.d[d];  // its cell when truncated, if that is an int
+      VPMG_CHECK(c >= 1.0 && c < (double)(g.n[d] - 2), VPMG_ERR_ARG, "a probe's M4' stencil leaves the mesh");
     }
 }
 

@@ -86,10 +86,11 @@ __global__ void k_keys(const double* __restrict__ x, const double* __restrict__ 
   const int i0 = cell_of(x[p], m.xmin[0], m.d[0]);
   const int j0 = cell_of(y[p], m.xmin[1], m.d[1]);
   const int k0 = cell_of(z[p], m.xmin[2], m.d[2]);
-  // stencil nodes (0-based) c - ips .. c + ipf must lie on the mesh
+  // stencil nodes (0-based) c - ips .. c + ipf must lie on the mesh; the cell of a
+  // distant position is the largest int, which nothing may be added to
   const bool ok = (x[p] - m.xmin[0] >= 0.0) && (y[p] - m.xmin[1] >= 0.0) && (z[p] - m.xmin[2] >= 0.0) &&
-                  i0 - m.ips >= 0 && j0 - m.ips >= 0 && k0 - m.ips >= 0 && i0 + m.ipf < m.n[0] &&
-                  j0 + m.ipf < m.n[1] && k0 + m.ipf < m.n[2];
+                  i0 >= m.ips && j0 >= m.ips && k0 >= m.ips && i0 < m.n[0] - m.ipf && j0 < m.n[1] - m.ipf &&
+                  k0 < m.n[2] - m.ipf;
   if (!ok) {
     key[p] = -1;
     atomicMax(err, kErrOutside);
