@@ -35,6 +35,20 @@ def test_run_after_define_sizes(gpulib):
         assert np.array_equal(a, b)
 
 
+def test_new_arrays_hold_no_particles(gpulib):
+    """Before set_particles, and after a mesh that needs larger arrays."""
+    V = gpulib
+    x1, q1, w = _ring(1.0)
+    x2, _, _ = _ring(1.4)
+    with V.VPM(V.VPMConfig.make(dpm=w["dpm"])) as h:
+        for x in (x1, x2):
+            h.define_sizes(x)
+            assert h.num_particles() == 0
+            h.run(1, w["dt"])
+            assert h.get_particles()[0].shape[0] == 0
+            h.set_particles(x1, q1)
+
+
 def test_gradient_after_define_sizes(gpulib):
     if gpulib.arith != "fp64":
         pytest.skip("one arithmetic")

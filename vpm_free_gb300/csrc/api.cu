@@ -218,7 +218,12 @@ void prepare(vpmg_handle* h) {
     h->ym.prepare(Y);
   }
   // particles: capacity for a full remesh of the global mesh
+  const int cap = h->parts.capacity;
   h->parts.ensure((int)std::min<size_t>(N, (size_t)INT32_MAX / 16));
+  if (h->parts.capacity != cap) {  // new arrays hold no particles
+    VPMG_CUDA(cudaMemsetAsync(h->parts.d_np.p, 0, sizeof(int), st));
+    h->np = 0;
+  }
   h->parts.arith = h->arith;
   h->bins.ensure(N);
   VPMG_CUDA(cudaStreamSynchronize(st));
@@ -615,7 +620,7 @@ int vpmg_create(const vpmg_config* cfg, int device, vpmg_handle** out) {
     VPMG_CUDA(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
     for (int i = 0; i < 10; ++i) VPMG_CUDA(cudaEventCreate(&h->ev[i]));
     h->bins.err.ensure(1);
-    VPMG_CUDA(cudaMemset(h->bins.err.p, 0, sizeof(int)));
+    VPMG_CUDA(cudaMemsetAsync(h->bins.err.p, 0, sizeof(int), h->stream));
     size_t fr = 0, tot = 0;
     VPMG_CUDA(cudaMemGetInfo(&fr, &tot));
     h->op_budget = std::min<long long>(100LL << 30, (long long)(0.6 * (double)fr));
